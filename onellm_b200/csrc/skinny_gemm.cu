@@ -9,6 +9,7 @@
 #include <mutex>
 #include <utility>
 
+#include "gemm_f32.h"
 #include "project.h"
 #include "skinny_common.cuh"
 
@@ -256,10 +257,16 @@ extern "C" int onellm_gemm_ld(int dtype, const void* x, const void* W, void* y, 
     if (M == 0) return ONELLM_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (dtype == ONELLM_F32) {
+        const bool nk = w_layout == ONELLM_W_NK;
+        const GemmF32 a = {(const float*)x, (const float*)W, (float*)y, M, N, K, K, nk ? K : N, ldy, nk, nullptr, 1.f, -1, 0.f};
+        if (gemm_f32_skinny_takes(a)) {
+            ONELLM_CUDA(gemm_f32_skinny(a, st));
+            return ONELLM_OK;
+        }
         const dim3 grid((N + 63) / 64, (M + 63) / 64);
         ONELLM_REQUIRE(grid.y <= 65535, ONELLM_ERR_UNSUPPORTED, "gemm: M too large for the fp32 path");
         note_launch();
-        if (w_layout == ONELLM_W_NK)
+        if (nk)
             sgemm_kernel<true><<<grid, 256, 0, st>>>((const float*)x, (const float*)W, (float*)y, M, N, K, K, K, ldy, nullptr, 1.f, -1, 0.f, RowGroups{});
         else
             sgemm_kernel<false><<<grid, 256, 0, st>>>((const float*)x, (const float*)W, (float*)y, M, N, K, K, N, ldy, nullptr, 1.f, -1, 0.f, RowGroups{});
@@ -301,6 +308,8 @@ static int project_f32(const onellm_projection& p, long ldy, cudaStream_t st)
     const long ldx = p.ldx ? p.ldx : p.K;
     const int ldw = p.ldw ? p.ldw : p.N;
     auto run = [&](const void* W, const float* resid, int gate) {
+        const GemmF32 a = {(const float*)p.x, (const float*)W, (float*)p.y, p.M, p.N, p.K, ldx, ldw, ldy, false, resid, p.scale, gate, p.limit};
+        if (!p.groups && gemm_f32_skinny_takes(a)) return gemm_f32_skinny(a, st);
         if (p.groups)
             return launch_pdl(sgemm_kernel<false, true>, grid, dim3(256), 0, st, (const float*)p.x, (const float*)W, (float*)p.y, p.M, p.N, p.K, ldx,
                               ldw, ldy, resid, p.scale, gate, p.limit, g);
