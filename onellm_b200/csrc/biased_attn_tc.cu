@@ -325,7 +325,7 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
 }
 
-static const TimeoutFlag timeout_flag(tc_flag_read_clear);
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
 template <bool WINDOWED>
 static int ba_launch(const BaParams& p, int B, int max_new, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t st)

@@ -22,8 +22,15 @@ long launches_noted();
 // Every file with kernels that have bounded waits registers the reader of its time-out flag (see tc_common.cuh);
 // onellm_gemm_timeout_flag asks them all.
 struct TimeoutFlag {
-    explicit TimeoutFlag(int (*read_and_clear)());
+    TimeoutFlag(int (*read_and_clear)(), const int* (*address)());
 };
+// Device addresses of these flags on the current device, for a kernel that reads them on its way (at most kMaxTimeoutFlags;
+// null behind the last one).
+constexpr int kMaxTimeoutFlags = 16;
+struct TimeoutFlags {
+    const int* at[kMaxTimeoutFlags];
+};
+TimeoutFlags timeout_flag_addresses();
 
 #define ONELLM_REQUIRE(cond, code, ...)          \
     do {                                         \

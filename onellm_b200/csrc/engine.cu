@@ -71,6 +71,23 @@ __global__ void half_to_float_kernel(const __half* in, float* out, size_t n)
         out[i] = __half2float(in[i]);
 }
 
+// The end of a pass in one piece, so that the host needs one copy and one wait (reading every time-out flag by a copy of its own
+// took 100 us of a short prompt's pass).
+__global__ void report_kernel(int* __restrict__ report, const int* __restrict__ bad, const int* __restrict__ ids, int n, const TimeoutFlags flags)
+{
+    pdl_wait();
+    if (threadIdx.x == 0) {
+        int any = 0;
+#pragma unroll
+        for (int i = 0; i < kMaxTimeoutFlags; i++)
+            if (flags.at[i]) any |= *flags.at[i];
+        report[0] = bad[0];
+        report[1] = bad[1];
+        report[2] = any;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) report[4 + i] = ids[i];
+}
+
 // ---- memory ------------------------------------------------------------------------------------------------
 void Engine::carve_common(Carver& cv)
 {
@@ -89,6 +106,7 @@ void Engine::carve_common(Carver& cv)
     d_skip = cv.take<uint32_t>(skip_table_words((int)B));
     d_cu = cv.take<int>(B + 1);
     d_hist = cv.take<int>(B);
+    d_report = cv.take<int>(4 + B);
     logits = cv.take_bytes(B * (size_t)vocab * dtype_size(logits_dtype));
 }
 
@@ -106,6 +124,8 @@ int Engine::allocate()
     ONELLM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     ONELLM_CUDA(cudaMemsetAsync(arena, 0, arena_bytes, stream));
     ONELLM_CUDA(cudaStreamSynchronize(stream));
+    ONELLM_CUDA(cudaMallocHost(&h_report, (4 + (size_t)max_batch) * sizeof(int)));
+    timeout_flags = timeout_flag_addresses();
     return build_skip_table(d_skip, max_batch, &skip_ok, stream);
 }
 
@@ -118,6 +138,8 @@ Engine::~Engine()
     if (scratch) cudaFree(scratch);
     if (row_logits) cudaFree(row_logits);
     if (d_rows) cudaFree(d_rows);
+    if (logits_f32) cudaFree(logits_f32);
+    if (h_report) cudaFreeHost(h_report);
 }
 
 int Engine::ensure_scratch(size_t bytes)
@@ -275,7 +297,7 @@ int Engine::prefill_context(int B, const int* lens)
     ONELLM_CUDA(cudaMemcpyAsync(d_cu, cu.data(), (B + 1) * sizeof(int), cudaMemcpyHostToDevice, stream));
     ONELLM_CUDA(cudaMemcpyAsync(d_hist, hist.data(), B * sizeof(int), cudaMemcpyHostToDevice, stream));
     ONELLM_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    ONELLM_CUDA(cudaStreamSynchronize(stream));  // the host arrays live on this stack frame
+    // (the host arrays are pageable: each copy has left them when its call returns)
     const long before = launches_noted();
     RC(context_layers(c));
     RC(sample(c.logits));  // seeded with the step counter, as the position-by-position path does
@@ -288,16 +310,42 @@ int Engine::prefill_context(int B, const int* lens)
 // The host's side of a context pass: first tokens out, then what the kernels recorded.
 int Engine::finish_context(int* host_first_ids, const char* where)
 {
-    if (host_first_ids) ONELLM_CUDA(cudaMemcpyAsync(host_first_ids, d_out_ids, (size_t)batch * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    note_launch();
+    report_kernel<<<1, 64, 0, stream>>>(d_report, d_bad_id, d_out_ids, host_first_ids ? batch : 0, timeout_flags);
+    ONELLM_CHECK_LAUNCH();
+    ONELLM_CUDA(cudaMemcpyAsync(h_report, d_report, (4 + (size_t)batch) * sizeof(int), cudaMemcpyDeviceToHost, stream));
     RC(queue_comm_check());
     ONELLM_CUDA(cudaStreamSynchronize(stream));
     RC(comm_check(where));
-    int bad[2] = {0, 0};
-    ONELLM_CUDA(cudaMemcpy(bad, d_bad_id, 2 * sizeof(int), cudaMemcpyDeviceToHost));
-    ONELLM_REQUIRE(bad[0] == 0, ONELLM_ERR_ARG, "%s: token id outside [0, vocab_size)", where);
-    ONELLM_REQUIRE(bad[1] == 0, ONELLM_ERR_STATE, "%s: a position beyond max_seq_len was refused by the cache", where);
-    ONELLM_REQUIRE(onellm_gemm_timeout_flag() <= 0, ONELLM_ERR_CUDA, "%s: a tensor-core GEMM block timed out", where);
+    ONELLM_REQUIRE(h_report[0] == 0, ONELLM_ERR_ARG, "%s: token id outside [0, vocab_size)", where);
+    ONELLM_REQUIRE(h_report[1] == 0, ONELLM_ERR_STATE, "%s: a position beyond max_seq_len was refused by the cache", where);
+    if (h_report[2]) {
+        (void)onellm_gemm_timeout_flag();  // clears it
+        ONELLM_REQUIRE(false, ONELLM_ERR_CUDA, "%s: a tensor-core GEMM block timed out", where);
+    }
+    if (host_first_ids) memcpy(host_first_ids, h_report + 4, (size_t)batch * sizeof(int));
     return ONELLM_OK;
+}
+
+// n rows of logits from row `first` of the last pass, as float on the host.  16-bit logits go through a buffer of max_batch rows
+// that the engine keeps (allocated and freed on every call it cost 0.8 ms and more, with a wait for the whole device).
+int Engine::copy_logits(size_t first, size_t rows, float* host_logits)
+{
+    const char* src = static_cast<const char*>(last_logits) + first * vocab * dtype_size(logits_dtype);
+    if (logits_dtype == ONELLM_F32) {
+        ONELLM_CUDA(cudaMemcpyAsync(host_logits, src, rows * vocab * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    } else {
+        if (!logits_f32) ONELLM_CUDA(cudaMalloc(&logits_f32, (size_t)max_batch * vocab * sizeof(float)));
+        for (size_t r = 0; r < rows; r += (size_t)max_batch) {
+            const size_t n = std::min(rows - r, (size_t)max_batch) * vocab;
+            half_to_float_kernel<<<blocks_for(n), 256, 0, stream>>>(reinterpret_cast<const __half*>(src) + r * vocab, logits_f32, n);
+            ONELLM_CHECK_LAUNCH();
+            ONELLM_CUDA(cudaMemcpyAsync(host_logits + r * vocab, logits_f32, n * sizeof(float), cudaMemcpyDeviceToHost, stream));
+        }
+    }
+    RC(queue_comm_check());
+    ONELLM_CUDA(cudaStreamSynchronize(stream));
+    return comm_check("llama_get_logits");
 }
 
 }  // namespace onellm
@@ -397,7 +445,6 @@ extern "C" int onellm_llama_prefill(onellm_llama* h, const int* host_ids, int ba
     ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
     ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
     ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
-    ONELLM_CUDA(cudaStreamSynchronize(st));  // `first_step` lives on this stack frame
     if (m->prefill_by_decode) {
         ONELLM_REQUIRE(m->want_rows.empty(), ONELLM_ERR_STATE, "llama_prefill: logits of single rows need the context-phase kernels");
         // one position at a time through the decode kernels; only the last position needs the LM head
@@ -438,7 +485,6 @@ extern "C" int onellm_llama_prefill_ragged(onellm_llama* h, const int* host_ids,
     ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
     ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
     ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
-    ONELLM_CUDA(cudaStreamSynchronize(st));  // `longest` lives on this stack frame
     RC(m->prefill_context(batch, lens));
     return m->finish_context(host_first_ids, "llama_prefill_ragged");
 }
@@ -456,7 +502,6 @@ extern "C" int onellm_llama_extend(onellm_llama* h, const int* host_ids, int n_n
     const int batch = m->batch, new_len = m->cur_len + n_new;
     ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * n_new * sizeof(int), cudaMemcpyHostToDevice, st));
     ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &new_len, sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaStreamSynchronize(st));  // `new_len` lives on this stack frame
     const std::vector<int> lens(batch, n_new);
     RC(m->prefill_context(batch, lens.data()));
     return m->finish_context(host_first_ids, "llama_extend");
@@ -506,9 +551,10 @@ extern "C" int onellm_llama_decode_step(onellm_llama* h, const int* host_in_ids,
         ONELLM_CUDA(cudaMemcpyAsync(m->d_ids, host_in_ids, (size_t)m->batch * sizeof(int), cudaMemcpyHostToDevice, st));
     RC(m->run_step(MODE_HEAD, 0));
     if (host_out_ids) {
-        ONELLM_CUDA(cudaMemcpyAsync(host_out_ids, m->d_out_ids, (size_t)m->batch * sizeof(int), cudaMemcpyDeviceToHost, st));
+        ONELLM_CUDA(cudaMemcpyAsync(m->h_report, m->d_out_ids, (size_t)m->batch * sizeof(int), cudaMemcpyDeviceToHost, st));
         RC(m->queue_comm_check());
         ONELLM_CUDA(cudaStreamSynchronize(st));
+        memcpy(host_out_ids, m->h_report, (size_t)m->batch * sizeof(int));
         RC(m->comm_check("llama_decode_step"));
     }
     return ONELLM_OK;
@@ -537,34 +583,12 @@ extern "C" int onellm_llama_generate(onellm_llama* h, const int* host_prompt, in
     return ONELLM_OK;
 }
 
-// n rows of logits from row `first` of the last pass, as float on the host.
-static int copy_logits(Engine* m, size_t first, size_t rows, float* host_logits)
-{
-    const size_t n = rows * m->vocab;
-    const char* src = static_cast<const char*>(m->last_logits) + first * m->vocab * dtype_size(m->logits_dtype);
-    cudaError_t e;
-    float* tmp = nullptr;
-    if (m->logits_dtype == ONELLM_F32) {
-        e = cudaMemcpyAsync(host_logits, src, n * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
-    } else {
-        ONELLM_CUDA(cudaMalloc(&tmp, n * sizeof(float)));
-        half_to_float_kernel<<<blocks_for(n), 256, 0, m->stream>>>(reinterpret_cast<const __half*>(src), tmp, n);
-        e = cudaMemcpyAsync(host_logits, tmp, n * sizeof(float), cudaMemcpyDeviceToHost, m->stream);
-    }
-    const int qrc = m->queue_comm_check();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    if (tmp) cudaFree(tmp);
-    ONELLM_REQUIRE(e == cudaSuccess, ONELLM_ERR_CUDA, "llama_get_logits: %s", cudaGetErrorString(e));
-    RC(qrc);
-    return m->comm_check("llama_get_logits");
-}
-
 extern "C" int onellm_llama_get_logits(onellm_llama* h, float* host_logits)
 {
     Engine* m = engine_of(h);
     ONELLM_REQUIRE(m && host_logits, ONELLM_ERR_ARG, "llama_get_logits: null pointer");
     ONELLM_REQUIRE(m->batch > 0 && m->last_logits, ONELLM_ERR_STATE, "llama_get_logits: nothing computed yet");
-    return copy_logits(m, 0, m->batch, host_logits);
+    return m->copy_logits(0, m->batch, host_logits);
 }
 
 extern "C" int onellm_llama_get_row_logits(onellm_llama* h, float* host_logits, int n_rows)
@@ -573,7 +597,7 @@ extern "C" int onellm_llama_get_row_logits(onellm_llama* h, float* host_logits, 
     ONELLM_REQUIRE(m && host_logits && n_rows >= 1, ONELLM_ERR_ARG, "llama_get_row_logits: bad argument");
     ONELLM_REQUIRE(m->row_have == (size_t)n_rows && m->last_logits == m->row_logits, ONELLM_ERR_STATE,
                    "llama_get_row_logits: the last pass was not a context pass with %d wanted rows", n_rows);
-    return copy_logits(m, m->batch, n_rows, host_logits);
+    return m->copy_logits(m->batch, n_rows, host_logits);
 }
 
 extern "C" int onellm_llama_get_state(onellm_llama* h, int* cur_len, long* kernel_launches, int* host_seqlen, unsigned char* host_finished)

@@ -68,6 +68,10 @@ struct Engine {
     void* row_logits = nullptr;  // [max_batch + wanted, vocab]
     size_t row_cap = 0, row_have = 0;
     const void* last_logits = nullptr;
+    float* logits_f32 = nullptr;   // [max_batch, vocab], made by the first call that asks for 16-bit logits
+    // what the host reads at the end of a pass: bad_id [2], whether a bounded wait gave up, sampled ids [max_batch]
+    int *d_report = nullptr, *h_report = nullptr;  // h_report: pinned
+    TimeoutFlags timeout_flags = {};
     // state
     int batch = 0, cur_len = 0, graph_prompt_len = 0;
     int top_k = 1, literal_walk = 0;  // top_k 0: logits only, nothing is sampled
@@ -107,6 +111,7 @@ struct Engine {
     int run_step(int mode, int prompt_len);
     int prefill_context(int B, const int* lens);
     int finish_context(int* host_first_ids, const char* where);
+    int copy_logits(size_t first, size_t rows, float* host_logits);
 
   private:
     void carve_common(Carver& cv);

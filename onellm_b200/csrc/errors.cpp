@@ -39,12 +39,27 @@ cudaError_t prefer_max_shared(const void* kernel)
     return e;
 }
 
-static std::vector<int (*)()>& timeout_flags()
+struct FlagReaders {
+    int (*read_and_clear)();
+    const int* (*address)();
+};
+static std::vector<FlagReaders>& timeout_flags()
 {
-    static std::vector<int (*)()> v;
+    static std::vector<FlagReaders> v;
     return v;
 }
-TimeoutFlag::TimeoutFlag(int (*read_and_clear)()) { timeout_flags().push_back(read_and_clear); }
+TimeoutFlag::TimeoutFlag(int (*read_and_clear)(), const int* (*address)()) { timeout_flags().push_back({read_and_clear, address}); }
+
+TimeoutFlags timeout_flag_addresses()
+{
+    TimeoutFlags f = {};
+    int n = 0;
+    for (const auto& r : timeout_flags()) {
+        const int* p = r.address();
+        if (p && n < kMaxTimeoutFlags) f.at[n++] = p;
+    }
+    return f;
+}
 
 }  // namespace onellm
 
@@ -52,8 +67,8 @@ TimeoutFlag::TimeoutFlag(int (*read_and_clear)()) { timeout_flags().push_back(re
 extern "C" int onellm_gemm_timeout_flag(void)
 {
     int any = 0;
-    for (auto read : onellm::timeout_flags()) {
-        const int v = read();
+    for (const auto& r : onellm::timeout_flags()) {
+        const int v = r.read_and_clear();
         any = (v < 0 || any < 0) ? -1 : (any | v);
     }
     return any;

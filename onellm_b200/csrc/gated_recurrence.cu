@@ -379,7 +379,7 @@ gated_recurrence_scan_kernel(const GrParams pp, int tokens, const float* __restr
         }
     }
 }
-static const TimeoutFlag timeout_flag(tc_flag_read_clear);
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
 // one warp per (token, head), at most 32 NJ columns
 template <typename T, int NJ>

@@ -468,6 +468,6 @@ int gemm_bf16_large(const onellm_projection& p, cudaStream_t st)
     return gemm_tc_launch<bf16>((const bf16*)p.x, (const bf16*)p.W, (const bf16*)p.W2, static_cast<bf16*>(p.y), p.M, p.N, p.K, p.W2 ? 2 : 0, st, epi);
 }
 
-static const TimeoutFlag timeout_flag(tc_flag_read_clear);
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
 }  // namespace onellm

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(128) latent_attn_tc_merge_kernel(const LtParam
         make_uint2(pack2<__nv_bfloat16>(o.x * f, o.y * f), pack2<__nv_bfloat16>(o.z * f, o.w * f));
 }
 
-static const TimeoutFlag timeout_flag(tc_flag_read_clear);
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
 bool latent_attn_tc_takes(const LatentAttn& a, const TokenPositions& tp)
 {

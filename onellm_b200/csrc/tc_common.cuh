@@ -139,6 +139,16 @@ static inline int tc_flag_read_clear()
     return v;
 }
 
+static inline const int* tc_flag_address()
+{
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_tc_timeout_flag) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return static_cast<const int*>(p);
+}
+
 // 2-D tensor map of 16-bit elements: `inner` contiguous elements, `outer` rows of `inner` elements; box {64, box_outer}; 128-byte swizzle
 // (defined in gemm_tc.cu)
 int make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_outer);
