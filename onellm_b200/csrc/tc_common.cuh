@@ -125,6 +125,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                  : "memory");
 }
 
+// One lane of a converged warp, for the instructions that a single thread issues (tcgen05.mma, TMA loads).  The warp stays
+// together around them: descriptors and addresses are then in uniform registers, which is where these instructions take them
+// from; behind a divergent `lane == 0` every operand is moved there one by one, about 100 cycles an instruction.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
