@@ -34,6 +34,15 @@ __device__ __forceinline__ float4 ld_stream4(const float* p)
     return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 
+// x comes from the kernel in front of this one: a load that stays behind the dependency wait (a read-only one, __ldg, the
+// compiler may move in front of it)
+__device__ __forceinline__ float4 ld_dependent4(const float* p)
+{
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void store_f32(const GemmF32& a, int m, int n, float v)
 {
     const size_t at = (size_t)m * a.ldy + n;
@@ -79,7 +88,7 @@ gemv_kn_f32_kernel(const GemmF32 a, int rows_per_block)
             const bool in = k + r4 < k_end;  // K and the rows of a block are multiples of 4
 #pragma unroll
             for (int m = 0; m < MT; m++) {
-                const float4 xv = in ? __ldg(reinterpret_cast<const float4*>(x + (size_t)min(m, m_rows - 1) * a.ldx + k + r4)) : zero;
+                const float4 xv = in ? ld_dependent4(x + (size_t)min(m, m_rows - 1) * a.ldx + k + r4) : zero;
                 const float xs[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
@@ -161,7 +170,7 @@ gemv_nk_f32_kernel(const GemmF32 a, int wk)
             fetch(k + wk * 128, next);
 #pragma unroll
             for (int m = 0; m < MT; m++) {
-                const float4 xv = k < a.K ? __ldg(reinterpret_cast<const float4*>(x + (size_t)min(m, m_rows - 1) * a.ldx + k)) : zero;
+                const float4 xv = k < a.K ? ld_dependent4(x + (size_t)min(m, m_rows - 1) * a.ldx + k) : zero;
 #pragma unroll
                 for (int r = 0; r < 4; r++)
                     acc[r][m] = fmaf(xv.x, cur[r].x, fmaf(xv.y, cur[r].y, fmaf(xv.z, cur[r].z, fmaf(xv.w, cur[r].w, acc[r][m]))));
