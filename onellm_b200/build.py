@@ -23,7 +23,7 @@ NVCC_FLAGS = [
 ]
 
 # What a design opened with onellm_model_open is linked from: the engine, the projections, sampling, and its own files.
-ENGINE_SOURCES = ["elementwise.cu", "engine.cu", "errors.cpp", "gemm_f32.cu", "gemm_tc.cu", "model_files.cpp", "norm.cu", "sampling.cu",
+ENGINE_SOURCES = ["elementwise.cu", "engine.cu", "errors.cpp", "gemm_f32.cu", "gemm_f32_tc.cu", "gemm_tc.cu", "model_files.cpp", "norm.cu", "sampling.cu",
                   "skinny_gemm.cu", "skinny_gemm_staged.cu", "skinny_gemm_tc.cu", "weight_placer.cu"]
 DESIGN_SOURCES = {
     "Finuvik": ["biased_attn.cu", "biased_attn_tc.cu", "finuvik.cu", "gated_recurrence.cu"],

@@ -1,4 +1,4 @@
-// float32 projections: the kernel for few tokens and its arguments (gemm_f32.cu).
+// float32 projections: the kernels for few tokens (gemm_f32.cu) and for many (gemm_f32_tc.cu) and their arguments.
 #pragma once
 #include "common.cuh"
 
@@ -22,5 +22,7 @@ constexpr int kF32SkinnyTokens = 64;
 // Sizes, strides and alignment that gemm_f32_skinny covers: 16-byte rows.
 bool gemm_f32_skinny_takes(const GemmF32& a);
 cudaError_t gemm_f32_skinny(const GemmF32& a, cudaStream_t st);
+bool gemm_f32_tc_takes(const GemmF32& a);
+cudaError_t gemm_f32_tc(const GemmF32& a, cudaStream_t st);
 
 }  // namespace onellm

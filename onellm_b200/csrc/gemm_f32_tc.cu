@@ -1,0 +1,380 @@
+// float32 projections of more than 64 tokens on the tensor cores, with the precision of float.
+//
+// Replaces the cuBLAS SGEMM behind launchLinearGemm (src/kernels/qkv_linear.cu:8-65 of the reference) for context passes of
+// float32 callers.  A float is split exactly into three bf16 values, eight bits of its mantissa each (by truncation, so that
+// they have its sign and the first cannot overflow): x = x0 + x1 + x2.  Of the nine products of two such sums six are computed,
+// x0 w0, x0 w1, x1 w0, x0 w2, x1 w1, x2 w0; the other three are below 2^-24 of the result.
+//
+// A block computes y^T: 128 columns of W are the rows of the MMA, the tokens (at most 192) its columns, so that a token count
+// that is no multiple of 128 costs no padding.
+//   W      lane = column: a thread splits 16 rows of its column and stores the pieces to tensor memory, where the MMA takes its A
+//          operand from: no transposition.
+//   x      8 threads split the 32 values of a token's stage; the pieces go to shared memory in the 128-byte swizzled form
+//          ([x0 | x1] in one tile of 128-byte rows, [x2 | unused] in a second one).
+//          Both come as floats by TMA, three stages ahead.
+//   sums   the tensor cores add into a float with truncation, so an accumulator is not kept for long: every stage of 32 rows
+//          starts a new one, the five small products go in before x0 w0, and the warps then add it to their
+//          registers, rounding to nearest.  Two accumulators, two buffers of each operand: the warps add stage s - 1 and
+//          convert stage s + 1 while the MMAs of stage s run.
+// K is split over the blocks of a cluster where the tiles alone would not fill the GPU; the partial sums meet in distributed
+// shared memory in rank order.
+// What bounds it: the MMAs of a stage of 176 tokens take 1060 cycles, splitting its floats 1000 and adding an accumulator 400 in
+// every warp, the last two one after the other.  Measured, 352 tokens of the 7B shapes, us (the 64 x 64 tiled kernel before): QKV
+// 277 (3000), o_proj 99 (890), gate or up 254 (2600), down 230 (2400), 120 to 138 TFLOP/s of float32; error against 64 bits
+// 1.8e-7 (2.6e-7 at K = 11008), a layer 7e-7 instead of 2.8e-6.
+// A value that is not finite makes its remainders NaN and so every result it enters; a result that is not finite (also one
+// whose partial sums overflowed) is computed again with plain multiply-adds.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <tuple>
+
+#include "gemm_f32.h"
+#include "tc_common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace onellm {
+
+constexpr int kFtCols = 128;                    // columns of W per block
+constexpr int kFtTok = 192;                     // most tokens per block
+constexpr int kFtK = 32;                        // rows of W per stage
+constexpr int kFtWarps = 8;                     // warps that convert and add
+constexpr int kFtThreads = kFtWarps * 32 + 32;  // and one that issues loads and MMAs
+constexpr int kFtTile = kFtTok * 128;           // bytes: a 128-byte row per token
+constexpr int kFtPiecesBytes = 4 * kFtTile;     // two stages of two tiles; the partial sums of the cluster afterwards
+constexpr int kFtDepth = 3;                     // stages of floats on their way
+constexpr int kFtRawW = kFtK * kFtCols * 4, kFtRaw = kFtRawW + kFtTok * kFtK * 4;
+constexpr int kFtSmem = kFtPiecesBytes + kFtDepth * kFtRaw;
+constexpr int kFtGroup = kFtTok / 2 / 3;        // accumulator columns read at a time
+constexpr uint32_t kFtPieces = 2 * kFtTok;      // tensor memory: two accumulators, then two stages of 3 pieces x 16 columns
+static_assert(kFtGroup == 32 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
+
+__device__ __forceinline__ void umma_f16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+// the three bf16 pieces of two floats, packed piece by piece (lo in the low half)
+__device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2)
+{
+    constexpr uint32_t kTop = 0xffff0000u;
+    const uint32_t l0 = __float_as_uint(lo) & kTop, h0 = __float_as_uint(hi) & kTop;
+    const float lr = lo - __uint_as_float(l0), hr = hi - __uint_as_float(h0);
+    const uint32_t l1 = __float_as_uint(lr) & kTop, h1 = __float_as_uint(hr) & kTop;
+    const float lq = lr - __uint_as_float(l1), hq = hr - __uint_as_float(h1);
+    p0 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+    p1 = __byte_perm(__float_as_uint(lr), __float_as_uint(hr), 0x7632);
+    p2 = __byte_perm(__float_as_uint(lq), __float_as_uint(hq), 0x7632);
+}
+
+template <bool NK>
+__device__ __noinline__ float plain_dot(const GemmF32& a, int m, int n)
+{
+    const float *x = a.x + (size_t)m * a.ldx, *w = NK ? a.W + (size_t)n * a.ldw : a.W + n;
+    float s = 0.f;
+    for (int k = 0; k < a.K; k++) s = fmaf(x[k], NK ? w[k] : w[(size_t)k * a.ldw], s);
+    return s;
+}
+template <bool NK>
+__device__ __forceinline__ void finish_f32(const GemmF32& a, int m, int n, float v)
+{
+    if (!isfinite(v)) v = plain_dot<NK>(a, m, n);
+    const size_t at = (size_t)m * a.ldy + n;
+    if (a.resid) v = fmaf(v, a.scale, a.resid[at]);
+    if (a.gate >= 0) v = gate_pair<true>(a.y[at], v, a.gate, a.limit);
+    a.y[at] = v;
+}
+
+// grid (ceil(N / 128), K split, ceil(M / nt)), cluster (1, K split, 1); nt: tokens per block, a multiple of 16; every block has a stage
+template <bool NK>
+__global__ void __launch_bounds__(kFtThreads, 1)
+gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int nt, int stages_per_block)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bars[4 + kFtDepth];  // pieces of a stage are there (2), its products are done (2), its floats are there
+    __shared__ uint32_t tmem_slot;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n0 = blockIdx.x * kFtCols, m0 = blockIdx.z * nt, m_rows = min(nt, a.M - m0);
+    const int k_begin = blockIdx.y * stages_per_block * kFtK, k_end = min(k_begin + stages_per_block * kFtK, a.K);
+    const int n_stages = (k_end - k_begin + kFtK - 1) / kFtK;
+    const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + 2), raw0 = smem_u32(bars + 4);
+    bool ok = (smem_u32(smem_raw) & 1023u) == 0;  // the swizzle works on address bits
+    if (!ok && tid == 0) atomicExch(&g_tc_timeout_flag, 1);
+    if (tid == 0) {
+        for (int s = 0; s < 2; s++) {
+            mbar_init(full0 + 8 * s, kFtWarps);
+            mbar_init(done0 + 8 * s, 1);
+        }
+        for (int s = 0; s < kFtDepth; s++) mbar_init(raw0 + 8 * s, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    pdl_wait();
+
+    const int half = warp >> 2, nh = nt / 2;  // a warp adds the accumulator columns [half * nh, half * nh + nh) of its 32 lanes
+    float acc[3 * kFtGroup];
+#pragma unroll
+    for (int i = 0; i < 3 * kFtGroup; i++) acc[i] = 0.f;
+
+    if (warp == kFtWarps) {
+        // Issues the loads of the floats and the MMAs (the whole warp runs this; one elected lane issues)
+        const uint64_t desc = umma_desc(smem_u32(smem_raw), 16, 1024);
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kFtCols >> 4) << 24);
+        const uint32_t raw = smem_u32(smem_raw) + kFtPiecesBytes;
+        const bool leader = elect_one();
+        auto fetch = [&](int s, int slot) {
+            if (!leader || s >= n_stages) return;
+            const int k0 = k_begin + s * kFtK;
+            const uint32_t bar = raw0 + 8 * slot, dst = raw + (uint32_t)(slot * kFtRaw);
+            mbar_expect_tx(bar, (uint32_t)(kFtRawW + nt * kFtK * 4));
+            if constexpr (NK) tma_load_2d(dst, &map_w, k0, n0, bar);
+            else tma_load_2d(dst, &map_w, n0, k0, bar);
+            tma_load_2d(dst + kFtRawW, &map_x, k0, m0, bar);
+        };
+        if (ok)
+            for (int s = 0; s < kFtDepth; s++) fetch(s, s);
+        int slot = 0;
+        for (int s = 0; s < n_stages && ok; s++) {
+            ok = mbar_wait_warp(full0 + 8 * (s & 1), (uint32_t)(s >> 1) & 1u);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            fetch(s + kFtDepth, slot);  // every warp has split the floats of this stage
+            slot = slot + 1 == kFtDepth ? 0 : slot + 1;
+            if (leader) {
+                const uint32_t d = tmem + (uint32_t)((s & 1) * kFtTok), wp = tmem + kFtPieces + (uint32_t)((s & 1) * 48);
+                const uint64_t xd = desc + (uint64_t)((s & 1) * (2 * kFtTile >> 4));
+                constexpr int kW[6] = {2, 0, 1, 1, 0, 0}, kX[6] = {0, 2, 1, 0, 1, 0};  // pieces of the products, small ones first
+#pragma unroll
+                for (int i = 0; i < 6; i++)
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++)
+                        umma_f16_tmem_a(d, wp + kW[i] * 16 + kk * 8, xd + (uint64_t)(((kX[i] >> 1) * kFtTile + (kX[i] & 1) * 64 + kk * 32) >> 4), idesc,
+                                        i + kk > 0 ? 1u : 0u);
+                umma_commit(done0 + 8 * (s & 1));
+            }
+            __syncwarp();
+        }
+    } else {
+        const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const int col = (warp & 3) * 32 + lane;
+        // x: rows r and r + 4 of a group of 8 side by side, so that a warp's stores fill all banks
+        const int quad = tid & 7, row0 = (warp * 4 & ~7) + ((tid >> 3) & 1) * 4 + ((tid >> 4) & 1) + (warp & 1) * 2;
+        const uint32_t x_at = (uint32_t)row0 * 128 + (((quad >> 1) ^ (row0 & 7)) << 4) + (quad & 1) * 8;  // + 32 rows: + 4096
+        auto add = [&](int s) {
+            if (!mbar_wait_warp(done0 + 8 * (s & 1), (uint32_t)(s >> 1) & 1u)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int g = 0; g < 3; g++) {
+                if (g * kFtGroup < nh) {
+                    uint32_t v[32];
+                    tmem_ld32(t_lane + (uint32_t)((s & 1) * kFtTok + half * nh + g * kFtGroup), v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 32; i++) acc[g * kFtGroup + i] += __uint_as_float(v[i]);
+                }
+            }
+            return true;
+        };
+        int slot = 0;
+        uint32_t phase = 0;
+        for (int s = 0; s < n_stages && ok; s++) {
+            ok = mbar_wait_warp(raw0 + 8 * slot, phase);
+            if (!ok) break;
+            const unsigned char* raw = smem_raw + kFtPiecesBytes + slot * kFtRaw;
+            // the buffers of this stage were last read by the MMAs of stage s - 2, whose accumulator has been added
+            uint32_t p0[8], p1[8], p2[8];
+            if constexpr (NK) {  // [128 columns][32 k], 128-byte swizzled
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float4 v = *reinterpret_cast<const float4*>(raw + col * 128 + (((half * 4 + i) ^ (col & 7)) << 4));
+                    split_pair(v.x, v.y, p0[2 * i], p1[2 * i], p2[2 * i]);
+                    split_pair(v.z, v.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1]);
+                }
+            } else {  // [32 k][128 columns]
+                const float* wr = reinterpret_cast<const float*>(raw) + half * 16 * kFtCols + col;
+#pragma unroll
+                for (int i = 0; i < 8; i++) split_pair(wr[2 * i * kFtCols], wr[(2 * i + 1) * kFtCols], p0[i], p1[i], p2[i]);
+            }
+            const uint32_t t_w = t_lane + kFtPieces + (uint32_t)((s & 1) * 48 + half * 8);
+            tmem_st8(t_w, p0);
+            tmem_st8(t_w + 16, p1);
+            tmem_st8(t_w + 32, p2);
+            const unsigned char* xr = raw + kFtRawW + row0 * 128 + quad * 16;
+            unsigned char* xs = smem_raw + (s & 1) * 2 * kFtTile;
+#pragma unroll
+            for (int j = 0; j < kFtTok / 32; j++) {
+                if (row0 + 32 * j < nt) {
+                    const float4 v = *reinterpret_cast<const float4*>(xr + j * 4096);
+                    uint2 q0, q1, q2;
+                    split_pair(v.x, v.y, q0.x, q1.x, q2.x);
+                    split_pair(v.z, v.w, q0.y, q1.y, q2.y);
+                    *reinterpret_cast<uint2*>(xs + x_at + j * 4096) = q0;
+                    *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 4096) = q1;  // 16-byte chunk + 4, swizzled
+                    *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 4096) = q2;
+                }
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full0 + 8 * (s & 1));
+            if (++slot == kFtDepth) {
+                slot = 0;
+                phase ^= 1;
+            }
+            if (s > 0) ok = add(s - 1);
+        }
+        if (ok) ok = add(n_stages - 1);
+    }
+    pdl_launch_dependents();
+
+    const int ks = gridDim.y, q = warp & 3;
+    if (ks == 1) {
+        const int n = n0 + q * 32 + lane;
+        if (warp < kFtWarps && n < a.N) {
+#pragma unroll
+            for (int i = 0; i < 3 * kFtGroup; i++)
+                if (i < nh && half * nh + i < m_rows) finish_f32<NK>(a, m0 + half * nh + i, n, acc[i]);
+        }
+    } else {
+        float* red = reinterpret_cast<float*>(smem_raw);  // [nt][128]
+        __syncthreads();                                  // every warp has seen the last products: the operands are not read any more
+        if (warp < kFtWarps) {
+#pragma unroll
+            for (int i = 0; i < 3 * kFtGroup; i++)
+                if (i < nh) red[(half * nh + i) * kFtCols + q * 32 + lane] = acc[i];
+        }
+        cluster.sync();
+        const int rank = blockIdx.y, total = m_rows * kFtCols;
+        for (int e = rank * kFtThreads + tid; e < total; e += ks * kFtThreads) {
+            float p[8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) p[r] = r < ks ? cluster.map_shared_rank(red, r)[e] : 0.f;
+            float v = p[0];
+#pragma unroll
+            for (int r = 1; r < 8; r++) v += p[r];
+            const int n = n0 + e % kFtCols;
+            if (n < a.N) finish_f32<NK>(a, m0 + e / kFtCols, n, v);
+        }
+        cluster.sync();  // peers may still be reading this block's sums
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
+
+template <bool NK>
+static cudaLaunchConfig_t ft_config(dim3 grid, cudaStream_t st, cudaLaunchAttribute (&at)[2])
+{
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = grid.y;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kFtThreads);
+    cfg.dynamicSmemBytes = kFtSmem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+
+// Blocks of clusters of `ks` that are resident at once, asked once per device.
+template <bool NK>
+static int ft_slots(int ks)
+{
+    static std::mutex mu;
+    static int known[kMaxDevices][9] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[current_device()][ks];
+    if (n == 0) {
+        cudaLaunchAttribute at[2];
+        cudaLaunchConfig_t cfg = ft_config<NK>(dim3(1024, ks, 1), nullptr, at);
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_f32_tc_kernel<NK>, &cfg) != cudaSuccess || clusters < 1) {
+            (void)cudaGetLastError();
+            clusters = num_sms() / ks;
+        }
+        n = std::max(1, clusters) * ks;
+    }
+    return n;
+}
+
+template <bool NK>
+static cudaError_t launch_ft(const GemmF32& a, cudaStream_t st)
+{
+    auto kern = gemm_f32_tc_kernel<NK>;
+    static DeviceOnce attr;
+    const cudaError_t e = attr.run([kern] {
+        const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kFtSmem);
+        return r != cudaSuccess ? r : prefer_max_shared((const void*)kern);
+    });
+    if (e != cudaSuccess) return e;
+    // Tokens per block and K split by an estimate: waves of blocks x (stages of a block x time of a stage + what a block costs
+    // besides, both in cycles).
+    const int cols = (a.N + kFtCols - 1) / kFtCols, total = (a.K + kFtK - 1) / kFtK, z_least = (a.M + kFtTok - 1) / kFtTok;
+    int best_nt = 0, best_per = 0, best_ks = 1;
+    double best = 0.0;
+    for (int z = z_least; z <= z_least + 2; z++) {
+        const int nt = ((a.M + z - 1) / z + 15) / 16 * 16, blocks_z = (a.M + nt - 1) / nt;
+        for (int ks = 1; ks <= std::min(8, total); ks++) {
+            const int per = (total + ks - 1) / ks;
+            if (per * (ks - 1) >= total) continue;
+            const long slots = ft_slots<NK>(ks), blocks = (long)cols * blocks_z * ks;
+            const double cost = (double)((blocks + slots - 1) / slots) * (per * (300.0 + 5.5 * nt) + 4000.0 + (ks > 1 ? 3000.0 : 0.0));
+            if (best_nt == 0 || cost < best) {
+                best = cost;
+                best_nt = nt;
+                best_per = per;
+                best_ks = ks;
+            }
+        }
+    }
+    const long z = (a.M + best_nt - 1) / best_nt;
+    CUtensorMap map_x, map_w;
+    if (make_map_f32(&map_x, a.x, a.K, a.M, a.ldx, kFtK, best_nt, false) != ONELLM_OK ||
+        make_map_f32(&map_w, a.W, NK ? a.K : a.N, NK ? a.N : a.K, a.ldw, NK ? kFtK : kFtCols, NK ? kFtCols : kFtK, NK) != ONELLM_OK)
+        return cudaErrorInvalidValue;
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = ft_config<NK>(dim3(cols, best_ks, (unsigned)z), st, at);
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kern, a, map_x, map_w, best_nt, best_per);
+}
+
+// Sizes, strides and alignment it covers: 16-byte rows.
+bool gemm_f32_tc_takes(const GemmF32& a)
+{
+    return a.M > kF32SkinnyTokens && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W) &&
+           ((long)a.M + 15) / 16 <= 65535;
+}
+
+cudaError_t gemm_f32_tc(const GemmF32& a, cudaStream_t st) { return a.w_nk ? launch_ft<true>(a, st) : launch_ft<false>(a, st); }
+
+}  // namespace onellm

@@ -664,6 +664,21 @@ int make_chunk_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t 
     return ONELLM_OK;
 }
 
+int make_map_f32(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer, bool swizzled)
+{
+    EncodeTiledFn enc = encode_tiled();
+    ONELLM_REQUIRE(enc, ONELLM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    const cuuint64_t dims[2] = {inner, outer};
+    const cuuint64_t strides[1] = {ld * sizeof(float)};
+    const cuuint32_t box[2] = {box_inner, box_outer};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    ONELLM_REQUIRE(r == CUDA_SUCCESS, ONELLM_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
+    return ONELLM_OK;
+}
+
 int gemm_f16_skinny(const __half* x, const __half* W, __half* y, int M, int N, int K, int w_layout, cudaStream_t st);
 
 // K split of a projection with few tiles; ks 0: the persistent kernel.

@@ -263,6 +263,10 @@ extern "C" int onellm_gemm_ld(int dtype, const void* x, const void* W, void* y, 
             ONELLM_CUDA(gemm_f32_skinny(a, st));
             return ONELLM_OK;
         }
+        if (gemm_f32_tc_takes(a)) {
+            ONELLM_CUDA(gemm_f32_tc(a, st));
+            return ONELLM_OK;
+        }
         const dim3 grid((N + 63) / 64, (M + 63) / 64);
         ONELLM_REQUIRE(grid.y <= 65535, ONELLM_ERR_UNSUPPORTED, "gemm: M too large for the fp32 path");
         note_launch();
@@ -310,6 +314,7 @@ static int project_f32(const onellm_projection& p, long ldy, cudaStream_t st)
     auto run = [&](const void* W, const float* resid, int gate) {
         const GemmF32 a = {(const float*)p.x, (const float*)W, (float*)p.y, p.M, p.N, p.K, ldx, ldw, ldy, false, resid, p.scale, gate, p.limit};
         if (!p.groups && gemm_f32_skinny_takes(a)) return gemm_f32_skinny(a, st);
+        if (!p.groups && gemm_f32_tc_takes(a)) return gemm_f32_tc(a, st);
         if (p.groups)
             return launch_pdl(sgemm_kernel<false, true>, grid, dim3(256), 0, st, (const float*)p.x, (const float*)W, (float*)p.y, p.M, p.N, p.K, ldx,
                               ldw, ldy, resid, p.scale, gate, p.limit, g);

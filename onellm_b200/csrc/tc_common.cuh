@@ -166,5 +166,7 @@ int make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer,
 // The same matrix seen as 64-column chunks: coordinates (column in the chunk, row, chunk), box {64, box_rows, box_chunks}, so that
 // one load brings whole rows and lays them out chunk by chunk.  inner % 64 == 0.
 int make_chunk_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint32_t box_rows, uint32_t box_chunks);
+// 2-D tensor map of floats, rows `ld` elements apart; box {box_inner, box_outer}, swizzled (box_inner 32) or plain
+int make_map_f32(CUtensorMap* map, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner, uint32_t box_outer, bool swizzled);
 
 }  // namespace onellm

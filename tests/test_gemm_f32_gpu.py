@@ -7,7 +7,9 @@ pytestmark = pytest.mark.gpu
 # (M, N, K): one and the most tokens of a kernel, token counts between its templates, columns and rows that end inside a tile,
 # a K that leaves warps and blocks of the split without rows
 SHAPES = [(1, 4096, 4096), (2, 132, 4), (3, 260, 72), (8, 12288, 4096), (9, 128, 1000), (16, 4, 4096), (17, 1024, 36), (31, 36, 11008), (64, 516, 260),
-          (5, 70, 33), (65, 70, 33), (33, 4100, 100)]
+          (5, 70, 33), (65, 70, 33), (33, 4100, 100),
+          # the tensor-core kernel: token counts at and beside its blocks, ends inside a tile, a stage and a split
+          (65, 4, 4), (80, 260, 72), (192, 128, 64), (193, 516, 2048), (352, 4096, 512), (400, 36, 11008), (1000, 384, 96)]
 
 
 def worst(got, x, w):
@@ -35,7 +37,7 @@ def test_gemm_f32_against_64_bits(ob, cuda, M, N, K, nk, pad):
     assert (got[:, N:] == 7.0).all()
 
 
-@pytest.mark.parametrize("M", [3, 40, 70])
+@pytest.mark.parametrize("M", [3, 40, 70, 200])
 def test_gemm_f32_keeps_infinities_and_nan(ob, cuda, M):
     torch = cuda
     g = torch.Generator(device="cuda").manual_seed(M)
@@ -49,7 +51,7 @@ def test_gemm_f32_keeps_infinities_and_nan(ob, cuda, M):
         assert torch.equal(same(y), same(ref))
 
 
-@pytest.mark.parametrize("M", [1, 6, 30])
+@pytest.mark.parametrize("M", [1, 6, 30, 100])
 def test_projection_f32_gate_and_residual(ob, cuda, M):
     torch = cuda
     g = torch.Generator(device="cuda").manual_seed(M)
