@@ -219,7 +219,7 @@ topk_reg_kernel(const T* __restrict__ logits, int vocab, int K, float* __restric
 
     // 0. The short way, which nearly every row of logits takes.  The K-th largest of the 1024 per-thread maxima is
     // a lower bound of the K-th largest key (K threads hold a key that large), and for logits hardly more than K
-    // keys reach it.  One bisection over ONE key per thread finds it (a ballot per warp, one block barrier per bit);
+    // keys reach it.  A bisection over ONE key per thread finds it (a ballot per warp, one block barrier per bit);
     // the keys that reach it are gathered (a few dozen shared-memory atomics) and ranked against each other, larger
     // key first, lower column first among equals: rank r < K is output slot r.  Rows with many equal keys, where
     // the gathered set would be large, take the bisection over all keys below instead.
@@ -228,13 +228,34 @@ topk_reg_kernel(const T* __restrict__ logits, int vocab, int K, float* __restric
 #pragma unroll
         for (int j = 0; j < kTopkPer; j++) mk = max(mk, key[j]);
         uint32_t low = 0u;
-#pragma unroll 1
-        for (int bit = 31; bit >= kLowBit; bit--, it++) {
-            const uint32_t t = low | (1u << bit);
-            const int c = __popc(__ballot_sync(0xffffffffu, mk >= t));
-            if (lane == 0) bit_tot[it & 1][wid] = c;
+        // With K no larger than the number of warps that have columns, the K-th largest of the 32 warp maxima is such a bound too:
+        // two barriers instead of one per bit.  It is lower, and where more threads than a few per warp reach it (the large logits
+        // side by side in few warps) the bisection takes over.
+        bool found = false;
+        if (K <= (vocab + 32 * kTopkPer - 1) / (32 * kTopkPer)) {
+            const uint32_t wm = __reduce_max_sync(0xffffffffu, mk);
+            if (lane == 0) warp_tot[wid] = (int)wm;
             __syncthreads();
-            if (__reduce_add_sync(0xffffffffu, bit_tot[it & 1][lane]) >= K) low = t;
+            const uint32_t v = (uint32_t)warp_tot[lane];
+            int r = 0;
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const uint32_t u = __shfl_sync(0xffffffffu, v, j);
+                r += u > v || (u == v && j < lane);
+            }
+            low = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, r == K - 1)) - 1);
+            found = __syncthreads_count(mk >= low) <= kTopkCand / 4;
+        }
+        if (!found) {
+            low = 0u;
+#pragma unroll 1
+            for (int bit = 31; bit >= kLowBit; bit--, it++) {
+                const uint32_t t = low | (1u << bit);
+                const int c = __popc(__ballot_sync(0xffffffffu, mk >= t));
+                if (lane == 0) bit_tot[it & 1][wid] = c;
+                __syncthreads();
+                if (__reduce_add_sync(0xffffffffu, bit_tot[it & 1][lane]) >= K) low = t;
+            }
         }
         if (mk >= low) {
 #pragma unroll
