@@ -139,6 +139,20 @@ def test_batched_gemm_layouts(ob, cuda, ta, tb):
     assert float((Cm.double() - ref).abs().max() / ref.abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (16, 65, 16), (17, 16, 33), (64, 64, 15), (65, 130, 128), (255, 5, 31)])
+def test_batched_gemm_edges_of_tiles(ob, cuda, ta, tb, m, n, k):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    A, Bm = torch.randn(2, m, k, device="cuda", generator=g), torch.randn(2, k, n, device="cuda", generator=g)
+    Cm = torch.full((2, m, n), 7.0, device="cuda")
+    at, bt = (A.transpose(1, 2).contiguous() if ta else A), (Bm.transpose(1, 2).contiguous() if tb else Bm)
+    ob.batched_gemm(ob.F32, at, bt, Cm, 2, m, n, k, trans_a=ta, trans_b=tb)
+    ref, size = A.double() @ Bm.double(), (A.double() ** 2 @ Bm.double() ** 2).sqrt()
+    # sqrt(k) sums, each off by at most 2^-24 of a partial sum
+    assert float(((Cm.double() - ref).abs() / size).max()) < 4 * k ** 0.5 * 2.0 ** -24 + 2.0 ** -22
+
+
 def test_softmax_fully_masked_row_is_zero(ob, cuda):
     torch = cuda
     qk = torch.randn(1, 2, 3, 40, device="cuda")
