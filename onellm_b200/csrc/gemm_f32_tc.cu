@@ -18,10 +18,10 @@
 //          convert stage s + 1 while the MMAs of stage s run.
 // K is split over the blocks of a cluster where the tiles alone would not fill the GPU; the partial sums meet in distributed
 // shared memory in rank order.
-// What bounds it: the MMAs of a stage of 176 tokens take 1060 cycles, splitting its floats 1000 and adding an accumulator 400 in
-// every warp, the last two one after the other.  Measured, 352 tokens of the 7B shapes, us (the 64 x 64 tiled kernel before): QKV
-// 277 (3000), o_proj 99 (890), gate or up 254 (2600), down 230 (2400), 120 to 138 TFLOP/s of float32; error against 64 bits
-// 1.8e-7 (2.6e-7 at K = 11008), a layer 7e-7 instead of 2.8e-6.
+// What bounds it: the MMAs of a stage of 176 tokens take about 1000 cycles, splitting its floats 1200, adding an accumulator 400 and
+// the waits between them 450, the last three one after the other in every warp.  Measured, 352 tokens of the 7B shapes, us (the 64 x
+// 64 tiled kernel before): QKV 262 (3000), o_proj 93 (890), gate or up 240 (2600), down 215 (2400), 127 to 147 TFLOP/s of float32;
+// error against 64 bits 1.8e-7 (2.6e-7 at K = 11008), a layer 7e-7 instead of 2.8e-6.
 // A value that is not finite makes its remainders NaN and so every result it enters; a result that is not finite (also one
 // whose partial sums overflowed) is computed again with plain multiply-adds.
 #include <cooperative_groups.h>
@@ -220,16 +220,27 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             tmem_st8(t_w + 32, p2);
             const unsigned char* xr = raw + kFtRawW + row0 * 128 + quad * 16;
             unsigned char* xs = smem_raw + (s & 1) * 2 * kFtTile;
+            // three token groups at a time, so that their latencies overlap; what lies behind the last token is read but not stored
 #pragma unroll
-            for (int j = 0; j < kFtTok / 32; j++) {
-                if (row0 + 32 * j < nt) {
-                    const float4 v = *reinterpret_cast<const float4*>(xr + j * 4096);
-                    uint2 q0, q1, q2;
-                    split_pair(v.x, v.y, q0.x, q1.x, q2.x);
-                    split_pair(v.z, v.w, q0.y, q1.y, q2.y);
-                    *reinterpret_cast<uint2*>(xs + x_at + j * 4096) = q0;
-                    *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 4096) = q1;  // 16-byte chunk + 4, swizzled
-                    *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 4096) = q2;
+            for (int j0 = 0; j0 < kFtTok / 32; j0 += 3) {
+                if (32 * j0 >= nt) break;
+                float4 v[3];
+                uint2 q0[3], q1[3], q2[3];
+#pragma unroll
+                for (int i = 0; i < 3; i++) v[i] = *reinterpret_cast<const float4*>(xr + (j0 + i) * 4096);
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    split_pair(v[i].x, v[i].y, q0[i].x, q1[i].x, q2[i].x);
+                    split_pair(v[i].z, v[i].w, q0[i].y, q1[i].y, q2[i].y);
+                }
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const int j = j0 + i;
+                    if ((warp >> 1) * 8 + 32 * j < nt) {  // the 8 rows of the warp's group: nt is a multiple of 16
+                        *reinterpret_cast<uint2*>(xs + x_at + j * 4096) = q0[i];
+                        *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 4096) = q1[i];  // 16-byte chunk + 4, swizzled
+                        *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 4096) = q2[i];
+                    }
                 }
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -338,7 +349,7 @@ static cudaError_t launch_ft(const GemmF32& a, cudaStream_t st)
     });
     if (e != cudaSuccess) return e;
     // Tokens per block and K split by an estimate: waves of blocks x (stages of a block x time of a stage + what a block costs
-    // besides, both in cycles).
+    // besides, both in cycles, fitted to 80 and 176 tokens).
     const int cols = (a.N + kFtCols - 1) / kFtCols, total = (a.K + kFtK - 1) / kFtK, z_least = (a.M + kFtTok - 1) / kFtTok;
     int best_nt = 0, best_per = 0, best_ks = 1;
     double best = 0.0;
@@ -348,7 +359,7 @@ static cudaError_t launch_ft(const GemmF32& a, cudaStream_t st)
             const int per = (total + ks - 1) / ks;
             if (per * (ks - 1) >= total) continue;
             const long slots = ft_slots<NK>(ks), blocks = (long)cols * blocks_z * ks;
-            const double cost = (double)((blocks + slots - 1) / slots) * (per * (300.0 + 5.5 * nt) + 4000.0 + (ks > 1 ? 3000.0 : 0.0));
+            const double cost = (double)((blocks + slots - 1) / slots) * (per * (1400.0 + 5.7 * nt) + 5000.0 + (ks > 1 ? 4000.0 : 0.0));
             if (best_nt == 0 || cost < best) {
                 best = cost;
                 best_nt = nt;
