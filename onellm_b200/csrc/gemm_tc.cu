@@ -11,6 +11,9 @@
 // cluster multicast anywhere); one thread of warp 1 issues tcgen05.mma (M = 128, N = 256, K = 16, kind::f16)
 // and releases each stage with tcgen05.commit; tensor memory holds two 256-column accumulators, so warps 2-5
 // (tcgen05.ld, convert, store) drain tile i while the MMAs of tile i + 1 run.
+// Where it is the faster (persistent_us) two blocks work as a pair on a tile of 256 rows (cta_group::2): an SM then takes in 32 KB
+// a slice instead of 48, the operand traffic being what bounds the single form (128 x 256: 0.40 us a slice, pairs 0.37, which is
+// 1.54 PFLOP/s on long prompts).
 // The [K,N] weight is used as it lies in memory: it is the "MN-major" B operand of the MMA
 // (four 64-column TMA boxes per stage), so no transposed copy of the weights is ever made.
 // Every wait on an mbarrier is bounded; on a time-out the block records it in a device flag,
@@ -32,6 +35,7 @@ namespace onellm {
 
 constexpr int kTcBM = 128, kTcBN = 256, kTcBK = 64;
 constexpr int kTcStages = 4;
+constexpr int kTcPairStages = 6;     // of 32 KB: the same shared memory
 constexpr int kTcBand = 16;  // row tiles per band of the tile order
 constexpr int kTcThreads = 192;      // producer warp, MMA warp, four epilogue warps
 constexpr int kTcEpiThreads = 128;
@@ -79,7 +83,9 @@ struct TcEpilogue {
     float scale = 1.f, limit = 0.f;
 };
 
-template <typename T, int MODE, bool GROUPED = false>
+// PAIR: the two blocks of a cluster share a tile of 256 rows (cta_group::2): a block loads its 128 rows of x and half the columns of W
+// (two weights: one of them), 32 KB a slice instead of 48, and finishes its rows.
+template <typename T, int MODE, bool GROUPED = false, bool PAIR = false>
 __global__ void __launch_bounds__(kTcThreads)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_b2, T* y, int M, int N, int K, const TcEpilogue epi, const RowGroups grp)
@@ -87,27 +93,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     constexpr bool W_NK = MODE == 1;
     constexpr bool DUAL = MODE == 2;
     constexpr int kOutN = DUAL ? kTcBN / 2 : kTcBN;  // output columns per tile
+    static_assert(!(PAIR && GROUPED), "the tiles of groups have 128 rows");
+    constexpr int kStages = PAIR ? kTcPairStages : kTcStages, kStageBytes = kTcATile + (PAIR ? kTcBTile / 2 : kTcBTile);
+    constexpr int kTileM = PAIR ? 2 * kTcBM : kTcBM, kBand = PAIR ? kTcBand / 2 : kTcBand;
+    const uint32_t rank = PAIR ? (uint32_t)cg::this_cluster().block_rank() : 0u;
+    const int tile0 = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, tile_step = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
     extern __shared__ unsigned char smem_raw[];
     // 1024-byte alignment for the 128-byte swizzle pattern
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kTcStages * kTcStageBytes);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kTcStages + 4);
-    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kTcStages);
-    const uint32_t acc_full0 = smem_u32(bars + 2 * kTcStages), acc_empty0 = smem_u32(bars + 2 * kTcStages + 2);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+    const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kStages);
+    const uint32_t acc_full0 = smem_u32(bars + 2 * kStages), acc_empty0 = smem_u32(bars + 2 * kStages + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Tile order: the linear tile index walks down a band of kTcBand row tiles, then moves one column
     // tile to the right, so the tiles in flight at one time (one per SM) cover a near-square patch
     // of the output and share their A row blocks and B column blocks in L2.  (Row-major order made every
     // wave touch all column tiles of B: operands were read from DRAM seven times over.)
-    int tiles_m = (M + kTcBM - 1) / kTcBM;
+    int tiles_m = (M + kTileM - 1) / kTileM;
     const int tiles_n = (N + kOutN - 1) / kOutN;
     int n_tiles = tiles_m * tiles_n;
     // first row and column of a tile, the row of the stacked weights it starts at, the end of its rows
     auto tile_origin = [&](int t, int& m0, int& n0, int& k0, int& m_end) {
-        const int per_band = kTcBand * tiles_n;
+        const int per_band = kBand * tiles_n;
         const int band = t / per_band, in_band = t % per_band;
-        const int band_rows = min(kTcBand, tiles_m - band * kTcBand);
-        const int mt = band * kTcBand + in_band % band_rows;
+        const int band_rows = min(kBand, tiles_m - band * kBand);
+        const int mt = band * kBand + in_band % band_rows;
         n0 = (in_band / band_rows) * kOutN;
         if constexpr (GROUPED) {
             const int g = grp.tile_group[mt];
@@ -115,7 +126,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             k0 = g * K;
             m_end = grp.off[g + 1];
         } else {
-            m0 = mt * kTcBM;
+            m0 = mt * kTileM + (int)rank * kTcBM;
             k0 = 0;
             m_end = M;
         }
@@ -124,23 +135,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t ring = smem_u32(smem);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kTcStages; s++) {
+        for (int s = 0; s < kStages; s++) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(acc_full0 + 8 * a, 1);
-            mbar_init(acc_empty0 + 8 * a, kTcEpiThreads);
+            mbar_init(acc_empty0 + 8 * a, PAIR ? 2 * kTcEpiThreads / 32 : kTcEpiThreads);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * kTcBN)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * kTcBN) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2u * kTcBN) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cg::this_cluster().sync();  // the other block's barriers
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
@@ -155,15 +171,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool leader = elect_one();
         uint32_t s = 0, round = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+        for (int t = tile0; t < n_tiles && ok; t += tile_step) {
             int m0, n0, k0, m_end;
             tile_origin(t, m0, n0, k0, m_end);
             for (int ks = 0; ks < k_steps; ks++) {
                 if (round > 0) ok = mbar_wait_warp(empty0 + 8 * s, (round - 1) & 1);
                 if (!ok) break;
-                if (leader) {
-                    const uint32_t bar = full0 + 8 * s, a_dst = ring + s * kTcStageBytes, b_dst = a_dst + kTcATile;
-                    mbar_expect_tx(bar, kTcStageBytes);
+                if (PAIR && leader) {
+                    const uint32_t bar = map_to_rank(full0 + 8 * s, 0), a_dst = ring + s * kStageBytes, b_dst = a_dst + kTcATile;
+                    if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * kStageBytes);  // what both blocks load
+                    tma_load_2d_pair(a_dst, &map_a, ks * kTcBK, m0, bar);
+                    if (W_NK) {
+                        tma_load_2d_pair(b_dst, &map_b, ks * kTcBK, n0 + (int)rank * (kTcBN / 2), bar);
+                    } else {
+                        // one weight: the 128 columns of this rank; two: the rank's weight
+                        const int n = DUAL ? n0 : n0 + (int)rank * (kTcBN / 2);
+#pragma unroll
+                        for (int c = 0; c < 2; c++)
+                            tma_load_2d_pair(b_dst + c * kTcBChunk, DUAL && rank == 1 ? &map_b2 : &map_b, n + 64 * c, ks * kTcBK, bar);
+                    }
+                } else if (leader) {
+                    const uint32_t bar = full0 + 8 * s, a_dst = ring + s * kStageBytes, b_dst = a_dst + kTcATile;
+                    mbar_expect_tx(bar, kStageBytes);
                     tma_load_2d(a_dst, &map_a, ks * kTcBK, m0, bar);
                     if (W_NK) {
                         tma_load_2d(b_dst, &map_b, ks * kTcBK, n0, bar);
@@ -178,15 +207,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int c = 0; c < kTcBN / 64; c++) tma_load_2d(b_dst + c * kTcBChunk, &map_b, n0 + 64 * c, k0 + ks * kTcBK, bar);
                     }
                 }
-                if (++s == kTcStages) {
+                if (++s == kStages) {
                     s = 0;
                     round++;
                 }
             }
         }
-    } else if (warp == 1) {
-        // instruction descriptor: D = f32, A and B of type T, A K-major, B MN-major unless W_NK, N = 256, M = 128
-        const uint32_t idesc = (1u << 4) | umma_operand_bits<T>() | ((W_NK ? 0u : 1u) << 16) | ((uint32_t)(kTcBN >> 3) << 17) | ((uint32_t)(kTcBM >> 4) << 24);
+        if (PAIR && rank == 1) pdl_launch_dependents();
+    } else if (warp == 1 && rank == 0) {
+        // instruction descriptor: D = f32, A and B of type T, A K-major, B MN-major unless W_NK, N = 256, M = 128 (256 of a pair)
+        const uint32_t idesc = (1u << 4) | umma_operand_bits<T>() | ((W_NK ? 0u : 1u) << 16) | ((uint32_t)(kTcBN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
         // A: K-major, rows of 128 bytes, 8-row groups 1024 bytes apart; 16 k = 32 bytes further in the row
         // B [N,K]: same form.  B [K,N]: MN-major, 64-column chunks 8192 bytes apart (LBO), 8-row k groups
         // 1024 bytes apart (SBO); 16 k = two groups further
@@ -196,7 +226,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int lt = 0;
         uint32_t s = 0, phase = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, lt++) {
+        for (int t = tile0; t < n_tiles && ok; t += tile_step, lt++) {
             const int acc = lt & 1, use = lt >> 1;
             // the accumulator must have been drained by the epilogue of the tile that used it before
             if (use >= 1) ok = mbar_wait_warp(acc_empty0 + 8 * acc, (use - 1) & 1);
@@ -208,20 +238,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (leader) {
-                    const uint64_t at = (uint64_t)(s * (kTcStageBytes >> 4));
+                    const uint64_t at = (uint64_t)(s * (kStageBytes >> 4));
 #pragma unroll
-                    for (int kk = 0; kk < kTcBK / 16; kk++)
-                        umma_f16(tmem_d, da + at + (uint64_t)((kk * 32) >> 4), db + at + (uint64_t)((W_NK ? kk * 32 : kk * 2048) >> 4), idesc,
-                                 (ks > 0 || kk > 0) ? 1u : 0u);
-                    umma_commit(empty0 + 8 * s);  // frees the stage when these MMAs have read it
+                    for (int kk = 0; kk < kTcBK / 16; kk++) {
+                        const uint64_t ad = da + at + (uint64_t)((kk * 32) >> 4), bd = db + at + (uint64_t)((W_NK ? kk * 32 : kk * 2048) >> 4);
+                        if constexpr (PAIR) umma_f16_pair(tmem_d, ad, bd, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
+                        else umma_f16(tmem_d, ad, bd, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    // frees the stage when these MMAs have read it
+                    if constexpr (PAIR) umma_commit_pair(empty0 + 8 * s);
+                    else umma_commit(empty0 + 8 * s);
                 }
                 __syncwarp();
-                if (++s == kTcStages) {
+                if (++s == kStages) {
                     s = 0;
                     phase ^= 1;
                 }
             }
-            if (ok && leader) umma_commit(acc_full0 + 8 * acc);  // the tile is complete when everything issued so far has run
+            if (ok && leader) {  // the tile is complete when everything issued so far has run
+                if constexpr (PAIR) umma_commit_pair(acc_full0 + 8 * acc);
+                else umma_commit(acc_full0 + 8 * acc);
+            }
         }
         pdl_launch_dependents();
     } else if (warp >= 2) {
@@ -230,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const size_t ldy = epi.ldy ? (size_t)epi.ldy : (size_t)N;
         int lt = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, lt++) {
+        for (int t = tile0; t < n_tiles && ok; t += tile_step, lt++) {
             const int acc = lt & 1, use = lt >> 1;
             int m0, n0, k0, m_end;
             tile_origin(t, m0, n0, k0, m_end);
@@ -319,13 +356,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (epi.ss_out && row_ok) epi.ss_out[(size_t)row * tiles_n + n0 / kOutN] = sq;
             // this thread's reads of the accumulator are over: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(acc_empty0 + 8 * acc);
+            if constexpr (PAIR) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(acc_empty0 + 8 * acc, 0));
+            } else {
+                mbar_arrive(acc_empty0 + 8 * acc);
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (PAIR) cg::this_cluster().sync();  // neither leaves while the other may reach its barriers or tensor memory
     if (warp == 2) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * kTcBN) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * kTcBN) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * kTcBN) : "memory");
     }
 }
 
@@ -686,21 +730,37 @@ struct SplitPlan {
     int ks, per;
 };
 
+// Estimated time in us of the persistent kernel, blocks alone or in pairs: a slice of 64 k takes 0.33 us (pairs 0.35), 0.40 (0.37) when
+// blocks take several tiles, the weights come in at 6.2 TB/s.  Pairs have half as many tiles of twice the rows, so that a token
+// count just above a multiple of 256 or a last wave of few tiles can cost them more than they gain.
+// Measured alone | in pairs: 3817 tokens, QKV of the 7B shape 282 | 249 us, gate/up 484 | 445, down 312 | 268; 238 tokens, QKV 33.4 |
+// 29.8, gate/up 65 | 56; 1030 tokens, o_proj 31 | 47 (144 tiles, 80 pairs).
+static double persistent_us(int M, int N, int K, bool dual, bool pairs)
+{
+    const long columns = dual ? 2L * N : N, slices = (K + kTcBK - 1) / kTcBK;
+    const long rows = pairs ? 2 * kTcBM : kTcBM, at_once = pairs ? num_sms() / 2 : num_sms();
+    const long waves = ((M + rows - 1) / rows * ((columns + kTcBN - 1) / kTcBN) + at_once - 1) / at_once;
+    const double slice = pairs ? (waves == 1 ? 0.35 : 0.37) : (waves == 1 ? 0.33 : 0.40);
+    return 8.0 + std::max((double)columns * K * 2 / 6.2e6, waves * slices * slice);
+}
+static bool takes_pairs(int M, int N, int K, bool dual)
+{
+    return M > kTcBM && persistent_us(M, N, K, dual, true) < persistent_us(M, N, K, dual, false);
+}
+
 // The plan with the least estimated time in us, from a sweep on B200 over 70 to 1000 tokens of the 2048- and 4096-wide shapes
-// (the estimate is within 15 % of all but the largest).  Either kernel needs about 8 us around its slices of 64 k.  A slice of
-// the persistent kernel takes 0.33 us, 0.40 when blocks take several tiles.  A slice here takes 0.32 us, 0.45 when two blocks
+// (the estimate is within 15 % of all but the largest).  Either kernel needs about 8 us around its slices of 64 k.  A slice here takes 0.32 us, 0.45 when two blocks
 // share an SM; the operands of all blocks come in at no more than 15 TB/s, the weights at 6.2.  Clusters leave some slots of two
 // blocks an SM unused, and a second wave of blocks costs another start.
 static SplitPlan plan_split(int M, int N, int K, bool dual, bool pairs)
 {
     const int slices = (K + kTcBK - 1) / kTcBK, tiles_m = (M + kTcBM - 1) / kTcBM, columns = dual ? 2 * N : N;
     SplitPlan plan = {0, slices};
-    const long tiles = (long)tiles_m * ((columns + kSplitBN - 1) / kSplitBN), wide = (long)tiles_m * ((columns + kTcBN - 1) / kTcBN);
+    const long tiles = (long)tiles_m * ((columns + kSplitBN - 1) / kSplitBN);
     const long sms = num_sms();
     if (tiles > 5 * sms) return plan;
     const double weights = (double)columns * K * 2 / 6.2e6;
-    const long waves = (wide + sms - 1) / sms;
-    double best = 8.0 + std::max(weights, waves * slices * (waves == 1 ? 0.33 : 0.40));
+    double best = persistent_us(M, N, K, dual, takes_pairs(M, N, K, dual));
     for (int ks = 1; ks <= (pairs ? 4 : 8); ks++) {
         const int per = (slices + ks - 1) / ks;
         if (ks > 1 && (per < 2 || per * (ks - 1) >= slices)) continue;  // every rank has slices
@@ -750,6 +810,37 @@ static cudaError_t launch_split(const CUtensorMap& a, const CUtensorMap& b, cons
     return cudaLaunchKernelEx(&cfg, kern, a, b, b2, y, M, N, K, epi, tiles_n, plan.per);
 }
 
+template <typename T, int MODE>
+static cudaError_t launch_pairs(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2, T* y, int M, int N, int K, const TcEpilogue& epi,
+                                cudaStream_t st)
+{
+    auto kern = gemm_tc_kernel<T, MODE, false, true>;
+    static DeviceOnce attr;
+    const cudaError_t e = attr.run([kern] {
+        const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes);
+        return r != cudaSuccess ? r : prefer_max_shared((const void*)kern);
+    });
+    if (e != cudaSuccess) return e;
+    constexpr int kOutN = MODE == 2 ? kTcBN / 2 : kTcBN;
+    const long tiles = (long)((N + kOutN - 1) / kOutN) * ((M + 2 * kTcBM - 1) / (2 * kTcBM));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(2 * (unsigned)std::min<long>(tiles, num_sms() / 2));
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = kTcSmemBytes;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kern, a, b, b2, y, M, N, K, epi, RowGroups{});
+}
+
 // mode 0: W [K,N]; 1: W [N,K]; 2: W and W2 [K,N], y = silu(x.W) * (x.W2)
 template <typename T>
 static int gemm_tc_launch(const T* x, const T* W, const T* W2, T* y, int M, int N, int K, int mode, cudaStream_t st,
@@ -773,6 +864,13 @@ static int gemm_tc_launch(const T* x, const T* W, const T* W2, T* y, int M, int 
         ONELLM_CUDA(mode == 0   ? (launch_split<T, 0>(map_a, map_b, map_b2, y, M, N, K, epi, plan, st))
                     : mode == 1 ? (launch_split<T, 1>(map_a, map_b, map_b2, y, M, N, K, epi, plan, st))
                                 : (launch_split<T, 2>(map_a, map_b, map_b2, y, M, N, K, epi, plan, st)));
+        return ONELLM_OK;
+    }
+    if (takes_pairs(M, N, K, mode == 2)) {
+        if (mode == 1) RC(make_map(&map_b, W, (uint64_t)K, (uint64_t)N, kTcBN / 2));
+        ONELLM_CUDA(mode == 0   ? (launch_pairs<T, 0>(map_a, map_b, map_b2, y, M, N, K, epi, st))
+                    : mode == 1 ? (launch_pairs<T, 1>(map_a, map_b, map_b2, y, M, N, K, epi, st))
+                                : (launch_pairs<T, 2>(map_a, map_b, map_b2, y, M, N, K, epi, st)));
         return ONELLM_OK;
     }
     static DeviceOnce smem_attr[3];

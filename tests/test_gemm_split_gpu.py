@@ -5,7 +5,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # tokens at the edges of one and two row tiles, K that leaves ranks uneven slices and a last slice cut short, columns that end inside a tile
-SHAPES = [(65, 256, 4096), (128, 8, 4096), (129, 264, 1032), (238, 4096, 4096), (256, 1000, 11008), (257, 520, 512), (300, 4096, 136), (1000, 32, 4096)]
+SHAPES = [(65, 256, 4096), (128, 8, 4096), (129, 264, 1032), (238, 4096, 4096), (256, 1000, 11008), (257, 520, 512), (300, 4096, 136), (1000, 32, 4096),
+          # many tiles: blocks in pairs on 256 rows, the last of which only one of them has, and several tiles per pair
+          (1290, 8712, 224), (1500, 8008, 1056)]
 
 
 def err(got, ref):
