@@ -407,6 +407,9 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     constexpr int kOutN = DUAL ? BN / 2 : BN;
     constexpr int NV = BN / 32;                    // accumulator values of a lane in the epilogue
     constexpr int kLaneCols = kOutN / 32;          // output columns of a lane
+    using Floats = typename std::conditional<DUAL, float2, float4>::type;  // a lane's part of a row, in float
+    using Halves = typename std::conditional<DUAL, uint32_t, uint2>::type;  // and in T
+    static_assert(sizeof(Floats) == kLaneCols * sizeof(float), "the stores of a lane");
     extern __shared__ unsigned char smem_raw[];
     __shared__ float s_sq[kTcBM];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -514,55 +517,45 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const bool in = n < N;  // N is a multiple of 8
         const size_t at = (size_t)m * ldy + n;
         float sq = 0.f;
-        if (DUAL) {
-            if (in) {
-                uint32_t w[kLaneCols / 2];
+        if (in) {
+            if constexpr (DUAL) {
 #pragma unroll
-                for (int e = 0; e < kLaneCols / 2; e++)
-                    w[e] = pack2<T>(gate_pair(v[2 * e], v[kLaneCols + 2 * e], epi.act, epi.limit),
-                                    gate_pair(v[2 * e + 1], v[kLaneCols + 2 * e + 1], epi.act, epi.limit));
-                *reinterpret_cast<uint32_t*>(y + at) = w[0];
+                for (int e = 0; e < kLaneCols; e++) v[e] = gate_pair(v[e], v[kLaneCols + e], epi.act, epi.limit);
             }
-        } else if (in) {
             if (epi.bias) {
 #pragma unroll
-                for (int e = 0; e < NV; e += 2) {
+                for (int e = 0; e < kLaneCols; e += 2) {
                     const float2 a = unpack2<T>(*reinterpret_cast<const uint32_t*>(static_cast<const T*>(epi.bias) + n + e));
                     v[e] += a.x;
                     v[e + 1] += a.y;
                 }
             }
             if (epi.f32) {
-#pragma unroll
-                for (int e = 0; e < NV; e += 4) {
-                    if (epi.resid) {
-                        const float4 r = *reinterpret_cast<const float4*>(static_cast<const float*>(epi.resid) + at + e);
-                        v[e] = fmaf(v[e], epi.scale, r.x);
-                        v[e + 1] = fmaf(v[e + 1], epi.scale, r.y);
-                        v[e + 2] = fmaf(v[e + 2], epi.scale, r.z);
-                        v[e + 3] = fmaf(v[e + 3], epi.scale, r.w);
-                    }
-                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + at + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-                }
-            } else {
-                uint32_t w[NV / 2];
                 if (epi.resid) {
-                    const T* rs = static_cast<const T*>(epi.resid) + at;
-                    *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(rs);
+                    __align__(16) float r[kLaneCols];
+                    *reinterpret_cast<Floats*>(r) = *reinterpret_cast<const Floats*>(static_cast<const float*>(epi.resid) + at);
 #pragma unroll
-                    for (int e = 0; e < NV / 2; e++) {
+                    for (int e = 0; e < kLaneCols; e++) v[e] = fmaf(v[e], epi.scale, r[e]);
+                }
+                *reinterpret_cast<Floats*>(reinterpret_cast<float*>(y) + at) = *reinterpret_cast<const Floats*>(v);
+            } else {
+                __align__(8) uint32_t w[kLaneCols / 2];
+                if (epi.resid) {
+                    *reinterpret_cast<Halves*>(w) = *reinterpret_cast<const Halves*>(static_cast<const T*>(epi.resid) + at);
+#pragma unroll
+                    for (int e = 0; e < kLaneCols / 2; e++) {
                         const float2 a = unpack2<T>(w[e]);
                         v[2 * e] += a.x;
                         v[2 * e + 1] += a.y;
                     }
                 }
 #pragma unroll
-                for (int e = 0; e < NV / 2; e++) {
+                for (int e = 0; e < kLaneCols / 2; e++) {
                     w[e] = pack2<T>(v[2 * e], v[2 * e + 1]);
                     const float2 a = unpack2<T>(w[e]);  // what the next projection will read
                     sq = fmaf(a.x, a.x, fmaf(a.y, a.y, sq));
                 }
-                *reinterpret_cast<uint2*>(y + at) = make_uint2(w[0], w[1]);
+                *reinterpret_cast<Halves*>(y + at) = *reinterpret_cast<const Halves*>(w);
             }
         }
         if (epi.ss_out) {
@@ -627,7 +620,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
         }
-        float v[NV], u[NV];
+        __align__(16) float v[NV], u[NV];
 #pragma unroll
         for (int e = 0; e < NV; e++) v[e] = u[e] = 0.f;
 #pragma unroll

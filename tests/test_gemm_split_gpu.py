@@ -67,6 +67,23 @@ def test_bfloat16_into_a_float_stream(ob, cuda, M, N, K):
     assert err(y[:, :N], ref) < 2e-6 and torch.equal(y[:, N:], side)  # float sums of exact products
 
 
+# every kernel a gated projection can take: few tokens, K split, blocks alone and in pairs
+@pytest.mark.parametrize("M,N,K", [(64, 256, 512), (65, 256, 512), (100, 1024, 1024), (128, 5632, 2048), (300, 200, 176)] + [s for s in SHAPES if s[2] % 16 == 0])
+@pytest.mark.parametrize("resid", [False, True])
+def test_gated_bfloat16_into_floats(ob, cuda, M, N, K, resid):
+    torch = cuda
+    x, (w, w2), rnd = operands(torch, M, N, K, torch.bfloat16, n=2)
+    y = rnd(M, N + 8)
+    side, start = y[:, N:].clone(), y[:, :N].double()
+    ref = (x.double() @ w.double()).clamp(min=0) * (x.double() @ w2.double())
+    if resid:
+        ob.project(ob.BF16, x, w, w2, y, M, N, K, ldy=N + 8, act=ob.GATE_RELU, f32=True, resid=y, scale=0.3)
+        ref = start + 0.3 * ref
+    else:
+        ob.project(ob.BF16, x, w, w2, y, M, N, K, ldy=N + 8, act=ob.GATE_RELU, f32=True)
+    assert err(y[:, :N], ref) < 4e-6 and torch.equal(y[:, N:], side)  # two float sums of exact products, multiplied
+
+
 def test_first_call_of_a_shape_inside_a_capture(ob, cuda):
     torch = cuda
     x, (w,), _ = operands(torch, 200, 776, 1000, torch.half)
