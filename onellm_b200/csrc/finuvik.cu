@@ -297,7 +297,7 @@ int Finuvik::layer(size_t i, const Buffers& buf, int tokens, const TokenPosition
     g.out_ld = w.n_cat;
     g.out_scale = (float)l.right_scale;
     g.work = buf.rec_work;
-    RC(gated_recurrence(g, tp, tp.B, tokens, stream));
+    RC(gated_recurrence(g, tp, tp.B, tokens, stream, /*settled=*/true));
     pj = Projection{};
     pj.dtype = dtype;
     pj.M = tokens;

@@ -496,7 +496,7 @@ int Fuposun::gla(size_t i, Pass& p)
     g.out_ld = w.n_out;
     g.out_scale = 1.f;
     g.work = b.rec_work;
-    RC(gated_recurrence(g, p.tp, p.tp.B, p.T, stream));
+    RC(gated_recurrence(g, p.tp, p.tp.B, p.T, stream, /*settled=*/true));
     return add_to_stream(p, b.cat, w.w_out, w.n_out);
 }
 

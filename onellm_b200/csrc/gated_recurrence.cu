@@ -104,6 +104,7 @@ __device__ __forceinline__ float decay(float z, float inv_tau) { return expm1f(i
 struct GrParams {
     GatedRecurrence g;
     TokenPositions tp;
+    int settled;  // see gated_recurrence (mixers.h)
 };
 
 // Layout of the work space of T tokens: the vectors of a head [H][T][n * dkp] (TIED n = 2: g, silu(q); KEYED n = 3: g, q, k),
@@ -443,8 +444,8 @@ __global__ void __launch_bounds__(256) gated_recurrence_norm_kernel(const GrPara
 }
 
 // One token per sequence.  A block owns `cols` value columns of one (sequence, head); cols / 4 threads share a row and
-// every thread walks the rows of its column group, 8 (KEYED 16) at a time.  What no earlier kernel of the step writes, the first
-// batch of the state, the gate matrix and the norm's weights, is requested in front of the dependency wait.
+// every thread walks the rows of its column group, 8 (KEYED 16) at a time.  For a caller whose state and weights are settled, the
+// first batch of the state, the gate matrix and the norm's weights are requested in front of the dependency wait.
 // 4 sequences, 8 heads of 256 x 512: 8.1 us (a batch of 8 and the gate matrix behind the wait: 16.1); the floor of its 34 MB is 5.
 constexpr int kGsThreads = 256;
 
@@ -460,6 +461,7 @@ __global__ void __launch_bounds__(kGsThreads) gated_recurrence_step_kernel(const
     const int tpr = cols / 4, rows_par = kGsThreads / tpr;  // threads per row, rows at a time
     const int r0 = tid / tpr, col = (tid % tpr) * 4;
     const bool works = r0 < rows_par;  // 256 need not be a multiple of tpr
+    if (!pp.settled) pdl_wait();  // the kernel in front may be the step that writes this state, and it lets this one start before it does
     const bool fresh = *pp.tp.step - 1 + pp.tp.off[b] == 0;
     float* base = p.state + (((size_t)b * p.H + h) * dk) * p.dv + c0 + col;
     float4 s[kGsBatch];
@@ -657,7 +659,7 @@ size_t gated_recurrence_workspace(int kind, int tokens, int H, int dk, int dv)
     return (size_t)tokens * H * (gr_vectors(kind) * gr_dkp(dk) + 2 * dv) * sizeof(float);
 }
 
-int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens, cudaStream_t st)
+int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens, cudaStream_t st, bool settled)
 {
     const bool keyed = g.kind == ONELLM_GR_KEYED;
     ONELLM_REQUIRE(g.kind == ONELLM_GR_TIED || keyed, ONELLM_ERR_ARG, "gated_recurrence: kind %d", g.kind);
@@ -668,7 +670,7 @@ int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, 
     ONELLM_REQUIRE(!keyed || (g.rank > 0 && g.rank <= 1024), ONELLM_ERR_UNSUPPORTED, "gated_recurrence: gate rank %d", g.rank);
     ONELLM_REQUIRE(g.H > 0 && g.H <= 65535 && B > 0 && B <= 65535 && g.ld % 8 == 0 && (tp.cu ? tp.hist && g.work && aligned16(g.work) : tp.step && tp.off),
                    ONELLM_ERR_ARG, "gated_recurrence: bad argument");
-    const GrParams p = {g, tp};
+    const GrParams p = {g, tp, settled};
     return g.dtype == ONELLM_F32 ? dispatch_gr<float>(p, B, tokens, st) : dispatch_gr<__nv_bfloat16>(p, B, tokens, st);
 }
 
@@ -682,5 +684,5 @@ extern "C" size_t onellm_gated_recurrence_workspace(int kind, int tokens, int H,
 extern "C" int onellm_gated_recurrence_run(const onellm_gated_recurrence* g, const onellm_token_positions* tp, int tokens, void* stream)
 {
     ONELLM_REQUIRE(g && tp && tokens >= 0, ONELLM_ERR_ARG, "gated_recurrence: bad argument");
-    return onellm::gated_recurrence(*g, *tp, tp->B, tokens, reinterpret_cast<cudaStream_t>(stream));
+    return onellm::gated_recurrence(*g, *tp, tp->B, tokens, reinterpret_cast<cudaStream_t>(stream), /*settled=*/false);
 }

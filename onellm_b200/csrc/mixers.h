@@ -46,7 +46,10 @@ inline int gated_recurrence_pad_dv(int dv)
     return (dv + m - 1) / m * m;
 }
 size_t gated_recurrence_workspace(int kind, int tokens, int H, int dk, int dv);
-int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens, cudaStream_t st);
+// settled: state, step counter and weights were written by work that is complete before the kernel enqueued just before this one
+// begins (the engine's first kernel of a step waits for everything in front of it).  A decode step then reads them before it waits
+// for that kernel; a caller that cannot say so gets every read behind the wait.
+int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens, cudaStream_t st, bool settled);
 
 // max_hist: most positions a sequence has before this pass; max_new: most new tokens of one
 inline int latent_pad(int rank) { return (rank + 63) / 64 * 64; }

@@ -463,6 +463,43 @@ def test_a_decode_step_at_the_first_position_starts_from_zero(cuda, ob):
     assert rel_err(got, ref_gla(x, A, zb, w, np.zeros((2, 32, 64)), 16.0, 1.0)) < 2e-5
 
 
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+@pytest.mark.parametrize("mode", ["tied", "keyed"])
+def test_decode_steps_with_nothing_between_them(cuda, ob, kind, mode):
+    """A step reads the state that the launch right in front of it writes, and norm weights that the one in front of both wrote."""
+    d = Dev(cuda, ob, kind)
+    rng = np.random.default_rng(8)
+    B, H, dk, dv, rank, n = 3, 4, 256, 256, 16, 12
+    keyed = mode == "keyed"
+    A, zb, lower = d.f32(rng.standard_normal((H * dk, rank)) / 4), d.f32(rng.uniform(-1, 3, H * dk)), d.f32(np.zeros(H * dk))
+    raw, ones, start = d.f32(rng.standard_normal((40, dv))), d.f32(np.ones(dv)), rng.standard_normal((B, H, dk, dv))
+    ld = H * (2 * dk + 2 * dv) + rank
+    rows = [d.up(rng.standard_normal((B, ld))) for _ in range(n)]
+    tp = ob.TokenPositions(None, None, B, d.i32([50]).data_ptr(), d.i32([0, -3, -9]).data_ptr())
+
+    def run(alone):
+        state, w, out = d.f32(start), d.zeros(40, dv, f32=True), [d.zeros(B, H * dv) for _ in range(n)]
+        es = rows[0].element_size()
+        calls = []
+        for x, o in zip(rows, out):
+            at = [x.data_ptr() + es * c for c in (0, H * dk, 2 * H * dk, 2 * H * dk + H * dv, 2 * H * (dk + dv))]
+            form = dict(kind=ob.GR_KEYED, k=at[1], r=at[4], rank=rank, A=A.data_ptr(), inv_tau=0.2, q_scale=0.1, g=at[3]) if keyed else \
+                dict(z=at[1], lower=lower.data_ptr())
+            calls.append(ob.GatedRecurrence(d.dtype, H, dk, dv, q=at[0], v=at[2], ld=ld, zb=zb.data_ptr(), w=w.data_ptr() + 4 * 39 * dv, eps=1e-5,
+                                            norm_width=dv, state=state.data_ptr(), out=o.data_ptr(), out_ld=H * dv, out_scale=1.0, **form))
+        cuda.cuda.synchronize()
+        ob.norm_rows(ob.F32, raw, None, 40, ones, None, w, None, 1e-5, dv, dv)
+        for c in calls:
+            if alone:
+                cuda.cuda.synchronize()
+            ob.gated_recurrence(c, tp, B)
+        cuda.cuda.synchronize()
+        return [state] + out
+
+    for a, b in zip(run(True), run(False)):
+        assert cuda.equal(a, b)
+
+
 def test_gated_linear_attention_remembers_through_a_slow_decay(cuda, ob):
     # a decay within 1e-6 of one (a large tau): what the first tokens wrote must still be there after thousands
     d = Dev(cuda, ob, "f32")
