@@ -224,7 +224,7 @@ void Finuvik::carve(Carver& cv)
 
 int Finuvik::norm(float* stream_rows, const int* rows, int n_rows, const float* w1, const float* w2, void* out1, void* out2)
 {
-    return norm_rows({dtype, stream_rows, rows, n_rows, w1, w2, out1, out2, (float)c.eps, 1.f, c.width, width, nullptr, nullptr, 0, 0.f}, stream);
+    return norm_rows({dtype, stream_rows, rows, n_rows, w1, w2, out1, out2, (float)c.eps, 1.f, c.width, width, nullptr, nullptr, 0, 0.f}, stream, /*settled=*/true);
 }
 
 // One layer over `tokens` tokens: a context pass (tp.cu) or a decode step.

@@ -386,13 +386,13 @@ int Fuposun::norm(Pass& p, const int* rows, int n_rows, const float* w, void* ou
         sum.add_n = p.add_n;
         sum.add_scale = (float)c.residual_mult;
         p.add_rows = nullptr;
-        if (!rows) return norm_rows(sum, stream);
+        if (!rows) return norm_rows(sum, stream, /*settled=*/true);
         sum.rows = nullptr;
         sum.n_rows = p.T;
         sum.out1 = nullptr;
-        RC(norm_rows(sum, stream));
+        RC(norm_rows(sum, stream, /*settled=*/true));
     }
-    return norm_rows(n, stream);
+    return norm_rows(n, stream, /*settled=*/true);
 }
 
 int Fuposun::latent_attention(size_t i, Pass& p)

@@ -63,7 +63,8 @@ int window_attn(const WindowAttn& a, const TokenPositions& tp, int max_new, cuda
 int route_max_tiles(int T, int experts, int top);
 int route(const Route& r, cudaStream_t st);
 // norm.cu
-int norm_rows(const NormRows& n, cudaStream_t st);
+// settled: the weights were written by work that is complete before the kernel enqueued just before this one begins
+int norm_rows(const NormRows& n, cudaStream_t st, bool settled);
 // elementwise.cu
 int embedding_norm_launch(int dtype, const int* ids, float* out, const void* table, const float* w, float eps, int n_tokens, int width, int ld,
                           int vocab, int* bad, cudaStream_t st);

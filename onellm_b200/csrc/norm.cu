@@ -179,9 +179,10 @@ namespace onellm {
 // ADD: the stream first takes add_scale times the sum of add_n rows of `add` (what the experts of a token made of it), so
 // that a feed-forward's last step and the next norm are one pass; out1 may be NULL then.
 constexpr int kPairVec = 8;  // float4 per thread kept in registers
-// EARLY: the weights, nobody's output, are requested in front of the dependency wait; behind the sum of a row they came from memory,
-// a fifth of a decode step's launch.  Only while every row has a place at once: the registers they take (126 instead of 64) cost
-// 2000 rows more than that.  Generation of 4 sequences, width 4096: 5.93 -> 5.84 ms; prompts of 2000 tokens lost 1.3 % with it.
+// EARLY: the weights are requested in front of the dependency wait, which only a caller whose weights are settled may ask for; behind
+// the sum of a row they came from memory, a fifth of a decode step's launch.  Only while every row has a place at once: the
+// registers they take (126 instead of 64) cost 2000 rows more than that.  Generation of 4 sequences, width 4096: 5.93 -> 5.84 ms;
+// prompts of 2000 tokens lost 1.3 % with it.
 template <typename T, bool ADD, bool EARLY>
 __global__ void __launch_bounds__(kNormThreads) norm_rows_kernel(const NormRows p)
 {
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(kNormThreads) norm_rows_kernel(const NormRows 
     for (int i = threadIdx.x + kPairVec * kNormThreads; i < nvec; i += kNormThreads) emit(i, xr[i], reinterpret_cast<const float4*>(p.w1)[i]);
 }
 
-int norm_rows(const NormRows& n, cudaStream_t st)
+int norm_rows(const NormRows& n, cudaStream_t st, bool settled)
 {
     ONELLM_REQUIRE(n.x && (n.out1 ? n.w1 != nullptr : n.add != nullptr) && (!n.out2 || (n.out1 && n.w2)) && (!n.add || n.add_rows), ONELLM_ERR_ARG,
                    "norm_rows: null pointer");
@@ -261,7 +262,7 @@ int norm_rows(const NormRows& n, cudaStream_t st)
     ONELLM_REQUIRE(n.dtype == ONELLM_BF16 || n.dtype == ONELLM_F32, ONELLM_ERR_UNSUPPORTED, "norm_rows: dtype %d", n.dtype);
     if (n.n_rows <= 0) return ONELLM_OK;
     const dim3 grid(n.n_rows), block(kNormThreads);
-    const bool early = n.n_rows <= 2 * num_sms() && !n.add;
+    const bool early = settled && n.n_rows <= 2 * num_sms() && !n.add;
     if (n.dtype == ONELLM_F32) {
         if (n.add) ONELLM_CUDA(launch_pdl(norm_rows_kernel<float, true, false>, grid, block, 0, st, n));
         else ONELLM_CUDA(launch_pdl(early ? norm_rows_kernel<float, false, true> : norm_rows_kernel<float, false, false>, grid, block, 0, st, n));
@@ -310,5 +311,5 @@ extern "C" int onellm_add_residual_rmsnorm(int dtype, void* residual, void* deco
 extern "C" int onellm_norm_rows_run(const onellm_norm_rows* n, void* stream)
 {
     ONELLM_REQUIRE(n, ONELLM_ERR_ARG, "norm_rows: null pointer");
-    return norm_rows(*n, reinterpret_cast<cudaStream_t>(stream));
+    return norm_rows(*n, reinterpret_cast<cudaStream_t>(stream), /*settled=*/false);
 }

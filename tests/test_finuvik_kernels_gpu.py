@@ -29,6 +29,26 @@ def test_two_zero_centred_norms(cuda, ob, kind, width, ld):
         assert np.all(host(o)[:, width:] == 0)
 
 
+def test_norm_weights_from_the_launch_in_front(cuda, ob):
+    d = Dev(cuda, ob, "f32")
+    rng = np.random.default_rng(2)
+    width, rows = 4096, 250
+    x, first, ones = d.f32(rng.standard_normal((5, width))), d.f32(rng.standard_normal((rows, width))), d.f32(np.ones(width))
+
+    def run(alone):
+        w, out = d.zeros(rows, width, f32=True), d.zeros(5, width, f32=True)
+        cuda.cuda.synchronize()
+        ob.norm_rows(ob.F32, first, None, rows, ones, None, w, None, 1e-5, width, width)
+        if alone:
+            cuda.cuda.synchronize()
+        ob.norm_rows(ob.F32, x, None, 5, w.data_ptr() + 4 * (rows - 1) * width, None, out, None, 1e-5, width, width)
+        cuda.cuda.synchronize()
+        return out
+
+    want = run(True)
+    assert all(cuda.equal(run(False), want) for _ in range(5))
+
+
 @pytest.mark.parametrize("kind", ["f32", "bf16"])
 @pytest.mark.parametrize("M", [1, 7, 16, 33, 64, 65, 300])
 def test_projection_forms(cuda, ob, kind, M):
