@@ -428,6 +428,26 @@ def test_topk_runs_of_equal_keys_on_both_ways_through_the_kernel(ob, cuda, orc, 
     assert np.array_equal(val.cpu().numpy(), rv)
 
 
+@pytest.mark.parametrize("dt", ["f16", "f32"])
+@pytest.mark.parametrize("V", [32000, 5000])
+@pytest.mark.parametrize("K", [1, 2, 3, 5, 10, 16, 17])
+def test_topk_with_the_large_logits_side_by_side(ob, cuda, orc, dt, V, K):
+    """Where the warp maxima are a poor bound: sorted rows, a few dozen threads full of large values, one warp that holds them all."""
+    torch = cuda
+    rng = np.random.default_rng(K)
+    x = rng.standard_normal((4, V)).astype(np.float32)
+    x[0], x[1] = np.sort(x[0]), np.sort(x[1])[::-1]
+    x[2, 640:640 + 32 * 40] += 20.0
+    x[3, 1024:2048] += 20.0
+    x = _round(x, dt)
+    val = torch.zeros(4, K, device="cuda")
+    idx = torch.zeros(4, K, device="cuda", dtype=torch.int32)
+    ob.topk(ob.F16 if dt == "f16" else ob.F32, _dev(torch, x, dt), 4, V, K, val, idx)
+    rv, ri = orc.topk(x, K)
+    assert np.array_equal(idx.cpu().numpy(), ri)
+    assert np.array_equal(val.cpu().numpy(), rv)
+
+
 def test_topk_reference_case(ob, cuda):
     # tests/unittests/test_beamsearch_topK.cu:12-25: probs[i] = i, V = 30000, K = 2, ids are row*V + column
     torch = cuda
