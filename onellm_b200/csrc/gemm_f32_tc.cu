@@ -1,9 +1,10 @@
 // float32 projections of more than 64 tokens on the tensor cores, with the precision of float.
 //
 // Replaces the cuBLAS SGEMM behind launchLinearGemm (src/kernels/qkv_linear.cu:8-65 of the reference) for context passes of
-// float32 callers.  A float is split exactly into three bf16 values, eight bits of its mantissa each (by truncation, so that
-// they have its sign and the first cannot overflow): x = x0 + x1 + x2.  Of the nine products of two such sums six are computed,
-// x0 w0, x0 w1, x1 w0, x0 w2, x1 w1, x2 w0; the other three are below 2^-24 of the result.
+// float32 callers.  A float is the sum of three bf16 values, each the nearest to what the ones before it leave (the method of Henry,
+// Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019):
+// x = x0 + x1 + x2, |x1| <= 2^-8 |x|, |x2| <= 2^-17 |x|.  Of the nine products of two such sums eight are computed; x2 w2, below
+// 2^-34 of x w, is not.
 //
 // A block computes y^T: 128 columns of W are the rows of the MMA, the tokens (at most 192) its columns, so that a token count
 // that is no multiple of 128 costs no padding.
@@ -13,7 +14,7 @@
 //          ([x0 | x1] in one tile of 128-byte rows, [x2 | unused] in a second one).
 //          Both come as floats by TMA, three stages ahead.
 //   sums   the tensor cores add into a float with truncation, so an accumulator is not kept for long: every stage of 32 rows
-//          starts a new one, the five small products go in before x0 w0, and the warps then add it to their
+//          starts a new one, the seven small products go in before x0 w0, and the warps then add it to their
 //          registers, rounding to nearest.  Two accumulators, two buffers of each operand: the warps add stage s - 1 and
 //          convert stage s + 1 while the MMAs of stage s run.
 // K is split over the blocks of a cluster where the tiles alone would not fill the GPU; the partial sums meet in distributed
@@ -69,12 +70,10 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
 __device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2)
 {
     constexpr uint32_t kTop = 0xffff0000u;
-    const uint32_t l0 = __float_as_uint(lo) & kTop, h0 = __float_as_uint(hi) & kTop;
-    const float lr = lo - __uint_as_float(l0), hr = hi - __uint_as_float(h0);
-    const uint32_t l1 = __float_as_uint(lr) & kTop, h1 = __float_as_uint(hr) & kTop;
-    const float lq = lr - __uint_as_float(l1), hq = hr - __uint_as_float(h1);
-    p0 = __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
-    p1 = __byte_perm(__float_as_uint(lr), __float_as_uint(hr), 0x7632);
+    p0 = pack2<__nv_bfloat16>(lo, hi);
+    const float lr = lo - __uint_as_float(p0 << 16), hr = hi - __uint_as_float(p0 & kTop);
+    p1 = pack2<__nv_bfloat16>(lr, hr);
+    const float lq = lr - __uint_as_float(p1 << 16), hq = hr - __uint_as_float(p1 & kTop);
     p2 = __byte_perm(__float_as_uint(lq), __float_as_uint(hq), 0x7632);
 }
 
@@ -162,9 +161,9 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             if (leader) {
                 const uint32_t d = tmem + (uint32_t)((s & 1) * kFtTok), wp = tmem + kFtPieces + (uint32_t)((s & 1) * 48);
                 const uint64_t xd = desc + (uint64_t)((s & 1) * (2 * kFtTile >> 4));
-                constexpr int kW[6] = {2, 0, 1, 1, 0, 0}, kX[6] = {0, 2, 1, 0, 1, 0};  // pieces of the products, small ones first
+                constexpr int kW[8] = {1, 2, 2, 0, 1, 1, 0, 0}, kX[8] = {2, 1, 0, 2, 1, 0, 1, 0};  // pieces of the products, small ones first
 #pragma unroll
-                for (int i = 0; i < 6; i++)
+                for (int i = 0; i < 8; i++)
 #pragma unroll
                     for (int kk = 0; kk < 2; kk++)
                         umma_f16_tmem_a(d, wp + kW[i] * 16 + kk * 8, xd + (uint64_t)(((kX[i] >> 1) * kFtTile + (kX[i] & 1) * 64 + kk * 32) >> 4), idesc,
@@ -379,10 +378,15 @@ static cudaError_t launch_ft(const GemmF32& a, cudaStream_t st)
     return cudaLaunchKernelEx(&cfg, kern, a, map_x, map_w, best_nt, best_per);
 }
 
+// Below, the chain of sgemm_kernel is as close or closer for some operands (equal ones, ones of very unequal size); from here on this
+// kernel is the closer for every kind that was tried.  256 products, error against 64 bits of the chain | here: normal 2.9e-7 | 8.0e-8,
+// positive 2.2e-7 | 7.0e-8, log-normal 8.7e-8 | 5.7e-8, all equal 1.19e-7 | 1.16e-7.
+constexpr int kFtLeastK = 256;
+
 // Sizes, strides and alignment it covers: 16-byte rows.
 bool gemm_f32_tc_takes(const GemmF32& a)
 {
-    return a.M > kF32SkinnyTokens && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W) &&
+    return a.M > kF32SkinnyTokens && a.K >= kFtLeastK && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W) &&
            ((long)a.M + 15) / 16 <= 65535;
 }
 

@@ -51,6 +51,38 @@ def test_gemm_f32_keeps_infinities_and_nan(ob, cuda, M):
         assert torch.equal(same(y), same(ref))
 
 
+def both_ways(ob, torch, x, w, nk):
+    """The product by the kernel that takes the call, and by the chain of multiply-adds of the tiled kernel, which takes unaligned rows."""
+    (M, K), N = x.shape, w.shape[1]
+    shifted = torch.empty(M * K + 1, device="cuda")[1:].view(M, K)
+    shifted.copy_(x)
+    dw, out = w.T.contiguous() if nk else w, []
+    for a in (x, shifted):
+        y = torch.empty(M, N, device="cuda")
+        ob.gemm(ob.F32, a, dw, y, M, N, K, ob.W_NK if nk else ob.W_KN)
+        out.append(y)
+    return out
+
+
+def off(y, x, w):
+    ref = x.double() @ w.double()
+    return float((y.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("K", [4, 16, 64, 252, 256, 260, 1024, 4096])
+@pytest.mark.parametrize("kind", ["normal", "positive", "constant", "ends"])
+@pytest.mark.parametrize("nk", [False, True])
+def test_more_than_64_tokens_are_no_less_exact_than_a_chain(ob, cuda, K, kind, nk):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(K)
+    make = {"normal": lambda *s: torch.randn(*s, generator=g, device="cuda"), "positive": lambda *s: torch.rand(*s, generator=g, device="cuda"),
+            "constant": lambda *s: torch.full(s, 1.0078124, device="cuda"), "ends": lambda *s: torch.full(s, 1 + 2.0 ** -7 - 2.0 ** -23, device="cuda")}[kind]
+    x, w = make(130, K), make(K, 260)
+    fast, chain = (off(y, x, w) for y in both_ways(ob, torch, x, w, nk))
+    # equal operands are the chain's good or bad luck: one step of the result's last place is let pass
+    assert fast <= (1.02 * chain if kind in ("normal", "positive") else max(chain, 2.0 ** -23))
+
+
 @pytest.mark.parametrize("M", [1, 6, 30, 100])
 def test_projection_f32_gate_and_residual(ob, cuda, M):
     torch = cuda
