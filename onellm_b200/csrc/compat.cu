@@ -13,6 +13,8 @@
 //   onellm_transpose_remove_padding launchTransposeOutRemovePadding  src/kernels/fused_transpose_reshape_remv_pad.cu:5-51
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace onellm {
@@ -129,8 +131,10 @@ struct GemmStrides {
 
 // 16 TM x 16 TN outputs per block, TM x TN per thread, so that a value read from shared memory serves TN or TM multiply-adds; the
 // next 16 steps of k are requested while the present ones are added.  Threads run along whichever index an operand has
-// contiguous.  Bound by the multiply-adds and shared-memory reads (one output per thread, as this was before, by the latter
-// alone).  Each output is one chain of multiply-adds in the order of k.  64 heads of 255 x 295 x 128 and of 255 x 128 x 295: 44 us each, before 185.
+// contiguous.  Bound by the multiply-adds and shared-memory reads where blocks fill the GPU, by the steps of k one after the other
+// where they do not.  Each output is one chain of multiply-adds in the order of k.
+// Before (one output per thread, loads and adds in turn) | now, us, float: 64 heads of 255 x 295 x 128 and of 255 x 128 x 295: 190 | 52;
+// one of 255 x 128 x 295: 8.9 | 6.5; 64 x 64 x 2048: 48 | 33; 20 x 20 x 4096: 94 | 64.
 template <typename T, int TM, int TN>
 __global__ void __launch_bounds__(256)
 strided_gemm_kernel(const T* __restrict__ A, const T* __restrict__ Bm, T* __restrict__ Cm, int m, int n, int k, GemmStrides s, float alpha, float beta)
@@ -154,19 +158,19 @@ strided_gemm_kernel(const T* __restrict__ A, const T* __restrict__ Bm, T* __rest
         j = b_along_k ? e / BK : e % BN;
         kk = b_along_k ? e % BK : e / BN;
     };
-    float av[TM], bv[TN];
+    T av[TM], bv[TN];  // as they come: a conversion here would wait for the load
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < TM; i++) {
             int r, kk;
             a_at(i, r, kk);
-            av[i] = m0 + r < m && k0 + kk < k ? (float)a[(m0 + r) * s.a_i + (k0 + kk) * s.a_k] : 0.f;
+            av[i] = m0 + r < m && k0 + kk < k ? a[(m0 + r) * s.a_i + (k0 + kk) * s.a_k] : (T)0.f;
         }
 #pragma unroll
         for (int i = 0; i < TN; i++) {
             int j, kk;
             b_at(i, j, kk);
-            bv[i] = n0 + j < n && k0 + kk < k ? (float)b[(k0 + kk) * s.b_k + (n0 + j) * s.b_j] : 0.f;
+            bv[i] = n0 + j < n && k0 + kk < k ? b[(k0 + kk) * s.b_k + (n0 + j) * s.b_j] : (T)0.f;
         }
     };
     const int ty = tid >> 4, tx = tid & 15;
@@ -177,13 +181,13 @@ strided_gemm_kernel(const T* __restrict__ A, const T* __restrict__ Bm, T* __rest
         for (int i = 0; i < TM; i++) {
             int r, kk;
             a_at(i, r, kk);
-            as[kk][r] = av[i];
+            as[kk][r] = (float)av[i];
         }
 #pragma unroll
         for (int i = 0; i < TN; i++) {
             int j, kk;
             b_at(i, j, kk);
-            bs[kk][j] = bv[i];
+            bs[kk][j] = (float)bv[i];
         }
         __syncthreads();
         if (k0 + BK < k) fetch(k0 + BK);
@@ -214,17 +218,26 @@ strided_gemm_kernel(const T* __restrict__ A, const T* __restrict__ Bm, T* __rest
     }
 }
 
+// What a step of 16 k takes a block that is alone on its SM, and for each block of an SM that is full (us), for 1 x 1, 1 x 4 (4 x 1) and
+// 4 x 4 outputs per thread.
+constexpr double kStep11 = 0.39, kBusy11 = 0.22, kStep14 = 0.44, kBusy14 = 0.30, kStep44 = 0.83, kBusy44 = 0.64;
+
 template <typename T>
 static cudaError_t launch_strided_gemm(const void* A, const void* Bm, void* Cm, int batch, int m, int n, int k, GemmStrides s,
                                        float alpha, float beta, cudaStream_t st)
 {
-    // few rows (or columns): blocks of 16 of them
-    if (m <= 16)
-        strided_gemm_kernel<T, 1, 4><<<dim3((n + 63) / 64, (m + 15) / 16, batch), 256, 0, st>>>((const T*)A, (const T*)Bm, (T*)Cm, m, n, k, s, alpha, beta);
-    else if (n <= 16)
-        strided_gemm_kernel<T, 4, 1><<<dim3((n + 15) / 16, (m + 63) / 64, batch), 256, 0, st>>>((const T*)A, (const T*)Bm, (T*)Cm, m, n, k, s, alpha, beta);
-    else
-        strided_gemm_kernel<T, 4, 4><<<dim3((n + 63) / 64, (m + 63) / 64, batch), 256, 0, st>>>((const T*)A, (const T*)Bm, (T*)Cm, m, n, k, s, alpha, beta);
+    auto blocks = [&](int tm, int tn) { return (long)((m + 16 * tm - 1) / (16 * tm)) * ((n + 16 * tn - 1) / (16 * tn)) * batch; };
+    // More outputs per thread pay once the small blocks no longer find places at the same time.
+    auto time = [&](int tm, int tn, double alone, double busy) { return std::max(alone, blocks(tm, tn) * busy / num_sms()); };
+    const double t11 = time(1, 1, kStep11, kBusy11), t14 = time(1, 4, kStep14, kBusy14), t41 = time(4, 1, kStep14, kBusy14), t44 = time(4, 4, kStep44, kBusy44);
+    auto launch = [&](auto kern, int tm, int tn) {
+        kern<<<dim3((n + 16 * tn - 1) / (16 * tn), (m + 16 * tm - 1) / (16 * tm), batch), 256, 0, st>>>((const T*)A, (const T*)Bm, (T*)Cm, m, n, k, s, alpha, beta);
+    };
+    const double least = std::min({t11, t14, t41, t44});
+    if (least == t11) launch(strided_gemm_kernel<T, 1, 1>, 1, 1);
+    else if (least == t14) launch(strided_gemm_kernel<T, 1, 4>, 1, 4);
+    else if (least == t41) launch(strided_gemm_kernel<T, 4, 1>, 4, 1);
+    else launch(strided_gemm_kernel<T, 4, 4>, 4, 4);
     return cudaPeekAtLastError();
 }
 

@@ -153,6 +153,22 @@ def test_batched_gemm_edges_of_tiles(ob, cuda, ta, tb, m, n, k):
     assert float(((Cm.double() - ref).abs() / size).max()) < 4 * k ** 0.5 * 2.0 ** -24 + 2.0 ** -22
 
 
+# 4 x 4, 1 x 4 and 4 x 1 outputs a thread, which calls with many blocks take, and the last small call
+@pytest.mark.parametrize("batch,m,n,k", [(300, 70, 90, 21), (900, 10, 130, 33), (900, 130, 10, 33), (64, 48, 48, 40), (12, 32, 33, 17)])
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True)])
+def test_batched_gemm_of_many_batches(ob, cuda, batch, m, n, k, half, ta, tb):
+    torch = cuda
+    g, t = torch.Generator(device="cuda").manual_seed(k), torch.half if half else torch.float32
+    A, Bm = (torch.randn(*s, device="cuda", generator=g).to(t) for s in ((batch, m, k), (batch, k, n)))
+    Cm = torch.full((batch, m, n), 7.0, device="cuda", dtype=t)
+    at, bt = (A.transpose(1, 2).contiguous() if ta else A), (Bm.transpose(1, 2).contiguous() if tb else Bm)
+    ob.batched_gemm(ob.F16 if half else ob.F32, at, bt, Cm, batch, m, n, k, trans_a=ta, trans_b=tb)
+    ref, size = A.double() @ Bm.double(), (A.double() ** 2 @ Bm.double() ** 2).sqrt()
+    bound = (4 * k ** 0.5 * 2.0 ** -24 + 2.0 ** -22) * size + (2.0 ** -11 * ref.abs() + 2.0 ** -24 if half else 0.0)  # half: one rounding more
+    assert bool(((Cm.double() - ref).abs() <= bound).all())
+
+
 def test_softmax_fully_masked_row_is_zero(ob, cuda):
     torch = cuda
     qk = torch.randn(1, 2, 3, 40, device="cuda")
