@@ -254,7 +254,11 @@ int Engine::prefill_context(int B, const int* lens)
 {
     ContextBatch c;
     c.B = B;
-    std::vector<int> cu(B + 1, 0), hist(B), off(B);
+    std::vector<int>&cu = h_cu, &hist = h_hist, &off = h_off, &rows = h_rows;
+    cu.assign(B + 1, 0);
+    hist.assign(B, 0);
+    off.assign(B, 0);
+    rows.clear();
     seq_off.resize(max_batch, 0);
     int new_max = 0;
     for (int b = 0; b < B; b++) {
@@ -266,7 +270,6 @@ int Engine::prefill_context(int B, const int* lens)
     }
     for (int b = 0; b < B; b++) off[b] = hist[b] + lens[b] - new_max;
     // the rows whose logits are computed: the last one of every sequence, then the ones asked for
-    std::vector<int> rows;
     for (int b = 0; b < B; b++) rows.push_back(cu[b + 1] - 1);
     for (int r : want_rows) {
         ONELLM_REQUIRE(r >= 0 && (size_t)r < c.T, ONELLM_ERR_ARG, "want_logits: row %d outside the %zu tokens of this call", r, c.T);
@@ -297,7 +300,6 @@ int Engine::prefill_context(int B, const int* lens)
     ONELLM_CUDA(cudaMemcpyAsync(d_cu, cu.data(), (B + 1) * sizeof(int), cudaMemcpyHostToDevice, stream));
     ONELLM_CUDA(cudaMemcpyAsync(d_hist, hist.data(), B * sizeof(int), cudaMemcpyHostToDevice, stream));
     ONELLM_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
-    // (the host arrays are pageable: each copy has left them when its call returns)
     const long before = launches_noted();
     RC(context_layers(c));
     RC(sample(c.logits));  // seeded with the step counter, as the position-by-position path does
@@ -421,6 +423,14 @@ extern "C" int onellm_llama_set_graphs(onellm_llama* h, int enabled)
     return ONELLM_OK;
 }
 
+// The end of a context pass.  One that failed may have left copies behind that read the caller's ids or the engine's host arrays:
+// they are waited for, as finish_context waits for those of a pass that went well.
+static int end_pass(Engine* m, int rc)
+{
+    if (rc != ONELLM_OK) (void)cudaStreamSynchronize(m->stream);
+    return rc;
+}
+
 extern "C" int onellm_llama_prefill(onellm_llama* h, const int* host_ids, int batch, int prompt_len, int* host_first_ids)
 {
     Engine* m = engine_of(h);
@@ -440,21 +450,23 @@ extern "C" int onellm_llama_prefill(onellm_llama* h, const int* host_ids, int ba
     m->seq_off.assign(m->max_batch, 0);
     ONELLM_CUDA(cudaMemsetAsync(m->d_step_off, 0, (size_t)m->max_batch * sizeof(int), st));
     const int first_step = m->prefill_by_decode ? 0 : prompt_len;  // the step kernels increment before use
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * prompt_len * sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &first_step, sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
-    if (m->prefill_by_decode) {
-        ONELLM_REQUIRE(m->want_rows.empty(), ONELLM_ERR_STATE, "llama_prefill: logits of single rows need the context-phase kernels");
-        // one position at a time through the decode kernels; only the last position needs the LM head
-        for (int p = 0; p < prompt_len; p++)
-            RC(m->run_step(MODE_GATHER | (p == prompt_len - 1 ? MODE_HEAD : 0), prompt_len));
-    } else {
-        const std::vector<int> lens(batch, prompt_len);
-        RC(m->prefill_context(batch, lens.data()));
-    }
-    return m->finish_context(host_first_ids, "llama_prefill");
+    return end_pass(m, [&]() -> int {
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * prompt_len * sizeof(int), cudaMemcpyHostToDevice, st));
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &first_step, sizeof(int), cudaMemcpyHostToDevice, st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
+        if (m->prefill_by_decode) {
+            ONELLM_REQUIRE(m->want_rows.empty(), ONELLM_ERR_STATE, "llama_prefill: logits of single rows need the context-phase kernels");
+            // one position at a time through the decode kernels; only the last position needs the LM head
+            for (int p = 0; p < prompt_len; p++)
+                RC(m->run_step(MODE_GATHER | (p == prompt_len - 1 ? MODE_HEAD : 0), prompt_len));
+        } else {
+            const std::vector<int> lens(batch, prompt_len);
+            RC(m->prefill_context(batch, lens.data()));
+        }
+        return m->finish_context(host_first_ids, "llama_prefill");
+    }());
 }
 
 // Prompts of different lengths: host_ids holds them packed one after the other, lens[b] tokens each.  Sequence b is
@@ -480,13 +492,15 @@ extern "C" int onellm_llama_prefill_ragged(onellm_llama* h, const int* host_ids,
     m->batch = batch;
     m->cur_len = 0;
     m->seq_off.assign(m->max_batch, 0);
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, total * sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &longest, sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
-    ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
-    RC(m->prefill_context(batch, lens));
-    return m->finish_context(host_first_ids, "llama_prefill_ragged");
+    return end_pass(m, [&]() -> int {
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, total * sizeof(int), cudaMemcpyHostToDevice, st));
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &longest, sizeof(int), cudaMemcpyHostToDevice, st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
+        ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
+        RC(m->prefill_context(batch, lens));
+        return m->finish_context(host_first_ids, "llama_prefill_ragged");
+    }());
 }
 
 // A further turn: n_new more tokens per sequence behind the cur_len positions already cached (history),
@@ -500,11 +514,13 @@ extern "C" int onellm_llama_extend(onellm_llama* h, const int* host_ids, int n_n
                    "llama_extend: %d cached + %d new positions exceed max_seq_len %d", m->cur_len, n_new, m->max_seq_len);
     cudaStream_t st = m->stream;
     const int batch = m->batch, new_len = m->cur_len + n_new;
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * n_new * sizeof(int), cudaMemcpyHostToDevice, st));
-    ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &new_len, sizeof(int), cudaMemcpyHostToDevice, st));
-    const std::vector<int> lens(batch, n_new);
-    RC(m->prefill_context(batch, lens.data()));
-    return m->finish_context(host_first_ids, "llama_extend");
+    return end_pass(m, [&]() -> int {
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * n_new * sizeof(int), cudaMemcpyHostToDevice, st));
+        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &new_len, sizeof(int), cudaMemcpyHostToDevice, st));
+        const std::vector<int> lens(batch, n_new);
+        RC(m->prefill_context(batch, lens.data()));
+        return m->finish_context(host_first_ids, "llama_extend");
+    }());
 }
 
 // The next prefill / extend call also computes the logits of these token rows (packed order of that call).

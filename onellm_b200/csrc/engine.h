@@ -72,6 +72,8 @@ struct Engine {
     // what the host reads at the end of a pass: bad_id [2], whether a bounded wait gave up, sampled ids [max_batch]
     int *d_report = nullptr, *h_report = nullptr;  // h_report: pinned
     TimeoutFlags timeout_flags = {};
+    // what the copies of a context pass read: kept until the next pass, which begins after the stream has been waited for
+    std::vector<int> h_off, h_cu, h_hist, h_rows;
     // state
     int batch = 0, cur_len = 0, graph_prompt_len = 0;
     int top_k = 1, literal_walk = 0;  // top_k 0: logits only, nothing is sampled

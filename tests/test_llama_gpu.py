@@ -155,6 +155,26 @@ def test_second_turn_with_history_matches_one_long_prompt(ob, cuda, orc, tmp_pat
     m.close()
 
 
+def test_a_context_pass_that_fails_has_read_its_ids(ob, cuda, tmp_path):
+    """An error behind the copy of the ids: the caller's (pinned) memory is free when the call returns, and the next pass is right."""
+    import ctypes as C
+    m, _ = _make(ob, tmp_path, CFG, seed=12)
+    ids = np.random.default_rng(7).integers(0, CFG["vocab_size"], (3, 40)).astype(np.int32)
+    want_first = m.prefill(ids)
+    want = m.logits(3)
+    for _ in range(3):
+        pinned = cuda.from_numpy(ids.copy()).pin_memory()
+        m.want_logits([3 * 40])
+        with pytest.raises(ob.OnellmError):
+            ob._check(ob.lib().onellm_llama_prefill(m._h, C.c_void_p(pinned.data_ptr()), C.c_int(3), C.c_int(40), None))
+        pinned.fill_(-1)
+        m.want_logits([])
+        assert np.array_equal(m.prefill(ids), want_first) and np.array_equal(m.logits(3), want)
+        with pytest.raises(ob.OnellmError):  # ids outside the vocabulary: the error comes behind the first tokens
+            m.prefill(np.where(ids == ids[0, 0], CFG["vocab_size"], ids))
+    m.close()
+
+
 def test_norm_free_context_phase_matches_the_one_with_norm_kernels(ob, cuda, tmp_path):
     """One GPU runs the context phase without norm kernels (row statistics handed from projection to projection);
     mode 2 keeps the norm kernels, as tensor-parallel runs do.  Same model, same prompt."""
