@@ -318,6 +318,7 @@ int Engine::finish_context(int* host_first_ids, const char* where)
     ONELLM_CUDA(cudaMemcpyAsync(h_report, d_report, (4 + (size_t)batch) * sizeof(int), cudaMemcpyDeviceToHost, stream));
     RC(queue_comm_check());
     ONELLM_CUDA(cudaStreamSynchronize(stream));
+    if (host_first_ids) memcpy(host_first_ids, h_report + 4, (size_t)batch * sizeof(int));
     RC(comm_check(where));
     ONELLM_REQUIRE(h_report[0] == 0, ONELLM_ERR_ARG, "%s: token id outside [0, vocab_size)", where);
     ONELLM_REQUIRE(h_report[1] == 0, ONELLM_ERR_STATE, "%s: a position beyond max_seq_len was refused by the cache", where);
@@ -325,7 +326,6 @@ int Engine::finish_context(int* host_first_ids, const char* where)
         (void)onellm_gemm_timeout_flag();  // clears it
         ONELLM_REQUIRE(false, ONELLM_ERR_CUDA, "%s: a tensor-core GEMM block timed out", where);
     }
-    if (host_first_ids) memcpy(host_first_ids, h_report + 4, (size_t)batch * sizeof(int));
     return ONELLM_OK;
 }
 
