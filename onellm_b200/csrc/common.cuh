@@ -24,13 +24,13 @@ long launches_noted();
 struct TimeoutFlag {
     TimeoutFlag(int (*read_and_clear)(), const int* (*address)());
 };
-// Device addresses of these flags on the current device, for a kernel that reads them on its way (at most kMaxTimeoutFlags;
-// null behind the last one).
+// Device addresses of these flags on the current device, for a kernel that reads them on its way (null behind the last one); false if
+// there are more than kMaxTimeoutFlags.
 constexpr int kMaxTimeoutFlags = 16;
 struct TimeoutFlags {
     const int* at[kMaxTimeoutFlags];
 };
-TimeoutFlags timeout_flag_addresses();
+bool timeout_flag_addresses(TimeoutFlags* out);
 
 #define ONELLM_REQUIRE(cond, code, ...)          \
     do {                                         \

@@ -125,7 +125,7 @@ int Engine::allocate()
     ONELLM_CUDA(cudaMemsetAsync(arena, 0, arena_bytes, stream));
     ONELLM_CUDA(cudaStreamSynchronize(stream));
     ONELLM_CUDA(cudaMallocHost(&h_report, (4 + (size_t)max_batch) * sizeof(int)));
-    timeout_flags = timeout_flag_addresses();
+    ONELLM_REQUIRE(timeout_flag_addresses(&timeout_flags), ONELLM_ERR_STATE, "%s: more than %d time-out flags", design(), kMaxTimeoutFlags);
     return build_skip_table(d_skip, max_batch, &skip_ok, stream);
 }
 

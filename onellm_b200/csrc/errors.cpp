@@ -50,15 +50,16 @@ static std::vector<FlagReaders>& timeout_flags()
 }
 TimeoutFlag::TimeoutFlag(int (*read_and_clear)(), const int* (*address)()) { timeout_flags().push_back({read_and_clear, address}); }
 
-TimeoutFlags timeout_flag_addresses()
+bool timeout_flag_addresses(TimeoutFlags* out)
 {
-    TimeoutFlags f = {};
+    *out = {};
     int n = 0;
     for (const auto& r : timeout_flags()) {
         const int* p = r.address();
-        if (p && n < kMaxTimeoutFlags) f.at[n++] = p;
+        if (p && n == kMaxTimeoutFlags) return false;
+        if (p) out->at[n++] = p;
     }
-    return f;
+    return true;
 }
 
 }  // namespace onellm
