@@ -23,14 +23,13 @@
 // the waits between them 450, the last three one after the other in every warp.  Measured, 352 tokens of the 7B shapes, us (the 64 x
 // 64 tiled kernel before): QKV 262 (3000), o_proj 93 (890), gate or up 240 (2600), down 215 (2400), 127 to 147 TFLOP/s of float32;
 // error against 64 bits 1.8e-7 (2.6e-7 at K = 11008), a layer 7e-7 instead of 2.8e-6.
-// A value that is not finite makes its remainders NaN and so every result it enters; a result that is not finite (also one
-// whose partial sums overflowed) is computed again with plain multiply-adds.
+// What the pieces do not hold: a value that is not finite, or whose first piece rounds to infinity, makes its remainders NaN and so
+// every result it enters; one below 2^-110 loses its last bits.  Blocks whose results that touches (see `stands`) compute them
+// again by plain multiply-adds, at the rate of the tiled kernel; the results are that kernel's to the bit.
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <map>
 #include <mutex>
-#include <tuple>
 
 #include "gemm_f32.h"
 #include "tc_common.cuh"
@@ -50,6 +49,10 @@ constexpr int kFtDepth = 3;                     // stages of floats on their way
 constexpr int kFtRawW = kFtK * kFtCols * 4, kFtRaw = kFtRawW + kFtTok * kFtK * 4;
 constexpr int kFtSmem = kFtPiecesBytes + kFtDepth * kFtRaw;
 constexpr int kFtGroup = kFtTok / 2 / 3;        // accumulator columns read at a time
+// The third piece of a float below 2^-110 falls among the subnormal bf16 values and loses up to 2^-133, on either side of a product: a
+// result of K products beside the largest operand then counts from 2^26 times K * 2^-132 of it.  Below kFtLeast the products of
+// the pieces themselves leave the range of float.
+constexpr float kFtLost = 0x1p-106f, kFtLeast = 0x1p-80f;
 constexpr uint32_t kFtPieces = 2 * kFtTok;      // tensor memory: two accumulators, then two stages of 3 pieces x 16 columns
 static_assert(kFtGroup == 32 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
 
@@ -66,8 +69,9 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                  "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-// the three bf16 pieces of two floats, packed piece by piece (lo in the low half)
-__device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2)
+// the three bf16 pieces of two floats, packed piece by piece (lo in the low half); rest: the ends of the third ones that bf16 has no
+// place for, in its low half
+__device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2, uint32_t& rest)
 {
     constexpr uint32_t kTop = 0xffff0000u;
     p0 = pack2<__nv_bfloat16>(lo, hi);
@@ -75,24 +79,113 @@ __device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uin
     p1 = pack2<__nv_bfloat16>(lr, hr);
     const float lq = lr - __uint_as_float(p1 << 16), hq = hr - __uint_as_float(p1 & kTop);
     p2 = __byte_perm(__float_as_uint(lq), __float_as_uint(hq), 0x7632);
+    rest |= __float_as_uint(lq) | __float_as_uint(hq);
 }
 
-template <bool NK>
-__device__ __noinline__ float plain_dot(const GemmF32& a, int m, int n)
-{
-    const float *x = a.x + (size_t)m * a.ldx, *w = NK ? a.W + (size_t)n * a.ldw : a.W + n;
-    float s = 0.f;
-    for (int k = 0; k < a.K; k++) s = fmaf(x[k], NK ? w[k] : w[(size_t)k * a.ldw], s);
-    return s;
-}
-template <bool NK>
 __device__ __forceinline__ void finish_f32(const GemmF32& a, int m, int n, float v)
 {
-    if (!isfinite(v)) v = plain_dot<NK>(a, m, n);
     const size_t at = (size_t)m * a.ldy + n;
     if (a.resid) v = fmaf(v, a.scale, a.resid[at]);
     if (a.gate >= 0) v = gate_pair<true>(a.y[at], v, a.gate, a.limit);
     a.y[at] = v;
+}
+
+// This thread's share of the largest operand of a block, 16 bytes at a time (K, and N of W [K,N], are multiples of 4)
+template <bool NK>
+__device__ __noinline__ float largest(const GemmF32& a, int m0, int rows, int n0, int k_begin, int k_end)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_end = min(n0 + kFtCols, a.N);
+    float top = 0.f;
+    auto take = [&](const float* p) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        top = fmaxf(fmaxf(top, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+    };
+    auto rows_of = [&](const float* p, int begin, int end, long ld) {
+        for (int r = begin + warp; r < end; r += kFtThreads / 32)
+#pragma unroll 8
+            for (int k = k_begin + 4 * lane; k < k_end; k += 128) take(p + (size_t)r * ld + k);
+    };
+    rows_of(a.x, m0, m0 + rows, a.ldx);
+    if constexpr (NK) {
+        rows_of(a.W, n0, n_end, a.ldw);
+    } else if (n0 + 4 * lane < n_end) {
+#pragma unroll 8
+        for (int k = k_begin + warp; k < k_end; k += kFtThreads / 32) take(a.W + (size_t)k * a.ldw + n0 + 4 * lane);
+    }
+    return top;
+}
+
+// The outputs of `rows` tokens from m0 on and the block's columns by multiply-adds in the order of k, as sgemm_kernel adds them: 64 tokens
+// at a time, 4 x 8 outputs a thread, the operands of the next 32 k on their way meanwhile.  All threads of the block call it (the last
+// warp for the barriers); buf: kFtPlainBytes of shared memory.
+constexpr int kFtPlainK = 32, kFtPlainTok = 64;
+constexpr int kFtPlainBytes = kFtPlainK * (kFtPlainTok + 4 + kFtCols + 4) * 4;
+static_assert(kFtPlainBytes <= kFtDepth * kFtRaw, "in place of the floats");
+template <bool NK>
+__device__ __noinline__ void plain_tile(const GemmF32& a, float* buf, int m0, int rows, int n0)
+{
+    float(*xs)[kFtPlainTok + 4] = reinterpret_cast<float(*)[kFtPlainTok + 4]>(buf);
+    float(*ws)[kFtCols + 4] = reinterpret_cast<float(*)[kFtCols + 4]>(buf + kFtPlainK * (kFtPlainTok + 4));
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const bool works = tid < 256;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t0 = 0; t0 < rows; t0 += kFtPlainTok) {
+        // four values of k of a token, or of a column; W [K,N]: four columns.  K, and N there, are multiples of 4.
+        float4 xv[2], wv[4];
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int e = tid + 256 * i, t = t0 + (e >> 3), k = k0 + (e & 7) * 4;
+                xv[i] = works && t < rows && k < a.K ? *reinterpret_cast<const float4*>(a.x + (size_t)(m0 + t) * a.ldx + k) : zero;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int e = tid + 256 * i, n = n0 + (NK ? e >> 3 : (e & 31) * 4), k = k0 + (NK ? (e & 7) * 4 : e >> 5);
+                wv[i] = works && n < a.N && k < a.K ? *reinterpret_cast<const float4*>(a.W + (NK ? (size_t)n * a.ldw + k : (size_t)k * a.ldw + n)) : zero;
+            }
+        };
+        float acc[4][8] = {};
+        fetch(0);
+        for (int k0 = 0; k0 < a.K; k0 += kFtPlainK) {
+            __syncthreads();
+            if (works) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int e = tid + 256 * i, t = e >> 3, k = (e & 7) * 4;
+                    xs[k][t] = xv[i].x, xs[k + 1][t] = xv[i].y, xs[k + 2][t] = xv[i].z, xs[k + 3][t] = xv[i].w;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int e = tid + 256 * i, c = e >> 3, k = (e & 7) * 4;
+                    if constexpr (NK) ws[k][c] = wv[i].x, ws[k + 1][c] = wv[i].y, ws[k + 2][c] = wv[i].z, ws[k + 3][c] = wv[i].w;
+                    else *reinterpret_cast<float4*>(&ws[e >> 5][(e & 31) * 4]) = wv[i];
+                }
+            }
+            __syncthreads();
+            if (k0 + kFtPlainK < a.K) fetch(k0 + kFtPlainK);
+            const int steps = works ? min(kFtPlainK, a.K - k0) : 0;
+#pragma unroll 4
+            for (int kk = 0; kk < steps; kk++) {
+                float x[4], w[8];
+                *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(&xs[kk][ty * 4]);
+                *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(&ws[kk][tx * 4]);
+                *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(&ws[kk][64 + tx * 4]);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) acc[i][j] = fmaf(x[i], w[j], acc[i][j]);
+            }
+        }
+        if (works) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int t = t0 + ty * 4 + i, n = n0 + (j >> 2) * 64 + tx * 4 + (j & 3);
+                    if (t < rows && n < a.N) finish_f32(a, m0 + t, n, acc[i][j]);
+                }
+        }
+    }
 }
 
 // grid (ceil(N / 128), K split, ceil(M / nt)), cluster (1, K split, 1); nt: tokens per block, a multiple of 16; every block has a stage
@@ -103,6 +196,8 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[4 + kFtDepth];  // pieces of a stage are there (2), its products are done (2), its floats are there
     __shared__ uint32_t tmem_slot;
+    __shared__ unsigned s_top;  // of the cluster: 0, or the largest operand of ranks that have one which is not the sum of its pieces
+                                // (bits of a float)
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * kFtCols, m0 = blockIdx.z * nt, m_rows = min(nt, a.M - m0);
@@ -117,6 +212,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             mbar_init(done0 + 8 * s, 1);
         }
         for (int s = 0; s < kFtDepth; s++) mbar_init(raw0 + 8 * s, 1);
+        s_top = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -127,6 +223,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
+    if (gridDim.y > 1) cluster_arrive();
     pdl_wait();
 
     const int half = warp >> 2, nh = nt / 2;  // a warp adds the accumulator columns [half * nh, half * nh + nh) of its 32 lanes
@@ -134,6 +231,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
 #pragma unroll
     for (int i = 0; i < 3 * kFtGroup; i++) acc[i] = 0.f;
 
+    bool lossy = false;  // pieces of this thread's operands do not add up to them
     if (warp == kFtWarps) {
         // Issues the loads of the floats and the MMAs (the whole warp runs this; one elected lane issues)
         const uint64_t desc = umma_desc(smem_u32(smem_raw), 16, 1024);
@@ -193,6 +291,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             }
             return true;
         };
+        uint32_t rest = 0u;
         int slot = 0;
         uint32_t phase = 0;
         for (int s = 0; s < n_stages && ok; s++) {
@@ -205,13 +304,13 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const float4 v = *reinterpret_cast<const float4*>(raw + col * 128 + (((half * 4 + i) ^ (col & 7)) << 4));
-                    split_pair(v.x, v.y, p0[2 * i], p1[2 * i], p2[2 * i]);
-                    split_pair(v.z, v.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1]);
+                    split_pair(v.x, v.y, p0[2 * i], p1[2 * i], p2[2 * i], rest);
+                    split_pair(v.z, v.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1], rest);
                 }
             } else {  // [32 k][128 columns]
                 const float* wr = reinterpret_cast<const float*>(raw) + half * 16 * kFtCols + col;
 #pragma unroll
-                for (int i = 0; i < 8; i++) split_pair(wr[2 * i * kFtCols], wr[(2 * i + 1) * kFtCols], p0[i], p1[i], p2[i]);
+                for (int i = 0; i < 8; i++) split_pair(wr[2 * i * kFtCols], wr[(2 * i + 1) * kFtCols], p0[i], p1[i], p2[i], rest);
             }
             const uint32_t t_w = t_lane + kFtPieces + (uint32_t)((s & 1) * 48 + half * 8);
             tmem_st8(t_w, p0);
@@ -219,23 +318,24 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             tmem_st8(t_w + 32, p2);
             const unsigned char* xr = raw + kFtRawW + row0 * 128 + quad * 16;
             unsigned char* xs = smem_raw + (s & 1) * 2 * kFtTile;
-            // three token groups at a time, so that their latencies overlap; what lies behind the last token is read but not stored
+            // three token groups at a time, so that their latencies overlap; the 8 rows of a warp's group are there or not: nt is a multiple of 16
 #pragma unroll
             for (int j0 = 0; j0 < kFtTok / 32; j0 += 3) {
                 if (32 * j0 >= nt) break;
                 float4 v[3];
                 uint2 q0[3], q1[3], q2[3];
 #pragma unroll
-                for (int i = 0; i < 3; i++) v[i] = *reinterpret_cast<const float4*>(xr + (j0 + i) * 4096);
+                for (int i = 0; i < 3; i++)
+                    v[i] = (warp >> 1) * 8 + 32 * (j0 + i) < nt ? *reinterpret_cast<const float4*>(xr + (j0 + i) * 4096) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
-                    split_pair(v[i].x, v[i].y, q0[i].x, q1[i].x, q2[i].x);
-                    split_pair(v[i].z, v[i].w, q0[i].y, q1[i].y, q2[i].y);
+                    split_pair(v[i].x, v[i].y, q0[i].x, q1[i].x, q2[i].x, rest);
+                    split_pair(v[i].z, v[i].w, q0[i].y, q1[i].y, q2[i].y, rest);
                 }
 #pragma unroll
                 for (int i = 0; i < 3; i++) {
                     const int j = j0 + i;
-                    if ((warp >> 1) * 8 + 32 * j < nt) {  // the 8 rows of the warp's group: nt is a multiple of 16
+                    if ((warp >> 1) * 8 + 32 * j < nt) {
                         *reinterpret_cast<uint2*>(xs + x_at + j * 4096) = q0[i];
                         *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 4096) = q1[i];  // 16-byte chunk + 4, swizzled
                         *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 4096) = q2[i];
@@ -254,36 +354,70 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             if (s > 0) ok = add(s - 1);
         }
         if (ok) ok = add(n_stages - 1);
+        lossy = (rest & 0xffffu) != 0u;
     }
     pdl_launch_dependents();
 
+    // A result stands if it is finite and so large that what its operands lost does not count; if one of a block's does not, the
+    // block computes all of its results again.
     const int ks = gridDim.y, q = warp & 3;
+    float* again = reinterpret_cast<float*>(smem_raw + kFtPiecesBytes);
+    auto stands = [](float v, float least, bool whole) { return (fabsf(v) >= least && isfinite(v)) || (whole && v == 0.f); };
+    auto least_of = [&](float top) { return fmaxf(kFtLeast, top * ((float)a.K * kFtLost)); };
+    __syncthreads();  // every warp has seen the last products: the operands are not read any more
+    if (ks > 1) cluster_wait();  // the other ranks have s_top
+    if (__syncthreads_or(lossy)) {
+        const unsigned top = __float_as_uint(largest<NK>(a, m0, m_rows, n0, k_begin, k_end));
+        const unsigned most = __reduce_max_sync(0xffffffffu, top);
+        if (lane < ks) atomicMax(cluster.map_shared_rank(&s_top, lane), most);
+    }
+    if (ks == 1) __syncthreads();
     if (ks == 1) {
         const int n = n0 + q * 32 + lane;
+        const float top = __uint_as_float(s_top), least = least_of(top);
+        bool bad = false;
         if (warp < kFtWarps && n < a.N) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
-                if (i < nh && half * nh + i < m_rows) finish_f32<NK>(a, m0 + half * nh + i, n, acc[i]);
+                if (i < nh && half * nh + i < m_rows) bad |= !stands(acc[i], least, top == 0.f);
+        }
+        if (__syncthreads_or(bad)) {
+            plain_tile<NK>(a, again, m0, m_rows, n0);
+        } else if (warp < kFtWarps && n < a.N) {
+#pragma unroll
+            for (int i = 0; i < 3 * kFtGroup; i++)
+                if (i < nh && half * nh + i < m_rows) finish_f32(a, m0 + half * nh + i, n, acc[i]);
         }
     } else {
         float* red = reinterpret_cast<float*>(smem_raw);  // [nt][128]
-        __syncthreads();                                  // every warp has seen the last products: the operands are not read any more
         if (warp < kFtWarps) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
                 if (i < nh) red[(half * nh + i) * kFtCols + q * 32 + lane] = acc[i];
         }
         cluster.sync();
-        const int rank = blockIdx.y, total = m_rows * kFtCols;
-        for (int e = rank * kFtThreads + tid; e < total; e += ks * kFtThreads) {
+        // this rank's tokens; their sums go into its own buffer, in the place that no other rank reads
+        const float top = __uint_as_float(s_top);
+        const int rank = blockIdx.y, per = (m_rows + ks - 1) / ks, r0 = min(rank * per, m_rows), r1 = min(r0 + per, m_rows);
+        const float least = least_of(top);
+        bool bad = false;
+        for (int e = r0 * kFtCols + tid; e < r1 * kFtCols; e += kFtThreads) {
             float p[8];
 #pragma unroll
             for (int r = 0; r < 8; r++) p[r] = r < ks ? cluster.map_shared_rank(red, r)[e] : 0.f;
             float v = p[0];
 #pragma unroll
             for (int r = 1; r < 8; r++) v += p[r];
-            const int n = n0 + e % kFtCols;
-            if (n < a.N) finish_f32<NK>(a, m0 + e / kFtCols, n, v);
+            red[e] = v;
+            bad |= n0 + e % kFtCols < a.N && !stands(v, least, top == 0.f);
+        }
+        if (__syncthreads_or(bad)) {
+            plain_tile<NK>(a, again, m0 + r0, r1 - r0, n0);
+        } else {
+            for (int e = r0 * kFtCols + tid; e < r1 * kFtCols; e += kFtThreads) {
+                const int n = n0 + e % kFtCols;
+                if (n < a.N) finish_f32(a, m0 + e / kFtCols, n, red[e]);
+            }
         }
         cluster.sync();  // peers may still be reading this block's sums
     }

@@ -168,6 +168,9 @@ __device__ __forceinline__ bool elect_one()
     return one != 0;
 }
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+// The two halves of a barrier of a cluster whose ranks only have to have come by (all threads)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {

@@ -83,6 +83,44 @@ def test_more_than_64_tokens_are_no_less_exact_than_a_chain(ob, cuda, K, kind, n
     assert fast <= (1.02 * chain if kind in ("normal", "positive") else max(chain, 2.0 ** -23))
 
 
+@pytest.mark.parametrize("K", [256, 1100])
+@pytest.mark.parametrize("sx,sw", [(1e-35, 1), (1e-39, 1), (1, 1e-38), (1e30, 1e-36), (1e-20, 1e-19), (1e-30, 1e-10), (3e37, 1e-3)])
+@pytest.mark.parametrize("nk", [False, True])
+def test_operands_at_the_ends_of_the_range(ob, cuda, K, sx, sw, nk):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rnd = lambda s, *n: (torch.randn(*n, generator=g, device="cuda", dtype=torch.double) * s).float()
+    x, w = rnd(sx, 70, K), rnd(sw, K, 132)
+    fast, chain = (off(y, x, w) for y in both_ways(ob, torch, x, w, nk))
+    assert fast <= 1.02 * chain
+
+
+@pytest.mark.parametrize("M,N,K", [(200, 384, 256), (300, 132, 4096)])
+def test_few_small_operands_among_others(ob, cuda, M, N, K):
+    # too small for three bf16 values, and of no weight in any result but one; a row of zeros and one whose results are tiny
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(K, N, generator=g, device="cuda")
+    x[3, ::7], x[M - 1, 5], w[2, ::3], x[9], x[M - 2] = 1.1e-36, -3e-40, 1.3e-37, 0.0, 1e-36 * x[0]
+    fast, chain = both_ways(ob, torch, x, w, False)
+    assert off(fast, x, w) <= 1.02 * off(chain, x, w)
+    assert off(fast[M - 2:M - 1], x[M - 2:M - 1], w) <= 1.02 * off(chain[M - 2:M - 1], x[M - 2:M - 1], w) and not fast[9].any()
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 200, 512), (70, 132, 8192)])
+def test_values_that_are_not_finite_beside_a_residual_in_place(ob, cuda, M, N, K):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w, r = (torch.randn(*s, generator=g, device="cuda") for s in ((M, K), (K, N), (M, N)))
+    x[4], x[60, K - 1], w[100, 7] = float("nan"), float("inf"), float("-inf")
+    y = r.clone()
+    ob.project(ob.F32, x, w, None, y, M, N, K, resid=y, scale=0.5)
+    ref = r.double() + 0.5 * (x.double() @ w.double())
+    finite = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(y), finite) and torch.equal(torch.isnan(y), torch.isnan(ref))
+    assert float((y.double() - ref)[finite].norm() / ref[finite].norm()) < 2e-6
+
+
 @pytest.mark.parametrize("M", [1, 6, 30, 100])
 def test_projection_f32_gate_and_residual(ob, cuda, M):
     torch = cuda
