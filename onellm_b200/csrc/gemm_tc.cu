@@ -166,11 +166,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         n_tiles = tiles_m * tiles_n;
     }
 
+    bool ok = true;
+    int used = 0;  // warp 0: stages it has loaded, warp 1: stages its products read
     if (warp == 0) {
         // producer: one 64-deep slice of A and of B per stage, tile after tile
         const bool leader = elect_one();
         uint32_t s = 0, round = 0;
-        bool ok = true;
         for (int t = tile0; t < n_tiles && ok; t += tile_step) {
             int m0, n0, k0, m_end;
             tile_origin(t, m0, n0, k0, m_end);
@@ -213,6 +214,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
             }
         }
+        used = (int)(round * kStages + s);
         if (PAIR && rank == 1) pdl_launch_dependents();
     } else if (warp == 1 && rank == 0) {
         // instruction descriptor: D = f32, A and B of type T, A K-major, B MN-major unless W_NK, N = 256, M = 128 (256 of a pair)
@@ -225,7 +227,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool leader = elect_one();
         int lt = 0;
         uint32_t s = 0, phase = 0;
-        bool ok = true;
         for (int t = tile0; t < n_tiles && ok; t += tile_step, lt++) {
             const int acc = lt & 1, use = lt >> 1;
             // the accumulator must have been drained by the epilogue of the tile that used it before
@@ -250,6 +251,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     else umma_commit(empty0 + 8 * s);
                 }
                 __syncwarp();
+                used++;
                 if (++s == kStages) {
                     s = 0;
                     phase ^= 1;
@@ -266,7 +268,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int q = warp & 3;
         const size_t ldy = epi.ldy ? (size_t)epi.ldy : (size_t)N;
         int lt = 0;
-        bool ok = true;
         for (int t = tile0; t < n_tiles && ok; t += tile_step, lt++) {
             const int acc = lt & 1, use = lt >> 1;
             int m0, n0, k0, m_end;
@@ -365,7 +366,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (!__syncthreads_and(ok)) {
+        // loads of a pair report to its even block, and the products are its own
+        if (warp <= 1 && rank == 0) ring_drain(warp == 0 ? full0 : empty0, kStages, used);
+        __syncthreads();
+    }
     if constexpr (PAIR) cg::this_cluster().sync();  // neither leaves while the other may reach its barriers or tensor memory
     if (warp == 2) {
         if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2u * kTcBN) : "memory");
@@ -412,6 +417,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     static_assert(sizeof(Floats) == kLaneCols * sizeof(float), "the stores of a lane");
     extern __shared__ unsigned char smem_raw[];
     __shared__ float s_sq[kTcBM];
+    __shared__ int s_gave_up;
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSplitStages * kSplitStage);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSplitStages + 1);
@@ -430,6 +436,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             mbar_init(empty0 + 8 * s, 1);
         }
         mbar_init(acc_full, 1);
+        s_gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
@@ -440,11 +447,13 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    cluster_arrive();
 
     pdl_wait();
+    bool ok = true;
+    int loaded = 0;
     if (warp == 0) {
         const bool leader = elect_one();
-        bool ok = true;
         uint32_t s = 0, round = 0;
         for (int it = 0; it < n_slices && ok; it++) {
             if (round > 0) ok = mbar_wait_warp(empty0 + 8 * s, (round - 1) & 1);
@@ -466,6 +475,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
                 tma_load_2d(a_dst, &map_a, k, m0, bar);
             }
+            loaded += ok;
             if (++s == kSplitStages) {
                 s = 0;
                 round++;
@@ -476,7 +486,6 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // descriptors of the first stage; a stage or a step inside it adds (bytes >> 4) to the address field
         const uint64_t da = umma_desc(ring, 16, 1024), db = umma_desc(ring + kTcATile, W_NK ? 16 : kTcBChunk, 1024);
         const bool leader = elect_one();
-        bool ok = true;
         uint32_t s = 0, phase = 0;
         for (int it = 0; it < n_slices && ok; it++) {
             ok = mbar_wait_warp(full0 + 8 * s, phase);
@@ -498,7 +507,14 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         if (leader) umma_commit(acc_full);  // arrives when everything issued has run (also when the loop gave up)
         pdl_launch_dependents();
     }
-    __syncwarp();  // the cluster barriers below are warp-wide
+    __syncwarp();  // the barriers below are warp-wide
+    if (warp >= 2) ok = mbar_wait_warp(acc_full, 0);  // the products have read the ring
+    const bool fine = __syncthreads_and(ok);
+    cluster_wait();  // the other ranks have s_gave_up
+    if (!fine) {     // nothing of the cluster's tiles is stored
+        if (warp == 0) ring_drain(full0, kSplitStages, loaded);
+        if (threadIdx.x < cluster.num_blocks()) *cluster.map_shared_rank(&s_gave_up, threadIdx.x) = 1;
+    }
 
     float* red = reinterpret_cast<float*>(smem);  // [128][kLd], in place of the ring
     const int rows_per_rank = (kTcBM + ks - 1) / ks;
@@ -563,8 +579,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             if (lane == 0) s_sq[tr] = sq;
         }
     };
-    if (warp >= 2) {
-        const bool ok = mbar_wait_warp(acc_full, 0);  // the products have read the ring
+    if (warp >= 2 && fine) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int q = warp & 3;  // this warp may touch TMEM lanes 32 q .. 32 q + 31, the rows of the same numbers
         const int half = (warp - 2) >> 2;
@@ -573,7 +588,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         for (int c = 0; c < BN / 2; c += 32) {
             const int c0 = half * (BN / 2) + c;
             uint32_t v[32];
-            if (ok && n_slices > 0) {
+            if (n_slices > 0) {
                 tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             } else {
@@ -587,6 +602,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
     }
     cluster.sync();
+    const bool gave_up = s_gave_up != 0;
     // This rank's rows, one warp a row, or two where at most four ranks leave room for their loads: all loads are on their
     // way before the first is used.
     const int at_once = ks <= 4 ? 2 : 1;
@@ -594,7 +610,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int peer_step = (int)cluster.dim_blocks().x;
     for (int i = warp * at_once; i < rows_per_rank; i += kSplitThreads / 32 * at_once) {
         const int tr = rank * rows_per_rank + i;
-        if (tr >= kTcBM || m0 + tr >= M) break;
+        if (tr >= kTcBM || m0 + tr >= M || gave_up) break;
         const bool second = at_once == 2 && i + 1 < rows_per_rank && tr + 1 < kTcBM && m0 + tr + 1 < M;
         float p[8][NV];
         const float* mine = red + (size_t)tr * kSplitLd + kLaneCols * lane;
@@ -636,7 +652,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     cluster.sync();  // peers may still be reading this block's sums
     if (epi.ss_out) {
         // the row statistics of 256 columns: two tiles side by side in the cluster
-        if (n_tile % 2 == 0 && n0 < N)
+        if (n_tile % 2 == 0 && n0 < N && !gave_up)
             for (int i = threadIdx.x; i < rows_per_rank; i += kSplitThreads) {
                 const int tr = rank * rows_per_rank + i;
                 if (tr >= kTcBM || m0 + tr >= M) break;

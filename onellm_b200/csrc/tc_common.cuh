@@ -171,6 +171,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) { 
 // The two halves of a barrier of a cluster whose ranks only have to have come by (all threads)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// For a block that gave up: what it has put on its way ends before it leaves, as far as the limit of a wait allows.  `used` phases of a
+// ring of `depth` barriers have been set going; the last ones of each are waited for.
+__device__ __forceinline__ void ring_drain(uint32_t bar0, int depth, int used)
+{
+    for (int i = used > depth ? used - depth : 0; i < used; i++) (void)mbar_wait(bar0 + 8 * (i % depth), (uint32_t)(i / depth) & 1u);
+}
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 {
