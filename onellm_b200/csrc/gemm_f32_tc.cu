@@ -53,6 +53,7 @@ constexpr int kFtGroup = kFtTok / 2 / 3;        // accumulator columns read at a
 // result of K products beside the largest operand then counts from 2^26 times K * 2^-132 of it.  Below kFtLeast the products of
 // the pieces themselves leave the range of float.
 constexpr float kFtLost = 0x1p-106f, kFtLeast = 0x1p-80f;
+constexpr unsigned kGaveUp = 0xffffffffu;  // above the bits of every float that is not NaN
 constexpr uint32_t kFtPieces = 2 * kFtTok;      // tensor memory: two accumulators, then two stages of 3 pieces x 16 columns
 static_assert(kFtGroup == 32 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
 
@@ -197,7 +198,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
     __shared__ __align__(8) uint64_t bars[4 + kFtDepth];  // pieces of a stage are there (2), its products are done (2), its floats are there
     __shared__ uint32_t tmem_slot;
     __shared__ unsigned s_top;  // of the cluster: 0, or the largest operand of ranks that have one which is not the sum of its pieces
-                                // (bits of a float)
+                                // (bits of a float), or kGaveUp
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * kFtCols, m0 = blockIdx.z * nt, m_rows = min(nt, a.M - m0);
@@ -231,7 +232,8 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
 #pragma unroll
     for (int i = 0; i < 3 * kFtGroup; i++) acc[i] = 0.f;
 
-    bool lossy = false;  // pieces of this thread's operands do not add up to them
+    int loaded = 0, issued = 0;  // stages, of the warp that issues
+    bool lossy = false;          // pieces of this thread's operands do not add up to them
     if (warp == kFtWarps) {
         // Issues the loads of the floats and the MMAs (the whole warp runs this; one elected lane issues)
         const uint64_t desc = umma_desc(smem_u32(smem_raw), 16, 1024);
@@ -249,12 +251,14 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
         };
         if (ok)
             for (int s = 0; s < kFtDepth; s++) fetch(s, s);
+        if (ok) loaded = min(n_stages, kFtDepth);
         int slot = 0;
         for (int s = 0; s < n_stages && ok; s++) {
             ok = mbar_wait_warp(full0 + 8 * (s & 1), (uint32_t)(s >> 1) & 1u);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             fetch(s + kFtDepth, slot);  // every warp has split the floats of this stage
+            loaded = min(n_stages, s + 1 + kFtDepth);
             slot = slot + 1 == kFtDepth ? 0 : slot + 1;
             if (leader) {
                 const uint32_t d = tmem + (uint32_t)((s & 1) * kFtTok), wp = tmem + kFtPieces + (uint32_t)((s & 1) * 48);
@@ -268,6 +272,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
                                         i + kk > 0 ? 1u : 0u);
                 umma_commit(done0 + 8 * (s & 1));
             }
+            issued++;
             __syncwarp();
         }
     } else {
@@ -364,9 +369,15 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
     float* again = reinterpret_cast<float*>(smem_raw + kFtPiecesBytes);
     auto stands = [](float v, float least, bool whole) { return (fabsf(v) >= least && isfinite(v)) || (whole && v == 0.f); };
     auto least_of = [&](float top) { return fmaxf(kFtLeast, top * ((float)a.K * kFtLost)); };
-    __syncthreads();  // every warp has seen the last products: the operands are not read any more
-    if (ks > 1) cluster_wait();  // the other ranks have s_top
-    if (__syncthreads_or(lossy)) {
+    const bool fine = __syncthreads_and(ok);  // every warp has seen the last products: the operands are not read any more
+    if (ks > 1) cluster_wait();               // the other ranks have s_top
+    if (!fine) {
+        if (warp == kFtWarps) {
+            ring_drain(raw0, kFtDepth, loaded);
+            ring_drain(done0, 2, issued);
+        }
+        if (tid < ks) atomicMax(cluster.map_shared_rank(&s_top, tid), kGaveUp);
+    } else if (__syncthreads_or(lossy)) {
         const unsigned top = __float_as_uint(largest<NK>(a, m0, m_rows, n0, k_begin, k_end));
         const unsigned most = __reduce_max_sync(0xffffffffu, top);
         if (lane < ks) atomicMax(cluster.map_shared_rank(&s_top, lane), most);
@@ -376,21 +387,21 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
         const int n = n0 + q * 32 + lane;
         const float top = __uint_as_float(s_top), least = least_of(top);
         bool bad = false;
-        if (warp < kFtWarps && n < a.N) {
+        if (fine && warp < kFtWarps && n < a.N) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
                 if (i < nh && half * nh + i < m_rows) bad |= !stands(acc[i], least, top == 0.f);
         }
         if (__syncthreads_or(bad)) {
             plain_tile<NK>(a, again, m0, m_rows, n0);
-        } else if (warp < kFtWarps && n < a.N) {
+        } else if (fine && warp < kFtWarps && n < a.N) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
                 if (i < nh && half * nh + i < m_rows) finish_f32(a, m0 + half * nh + i, n, acc[i]);
         }
     } else {
         float* red = reinterpret_cast<float*>(smem_raw);  // [nt][128]
-        if (warp < kFtWarps) {
+        if (fine && warp < kFtWarps) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
                 if (i < nh) red[(half * nh + i) * kFtCols + q * 32 + lane] = acc[i];
@@ -398,7 +409,8 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
         cluster.sync();
         // this rank's tokens; their sums go into its own buffer, in the place that no other rank reads
         const float top = __uint_as_float(s_top);
-        const int rank = blockIdx.y, per = (m_rows + ks - 1) / ks, r0 = min(rank * per, m_rows), r1 = min(r0 + per, m_rows);
+        const int tokens = s_top == kGaveUp ? 0 : m_rows;  // a rank that gave up: nothing of the tile is stored
+        const int rank = blockIdx.y, per = (tokens + ks - 1) / ks, r0 = min(rank * per, tokens), r1 = min(r0 + per, tokens);
         const float least = least_of(top);
         bool bad = false;
         for (int e = r0 * kFtCols + tid; e < r1 * kFtCols; e += kFtThreads) {
