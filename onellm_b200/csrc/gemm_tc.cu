@@ -778,7 +778,7 @@ static SplitPlan plan_split(int M, int N, int K, bool dual, bool pairs)
         const double time = full * per * 0.45 + (rest > sms ? per * 0.45 : rest ? per * 0.32 : 0.0);
         const double operands = (double)tiles * slices * kSplitStage / 15e6;
         const double t = 7.5 + 0.15 * ks + std::max({time, operands, weights}) + 6.0 * (full + (rest > 0) - 1);
-        if (t < 0.97 * best) {
+        if (t < (plan.ks == 0 ? best - 1.0 : 0.97 * best)) {
             best = t;
             plan = {ks, per};
         }
