@@ -1,4 +1,4 @@
-// Projections of float32 callers (the reference's own type) for few tokens: the weight is streamed once.
+// Projections of float32 callers (the reference's own type) for few tokens: the weight is streamed, once for every 16 tokens.
 //
 // Replaces the cuBLAS SGEMM behind launchLinearGemm (src/kernels/qkv_linear.cu:8-65 of the reference) for decode steps:
 // y[M,N] = x[M,K] . W with M of a few rows is bound by the bytes of W, so what matters is how many of them are on their way.
@@ -244,7 +244,7 @@ static cudaError_t launch_nk(const GemmF32& a, cudaStream_t st)
 
 bool gemm_f32_skinny_takes(const GemmF32& a)
 {
-    return a.M <= kF32SkinnyTokens && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W);
+    return a.M <= kF32SkinnyTokens && a.K >= kF32SkinnyK && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W);
 }
 
 cudaError_t gemm_f32_skinny(const GemmF32& a, cudaStream_t st)

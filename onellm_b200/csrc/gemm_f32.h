@@ -19,6 +19,7 @@ struct GemmF32 {
 };
 
 constexpr int kF32SkinnyTokens = 64;
+constexpr int kF32SkinnyK = 96;  // below, a warp of gemm_f32_skinny has no or few rows for all its lanes: the tiled kernel is as fast or faster
 // Sizes, strides and alignment that gemm_f32_skinny covers: 16-byte rows.
 bool gemm_f32_skinny_takes(const GemmF32& a);
 cudaError_t gemm_f32_skinny(const GemmF32& a, cudaStream_t st);
