@@ -482,35 +482,48 @@ static StagedPlan plan_staged(int N, int K, bool tp)
         }
     }
     if (!FUSED && !tp) {
-        // Two and a bit blocks for every SM (one block's barriers and its epilogue pass under the copies of another), by the
-        // fewest K ranges that give them, since every further range is one more block that meets at the end; then rings just
-        // deep enough for about 100 KB on their way to an SM, which is what the memory latency asks for: deeper ones only
-        // keep blocks out.  Every block is resident with 5 % to spare: a launch that only just fits is placed while blocks
-        // of its neighbours are still there, a cluster of eight then finds no room in any one GPC, and it runs after the others
-        // instead of beside them.
-        // Measured in decode steps and generation of the three designs, every projection over all splits and five depths: 0.8 %
-        // behind the best plan of each on average, 3.4 % at most.  The deepest-ring rule that stood here lost most where
-        // it only just fitted: 4096 outputs of 19200 (bfloat16, 8 tokens) 58 us instead of 36.
-        bool found = false;
+        // The K split with the least estimated time.  A block takes in so many bytes a second whatever else there is, and an SM hardly
+        // more with three or four blocks than with two; so the time of a split is that of the SM with the most weight to take
+        // in, plus what every further range costs when the blocks of a cluster meet.  The blocks have to be spread evenly for that,
+        // but a launch fills SM after SM: of 256 blocks that fit three to an SM 62 SMs get none (16384 x 4096, 4 tokens: 32.0 us
+        // instead of 27.0).  So the ring is as deep as it takes to keep more blocks off an SM than all of them need, and no
+        // deeper than that and 88 KB on their way to an SM call for: a launch whose blocks only just fit into an SM finds no room while
+        // blocks of its neighbours are still there.  3 % of the places, and two of its clusters, stay free for the same reason: 32
+        // clusters of eight where 33 fit took 10 us longer than 32 of seven in a design's decode steps (19200 x 4096, 16 tokens: as if
+        // in two waves), elsewhere about as long; called alone one right behind the other they are the faster by 9 %.
+        // Rates (KB a us and SM with one to four blocks) and cost per range (us) are fitted to a sweep over all splits and seven depths
+        // of 26 shapes with 4, 12 and 24 tokens, weights from memory.  Behind the best plan of each: 3 % on average, 12 % at most (two
+        // rules by blocks and bytes on their way alone: 8 % and 51 %, 7 % and 31 %).
+        constexpr int kClass = MB >= 4 ? 2 : MB >= 2 ? 1 : 0;
+        constexpr double kRange[3][2] = {{0.03, 0.20}, {0.05, 0.32}, {0.21, 0.81}};
+        constexpr double kRate[3][2][4] = {{{29, 46, 49, 49}, {43, 60, 54, 54}}, {{26, 41, 45, 45}, {38, 54, 50, 50}}, {{19.4, 29, 31.5, 33}, {32, 43, 41, 41}}};
+        const long sms = num_sms();
+        auto bytes = [&](int nst) { return std::max(stage * nst, red); };
+        auto on_an_sm = [&](int nst) { return std::max(1L, staged_slots(kern, 1, nst, bytes(nst), col_blocks) / sms); };
+        double best = 0.0;
         for (int ks = 1; ks <= 8; ks++) {
             const int per = (total_stages + ks - 1) / ks;
             if (ks > 1 && per < 4) break;
-            const long total = (long)col_blocks * ks, sms = num_sms();
-            const long in_ring = total * NW * kStageBytes;
-            int nst = (int)std::min<long>(12, (100L * 1024 * sms + in_ring - 1) / in_ring + 1);
-            nst = std::max(3, std::min({std::max(4, nst), per + 1, 12}));
-            while (nst >= 3 && (std::max(stage * nst, red) > smem_cap ||
-                                (long)staged_slots(kern, ks, nst, std::max(stage * nst, red), col_blocks) * 95 < total * 100))
-                nst--;
+            const long total = (long)col_blocks * ks;
+            int nst = 12;
+            auto holds = [&](int n) {
+                const long places = staged_slots(kern, ks, n, bytes(n), col_blocks);
+                return places * 97 >= total * 100 && places / ks >= col_blocks + 2;
+            };
+            while (nst >= 3 && (bytes(nst) > smem_cap || !holds(nst))) nst--;
             if (nst < 3) continue;
+            const long each = on_an_sm(nst);  // blocks of the SMs that have the most
+            while (nst > 3 && on_an_sm(nst - 1) == each && each * (nst - 2) * NW * kStageBytes >= 88 * 1024) nst--;
+            const double time = kRange[kClass][NW - 1] * ks +
+                                (double)N * K * sizeof(T) * NW / 1024 * each / total / kRate[kClass][NW - 1][std::min<long>(each, 4) - 1];
+            if (best > 0.0 && time >= best) continue;
+            best = time;
             plan.ks = ks;
-            plan.nst = nst;
+            plan.nst = std::min(nst, std::max(3, per + 1));
             plan.per_block = per;
-            plan.smem = std::max(stage * nst, red);
-            found = true;
-            if (total * 10 >= sms * 22) break;
+            plan.smem = bytes(plan.nst);
         }
-        if (found) {
+        if (best > 0.0) {
             plans[key] = plan;
             return plan;
         }

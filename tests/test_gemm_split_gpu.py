@@ -94,3 +94,18 @@ def test_first_call_of_a_shape_inside_a_capture(ob, cuda):
     g.replay()
     torch.cuda.synchronize()
     assert err(y, x.double() @ w.double()) < 3e-4
+
+
+# decode projections: every K split from one to eight, the last of them with fewer rows or none, columns that end inside a block
+@pytest.mark.parametrize("M", [1, 9, 17, 32])
+@pytest.mark.parametrize("N,K", [(4096, 16384), (4096, 4096), (2080, 4096), (4096, 928), (5632, 2048), (12304, 512), (32000, 256), (136, 48), (8, 4096)])
+def test_decode_projection_plans(ob, cuda, M, N, K):
+    torch = cuda
+    x, (w, w2), _ = operands(torch, M, N, K, torch.half, n=2)
+    y, ref = torch.empty(M, N, device="cuda", dtype=torch.half), x.double() @ w.double()
+    ob.gemm(ob.F16, x, w, y, M, N, K)
+    assert err(y, ref) < 3e-4
+    ob.gemm_swiglu(ob.F16, x, w, w2, y.zero_(), M, N, K)
+    assert err(y, torch.nn.functional.silu(ref) * (x.double() @ w2.double())) < 4e-4
+    k_split, ring, blocks = ob.gemm_plan_query(M, N, K)
+    assert 1 <= k_split <= 8 and ring >= 3 and blocks == k_split * -(-N // 128)
