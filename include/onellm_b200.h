@@ -197,7 +197,11 @@ ONELLM_API int onellm_gemm_fused(int dtype, const void* x, const void* W, const 
  * Replaces launchLinearGemm + cublasWrapper::Gemm
  * (src/kernels/qkv_linear.h:9-14, qkv_linear.cu:8-65, cublas_wrapper.cc:45-90).
  * w_layout selects [K,N] (layer weights) or [N,K] (LM head).  F16: tensor cores; M <= 64
- * takes the weight-streaming path, larger M the tiled path.  F32: plain fp32 arithmetic.
+ * takes the weight-streaming path, larger M the tiled path.  The weight-streaming kernels of this and
+ * the other F16 and BF16 projections request weights before they wait for the kernel enqueued just in
+ * front: weights must have been written by work that was complete before that kernel began.
+ * F32: the precision of plain fp32 arithmetic (more than 64 tokens and K >= 256: on tensor cores, every
+ * value as the sum of three bfloat16 ones; operands or results these cannot hold: plain arithmetic).
  * F16 constraints: [K,N] weights need K % 16 == 0 and N % 8 == 0; [N,K] weights K % 32 == 0.
  * ------------------------------------------------------------------------------------- */
 ONELLM_API int onellm_gemm(int dtype, const void* x, const void* W, void* y, int M, int N, int K,

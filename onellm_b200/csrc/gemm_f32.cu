@@ -14,6 +14,8 @@
 // Sums of products are in float throughout, in more and shorter chains than the tiled kernel's (error against 64 bits of a layer
 // and the head: 5.9e-7 instead of 2.7e-6).
 // Measured, 2 tokens, one 7B-shaped layer and its head (1.33 GB of weights, floor 0.20 ms): 6.65 ms in the tiled kernel, 0.33 here.
+// 4096 x 12288 (201 MB), us, [K,N] | [N,K] | tiled: 2 tokens 48 | 44 | 893, 16 tokens 247 | 109 | 937, 32 tokens 470 | 197 | 1014,
+// 64 tokens 935 | 361 | 1140.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -19,10 +19,11 @@
 //          convert stage s + 1 while the MMAs of stage s run.
 // K is split over the blocks of a cluster where the tiles alone would not fill the GPU; the partial sums meet in distributed
 // shared memory in rank order.
-// What bounds it: the MMAs of a stage of 176 tokens take about 1000 cycles, splitting its floats 1200, adding an accumulator 400 and
-// the waits between them 450, the last three one after the other in every warp.  Measured, 352 tokens of the 7B shapes, us (the 64 x
-// 64 tiled kernel before): QKV 262 (3000), o_proj 93 (890), gate or up 240 (2600), down 215 (2400), 127 to 147 TFLOP/s of float32;
-// error against 64 bits 1.8e-7 (2.6e-7 at K = 11008), a layer 7e-7 instead of 2.8e-6.
+// What bounds it, in cycles of a stage of 176 tokens with six products and pieces cut off instead of rounded: the MMAs 1000 (eight: a
+// third more), splitting its floats 1200, adding an accumulator 400 and the waits between them 450, the last three one after the
+// other in every warp.  The two products more cost 1 %, noticing what the pieces do not hold 1 to 2 %.  Measured, 352 tokens of the 7B
+// shapes, us (the 64 x 64 tiled kernel): QKV 276 (2209), o_proj 91 (911), gate or up 250 (2202), down 219 (2569), 127 to 145 TFLOP/s
+// of float32; error against 64 bits, normal operands, 1.1e-7 (chain 1.1e-6; K = 11008: 1.5e-7, 1.8e-6), a layer 6.9e-7 instead of 2.8e-6.
 // What the pieces do not hold: a value that is not finite, or whose first piece rounds to infinity, makes its remainders NaN and so
 // every result it enters; one below 2^-110 loses its last bits.  Blocks whose results that touches (see `stands`) compute them
 // again by plain multiply-adds, at the rate of the tiled kernel; the results are that kernel's to the bit.
@@ -532,8 +533,8 @@ constexpr int kFtLeastK = 256;
 // Sizes, strides and alignment it covers: 16-byte rows.
 bool gemm_f32_tc_takes(const GemmF32& a)
 {
-    return a.M > kF32SkinnyTokens && a.K >= kFtLeastK && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) && aligned16(a.x) && aligned16(a.W) &&
-           ((long)a.M + 15) / 16 <= 65535;
+    return a.M > kF32SkinnyTokens && a.K >= kFtLeastK && a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && (a.w_nk || a.N % 4 == 0) &&
+           aligned16(a.x) && aligned16(a.W) && ((long)a.M + 15) / 16 <= 65535;
 }
 
 cudaError_t gemm_f32_tc(const GemmF32& a, cudaStream_t st) { return a.w_nk ? launch_ft<true>(a, st) : launch_ft<false>(a, st); }

@@ -390,7 +390,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // about 60 bytes per cycle of operands.
 // Same operands, descriptors, epilogue options and row statistics as gemm_tc_kernel; the K ranges are added in float.
 // Measured beside the persistent kernel, 7B shape, 70 | 238 tokens: o_proj 28.9 -> 12.5 | 29.3 -> 15.6 us, down 65.2 -> 23.8 |
-// 66.2 -> 28.9, QKV 31.8 -> 24.5 | 33.1 (stays), 32 outputs (a router) 21.8 -> 6.1 | 21.5 -> 7.2.
+// 66.2 -> 28.9, QKV 31.8 -> 24.5 | 33.1 (stays; 29.8 in pairs), 32 outputs (a router) 21.8 -> 6.1 | 21.5 -> 7.2.
 constexpr int kSplitBN = 128;
 constexpr int kSplitStage = kTcATile + kSplitBN * kTcBK * 2;
 constexpr int kSplitStages = 3;
