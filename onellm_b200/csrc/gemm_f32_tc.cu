@@ -21,9 +21,10 @@
 // shared memory in rank order.
 // What bounds it, in cycles of a stage of 176 tokens with six products and pieces cut off instead of rounded: the MMAs 1000 (eight: a
 // third more), splitting its floats 1200, adding an accumulator 400 and the waits between them 450, the last three one after the
-// other in every warp.  The two products more cost 1 %, noticing what the pieces do not hold 1 to 2 %.  Measured, 352 tokens of the 7B
-// shapes, us (the 64 x 64 tiled kernel): QKV 276 (2209), o_proj 91 (911), gate or up 250 (2202), down 219 (2569), 127 to 145 TFLOP/s
-// of float32; error against 64 bits, normal operands, 1.1e-7 (chain 1.1e-6; K = 11008: 1.5e-7, 1.8e-6), a layer 6.9e-7 instead of 2.8e-6.
+// other in every warp.  The two products more and the notice of what the pieces do not hold cost 2 to 9 % of a call, 3 to 8 % of a
+// layer.  Measured, 352 tokens of the 7B shapes, us (the 64 x 64 tiled kernel): QKV 276 (2209), o_proj 91 (911), gate or up 250 (2202),
+// down 219 (2569), 127 to 145 TFLOP/s of float32; error against 64 bits, normal operands, 1.1e-7 (chain 1.1e-6; K = 11008: 1.5e-7,
+// 1.8e-6), a layer 6.9e-7 instead of 2.8e-6.
 // What the pieces do not hold: a value that is not finite, or whose first piece rounds to infinity, makes its remainders NaN and so
 // every result it enters; one below 2^-110 loses its last bits.  Blocks whose results that touches (see `stands`) compute them
 // again by plain multiply-adds, at the rate of the tiled kernel; the results are that kernel's to the bit.
