@@ -26,8 +26,8 @@ NVCC_FLAGS = [
 ENGINE_SOURCES = ["elementwise.cu", "engine.cu", "errors.cpp", "gemm_f32.cu", "gemm_f32_tc.cu", "gemm_tc.cu", "model_files.cpp", "norm.cu", "sampling.cu",
                   "skinny_gemm.cu", "skinny_gemm_staged.cu", "skinny_gemm_tc.cu", "weight_placer.cu"]
 DESIGN_SOURCES = {
-    "Finuvik": ["biased_attn.cu", "biased_attn_tc.cu", "finuvik.cu", "gated_recurrence.cu"],
-    "Fuposun": ["biased_attn_tc.cu", "fuposun.cu", "gated_recurrence.cu", "latent_attn.cu", "latent_attn_tc.cu", "route.cu"],
+    "Finuvik": ["biased_attn.cu", "biased_attn_tc.cu", "finuvik.cu", "gated_recurrence.cu", "gated_recurrence_tc.cu"],
+    "Fuposun": ["biased_attn_tc.cu", "fuposun.cu", "gated_recurrence.cu", "gated_recurrence_tc.cu", "latent_attn.cu", "latent_attn_tc.cu", "route.cu"],
 }
 
 

@@ -8,7 +8,7 @@
 //     which keeps the digits of a gate near one as well; the gate's logit comes through a low-rank projection, whose
 //     second matrix is applied in float here.
 //
-// Context pass, three launches:
+// Context pass, three launches (long prompts of bfloat16 callers: gated_recurrence_tc.cu):
 //   1. the prepare kernel turns the projections into the vectors of the recurrence (g and silu(q); or g, k and q), in
 //      float and head by head, so that the tokens of a head lie behind each other.
 //   2. gated_recurrence_scan_kernel.  A thread block owns 32 value columns of one (sequence, head) and keeps that part of
@@ -28,8 +28,7 @@
 
 #include <algorithm>
 
-#include "mixers.h"
-#include "tc_common.cuh"
+#include "gated_recurrence.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -64,66 +63,11 @@ __device__ __forceinline__ f32x2 sub_f2(f32x2 a, f32x2 b)
     return r;
 }
 
-// sigmoid(x) and 1 - sigmoid(x), both with full relative precision; the fast exponential and division where the
-// projections are bfloat16 (their error is far below the rounding of x)
-template <typename T>
-__device__ __forceinline__ void sigmoid_pair(float x, float& s, float& c)
-{
-    float e, r;
-    if constexpr (sizeof(T) == 2) {
-        e = __expf(-fabsf(x));
-        r = __fdividef(1.f, 1.f + e);
-    } else {
-        e = expf(-fabsf(x));
-        r = 1.f / (1.f + e);
-    }
-    s = x >= 0.f ? r : e * r;
-    c = x >= 0.f ? e * r : r;
-}
-template <typename T>
-__device__ __forceinline__ float silu_of(float x)
-{
-    float s, c;
-    sigmoid_pair<T>(x, s, c);
-    return x * s;
-}
-// 1 - f and silu(q) of one channel
-template <typename T>
-__device__ __forceinline__ void gate(float q, float z, float zb, float lower, float& g, float& qs)
-{
-    float s, c;
-    sigmoid_pair<T>(z + zb, s, c);
-    g = (1.f - lower) * c;
-    sigmoid_pair<T>(q, s, c);
-    qs = q * s;
-}
-
-// sigmoid(z) ^ inv_tau - 1 from the logarithm of the sigmoid
-__device__ __forceinline__ float decay(float z, float inv_tau) { return expm1f(inv_tau * (fminf(z, 0.f) - log1pf(expf(-fabsf(z))))); }
-
-struct GrParams {
-    GatedRecurrence g;
-    TokenPositions tp;
-    int settled;  // see gated_recurrence (mixers.h)
-};
-
 // Layout of the work space of T tokens: the vectors of a head [H][T][n * dkp] (TIED n = 2: g, silu(q); KEYED n = 3: g, q, k),
 // v [H][dv / 32][T][32], outputs before the norm [T][H][dv]; all float, dkp = dk padded to the rows of a block.
 static int gr_dkp(int dk) { return dk <= 64 ? 64 : dk <= 128 ? 128 : dk <= 256 ? 256 : 512; }
 static int gr_vectors(int kind) { return kind == ONELLM_GR_KEYED ? 3 : 2; }
 
-template <typename T>
-__device__ __forceinline__ void gr_load4(const T* src, float (&f)[4])
-{
-    if constexpr (sizeof(T) == 4) {
-        const float4 x = *reinterpret_cast<const float4*>(src);
-        f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w;
-    } else {
-        const uint2 x = *reinterpret_cast<const uint2*>(src);
-        const float2 a = unpack2<T>(x.x), b = unpack2<T>(x.y);
-        f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-    }
-}
 // the values of one token, 32-column tile by tile
 template <typename T>
 __device__ __forceinline__ void gr_values(const GatedRecurrence& p, int t, int tokens, float* __restrict__ vf)
@@ -257,12 +201,6 @@ __global__ void __launch_bounds__(256) gated_recurrence_prepare_kernel(const GrP
         *reinterpret_cast<float4*>(dst + dkp) = make_float4(qs[0], qs[1], qs[2], qs[3]);
     }
     gr_values<T>(p, t, tokens, vf);
-}
-
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
 }
 
 template <int NV, int R, int TOK>
@@ -636,6 +574,7 @@ static int dispatch_gr(const GrParams& p, int B, int tokens, cudaStream_t st)
                      : launch_cluster(gated_recurrence_step_kernel<T, false>, grid, kGsThreads, 0, st, p, cols);
     }
     if (tokens <= 0) return ONELLM_OK;
+    if (gr_chunked_takes(p.g, p.tp, B, tokens)) return gr_chunked(p, B, tokens, st);
     const int dkp = gr_dkp(p.g.dk), nv = gr_vectors(p.g.kind);
     float* gq = static_cast<float*>(p.g.work);
     float* vf = gq + (size_t)tokens * p.g.H * nv * dkp;
@@ -656,7 +595,7 @@ static int dispatch_gr(const GrParams& p, int B, int tokens, cudaStream_t st)
 
 size_t gated_recurrence_workspace(int kind, int tokens, int H, int dk, int dv)
 {
-    return (size_t)tokens * H * (gr_vectors(kind) * gr_dkp(dk) + 2 * dv) * sizeof(float);
+    return std::max((size_t)tokens * H * (gr_vectors(kind) * gr_dkp(dk) + 2 * dv) * sizeof(float), gr_chunked_workspace(tokens, H, dk, dv));
 }
 
 int gated_recurrence(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens, cudaStream_t st, bool settled)

@@ -59,32 +59,6 @@ constexpr unsigned kGaveUp = 0xffffffffu;  // above the bits of every float that
 constexpr uint32_t kFtPieces = 2 * kFtTok;      // tensor memory: two accumulators, then two stages of 3 pieces x 16 columns
 static_assert(kFtGroup == 32 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
 
-__device__ __forceinline__ void umma_f16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-// the three bf16 pieces of two floats, packed piece by piece (lo in the low half); rest: the ends of the third ones that bf16 has no
-// place for, in its low half
-__device__ __forceinline__ void split_pair(float lo, float hi, uint32_t& p0, uint32_t& p1, uint32_t& p2, uint32_t& rest)
-{
-    constexpr uint32_t kTop = 0xffff0000u;
-    p0 = pack2<__nv_bfloat16>(lo, hi);
-    const float lr = lo - __uint_as_float(p0 << 16), hr = hi - __uint_as_float(p0 & kTop);
-    p1 = pack2<__nv_bfloat16>(lr, hr);
-    const float lq = lr - __uint_as_float(p1 << 16), hq = hr - __uint_as_float(p1 & kTop);
-    p2 = __byte_perm(__float_as_uint(lq), __float_as_uint(hq), 0x7632);
-    rest |= __float_as_uint(lq) | __float_as_uint(hq);
-}
-
 __device__ __forceinline__ void finish_f32(const GemmF32& a, int m, int n, float v)
 {
     const size_t at = (size_t)m * a.ldy + n;

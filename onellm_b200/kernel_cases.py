@@ -156,7 +156,7 @@ def make_mechanism_case(name, torch, m, B, ctx, plain=False) -> Case:
         fn = lambda i: ob.gated_recurrence(g[i], tp, T)
         keep = (mix, cat, cu, hist, off, step, state, zb, lower, w, work)
         if prefill:  # decay and write (a product and a multiply-add), read (a multiply-add) per state element and token
-            return Case(fn, rot, 5.0 * T * RH * RK * RV, "flop", "gated_recurrence_scan_kernel", launches=3, keep=keep)
+            return Case(fn, rot, 5.0 * T * RH * RK * RV, "flop", "gr_chunk_output_kernel", launches=3, keep=keep)
         return Case(fn, rot, 2 * B * RH * RK * RV * 4 + B * RH * (2 * RK + 2 * RV) * 2, "B", "gated_recurrence_step_kernel", keep=keep)
     raise ValueError(f"unknown case {name}")
 
@@ -277,7 +277,7 @@ def make_latent_case(name, torch, m, B, ctx, plain=False) -> Case:
         fn = lambda i: ob.gated_recurrence(g[i], tp, T)
         keep = (state, row, out, A, zb, w, work, cu, hist, off, step)
         if prefill:  # decay, write and read of a state element and token, as counted for fv_rec
-            return Case(fn, rot, 5.0 * T * RH * RK * RV, "flop", "gated_recurrence_scan_kernel", launches=3, keep=keep)
+            return Case(fn, rot, 5.0 * T * RH * RK * RV, "flop", "gr_chunk_output_kernel", launches=3, keep=keep)
         return Case(fn, rot, 2 * B * RH * RK * RV * 4 + B * RH * (2 * RK + 3 * RV) * 2, "B", "gated_recurrence_step_kernel", keep=keep)
     raise ValueError(f"unknown case {name}")
 

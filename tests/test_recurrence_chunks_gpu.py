@@ -1,0 +1,94 @@
+"""Context passes of the gated recurrences in chunks of 128 tokens on the tensor cores, against the token by token sums in 64 bits."""
+import numpy as np
+import pytest
+
+from oracle import finuvik_ref as fr
+from tests.conftest import rel_err
+from tests.device import Dev, host, rounded
+from tests.test_finuvik_kernels_gpu import ref_recurrence, run_recurrence
+from tests.test_fuposun_kernels_gpu import ref_gla, run_gla
+
+pytestmark = pytest.mark.gpu
+TOL = 1.2e-2
+# The state is float and its sums are taken as closely as float adds them; the outputs are rounded to bfloat16.
+STATE = 2e-6
+
+
+def positions(ob, d, counts, hist):
+    return ob.TokenPositions(d.i32(np.concatenate([[0], np.cumsum(counts)])).data_ptr(), d.i32(hist).data_ptr(), len(counts), None, None)
+
+
+# sequences that end at, in front of and behind the edges of a chunk; the second portion starts from the state of the first
+COUNTS = [([384, 640, 129], [1, 500, 512]), ([300], [1031]), ([255, 257, 640, 128], [511, 1, 513, 127])]
+
+
+@pytest.mark.parametrize("H,dk,dv", [(2, 64, 128), (3, 128, 128), (1, 192, 256), (2, 256, 384)])
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("gates", ["learned", "slow", "fast"])
+def test_tied(cuda, ob, H, dk, dv, counts, gates):
+    # slow: nearly every gate is the same one close to 1; fast: chunks forget channels far below 2^-80, others hardly anything
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(dk + dv)
+    zb = fr.round_bf16({"learned": rng.uniform(-1, 6, H * dk), "slow": np.full(H * dk, 9.0), "fast": rng.uniform(-12, 8, H * dk)}[gates])
+    lower = fr.round_bf16(rng.uniform(0, 0.95, H * dk) * (rng.uniform(size=H * dk) > 0.3)) if gates == "learned" else np.zeros(H * dk)
+    w = fr.round_bf16(1 + 0.3 * rng.standard_normal(dv))
+    B = len(counts[0])
+    state = d.zeros(B, H, dk, dv, f32=True) + float("nan")  # what a freed sequence left behind: a new one must not see it
+    ref_state, hist = [np.zeros((H, dk, dv)) for _ in range(B)], [0] * B
+    for portion in counts:
+        z_std = 0.0 if gates == "slow" else 1.0
+        q, z, v = (rounded(rng.standard_normal((sum(portion), H, m)) * s, "bf16") for m, s in ((dk, 1.0), (dk, z_std), (dv, 1.0)))
+        got = run_recurrence(ob, d, H, dk, dv, q, z, v, zb, lower, w, state, positions(ob, d, portion, hist), B, scale_out=0.6)
+        assert ob.lib().onellm_gemm_timeout_flag() == 0
+        at = 0
+        for b, n in enumerate(portion):
+            s = slice(at, at + n)
+            assert rel_err(got[s], 0.6 * ref_recurrence(q[s], z[s], v[s], zb, lower, w, ref_state[b])) < TOL, (portion, b)
+            at += n
+            hist[b] += n
+    for b in range(B):
+        assert rel_err(host(state[b]), ref_state[b]) < STATE
+
+
+@pytest.mark.parametrize("H,dk,dv,rank", [(2, 64, 128, 5), (1, 128, 128, 16), (2, 256, 512, 16), (1, 192, 1024, 64)])
+@pytest.mark.parametrize("tau,gated", [(16.0, True), (0.3, False)])
+def test_keyed(cuda, ob, H, dk, dv, rank, tau, gated):
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(dk + dv)
+    A, zb = (fr.round_bf16(x) for x in (rng.standard_normal((H * dk, rank)) / np.sqrt(rank), rng.uniform(-1, 6, H * dk)))
+    w, qs = fr.round_bf16(1 + 0.3 * rng.standard_normal(dv)), dk ** -0.5
+    for counts in COUNTS[:2]:
+        B = len(counts[0])
+        state = d.zeros(B, H, dk, dv, f32=True) + float("nan")
+        ref_state, hist = [np.zeros((H, dk, dv)) for _ in range(B)], [0] * B
+        for portion in counts:
+            T = sum(portion)
+            x = tuple(rounded(rng.standard_normal(s), "bf16") for s in ((T, H, dk), (T, H, dk), (T, H, dv), (T, rank), (T, H, dv)))
+            got = run_gla(ob, d, H, dk, dv, x, A, zb, w, state, positions(ob, d, portion, hist), tau, qs, scale_out=0.6, gated=gated)
+            at = 0
+            for b, n in enumerate(portion):
+                ref = 0.6 * ref_gla([y[at:at + n] for y in x], A, zb, w, ref_state[b], tau, qs, gated=gated)
+                assert rel_err(got[at:at + n], ref) < TOL, (portion, b)
+                at += n
+                hist[b] += n
+        for b in range(B):
+            assert rel_err(host(state[b]), ref_state[b]) < STATE
+
+
+@pytest.mark.parametrize("what", ["value", "query", "gate", "key"])
+def test_what_is_not_finite_reaches_its_own_and_later_tokens_only(cuda, ob, what):
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(1)
+    H, dk, dv, n, rank, t = 1, 64, 128, 300, 4, 200
+    x = [rounded(rng.standard_normal(s), "bf16") for s in ((n, H, dk), (n, H, dk), (n, H, dv), (n, rank), (n, H, dv))]
+    A, zb, w = rng.standard_normal((dk, rank)).astype(np.float32), np.ones(dk), np.ones(dv)
+    run = lambda state: run_gla(ob, d, H, dk, dv, x, A, zb, w, state, positions(ob, d, [n], [0]), 16.0, 1.0, gated=False)
+    states = [d.zeros(1, H, dk, dv, f32=True) for _ in range(2)]
+    clean = run(states[0])
+    x[{"value": 2, "query": 0, "gate": 3, "key": 1}[what]][(t,) + (0,) * (1 if what == "gate" else 2)] = np.inf if what == "value" else np.nan
+    got = run(states[1])
+    assert rel_err(got[:t], clean[:t]) < TOL and np.all(np.isnan(got[t]).any(-1))
+    if what == "query":
+        assert rel_err(got[t + 1:], clean[t + 1:]) < TOL and rel_err(host(states[1]), host(states[0])) < STATE
+    else:
+        assert np.isnan(got[t + 1:]).any(-1).all() and not np.isfinite(host(states[1])).all()
