@@ -294,16 +294,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     uint32_t u[32];
                     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTcBN + kOutN + c0), u);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    // rows that are stored only: the zeros behind the last row send every division of the gate down its slow
-                    // path (16 us of a 5632 x 2 projection of 238 tokens)
-                    if (row_ok) {
-#pragma unroll
-                        for (int i = 0; i < 32; i++) {
-                            const float g = __uint_as_float(r[i]) * inv;
-                            r[i] = __float_as_uint(gate_pair(g, __uint_as_float(u[i]) * inv, epi.act, epi.limit));
-                        }
-                    }
-                    __syncwarp();
+                    gate_row(reinterpret_cast<float(&)[32]>(r), reinterpret_cast<const float(&)[32]>(u), inv, epi.act, epi.limit);
                 } else {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (scaled) {
