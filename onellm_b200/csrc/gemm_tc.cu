@@ -43,7 +43,8 @@ constexpr int kTcATile = kTcBM * kTcBK * 2;        // 16 KB: 128 rows x 128 byte
 constexpr int kTcBTile = kTcBN * kTcBK * 2;        // 32 KB: [K,N] four boxes of 64 k-rows x 128 bytes; [N,K] 256 rows x 128 bytes
 constexpr int kTcBChunk = 64 * kTcBK * 2;          // 8 KB: one 64-column chunk of a [K,N] stage
 constexpr int kTcStageBytes = kTcATile + kTcBTile;
-constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024 /* alignment slack */ + 256 /* barriers, TMEM address */;
+constexpr int kTcTurnBytes = 32 * 32 * 4;  // a warp's 32 x 32 values on their way to memory
+constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + 1024 /* alignment slack */ + 256 /* barriers, TMEM address */ + kTcEpiThreads / 32 * kTcTurnBytes;
 
 // W_NK = false: W [K,N] (B operand MN-major);  W_NK = true: W [N,K] (B operand K-major).
 // Persistent: grid = min(tiles, SMs) blocks of six warps; block c works on tiles c, c + grid, ... in band
@@ -267,18 +268,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31, which are the tile rows of the same numbers
         const int q = warp & 3;
         const size_t ldy = epi.ldy ? (size_t)epi.ldy : (size_t)N;
+        float4* turn = reinterpret_cast<float4*>(smem + kStages * kStageBytes + 256 + (warp - 2) * kTcTurnBytes);
+        auto turned = [&](int r, int chunk) { return turn + r * 8 + (chunk ^ (r & 7)); };  // 16 bytes of row r, free of bank conflicts both ways
         int lt = 0;
         for (int t = tile0; t < n_tiles && ok; t += tile_step, lt++) {
             const int acc = lt & 1, use = lt >> 1;
             int m0, n0, k0, m_end;
             tile_origin(t, m0, n0, k0, m_end);
+            // In memory a lane has 16 bytes of a row: of every fourth row (f32), of every eighth (16-bit elements)
+            const int r_step = epi.f32 ? 4 : 8, r_lane = epi.f32 ? lane >> 3 : lane >> 2, c_lane = epi.f32 ? (lane & 7) * 4 : (lane & 3) * 8;
+            const int m_lane = m0 + q * 32 + r_lane, n_lane = n0 + c_lane, turns = 32 / r_step, size = epi.f32 ? 4 : (int)sizeof(T);
+            auto inside = [&](int c0, int i) { return m_lane + i * r_step < m_end && n_lane + c0 < N; };  // N is a multiple of 8
+            auto element = [&](int c0, int i) { return ((size_t)(m_lane + i * r_step) * ldy + n_lane + c0) * size; };
+            uint4 rs[8];  // the residual of the next 32 columns, asked for one turn ahead
+            auto fetch = [&](int c0) {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (i < turns && c0 < kOutN && inside(c0, i)) rs[i] = *reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(epi.resid) + element(c0, i));
+            };
+            if (epi.resid) fetch(0);
             ok = mbar_wait(acc_full0 + 8 * acc, use & 1);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + q * 32 + lane;
             const bool row_ok = row < m_end;
-            float inv = 1.f, sq = 0.f;
+            float inv = 1.f, sq[4] = {0.f, 0.f, 0.f, 0.f};
             const bool scaled = GROUPED ? grp.row_scale != nullptr : epi.row_ss != nullptr;
             if (GROUPED && scaled && row_ok) inv = grp.row_scale[row];
             if (epi.row_ss && row_ok) {
@@ -302,50 +317,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         for (int i = 0; i < 32; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * inv);
                     }
                 }
-                if (row_ok) {
-                    const size_t at = (size_t)row * ldy + n0 + c0;
+                // A lane has a row of the accumulator; written from there, every store of a warp would touch 32 lines (2000 tokens, K 9728, 2048
+                // float outputs on top of a residual: 20 us behind the last product).  Turned around in shared memory, a warp's
+                // accesses cover whole 64- or 128-byte parts of rows.
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (n0 + c0 + 8 * j < N) {  // N is a multiple of 8
-                            float v[8];
+                for (int i = 0; i < 8; i++) *turned(lane, i) = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+                __syncwarp();
+                if (epi.f32) {
+                    float a[4] = {0.f, 0.f, 0.f, 0.f};
+                    if (epi.bias && n_lane + c0 < N) {
 #pragma unroll
-                            for (int e = 0; e < 8; e++) v[e] = __uint_as_float(r[8 * j + e]);
-                            float a[8];
-                            if (epi.bias) {
-                                Vec16<T>::load(static_cast<const T*>(epi.bias) + n0 + c0 + 8 * j, a);
+                        for (int e = 0; e < 4; e++) a[e] = to_float(static_cast<const T*>(epi.bias)[n_lane + c0 + e]);
+                    }
+                    const float sc = epi.scale;
 #pragma unroll
-                                for (int e = 0; e < 8; e++) v[e] += a[e];
-                            }
-                            if (epi.f32) {
-                                float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + at + 8 * j);
-                                if (epi.resid) {
-                                    const float4* rs = reinterpret_cast<const float4*>(static_cast<const float*>(epi.resid) + at + 8 * j);
-                                    const float4 r0 = rs[0], r1 = rs[1];
-                                    const float sc = epi.scale;
-                                    v[0] = fmaf(v[0], sc, r0.x); v[1] = fmaf(v[1], sc, r0.y); v[2] = fmaf(v[2], sc, r0.z); v[3] = fmaf(v[3], sc, r0.w);
-                                    v[4] = fmaf(v[4], sc, r1.x); v[5] = fmaf(v[5], sc, r1.y); v[6] = fmaf(v[6], sc, r1.z); v[7] = fmaf(v[7], sc, r1.w);
-                                }
-                                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-                                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-                                continue;
-                            }
-                            if (epi.resid) {
-                                Vec16<T>::load(static_cast<const T*>(epi.resid) + at + 8 * j, a);
+                    for (int i = 0; i < 8; i++) {
+                        float4 v = *turned(r_lane + 4 * i, c_lane / 4);
+                        if (epi.bias) v.x += a[0], v.y += a[1], v.z += a[2], v.w += a[3];
+                        if (epi.resid) {
+                            v.x = fmaf(v.x, sc, __uint_as_float(rs[i].x)), v.y = fmaf(v.y, sc, __uint_as_float(rs[i].y));
+                            v.z = fmaf(v.z, sc, __uint_as_float(rs[i].z)), v.w = fmaf(v.w, sc, __uint_as_float(rs[i].w));
+                        }
+                        if (inside(c0, i)) *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(y) + element(c0, i)) = v;
+                    }
+                    if (epi.resid) fetch(c0 + 32);
+                } else {
+                    float a[8];
+                    if (epi.bias && n_lane + c0 < N) Vec16<T>::load(static_cast<const T*>(epi.bias) + n_lane + c0, a);
 #pragma unroll
-                                for (int e = 0; e < 8; e++) v[e] += a[e];
-                            }
-                            const uint4 packed = Vec16<T>::pack(v);
-                            *reinterpret_cast<uint4*>(y + at + 8 * j) = packed;
+                    for (int i = 0; i < 4; i++) {
+                        float v[8];
+                        *reinterpret_cast<float4*>(v) = *turned(r_lane + 8 * i, c_lane / 4);
+                        *reinterpret_cast<float4*>(v + 4) = *turned(r_lane + 8 * i, c_lane / 4 + 1);
+                        if (epi.bias) {
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[e] += a[e];
+                        }
+                        if (epi.resid) {
+                            float x[8];
+                            Vec16<T>::unpack(rs[i], x);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) v[e] += x[e];
+                        }
+                        const uint4 packed = Vec16<T>::pack(v);
+                        if (inside(c0, i)) {
+                            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(y) + element(c0, i)) = packed;
                             if (epi.ss_out) {
                                 Vec16<T>::unpack(packed, v);  // what the next projection will read
 #pragma unroll
-                                for (int e = 0; e < 8; e++) sq = fmaf(v[e], v[e], sq);
+                                for (int e = 0; e < 8; e++) sq[i] = fmaf(v[e], v[e], sq[i]);
                             }
                         }
                     }
+                    if (epi.resid) fetch(c0 + 32);
+                }
+                __syncwarp();
+            }
+            if (epi.ss_out) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 1);
+                    sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], 2);
+                    if ((lane & 3) == 0 && m_lane + 8 * i < m_end) epi.ss_out[(size_t)(m_lane + 8 * i) * tiles_n + n0 / kOutN] = sq[i];
                 }
             }
-            if (epi.ss_out && row_ok) epi.ss_out[(size_t)row * tiles_n + n0 / kOutN] = sq;
             // this thread's reads of the accumulator are over: hand it back to the MMA warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if constexpr (PAIR) {
@@ -730,17 +765,19 @@ struct SplitPlan {
     int ks, per;
 };
 
-// Estimated time in us of the persistent kernel, blocks alone or in pairs: a slice of 64 k takes 0.33 us (pairs 0.35), 0.40 (0.37) when
-// blocks take several tiles, the weights come in at 6.2 TB/s.  Pairs have half as many tiles of twice the rows, so that a token
+// Estimated time in us of the persistent kernel, blocks alone or in pairs, from a sweep over 200 to 3817 tokens and 13 weights: 8 us around
+// the slices of 64 k; where no block has a second tile a slice takes 0.335 us, 0.38 when all SMs ask for operands (pairs 0.285 and 0.34),
+// else 0.40 (0.37); the weights come in at 6.2 TB/s.  Pairs have half as many tiles of twice the rows, so that a token
 // count just above a multiple of 256 or a last wave of few tiles can cost them more than they gain.
 // Measured alone | in pairs: 3817 tokens, QKV of the 7B shape 282 | 249 us, gate/up 484 | 445, down 312 | 268; 238 tokens, QKV 33.4 |
-// 29.8, gate/up 65 | 56; 1030 tokens, o_proj 31 | 47 (144 tiles, 80 pairs).
+// 29.8, gate/up 65 | 56; 2000 tokens, 9728 x 2048 65.2 | 58.6; 1030 tokens, o_proj 31 | 47 (144 tiles, 80 pairs).
 static double persistent_us(int M, int N, int K, bool dual, bool pairs)
 {
     const long columns = dual ? 2L * N : N, slices = (K + kTcBK - 1) / kTcBK;
     const long rows = pairs ? 2 * kTcBM : kTcBM, at_once = pairs ? num_sms() / 2 : num_sms();
-    const long waves = ((M + rows - 1) / rows * ((columns + kTcBN - 1) / kTcBN) + at_once - 1) / at_once;
-    const double slice = pairs ? (waves == 1 ? 0.35 : 0.37) : (waves == 1 ? 0.33 : 0.40);
+    const long tiles = (M + rows - 1) / rows * ((columns + kTcBN - 1) / kTcBN), waves = (tiles + at_once - 1) / at_once;
+    const double full = (double)tiles / at_once;
+    const double slice = waves > 1 ? (pairs ? 0.37 : 0.40) : pairs ? 0.285 + 0.055 * full : 0.335 + 0.045 * full;
     return 8.0 + std::max((double)columns * K * 2 / 6.2e6, waves * slices * slice);
 }
 static bool takes_pairs(int M, int N, int K, bool dual)
@@ -750,8 +787,9 @@ static bool takes_pairs(int M, int N, int K, bool dual)
 
 // The plan with the least estimated time in us, from a sweep on B200 over 70 to 1000 tokens of the 2048- and 4096-wide shapes
 // (the estimate is within 15 % of all but the largest).  Either kernel needs about 8 us around its slices of 64 k.  A slice here takes 0.32 us, 0.45 when two blocks
-// share an SM; the operands of all blocks come in at no more than 15 TB/s, the weights at 6.2.  Clusters leave some slots of two
-// blocks an SM unused, and a second wave of blocks costs another start.
+// share an SM; the operands of all blocks come in at no more than 15 TB/s, the weights at 6.2.  Clusters of more than two blocks leave some
+// slots of two blocks an SM unused (1030 tokens, 2048 outputs, K 5632, 288 blocks: clusters of two 28.1 us, the persistent kernel 37.0), and a
+// second wave of blocks costs another start.
 static SplitPlan plan_split(int M, int N, int K, bool dual, bool pairs)
 {
     const int slices = (K + kTcBK - 1) / kTcBK, tiles_m = (M + kTcBM - 1) / kTcBM, columns = dual ? 2 * N : N;
@@ -764,7 +802,7 @@ static SplitPlan plan_split(int M, int N, int K, bool dual, bool pairs)
     for (int ks = 1; ks <= (pairs ? 4 : 8); ks++) {
         const int per = (slices + ks - 1) / ks;
         if (ks > 1 && (per < 2 || per * (ks - 1) >= slices)) continue;  // every rank has slices
-        const long blocks = tiles * ks, slots = ks == 1 && !pairs ? 2 * sms : 2 * sms - 32;
+        const long blocks = tiles * ks, slots = ks <= 2 && !pairs ? 2 * sms : 2 * sms - 32;
         const long full = blocks / slots, rest = blocks % slots;
         const double time = full * per * 0.45 + (rest > sms ? per * 0.45 : rest ? per * 0.32 : 0.0);
         const double operands = (double)tiles * slices * kSplitStage / 15e6;

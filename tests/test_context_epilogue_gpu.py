@@ -1,8 +1,33 @@
-"""The end of a context projection: gates of any size."""
+"""The end of a context projection: gates of any size, float outputs on top of a residual, at the edges of tiles and forms."""
 import numpy as np
 import pytest
 
+from tests.conftest import rel_err
+
 pytestmark = pytest.mark.gpu
+
+
+# one tile, the last tile of rows and of columns cut, one wave and several, blocks alone and in pairs, K split
+@pytest.mark.parametrize("M,N,K", [(65, 8, 128), (129, 264, 192), (300, 5640, 512), (1030, 4096, 512), (2060, 2056, 1024)])
+@pytest.mark.parametrize("form", ["float", "element", "gated"])
+def test_outputs_at_the_edges(cuda, ob, M, N, K, form):
+    g = cuda.Generator(device="cuda").manual_seed(M + N)
+    rnd = lambda *s: cuda.randn(s, generator=g, device="cuda")
+    x, W, W2 = rnd(M, K).bfloat16(), (rnd(K, N) * 0.05).bfloat16(), (rnd(K, N) * 0.05).bfloat16()
+    ld, f32 = N + 24, form != "element"
+    y = rnd(M, ld) if f32 else rnd(M, ld).bfloat16()
+    old = y.double().clone()
+    ob.project(ob.BF16, x, W, W2 if form == "gated" else None, y, M, N, K, act=ob.GATE_SILU, resid=y if f32 else None, scale=0.5 if f32 else 1.0, ldy=ld,
+               f32=f32)
+    ref = x.double() @ W.double()
+    if form == "gated":
+        ref = cuda.nn.functional.silu(ref) * (x.double() @ W2.double())
+    if f32:  # on top of a residual
+        ref = old[:, :N] + 0.5 * ref
+    assert cuda.equal(y[:, N:].double(), old[:, N:])
+    # float: the order of sums of K products and the fast exponential; elements: one rounding to bfloat16
+    assert rel_err(y[:, :N].double().cpu().numpy(), ref.cpu().numpy()) < (1e-5 if f32 else 4e-3)
+    assert ob.lib().onellm_gemm_timeout_flag() == 0
 
 
 @pytest.mark.parametrize("act,name", [("GATE_SILU", "silu"), ("GATE_CLAMPED", "clamped"), ("GATE_RELU", "relu")])
