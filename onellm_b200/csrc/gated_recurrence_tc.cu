@@ -655,21 +655,6 @@ constexpr int kGoSmem = kGoRing * kGcTile;
 constexpr uint32_t kGoTable = 0, kGoTableLow = 128, kGoState = 256, kGoStateLow = 384;
 
 __device__ __forceinline__ void go_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kGoWarps * 32) : "memory"); }  // the warps that make the output
-// a wait for what the blocks of the cluster have written
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity)
-{
-    for (uint32_t i = 0; i < kSpinLimit; i++) {
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (ok) return true;
-    }
-    atomicExch(&g_tc_timeout_flag, 1);
-    return false;
-}
-
 // grid (dv / 128, clusters), cluster (dv / 128, 1, 1): a cluster has the value tiles of a head and takes every gridDim.y-th pair of chunk and head
 __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __grid_constant__ GrParams pp, const __grid_constant__ GrChunks ck)
 {

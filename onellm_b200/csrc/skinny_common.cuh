@@ -40,12 +40,18 @@ struct EpilogueArgs {
     const float* row_scale = nullptr;
 };
 
+// Elements of a tile of `tokens` rows that a rank of the cluster finishes: an even number.
+__host__ __device__ constexpr int splitk_share(int tokens, int ks) { return (((tokens * kBN + ks - 1) / ks) + 1) & ~1; }
+
 // `red` holds this block's partial tile as [NW][MP][kRedLd] floats followed by MP partial sums of squares (used
 // when ep.rms is set); the blocks of the cluster (rank = blockIdx.y of gridDim.y) hold the other K ranges of the
 // same tile.  Sums them in rank order and finishes the tile; every thread of the block (NT of them) calls it.
 // WIDE (tcgen05 kernel, no tensor-parallel exchange): the second half of `red` is not a second weight but the next
 // 128 output columns of the same weight (a block owns 256 columns and reads its activations once for both).
-template <typename T, int MP, bool DUAL, bool FUSED, int NT, bool WIDE = false>
+// PUSHED: every rank has put its values of the elements that this one finishes into `red` here, as [NW][KS][splitk_share] floats, and its sums
+// of squares behind them, [KS][MP], and the caller has waited for them: there is no barrier of the cluster here, and no block has to stay for
+// others.
+template <typename T, int MP, bool DUAL, bool FUSED, int NT, bool WIDE = false, bool PUSHED = false>
 __device__ __forceinline__ void splitk_epilogue(float* red, cg::cluster_group& cluster, T* y, int M, int N, int K, int n0,
                                                 const EpilogueArgs& ep)
 {
@@ -61,10 +67,11 @@ __device__ __forceinline__ void splitk_epilogue(float* red, cg::cluster_group& c
         *ctr = n;
         s_seq = 0x80000000u | (uint32_t)n;  // the high bit keeps these apart from the numbers of the stand-alone all-reduce
     }
-    cluster.sync();
+    if constexpr (!PUSHED) cluster.sync();
+    else if (tp) __syncthreads();
     const uint32_t seq = tp ? s_seq : 0u;
     // every rank of the cluster finishes an even-sized slice of the tile, two adjacent columns per thread
-    const int per_rank = (((MP * kBN + KS - 1) / KS) + 1) & ~1;
+    const int per_rank = splitk_share(MP, KS);
     const int e_begin = rank * per_rank, e_end = min(e_begin + per_rank, MP * kBN);
     const long long t_start = clock64();
     // The value this block contributes to elements (tok, c) and (tok, c + 1): the K ranges of the cluster added in rank
@@ -79,7 +86,13 @@ __device__ __forceinline__ void splitk_epilogue(float* red, cg::cluster_group& c
         for (int r = 0; r < 8; r++) {
             p0[r] = p1[r] = make_float2(0.f, 0.f);
             ps[r] = 0.f;
-            if (r < KS) {
+            if (PUSHED) {
+                if (r < KS) {
+                    p0[r] = *reinterpret_cast<const float2*>(red + r * per_rank + e - e_begin);
+                    if (NW == 2) p1[r] = *reinterpret_cast<const float2*>(red + (KS + r) * per_rank + e - e_begin);
+                    if (ep.rms) ps[r] = red[NW * KS * per_rank + r * MP + tok];
+                }
+            } else if (r < KS) {
                 const float* peer = cluster.map_shared_rank(red, r);
                 p0[r] = make_float2(peer[tok * kRedLd + c], peer[tok * kRedLd + c + 1]);
                 if (NW == 2) p1[r] = make_float2(peer[(MP + tok) * kRedLd + c], peer[(MP + tok) * kRedLd + c + 1]);

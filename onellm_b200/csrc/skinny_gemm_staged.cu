@@ -14,7 +14,10 @@
 // mma.m16n8k16 (the WEIGHT is the 16-row operand, the 8 tokens of a batch block the 8-column
 // operand, so a batch of 8 wastes nothing).  The eight warps of a block split the 128 columns,
 // so no cross-warp reduction is needed; K is split across the blocks of a thread-block
-// cluster and the partial sums meet in distributed shared memory in a fixed order.
+// cluster and the partial sums meet in distributed shared memory in a fixed order: a block sends every rank its values of the
+// elements that one finishes by stores that count on an mbarrier there, and sums what has come in from its own memory (up to 16
+// tokens; read from the peers' memory between two barriers of the cluster, as for more tokens, the end of a launch took 2.3 to 3.4 us
+// instead of 1.1 to 1.9).
 #include <cooperative_groups.h>
 #include <math.h>
 #include <stdio.h>
@@ -28,6 +31,7 @@
 
 #include "project.h"
 #include "skinny_common.cuh"
+#include "tc_common.cuh"
 
 namespace onellm {
 
@@ -35,6 +39,18 @@ constexpr int kStThreads = 256;
 constexpr int kKC = 32;                  // rows per stage
 constexpr int kStageBytes = kKC * kBN * 2;  // 8 KB per weight matrix
 constexpr int kXRowBytes = kKC * 2 + 16;   // activation rows of a stage, padded: conflict-free fragment reads
+
+// Whether the blocks of a cluster push their partial sums, and the shared memory behind the ring that takes them
+template <int MB, bool FUSED, bool GROUPED = false>
+constexpr bool pushes() { return MB <= 2 && !FUSED && !GROUPED; }
+template <int MB, int NW>
+constexpr size_t pushed_bytes() { return ((size_t)NW * (8 * MB * kBN + 2 * 8) + 8 * 8 * MB) * sizeof(float); }
+
+// a store into the memory of a block of the cluster that counts on a barrier of that block
+__device__ __forceinline__ void store_counted(uint32_t addr, float v, uint32_t bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar) : "memory");
+}
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr)
 {
@@ -183,6 +199,18 @@ skinny_kn_staged_kernel(const T* __restrict__ x, const T* __restrict__ W0, const
         issue_w(smem_base + (uint32_t)(s * STAGE));
         cp_async_commit();
     }
+    constexpr bool PUSH = pushes<MB, FUSED, GROUPED>();
+    __shared__ __align__(8) uint64_t sums_bar;
+    const uint32_t sums_there = smem_u32(&sums_bar);
+    if constexpr (PUSH) {
+        if (tid == 0) {
+            const int share = splitk_share(MP, KS), own = max(0, min(share, MP * kBN - rank * share));
+            mbar_init(sums_there, 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            mbar_expect_tx(sums_there, (uint32_t)(4 * KS * (NW * own + (ep.rms ? MP : 0))));
+        }
+        cluster_arrive();
+    }
     if (ep.early_dependents) pdl_launch_dependents();
     pdl_wait();
     // FUSED: normalised activations of this block's K range, [MP][xn_ld] halfs behind the ring
@@ -330,8 +358,39 @@ skinny_kn_staged_kernel(const T* __restrict__ x, const T* __restrict__ W0, const
     }
     cp_async_wait<0>();
     if (!ep.early_dependents) pdl_launch_dependents();
-    __syncthreads();
 
+    if constexpr (PUSH) {
+        cluster_wait();  // the barriers of all blocks
+        float* sums = reinterpret_cast<float*>(smem + (size_t)nst * STAGE);
+        const uint32_t to = smem_u32(sums);
+        const int share = splitk_share(MP, KS);
+        const uint32_t inv = 0xffffffffu / (uint32_t)share + 1u;  // i / share as the high word of i * inv: i < 2048
+#pragma unroll
+        for (int mb = 0; mb < MB; mb++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int i = (8 * mb + 2 * t + (e & 1)) * kBN + warp * 16 + g + ((e & 2) ? 8 : 0);
+                const int owner = (int)__umulhi((uint32_t)i, inv);
+                const uint32_t at = map_to_rank(to + 4u * (uint32_t)(rank * share + i - owner * share), (uint32_t)owner),
+                               bar = map_to_rank(sums_there, (uint32_t)owner);
+#pragma unroll
+                for (int w = 0; w < NW; w++) store_counted(at + 4u * (uint32_t)(w * KS * share), acc[w][mb][e], bar);
+            }
+        if (ep.rms && warp == 0) {
+#pragma unroll
+            for (int mb = 0; mb < MB; mb++) {
+                float v = ssq[mb];
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                for (int r = t; r < KS; r += 4)  // the four lanes of a token share out the ranks
+                    store_counted(map_to_rank(to + 4u * (uint32_t)(NW * KS * share + rank * MP + 8 * mb + g), (uint32_t)r), v, map_to_rank(sums_there, (uint32_t)r));
+            }
+        }
+        if (!mbar_wait_cluster(sums_there, 0)) return;  // never seen: the flag is up
+        splitk_epilogue<T, MP, DUAL, FUSED, kStThreads, false, true>(sums, cluster, y, M, N, K, n0, ep);
+        return;
+    }
+    __syncthreads();
     // this block's partial tile, then the cluster-wide sum in rank order
     float* red = reinterpret_cast<float*>(smem);  // [NW][MP][kRedLd]
 #pragma unroll
@@ -402,17 +461,15 @@ struct StagedPlan {
 };
 
 // Launch plans found by sweeping (K split, ring depth) with the decoder layer's five kernels as one CUDA graph as the
-// objective (batch 8, B200): the Llama-2-7B projections whole and sliced 2, 4 and 8 ways.  The general rule below
-// (most bytes in flight with every block resident) is within a few percent on the whole shapes but picks too few,
-// too deep blocks for the narrow slices (the 2-way gate/up slice: 129 blocks of 12 stages, 21 us; 215 blocks of
-// 4 stages, 10 us less for the layer).
+// objective (batch 8, B200): the Llama-2-7B projections sliced 2, 4 and 8 ways.  (Whole they take the general rule: the plans of
+// such a sweep, 32 clusters of eight for the down projection where 33 fit, left two of them without room behind the gate/up
+// projection in 45 % of the layers of a decode step, 35 instead of 20 us.)
 struct TunedPlan {
     int N, K;
     bool dual;
     int ks, nst;
 };
 static const TunedPlan kTunedPlans[] = {
-    {12288, 4096, false, 5, 5}, {4096, 4096, false, 8, 8},  {11008, 4096, true, 3, 6}, {4096, 11008, false, 8, 10},
     {6144, 4096, false, 8, 6},  {4096, 2048, false, 6, 5},  {5504, 4096, true, 5, 4},  {4096, 5504, false, 8, 10},
     {3072, 4096, false, 8, 10}, {4096, 1024, false, 6, 4},  {2752, 4096, true, 8, 5},  {4096, 2752, false, 8, 8},
     {1536, 4096, false, 8, 4},  {4096, 512, false, 4, 4},   {1376, 4096, true, 8, 5},  {4096, 1376, false, 8, 4},
@@ -433,6 +490,8 @@ static StagedPlan plan_staged(int N, int K, bool tp)
     constexpr int NW = DUAL ? 2 : 1;
     constexpr size_t stage = (size_t)NW * kStageBytes + (FUSED ? 0 : 8 * MB * kXRowBytes);
     constexpr size_t red = ((size_t)NW * 8 * MB * kRedLd + 8 * MB) * sizeof(float);
+    // a ring of n stages and what the partial sums take: behind it, or in its place
+    const auto bytes = [=](int n) { return pushes<MB, FUSED>() ? stage * n + pushed_bytes<MB, NW>() : std::max(stage * n, red); };
     constexpr size_t smem_cap = 226 * 1024;
     static DeviceOnce smem_attr;
     StagedPlan plan = {1, 3, 0, 0, cudaSuccess};
@@ -452,7 +511,7 @@ static StagedPlan plan_staged(int N, int K, bool tp)
             plan.nst = std::max(3, std::min(ov->second.second, 12));  // the prologue holds at most 11 stages of activations in registers
             plan.per_block = (total_stages + plan.ks - 1) / plan.ks;
             const size_t xn = FUSED ? (size_t)8 * MB * (plan.per_block * kKC + 8) * sizeof(T) : 0;
-            plan.smem = std::max(stage * plan.nst, red) + xn;
+            plan.smem = bytes(plan.nst) + xn;
             if (plan.smem > smem_cap) plan.status = cudaErrorInvalidConfiguration;
             return plan;
         }
@@ -469,9 +528,10 @@ static StagedPlan plan_staged(int N, int K, bool tp)
         for (const TunedPlan& t : kTunedPlans) {
             if (t.N != N || t.K != K || t.dual != DUAL || t.ks > total_stages) continue;
             const int per = (total_stages + t.ks - 1) / t.ks;
-            const size_t smem = std::max(stage * t.nst, red);
+            const size_t smem = bytes(t.nst);
             if (smem > smem_cap || per * (t.ks - 1) >= total_stages) break;
-            if (staged_slots(kern, t.ks, t.nst, smem, col_blocks) < (long)col_blocks * t.ks) break;
+            const long places = staged_slots(kern, t.ks, t.nst, smem, col_blocks), needed = (long)col_blocks * t.ks;
+            if (places < needed || (!tp && (places * 97 < needed * 100 || places / t.ks < col_blocks + 2))) break;  // room to spare, as below
             if (tp && (long)col_blocks * t.ks > kTpMaxBlocks) break;
             plan.ks = t.ks;
             plan.nst = t.nst;
@@ -498,7 +558,6 @@ static StagedPlan plan_staged(int N, int K, bool tp)
         constexpr double kRange[3][2] = {{0.03, 0.20}, {0.05, 0.32}, {0.21, 0.81}};
         constexpr double kRate[3][2][4] = {{{29, 46, 49, 49}, {43, 60, 54, 54}}, {{26, 41, 45, 45}, {38, 54, 50, 50}}, {{19.4, 29, 31.5, 33}, {32, 43, 41, 41}}};
         const long sms = num_sms();
-        auto bytes = [&](int nst) { return std::max(stage * nst, red); };
         auto on_an_sm = [&](int nst) { return std::max(1L, staged_slots(kern, 1, nst, bytes(nst), col_blocks) / sms); };
         double best = 0.0;
         for (int ks = 1; ks <= 8; ks++) {
@@ -539,7 +598,7 @@ static StagedPlan plan_staged(int N, int K, bool tp)
         const long total = (long)col_blocks * ks;
         const size_t xn_b = FUSED ? (size_t)8 * MB * (per * kKC + 8) * sizeof(T) : 0;
         for (int nst = std::min(12, std::max(3, per + 1)); nst >= 3; nst--) {
-            const size_t smem = std::max(stage * nst, red) + xn_b;
+            const size_t smem = bytes(nst) + xn_b;
             if (smem > smem_cap) continue;
             if (staged_slots(kern, ks, nst, smem, col_blocks) < total) continue;
             // FUSED: every block redoes the row statistics, so fewer blocks are better there
@@ -563,7 +622,7 @@ static StagedPlan plan_staged(int N, int K, bool tp)
     plan.nst = best_nst;
     plan.per_block = (total_stages + best_ks - 1) / best_ks;
     const size_t xn_final = FUSED ? (size_t)8 * MB * (plan.per_block * kKC + 8) * sizeof(T) : 0;
-    plan.smem = std::max(stage * best_nst, red) + xn_final;
+    plan.smem = bytes(best_nst) + xn_final;
     if (plan.status == cudaSuccess && plan.smem > smem_cap) plan.status = cudaErrorInvalidConfiguration;
     if (plan.status == cudaSuccess && tp && (long)col_blocks * best_ks > kTpMaxBlocks) plan.status = cudaErrorInvalidConfiguration;
     plans[key] = plan;
@@ -757,6 +816,8 @@ cudaError_t skinny_kn_staged_dispatch(const __half* x, const __half* W0, const _
     if (tp) ep.tp = *tp;
     return skinny_kn_project<__half>(x, W0, dual ? W1 : nullptr, y, M, N, K, ep, st);
 }
+
+static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
 }  // namespace onellm
 

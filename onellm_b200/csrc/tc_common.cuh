@@ -70,6 +70,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     atomicExch(&g_tc_timeout_flag, 1);
     return false;
 }
+// a wait for what the blocks of the cluster have written
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity)
+{
+    for (uint32_t i = 0; i < kSpinLimit; i++) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+    }
+    atomicExch(&g_tc_timeout_flag, 1);
+    return false;
+}
 // whether the phase has completed, without waiting
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity)
 {
