@@ -20,16 +20,17 @@
 //      multiply-adds along the gates: slower, never out of range.  Bound by the instructions (70 per channel and token).
 //   2. gr_chunk_state_kernel (29 | 24): a block keeps 32 or 64 key channels x 128 value columns of a state in registers and walks the
 //      chunks; it leaves the pieces of b_m S in front of every chunk.  Bound by the chain of a chunk: products into registers, update, split.
-//   3. gr_chunk_output_kernel (26 | 80): a block makes 128 tokens x 128 value columns of the output: q~ . k~, q~ . S, then, behind the mask,
+//   3. gr_chunk_output_kernel (26 | 58): a block makes 128 tokens x 128 value columns of the output: q~ . k~, q~ . S, then, behind the mask,
 //      the first times V with the pieces of the table in tensor memory; RMS norm over the head (a cluster's blocks share the sums) and gate.
 //      Bound by its operands: 6 bytes a float, 320 KB (608 KB) for 7680 (13800) cycles of products.
-// All three 83 | 144 us; token by token 254 | 246.  Error of the state against 64 bits 9.7e-8 | 8.2e-8 (9.3e-8 | 1.1e-7), of the outputs
+// All three 82 | 118 us; token by token 254 | 246.  Error of the state against 64 bits 9.7e-8 | 8.2e-8 (9.3e-8 | 1.1e-7), of the outputs
 // 1.66e-3 both, the rounding to bfloat16.
 // A value that is not finite would reach the chunk's earlier tokens through a product with zero: the copy has zero there, and the
 // column is NaN from its token on.
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "gated_recurrence.cuh"
 
@@ -548,17 +549,20 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
         float* state = p.state + (((size_t)b * p.H + h) * dk + blockIdx.x * COLS + c0) * dv + v;
         const bool fresh = pp.tp.hist[b] == 0;
         float S[kCols];
-        int notes = ck.notes[at0].y | ck.notes[at0].z;
+        int4 notes = ck.notes[at0];
 #pragma unroll
         for (int c = 0; c < kCols; c++) S[c] = fresh ? 0.f : state[(size_t)c * dv];
         for (int i = 0; i < n_chunk; i++) {
             const size_t at = at0 + i;
-            const int next = i + 1 < n_chunk ? ck.notes[at + 1].y | ck.notes[at + 1].z : 0;
+            const int4 next = i + 1 < n_chunk ? ck.notes[at + 1] : make_int4(0, 0, 0, 0);
             bool there = ok && mbar_wait_warp(vec0 + 8 * (i & 3), (uint32_t)(i >> 2) & 1u);
             const float4* vec = reinterpret_cast<const float4*>(s_vec + (i & 3) * kGsVec) + (from_col + c0) / 4;  // + 16: the next vector
-            // the pieces of the chunk in front have been read out of shared memory before anyone writes the next ones
-            if (COLS == 64 && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            gs_sync();
+            // the pieces of the chunk in front have been read out of shared memory before anyone writes the next ones; half rows have two places
+            const int place = COLS == 64 ? 0 : (i & 1) * 32;
+            if constexpr (COLS == 64) {
+                if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                gs_sync();
+            }
 #pragma unroll
             for (int g = 0; g < kCols / 8; g++) {
                 uint32_t p0[4], p1[4], p2[4], rest = 0u;
@@ -569,7 +573,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
                     split_pair(x[0] * bm.x, x[1] * bm.y, p0[2 * e], p1[2 * e], p2[2 * e], rest);
                     split_pair(x[2] * bm.z, x[3] * bm.w, p0[2 * e + 1], p1[2 * e + 1], p2[2 * e + 1], rest);
                 }
-                unsigned char* dst = s_out + gc_at(row, from_col + c0 + 8 * g);
+                unsigned char* dst = s_out + gc_at(row, place + c0 + 8 * g);
                 *reinterpret_cast<uint4*>(dst) = make_uint4(p0[0], p0[1], p0[2], p0[3]);
                 *reinterpret_cast<uint4*>(dst + kGcTile) = make_uint4(p1[0], p1[1], p1[2], p1[3]);
                 *reinterpret_cast<uint4*>(dst + 2 * kGcTile) = make_uint4(p2[0], p2[1], p2[2], p2[3]);
@@ -585,10 +589,9 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
             } else {
                 gs_sync();
 #pragma unroll
-                for (int e = 0; e < 3; e++) {  // four threads to the 64 bytes of a row
-                    const uint32_t from = e * kGcTile + gc_at(tid >> 2, from_col + (tid & 3) * 8);
-                    *reinterpret_cast<uint4*>(out + from) = *reinterpret_cast<const uint4*>(s_out + from);
-                }
+                for (int e = 0; e < 3; e++)  // four threads to the 64 bytes of a row
+                    *reinterpret_cast<uint4*>(out + e * kGcTile + gc_at(tid >> 2, from_col + (tid & 3) * 8)) =
+                        *reinterpret_cast<const uint4*>(s_out + e * kGcTile + gc_at(tid >> 2, place + (tid & 3) * 8));
             }
             there = there && mbar_wait_warp(done0 + 8 * slot(2 * i + 1), turn(2 * i + 1));
             if (!there) ok = false;  // goes on to the barriers of the others, with nothing stored at the end
@@ -625,7 +628,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(free0 + 8 * (i & 1));  // the accumulators and the vectors
-            if (notes && ck.bad[at * dv + v] < kGcTok) {
+            if ((notes.y | notes.z) && ck.bad[at * dv + v] < kGcTok) {
 #pragma unroll
                 for (int c = 0; c < kCols; c++) S[c] = __uint_as_float(0x7fffffffu);
             }
@@ -987,6 +990,36 @@ size_t gr_chunked_workspace(int tokens, int H, int dk, int dv)
     return (size_t)gc_slots(tokens, tokens / kGcLeastTokensFull) * H * gc_chunk_bytes(dk, dv) + 256;
 }
 
+// Clusters of `nv` output blocks that run at once, asked once per device: a GPC of 18 SMs has room for four clusters of four, and a
+// cluster more than there is room for would run when the others are through (4 heads of 256 x 512, 2 x 1030 tokens: 84 us instead of 42).
+static int go_clusters(int nv)
+{
+    static std::mutex mu;
+    static int known[kMaxDevices][kGcMaxDv / 128 + 1] = {};
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[current_device()][nv];
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute a[1];
+        a[0].id = cudaLaunchAttributeClusterDimension;
+        a[0].val.clusterDim.x = nv;
+        a[0].val.clusterDim.y = 1;
+        a[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(nv, 1024);
+        cfg.blockDim = dim3(kGoBlock);
+        cfg.dynamicSmemBytes = kGoSmem;
+        cfg.attrs = a;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gr_chunk_output_kernel, &cfg) != cudaSuccess || clusters < 1) {
+            (void)cudaGetLastError();
+            clusters = num_sms() / nv;
+        }
+        n = std::max(1, clusters);
+    }
+    return n;
+}
+
 template <typename... KArgs, typename... Args>
 static cudaError_t gc_launch(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, dim3 cluster, cudaStream_t st, Args... args)
 {
@@ -1046,7 +1079,7 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
             if (e == cudaSuccess) e = prefer_max_shared(k);
         return e;
     }));
-    const long clusters = std::min((long)std::max(1, num_sms() / nv), (long)slots * g.H);
+    const long clusters = std::min((long)go_clusters(nv), (long)slots * g.H);
     // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
     const bool narrow = (long)(dk / 32) * nv * g.H * B <= num_sms();
     ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
