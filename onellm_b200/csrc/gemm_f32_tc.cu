@@ -8,7 +8,7 @@
 //
 // A block computes y^T: 128 columns of W are the rows of the MMA, the tokens (at most 192) its columns, so that a token count
 // that is no multiple of 128 costs no padding.
-//   W      lane = column: a thread splits 16 rows of its column and stores the pieces to tensor memory, where the MMA takes its A
+//   W      lane = column: a thread splits 8 rows of its column and stores the pieces to tensor memory, where the MMA takes its A
 //          operand from: no transposition.
 //   x      8 threads split the 32 values of a token's stage; the pieces go to shared memory in the 128-byte swizzled form
 //          ([x0 | x1] in one tile of 128-byte rows, [x2 | unused] in a second one).
@@ -19,12 +19,11 @@
 //          convert stage s + 1 while the MMAs of stage s run.
 // K is split over the blocks of a cluster where the tiles alone would not fill the GPU; the partial sums meet in distributed
 // shared memory in rank order.
-// What bounds it, in cycles of a stage of 176 tokens with six products and pieces cut off instead of rounded: the MMAs 1000 (eight: a
-// third more), splitting its floats 1200, adding an accumulator 400 and the waits between them 450, the last three one after the
-// other in every warp.  The two products more and the notice of what the pieces do not hold cost 2 to 9 % of a call, 3 to 8 % of a
-// layer.  Measured, 352 tokens of the 7B shapes, us (the 64 x 64 tiled kernel): QKV 276 (2209), o_proj 91 (911), gate or up 250 (2202),
-// down 219 (2569), 127 to 145 TFLOP/s of float32; error against 64 bits, normal operands, 1.1e-7 (chain 1.1e-6; K = 11008: 1.5e-7,
-// 1.8e-6), a layer 6.9e-7 instead of 2.8e-6.
+// What bounds it: a stage of 176 tokens takes about 2100 cycles, 1400 of them its MMAs; the warps split its floats, add an accumulator
+// and wait for both one after the other.  Sixteen warps instead of eight shorten that chain, with half of the rows, columns and
+// registers each: 352 tokens of the 7B shapes, us (with eight | the 64 x 64 tiled kernel): QKV 266 (276 | 2209), o_proj 90 (91 | 911),
+// gate or up 245 (250 | 2202), down 217 (219 | 2569), 131 to 146 TFLOP/s of float32; a layer 1355 (1390).  Error against 64 bits, normal
+// operands, 1.1e-7 (chain 1.1e-6; K = 11008: 1.5e-7, 1.8e-6), a layer 6.9e-7 instead of 2.8e-6.
 // What the pieces do not hold: a value that is not finite, or whose first piece rounds to infinity, makes its remainders NaN and so
 // every result it enters; one below 2^-110 loses its last bits.  Blocks whose results that touches (see `stands`) compute them
 // again by plain multiply-adds, at the rate of the tiled kernel; the results are that kernel's to the bit.
@@ -43,21 +42,22 @@ namespace onellm {
 constexpr int kFtCols = 128;                    // columns of W per block
 constexpr int kFtTok = 192;                     // most tokens per block
 constexpr int kFtK = 32;                        // rows of W per stage
-constexpr int kFtWarps = 8;                     // warps that convert and add
+constexpr int kFtWarps = 16;                    // warps that convert and add, four to 32 columns of W
+constexpr int kFtParts = kFtWarps / 4;
 constexpr int kFtThreads = kFtWarps * 32 + 32;  // and one that issues loads and MMAs
 constexpr int kFtTile = kFtTok * 128;           // bytes: a 128-byte row per token
 constexpr int kFtPiecesBytes = 4 * kFtTile;     // two stages of two tiles; the partial sums of the cluster afterwards
 constexpr int kFtDepth = 3;                     // stages of floats on their way
 constexpr int kFtRawW = kFtK * kFtCols * 4, kFtRaw = kFtRawW + kFtTok * kFtK * 4;
 constexpr int kFtSmem = kFtPiecesBytes + kFtDepth * kFtRaw;
-constexpr int kFtGroup = kFtTok / 2 / 3;        // accumulator columns read at a time
+constexpr int kFtGroup = kFtTok / kFtParts / 3; // accumulator columns read at a time
 // The third piece of a float below 2^-110 falls among the subnormal bf16 values and loses up to 2^-133, on either side of a product: a
 // result of K products beside the largest operand then counts from 2^26 times K * 2^-132 of it.  Below kFtLeast the products of
 // the pieces themselves leave the range of float.
 constexpr float kFtLost = 0x1p-106f, kFtLeast = 0x1p-80f;
 constexpr unsigned kGaveUp = 0xffffffffu;  // above the bits of every float that is not NaN
 constexpr uint32_t kFtPieces = 2 * kFtTok;      // tensor memory: two accumulators, then two stages of 3 pieces x 16 columns
-static_assert(kFtGroup == 32 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
+static_assert(kFtGroup == 16 && kFtPieces + 2 * 48 <= 512 && kFtTok * kFtCols * 4 <= kFtPiecesBytes, "layout");
 
 __device__ __forceinline__ void finish_f32(const GemmF32& a, int m, int n, float v)
 {
@@ -203,7 +203,7 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
     if (gridDim.y > 1) cluster_arrive();
     pdl_wait();
 
-    const int half = warp >> 2, nh = nt / 2;  // a warp adds the accumulator columns [half * nh, half * nh + nh) of its 32 lanes
+    const int part = warp >> 2, np = nt / kFtParts;  // a warp adds the accumulator columns [part * np, part * np + np) of its 32 lanes
     float acc[3 * kFtGroup];
 #pragma unroll
     for (int i = 0; i < 3 * kFtGroup; i++) acc[i] = 0.f;
@@ -256,18 +256,18 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
         const int col = (warp & 3) * 32 + lane;
         // x: rows r and r + 4 of a group of 8 side by side, so that a warp's stores fill all banks
         const int quad = tid & 7, row0 = (warp * 4 & ~7) + ((tid >> 3) & 1) * 4 + ((tid >> 4) & 1) + (warp & 1) * 2;
-        const uint32_t x_at = (uint32_t)row0 * 128 + (((quad >> 1) ^ (row0 & 7)) << 4) + (quad & 1) * 8;  // + 32 rows: + 4096
+        const uint32_t x_at = (uint32_t)row0 * 128 + (((quad >> 1) ^ (row0 & 7)) << 4) + (quad & 1) * 8;  // + 64 rows: + 8192
         auto add = [&](int s) {
             if (!mbar_wait_warp(done0 + 8 * (s & 1), (uint32_t)(s >> 1) & 1u)) return false;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
             for (int g = 0; g < 3; g++) {
-                if (g * kFtGroup < nh) {
-                    uint32_t v[32];
-                    tmem_ld32(t_lane + (uint32_t)((s & 1) * kFtTok + half * nh + g * kFtGroup), v);
+                if (g * kFtGroup < np) {
+                    uint32_t v[kFtGroup];
+                    tmem_ld16(t_lane + (uint32_t)((s & 1) * kFtTok + part * np + g * kFtGroup), v);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int i = 0; i < 32; i++) acc[g * kFtGroup + i] += __uint_as_float(v[i]);
+                    for (int i = 0; i < kFtGroup; i++) acc[g * kFtGroup + i] += __uint_as_float(v[i]);
                 }
             }
             return true;
@@ -280,47 +280,39 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
             if (!ok) break;
             const unsigned char* raw = smem_raw + kFtPiecesBytes + slot * kFtRaw;
             // the buffers of this stage were last read by the MMAs of stage s - 2, whose accumulator has been added
-            uint32_t p0[8], p1[8], p2[8];
+            uint32_t p0[4], p1[4], p2[4];
             if constexpr (NK) {  // [128 columns][32 k], 128-byte swizzled
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float4 v = *reinterpret_cast<const float4*>(raw + col * 128 + (((half * 4 + i) ^ (col & 7)) << 4));
+                for (int i = 0; i < 2; i++) {
+                    const float4 v = *reinterpret_cast<const float4*>(raw + col * 128 + (((part * 2 + i) ^ (col & 7)) << 4));
                     split_pair(v.x, v.y, p0[2 * i], p1[2 * i], p2[2 * i], rest);
                     split_pair(v.z, v.w, p0[2 * i + 1], p1[2 * i + 1], p2[2 * i + 1], rest);
                 }
             } else {  // [32 k][128 columns]
-                const float* wr = reinterpret_cast<const float*>(raw) + half * 16 * kFtCols + col;
+                const float* wr = reinterpret_cast<const float*>(raw) + part * 8 * kFtCols + col;
 #pragma unroll
-                for (int i = 0; i < 8; i++) split_pair(wr[2 * i * kFtCols], wr[(2 * i + 1) * kFtCols], p0[i], p1[i], p2[i], rest);
+                for (int i = 0; i < 4; i++) split_pair(wr[2 * i * kFtCols], wr[(2 * i + 1) * kFtCols], p0[i], p1[i], p2[i], rest);
             }
-            const uint32_t t_w = t_lane + kFtPieces + (uint32_t)((s & 1) * 48 + half * 8);
-            tmem_st8(t_w, p0);
-            tmem_st8(t_w + 16, p1);
-            tmem_st8(t_w + 32, p2);
+            const uint32_t t_w = t_lane + kFtPieces + (uint32_t)((s & 1) * 48 + part * 4);
+            tmem_st4(t_w, p0);
+            tmem_st4(t_w + 16, p1);
+            tmem_st4(t_w + 32, p2);
             const unsigned char* xr = raw + kFtRawW + row0 * 128 + quad * 16;
             unsigned char* xs = smem_raw + (s & 1) * 2 * kFtTile;
-            // three token groups at a time, so that their latencies overlap; the 8 rows of a warp's group are there or not: nt is a multiple of 16
+            // all token groups at a time, so that their latencies overlap; the 8 rows of a warp's group are there or not: nt is a multiple of 16
+            float4 v[kFtTok / 64];
 #pragma unroll
-            for (int j0 = 0; j0 < kFtTok / 32; j0 += 3) {
-                if (32 * j0 >= nt) break;
-                float4 v[3];
-                uint2 q0[3], q1[3], q2[3];
+            for (int j = 0; j < kFtTok / 64; j++)
+                v[j] = (warp >> 1) * 8 + 64 * j < nt ? *reinterpret_cast<const float4*>(xr + j * 8192) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 3; i++)
-                    v[i] = (warp >> 1) * 8 + 32 * (j0 + i) < nt ? *reinterpret_cast<const float4*>(xr + (j0 + i) * 4096) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    split_pair(v[i].x, v[i].y, q0[i].x, q1[i].x, q2[i].x, rest);
-                    split_pair(v[i].z, v[i].w, q0[i].y, q1[i].y, q2[i].y, rest);
-                }
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    const int j = j0 + i;
-                    if ((warp >> 1) * 8 + 32 * j < nt) {
-                        *reinterpret_cast<uint2*>(xs + x_at + j * 4096) = q0[i];
-                        *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 4096) = q1[i];  // 16-byte chunk + 4, swizzled
-                        *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 4096) = q2[i];
-                    }
+            for (int j = 0; j < kFtTok / 64; j++) {
+                uint2 q0, q1, q2;
+                split_pair(v[j].x, v[j].y, q0.x, q1.x, q2.x, rest);
+                split_pair(v[j].z, v[j].w, q0.y, q1.y, q2.y, rest);
+                if ((warp >> 1) * 8 + 64 * j < nt) {
+                    *reinterpret_cast<uint2*>(xs + x_at + j * 8192) = q0;
+                    *reinterpret_cast<uint2*>(xs + (x_at ^ 64u) + j * 8192) = q1;  // 16-byte chunk + 4, swizzled
+                    *reinterpret_cast<uint2*>(xs + kFtTile + x_at + j * 8192) = q2;
                 }
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -366,21 +358,21 @@ gemm_f32_tc_kernel(const GemmF32 a, const __grid_constant__ CUtensorMap map_x, c
         if (fine && warp < kFtWarps && n < a.N) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
-                if (i < nh && half * nh + i < m_rows) bad |= !stands(acc[i], least, top == 0.f);
+                if (i < np && part * np + i < m_rows) bad |= !stands(acc[i], least, top == 0.f);
         }
         if (__syncthreads_or(bad)) {
             plain_tile<NK>(a, again, m0, m_rows, n0);
         } else if (fine && warp < kFtWarps && n < a.N) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
-                if (i < nh && half * nh + i < m_rows) finish_f32(a, m0 + half * nh + i, n, acc[i]);
+                if (i < np && part * np + i < m_rows) finish_f32(a, m0 + part * np + i, n, acc[i]);
         }
     } else {
         float* red = reinterpret_cast<float*>(smem_raw);  // [nt][128]
         if (fine && warp < kFtWarps) {
 #pragma unroll
             for (int i = 0; i < 3 * kFtGroup; i++)
-                if (i < nh) red[(half * nh + i) * kFtCols + q * 32 + lane] = acc[i];
+                if (i < np) red[(part * np + i) * kFtCols + q * 32 + lane] = acc[i];
         }
         cluster.sync();
         // this rank's tokens; their sums go into its own buffer, in the place that no other rank reads
