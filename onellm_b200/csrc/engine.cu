@@ -20,6 +20,32 @@ namespace onellm {
 // the new step.
 __global__ void advance_step_kernel(int* step) { *step += 1; }
 
+// The same, and the step's ids out of mapped host memory
+__global__ void advance_with_ids_kernel(int* step, const volatile int* in, int stride, int* __restrict__ ids, int B)
+{
+    const int next = *step + 1;
+    for (int b = threadIdx.x; b < B; b += blockDim.x) ids[b] = in[(next % Mail::kTurns) * stride + b];
+    __syncthreads();
+    if (threadIdx.x == 0) *step = next;
+}
+
+// The start of a context pass: cu [B + 1], hist [B], off [B] and rows [n_rows] out of mapped host memory, where they lie in that order,
+// the step counter, and the counters of sequences that begin here to zero.
+__global__ void begin_pass_kernel(const volatile int* in, int B, int n_rows, int at_step, bool first, int* step, int* __restrict__ cu, int* __restrict__ hist,
+                                  int* __restrict__ off, int* __restrict__ rows, int* __restrict__ seqlen, unsigned char* __restrict__ finished, int* __restrict__ bad)
+{
+    const int tid = threadIdx.x;
+    for (int b = tid; b <= B; b += blockDim.x) cu[b] = in[b];
+    for (int b = tid; b < B; b += blockDim.x) {
+        hist[b] = in[B + 1 + b];
+        off[b] = in[2 * B + 1 + b];
+        if (first) seqlen[b] = 0, finished[b] = 0;
+    }
+    for (int r = tid; r < n_rows; r += blockDim.x) rows[r] = in[3 * B + 1 + r];
+    if (tid == 0) *step = at_step;
+    if (first && tid < 4) bad[tid] = 0;
+}
+
 // ids[b] = prompt[b * prompt_len + (*step - 1)]; launched with a full stream dependency
 __global__ void gather_prompt_ids_kernel(const int* __restrict__ prompt, int prompt_len, const int* __restrict__ step,
                                          int* __restrict__ ids, int B)
@@ -71,9 +97,9 @@ __global__ void half_to_float_kernel(const __half* in, float* out, size_t n)
         out[i] = __half2float(in[i]);
 }
 
-// The end of a pass in one piece, so that the host needs one copy and one wait (reading every time-out flag by a copy of its own
+// The end of a pass in one piece, so that the host needs one wait and no copy (reading every time-out flag by a copy of its own
 // took 100 us of a short prompt's pass).
-__global__ void report_kernel(int* __restrict__ report, const int* __restrict__ bad, const int* __restrict__ ids, int n, const TimeoutFlags flags)
+__global__ void report_kernel(int* report, const int* __restrict__ bad, const int* __restrict__ ids, int n, const TimeoutFlags flags)
 {
     pdl_wait();
     if (threadIdx.x == 0) {
@@ -106,7 +132,6 @@ void Engine::carve_common(Carver& cv)
     d_skip = cv.take<uint32_t>(skip_table_words((int)B));
     d_cu = cv.take<int>(B + 1);
     d_hist = cv.take<int>(B);
-    d_report = cv.take<int>(4 + B);
     logits = cv.take_bytes(B * (size_t)vocab * dtype_size(logits_dtype));
 }
 
@@ -124,7 +149,11 @@ int Engine::allocate()
     ONELLM_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     ONELLM_CUDA(cudaMemsetAsync(arena, 0, arena_bytes, stream));
     ONELLM_CUDA(cudaStreamSynchronize(stream));
-    ONELLM_CUDA(cudaMallocHost(&h_report, (4 + (size_t)max_batch) * sizeof(int)));
+    const size_t B = max_batch;
+    ONELLM_CUDA(cudaHostAlloc(&mail.report, (4 + B + B + Mail::kTurns * B + 1 + 4 * B) * sizeof(int), cudaHostAllocMapped));
+    mail.out = mail.report + 4 + B;
+    mail.in = mail.out + B;
+    mail.pass = mail.in + Mail::kTurns * B;
     ONELLM_REQUIRE(timeout_flag_addresses(&timeout_flags), ONELLM_ERR_STATE, "%s: more than %d time-out flags", design(), kMaxTimeoutFlags);
     return build_skip_table(d_skip, max_batch, &skip_ok, stream);
 }
@@ -139,7 +168,7 @@ Engine::~Engine()
     if (row_logits) cudaFree(row_logits);
     if (d_rows) cudaFree(d_rows);
     if (logits_f32) cudaFree(logits_f32);
-    if (h_report) cudaFreeHost(h_report);
+    if (mail.report) cudaFreeHost(mail.report);
 }
 
 int Engine::ensure_scratch(size_t bytes)
@@ -169,7 +198,7 @@ int Engine::sample(const void* rows)
     if (top_k < 1) return ONELLM_OK;
     RC(onellm_topk(logits_dtype, rows, batch, vocab, top_k, d_topk_val, d_topk_id, 0, (void*)stream));
     return topk_sample_launch(d_topk_id, d_topk_val, batch, top_k, temperature, 0, d_step, vocab, eos_id, literal_walk, d_out_ids,
-                              d_seqlen, d_finished, d_u, d_ids, /*early_seed=*/true, skip_ok ? d_skip : nullptr, stream);
+                              d_seqlen, d_finished, d_u, d_ids, mail.out, /*early_seed=*/true, skip_ok ? d_skip : nullptr, stream);
 }
 
 // Enqueues one decode step for `batch` sequences on the stream.  `step_bound` sizes the attention grid; the real
@@ -182,7 +211,9 @@ int Engine::enqueue_step(int mode, int step_bound, int prompt_len)
     note_launch();
     (void)prefer_max_shared((const void*)advance_step_kernel);  // same L1 / shared-memory split as every kernel behind it
     (void)prefer_max_shared((const void*)gather_prompt_ids_kernel);
-    advance_step_kernel<<<1, 1, 0, stream>>>(d_step);
+    (void)prefer_max_shared((const void*)advance_with_ids_kernel);
+    if (mode & MODE_IDS) advance_with_ids_kernel<<<1, 128, 0, stream>>>(d_step, mail.in, max_batch, d_ids, batch);
+    else advance_step_kernel<<<1, 1, 0, stream>>>(d_step);
     if (mode & MODE_GATHER) {
         note_launch();
         gather_prompt_ids_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(d_prompt, prompt_len, d_step, d_ids, batch);
@@ -194,12 +225,26 @@ int Engine::enqueue_step(int mode, int step_bound, int prompt_len)
 }
 
 // Runs one step (attending cur_len + 1 rows) and advances cur_len.
-int Engine::run_step(int mode, int prompt_len)
+int Engine::run_step(int mode, int prompt_len, const int* host_ids)
 {
     const int step = cur_len + 1;
     last_logits = logits;
     ONELLM_REQUIRE(step <= max_seq_len, ONELLM_ERR_STATE, "decode: sequence length %d exceeds max_seq_len %d", step,
                    max_seq_len);
+    cudaPointerAttributes at = {};
+    if (host_ids) (void)cudaPointerGetAttributes(&at, host_ids);
+    if (host_ids && at.type != cudaMemoryTypeUnregistered) {  // pinned: read in the order of the stream
+        ONELLM_CUDA(cudaMemcpyAsync(d_ids, host_ids, (size_t)batch * sizeof(int), cudaMemcpyHostToDevice, stream));
+    } else if (host_ids) {
+        // the step kTurns positions ago read its ids from the same place
+        if (mail.unread >= Mail::kTurns - 1) {
+            ONELLM_CUDA(cudaStreamSynchronize(stream));
+            mail.unread = 0;
+        }
+        memcpy(mail.in + (size_t)(step % Mail::kTurns) * max_batch, host_ids, (size_t)batch * sizeof(int));
+        mode |= MODE_IDS;
+    }
+    mail.unread++;
     int bound = (step + 255) / 256 * 256;
     bound = std::min({bound, max_seq_len, span_cap});
     if (!use_graphs) {
@@ -250,7 +295,7 @@ int Engine::run_step(int mode, int prompt_len)
 // lens[b] new tokens of sequence b (packed in d_prompt in sequence order) behind the cur_len + seq_off[b] positions it
 // has cached: all tokens at once through the design's context kernels, then sampling from the last token of every
 // sequence.
-int Engine::prefill_context(int B, const int* lens)
+int Engine::prefill_context(int B, const int* lens, int step, bool first)
 {
     ContextBatch c;
     c.B = B;
@@ -296,11 +341,17 @@ int Engine::prefill_context(int B, const int* lens)
     c.hist = d_hist;
     c.host_hist = hist.data();
     c.rows = d_rows;
-    ONELLM_CUDA(cudaMemcpyAsync(d_step_off, off.data(), B * sizeof(int), cudaMemcpyHostToDevice, stream));
-    ONELLM_CUDA(cudaMemcpyAsync(d_cu, cu.data(), (B + 1) * sizeof(int), cudaMemcpyHostToDevice, stream));
-    ONELLM_CUDA(cudaMemcpyAsync(d_hist, hist.data(), B * sizeof(int), cudaMemcpyHostToDevice, stream));
-    ONELLM_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+    // a pass ends with a wait for the stream: nothing reads the last one's mail any more
+    int* m = std::copy(cu.begin(), cu.begin() + B + 1, mail.pass);
+    m = std::copy(hist.begin(), hist.begin() + B, m);
+    m = std::copy(off.begin(), off.begin() + B, m);
+    const int mailed = rows.size() <= (size_t)max_batch ? (int)rows.size() : 0;
+    std::copy(rows.begin(), rows.begin() + mailed, m);
+    if (!mailed) ONELLM_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
     const long before = launches_noted();
+    note_launch();
+    begin_pass_kernel<<<1, 128, 0, stream>>>(mail.pass, B, mailed, step, first, d_step, d_cu, d_hist, d_step_off, d_rows, d_seqlen, d_finished, d_bad_id);
+    ONELLM_CHECK_LAUNCH();
     RC(context_layers(c));
     RC(sample(c.logits));  // seeded with the step counter, as the position-by-position path does
     launches += launches_noted() - before;
@@ -313,16 +364,16 @@ int Engine::prefill_context(int B, const int* lens)
 int Engine::finish_context(int* host_first_ids, const char* where)
 {
     note_launch();
-    report_kernel<<<1, 64, 0, stream>>>(d_report, d_bad_id, d_out_ids, host_first_ids ? batch : 0, timeout_flags);
+    report_kernel<<<1, 64, 0, stream>>>(mail.report, d_bad_id, d_out_ids, host_first_ids ? batch : 0, timeout_flags);
     ONELLM_CHECK_LAUNCH();
-    ONELLM_CUDA(cudaMemcpyAsync(h_report, d_report, (4 + (size_t)batch) * sizeof(int), cudaMemcpyDeviceToHost, stream));
     RC(queue_comm_check());
     ONELLM_CUDA(cudaStreamSynchronize(stream));
-    if (host_first_ids) memcpy(host_first_ids, h_report + 4, (size_t)batch * sizeof(int));
+    mail.unread = 0;
+    if (host_first_ids) memcpy(host_first_ids, mail.report + 4, (size_t)batch * sizeof(int));
     RC(comm_check(where));
-    ONELLM_REQUIRE(h_report[0] == 0, ONELLM_ERR_ARG, "%s: token id outside [0, vocab_size)", where);
-    ONELLM_REQUIRE(h_report[1] == 0, ONELLM_ERR_STATE, "%s: a position beyond max_seq_len was refused by the cache", where);
-    if (h_report[2]) {
+    ONELLM_REQUIRE(mail.report[0] == 0, ONELLM_ERR_ARG, "%s: token id outside [0, vocab_size)", where);
+    ONELLM_REQUIRE(mail.report[1] == 0, ONELLM_ERR_STATE, "%s: a position beyond max_seq_len was refused by the cache", where);
+    if (mail.report[2]) {
         (void)onellm_gemm_timeout_flag();  // clears it
         ONELLM_REQUIRE(false, ONELLM_ERR_CUDA, "%s: a tensor-core GEMM block timed out", where);
     }
@@ -448,22 +499,21 @@ extern "C" int onellm_llama_prefill(onellm_llama* h, const int* host_ids, int ba
     m->graph_prompt_len = prompt_len;
     m->cur_len = 0;
     m->seq_off.assign(m->max_batch, 0);
-    ONELLM_CUDA(cudaMemsetAsync(m->d_step_off, 0, (size_t)m->max_batch * sizeof(int), st));
-    const int first_step = m->prefill_by_decode ? 0 : prompt_len;  // the step kernels increment before use
     return end_pass(m, [&]() -> int {
         ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * prompt_len * sizeof(int), cudaMemcpyHostToDevice, st));
-        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &first_step, sizeof(int), cudaMemcpyHostToDevice, st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
         if (m->prefill_by_decode) {
+            ONELLM_CUDA(cudaMemsetAsync(m->d_step_off, 0, (size_t)m->max_batch * sizeof(int), st));
+            ONELLM_CUDA(cudaMemsetAsync(m->d_step, 0, sizeof(int), st));  // the step kernels increment before use
+            ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
+            ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
+            ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
             ONELLM_REQUIRE(m->want_rows.empty(), ONELLM_ERR_STATE, "llama_prefill: logits of single rows need the context-phase kernels");
             // one position at a time through the decode kernels; only the last position needs the LM head
             for (int p = 0; p < prompt_len; p++)
                 RC(m->run_step(MODE_GATHER | (p == prompt_len - 1 ? MODE_HEAD : 0), prompt_len));
         } else {
             const std::vector<int> lens(batch, prompt_len);
-            RC(m->prefill_context(batch, lens.data()));
+            RC(m->prefill_context(batch, lens.data(), prompt_len, true));
         }
         return m->finish_context(host_first_ids, "llama_prefill");
     }());
@@ -494,11 +544,7 @@ extern "C" int onellm_llama_prefill_ragged(onellm_llama* h, const int* host_ids,
     m->seq_off.assign(m->max_batch, 0);
     return end_pass(m, [&]() -> int {
         ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, total * sizeof(int), cudaMemcpyHostToDevice, st));
-        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &longest, sizeof(int), cudaMemcpyHostToDevice, st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_seqlen, 0, (size_t)batch * sizeof(int), st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_finished, 0, (size_t)batch, st));
-        ONELLM_CUDA(cudaMemsetAsync(m->d_bad_id, 0, 4 * sizeof(int), st));
-        RC(m->prefill_context(batch, lens));
+        RC(m->prefill_context(batch, lens, longest, true));
         return m->finish_context(host_first_ids, "llama_prefill_ragged");
     }());
 }
@@ -516,9 +562,8 @@ extern "C" int onellm_llama_extend(onellm_llama* h, const int* host_ids, int n_n
     const int batch = m->batch, new_len = m->cur_len + n_new;
     return end_pass(m, [&]() -> int {
         ONELLM_CUDA(cudaMemcpyAsync(m->d_prompt, host_ids, (size_t)batch * n_new * sizeof(int), cudaMemcpyHostToDevice, st));
-        ONELLM_CUDA(cudaMemcpyAsync(m->d_step, &new_len, sizeof(int), cudaMemcpyHostToDevice, st));
         const std::vector<int> lens(batch, n_new);
-        RC(m->prefill_context(batch, lens.data()));
+        RC(m->prefill_context(batch, lens.data(), new_len, false));
         return m->finish_context(host_first_ids, "llama_extend");
     }());
 }
@@ -562,15 +607,15 @@ extern "C" int onellm_llama_decode_step(onellm_llama* h, const int* host_in_ids,
     Engine* m = engine_of(h);
     ONELLM_REQUIRE(m, ONELLM_ERR_ARG, "llama_decode_step: null handle");
     ONELLM_REQUIRE(m->batch > 0 && m->cur_len > 0, ONELLM_ERR_STATE, "llama_decode_step: call prefill first");
-    cudaStream_t st = m->stream;
-    if (host_in_ids)
-        ONELLM_CUDA(cudaMemcpyAsync(m->d_ids, host_in_ids, (size_t)m->batch * sizeof(int), cudaMemcpyHostToDevice, st));
-    RC(m->run_step(MODE_HEAD, 0));
+    RC(m->run_step(MODE_HEAD, 0, host_in_ids));
     if (host_out_ids) {
-        ONELLM_CUDA(cudaMemcpyAsync(m->h_report, m->d_out_ids, (size_t)m->batch * sizeof(int), cudaMemcpyDeviceToHost, st));
+        // nothing is sampled with top_k 0: the ids of the last step that sampled
+        if (m->top_k < 1)
+            ONELLM_CUDA(cudaMemcpyAsync(m->mail.out, m->d_out_ids, (size_t)m->batch * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
         RC(m->queue_comm_check());
-        ONELLM_CUDA(cudaStreamSynchronize(st));
-        memcpy(host_out_ids, m->h_report, (size_t)m->batch * sizeof(int));
+        ONELLM_CUDA(cudaStreamSynchronize(m->stream));
+        m->mail.unread = 0;
+        memcpy(host_out_ids, m->mail.out, (size_t)m->batch * sizeof(int));
         RC(m->comm_check("llama_decode_step"));
     }
     return ONELLM_OK;

@@ -28,7 +28,21 @@ struct Carver {
     void* take_bytes(size_t n) { return take<char>(n); }
 };
 
-enum StepMode { MODE_GATHER = 1, MODE_HEAD = 2 };
+enum StepMode { MODE_GATHER = 1, MODE_HEAD = 2, MODE_IDS = 4 };  // ids out of the prompt; logits; ids from the host
+
+// What host and device hand each other besides tensors, in mapped host memory (one pinned allocation per engine): kernels that a step or a
+// pass launches anyway read and write it.  As copies and fills of their own, one behind the other around the kernels, they took 30 us of
+// a context pass (ten of them) and 10 us of a decode step that is given its ids and waited for.  Measured, us: eight
+// steps of one sequence through four layers of width 2048, 1831 -> 1791; three ragged prompts of 238 tokens through four 7B layers, 891 -> 881;
+// prompts and 16 steps of the two other designs, two layers of width 4096, 5822 -> 5755 and 5680 -> 5590.
+struct Mail {
+    static constexpr int kTurns = 64;
+    int *report = nullptr;  // end of a context pass: bad ids [2], a bounded wait gave up, -, ids [max_batch]
+    int *out = nullptr;     // [max_batch] ids sampled last
+    int *in = nullptr;      // [kTurns][max_batch] ids for the step to position p at p % kTurns
+    int *pass = nullptr;    // start of a context pass, see begin_pass_kernel
+    int unread = 0;         // steps enqueued since the stream was last waited for
+};
 
 // One context pass: T new tokens of B sequences, packed in sequence order in Engine::d_prompt.
 struct ContextBatch {
@@ -69,10 +83,9 @@ struct Engine {
     size_t row_cap = 0, row_have = 0;
     const void* last_logits = nullptr;
     float* logits_f32 = nullptr;   // [max_batch, vocab], made by the first call that asks for 16-bit logits
-    // what the host reads at the end of a pass: bad_id [2], whether a bounded wait gave up, sampled ids [max_batch]
-    int *d_report = nullptr, *h_report = nullptr;  // h_report: pinned
+    Mail mail;
     TimeoutFlags timeout_flags = {};
-    // what the copies of a context pass read: kept until the next pass, which begins after the stream has been waited for
+    // of a context pass; the rows are read by a copy and kept until the next pass, which begins after the stream has been waited for
     std::vector<int> h_off, h_cu, h_hist, h_rows;
     // state
     int batch = 0, cur_len = 0, graph_prompt_len = 0;
@@ -110,8 +123,9 @@ struct Engine {
     // ---- the generation loop
     int sample(const void* row_logits);
     int enqueue_step(int mode, int step_bound, int prompt_len);
-    int run_step(int mode, int prompt_len);
-    int prefill_context(int B, const int* lens);
+    int run_step(int mode, int prompt_len, const int* host_ids = nullptr);  // host_ids: the step's input ids, else the ones sampled last
+    // step: what the step counter is to be; first: the sequences begin with this pass
+    int prefill_context(int B, const int* lens, int step, bool first);
     int finish_context(int* host_first_ids, const char* where);
     int copy_logits(size_t first, size_t rows, float* host_logits);
 
@@ -135,7 +149,7 @@ size_t skip_table_words(int rows);  // sampling.cu
 int build_skip_table(uint32_t* table, int rows, int* usable, cudaStream_t st);
 int topk_sample_launch(const int* topk_id, const float* topk_val, int B, int K, float temperature, int rng_step,
                        const int* rng_step_dev, int vocab_size, int end_id, int literal_walk, int* output_id,
-                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, bool early_seed,
+                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id, bool early_seed,
                        const uint32_t* skip_table, cudaStream_t st);
 int embedding_launch(int dtype, const int* ids, void* out, void* out2, const void* table, int n_tokens, int hidden,
                      int vocab, int* bad_id_flag, bool pdl, cudaStream_t st);

@@ -451,7 +451,7 @@ __global__ void sample_kernel(const int* __restrict__ topk_id, const float* __re
                               float temperature, int rng_step, const int* __restrict__ rng_step_dev,
                               int vocab_size, int end_id, int literal_walk, int* __restrict__ output_id, int* __restrict__ seqlen,
                               unsigned char* __restrict__ finished, float* __restrict__ u_out,
-                              int* __restrict__ output_id2, int early_seed, const uint32_t* __restrict__ skip_tab)
+                              int* __restrict__ output_id2, int* host_id, int early_seed, const uint32_t* __restrict__ skip_tab)
 {
     pdl_launch_dependents();
     const int b = blockIdx.x;
@@ -492,6 +492,7 @@ __global__ void sample_kernel(const int* __restrict__ topk_id, const float* __re
     const int id = topk_id[(size_t)b * K + pick] % vocab_size;
     output_id[b] = id;
     if (output_id2) output_id2[b] = id;
+    if (host_id) host_id[b] = id;
     if (seqlen && finished) {
         seqlen[b] = finished[b] ? seqlen[b] : seqlen[b] + 1;
         finished[b] = (id == end_id) ? 1 : 0;
@@ -526,10 +527,10 @@ extern "C" int onellm_topk(int dtype, const void* logits, int rows, int vocab, i
 
 namespace onellm {
 // Shared by the C entry point and the model driver; output_id2 (may be NULL) gets a second
-// copy of the sampled ids (the next step's input buffer).
+// copy of the sampled ids (the next step's input buffer), host_id (likewise) one in mapped host memory.
 int topk_sample_launch(const int* topk_id, const float* topk_val, int B, int K, float temperature, int rng_step,
                        const int* rng_step_dev, int vocab_size, int end_id, int literal_walk, int* output_id,
-                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, bool early_seed,
+                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id, bool early_seed,
                        const uint32_t* skip_table, cudaStream_t st)
 {
     ONELLM_REQUIRE(topk_id && topk_val && output_id, ONELLM_ERR_ARG, "topk_sample: null pointer");
@@ -540,7 +541,7 @@ int topk_sample_launch(const int* topk_id, const float* topk_val, int B, int K, 
     if (B == 0) return ONELLM_OK;
     ONELLM_CUDA(launch_pdl(sample_kernel, dim3(B), dim3(32), 0, st, topk_id, topk_val, K, temperature, rng_step,
                            rng_step_dev, vocab_size, end_id, literal_walk, output_id, seqlen, finished, u_out,
-                           output_id2, early_seed ? 1 : 0, skip_table));
+                           output_id2, host_id, early_seed ? 1 : 0, skip_table));
     return ONELLM_OK;
 }
 
@@ -577,6 +578,6 @@ extern "C" int onellm_topk_sample(const int* topk_id, const float* topk_val, int
                                   float* u_out, void* stream)
 {
     return topk_sample_launch(topk_id, topk_val, B, K, temperature, rng_step, rng_step_dev, vocab_size, end_id,
-                              literal_walk, output_id, seqlen, finished, u_out, nullptr, /*early_seed=*/false,
+                              literal_walk, output_id, seqlen, finished, u_out, nullptr, nullptr, /*early_seed=*/false,
                               /*skip_table=*/nullptr, reinterpret_cast<cudaStream_t>(stream));
 }
