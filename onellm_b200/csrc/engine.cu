@@ -35,13 +35,14 @@ __global__ void begin_pass_kernel(const volatile int* in, int B, int n_rows, int
                                   int* __restrict__ off, int* __restrict__ rows, int* __restrict__ seqlen, unsigned char* __restrict__ finished, int* __restrict__ bad)
 {
     const int tid = threadIdx.x;
-    for (int b = tid; b <= B; b += blockDim.x) cu[b] = in[b];
-    for (int b = tid; b < B; b += blockDim.x) {
-        hist[b] = in[B + 1 + b];
-        off[b] = in[2 * B + 1 + b];
-        if (first) seqlen[b] = 0, finished[b] = 0;
+    for (int i = tid; i < 3 * B + 1 + n_rows; i += blockDim.x) {  // one trip to the host and back, not one a table (4 us)
+        const int v = in[i];
+        if (i <= B) cu[i] = v;
+        else if (i <= 2 * B) hist[i - B - 1] = v;
+        else if (i <= 3 * B) off[i - 2 * B - 1] = v;
+        else rows[i - 3 * B - 1] = v;
     }
-    for (int r = tid; r < n_rows; r += blockDim.x) rows[r] = in[3 * B + 1 + r];
+    for (int b = tid; first && b < B; b += blockDim.x) seqlen[b] = 0, finished[b] = 0;
     if (tid == 0) *step = at_step;
     if (first && tid < 4) bad[tid] = 0;
 }
@@ -196,9 +197,8 @@ void Engine::drop_graphs()
 int Engine::sample(const void* rows)
 {
     if (top_k < 1) return ONELLM_OK;
-    RC(onellm_topk(logits_dtype, rows, batch, vocab, top_k, d_topk_val, d_topk_id, 0, (void*)stream));
-    return topk_sample_launch(d_topk_id, d_topk_val, batch, top_k, temperature, 0, d_step, vocab, eos_id, literal_walk, d_out_ids,
-                              d_seqlen, d_finished, d_u, d_ids, mail.out, /*early_seed=*/true, skip_ok ? d_skip : nullptr, stream);
+    return sample_logits(logits_dtype, rows, batch, vocab, top_k, d_topk_val, d_topk_id, temperature, d_step, eos_id, literal_walk, d_out_ids, d_seqlen,
+                         d_finished, d_u, d_ids, mail.out, skip_ok ? d_skip : nullptr, stream);
 }
 
 // Enqueues one decode step for `batch` sequences on the stream.  `step_bound` sizes the attention grid; the real

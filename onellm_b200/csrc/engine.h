@@ -147,10 +147,9 @@ struct ModelRegistration {
 // ---- kernels and launchers of other files --------------------------------------------------------------------
 size_t skip_table_words(int rows);  // sampling.cu
 int build_skip_table(uint32_t* table, int rows, int* usable, cudaStream_t st);
-int topk_sample_launch(const int* topk_id, const float* topk_val, int B, int K, float temperature, int rng_step,
-                       const int* rng_step_dev, int vocab_size, int end_id, int literal_walk, int* output_id,
-                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id, bool early_seed,
-                       const uint32_t* skip_table, cudaStream_t st);
+int sample_logits(int dtype, const void* logits, int B, int vocab, int K, float* topk_val, int* topk_id, float temperature, const int* step, int end_id,
+                  int literal_walk, int* output_id, int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id,
+                  const uint32_t* skip_table, cudaStream_t st);
 int embedding_launch(int dtype, const int* ids, void* out, void* out2, const void* table, int n_tokens, int hidden,
                      int vocab, int* bad_id_flag, bool pdl, cudaStream_t st);
 // w[i] = mean + std * N(0,1) of element type dtype, counter-based (seed, tensor tag, index); see engine.cu

@@ -6,13 +6,16 @@
 // SamplingKernel (src/kernels/topK_sampling.cu:6-41) with the same cuRAND call sequence.
 //
 // One thread block per row, over an order-preserving integer image of the logits (NaN lowest).  Rows of up to
-// 32768 logits (topk_reg_kernel) are read once, 32 consecutive keys per thread in registers: the K-th largest of
-// the per-thread maxima bounds the K-th largest key from below, the few keys that reach it are gathered and ranked
+// 32768 logits (topk_reg_kernel) are read once, 32 keys per thread in registers: the K-th largest of
+// the maxima of groups of keys bounds the K-th largest key from below, the few keys that reach it are gathered and ranked
 // against each other; rows with long runs of equal keys fall back to a bisection over all keys.  Neither step
 // uses a histogram: logits share their leading bits, and a 256-bin histogram in shared memory serialises on a
 // handful of bins.  Longer rows (topk_kernel) are a radix select, 8 bits per pass, re-reading the logits from L2.
 #include <curand_kernel.h>
 #include <math.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -175,200 +178,6 @@ __device__ __forceinline__ float key_value<__half>(uint32_t k)
     return __half2float(__ushort_as_half((unsigned short)u));
 }
 
-constexpr int kTopkPer = 32;  // keys per thread held in registers
-constexpr int kTopkCand = 512;  // gathered keys the short way ranks; >= kMaxK
-
-template <typename T>
-__global__ void __launch_bounds__(kTopkThreads)
-topk_reg_kernel(const T* __restrict__ logits, int vocab, int K, float* __restrict__ out_val, int* __restrict__ out_id,
-                int global_ids)
-{
-    pdl_launch_dependents();
-    pdl_wait();
-    const int row = blockIdx.x;
-    const T* x = logits + (size_t)row * vocab;
-    __shared__ int s_count;
-    __shared__ int warp_tot[kTopkThreads / 32];
-    __shared__ uint32_t cand_key[kTopkCand];
-    __shared__ int cand_id[kTopkCand];
-
-    // thread t owns columns [t*32, t*32 + 32): a contiguous slice, so ranks inside a tie follow the columns
-    const int c0 = threadIdx.x * kTopkPer;
-    const int n_mine = max(0, min(kTopkPer, vocab - c0));
-    uint32_t key[kTopkPer];
-    constexpr int VEC = 16 / sizeof(T);
-    if (n_mine == kTopkPer && ((reinterpret_cast<uintptr_t>(x + c0) & 15u) == 0)) {
-#pragma unroll
-        for (int j = 0; j < kTopkPer; j += VEC) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(x + c0 + j);
-            const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-            for (int q = 0; q < VEC; q++) key[j + q] = logit_key<T>(e[q]);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kTopkPer; j++) key[j] = j < n_mine ? logit_key<T>(x[c0 + j]) : 0u;
-    }
-    if (threadIdx.x == 0) s_count = 0;
-    __syncthreads();
-
-    constexpr int kLowBit = sizeof(T) == 2 ? 16 : 0;  // fp16 keys live in the upper half
-    __shared__ int bit_tot[2][kTopkThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int it = 0;
-
-    // 0. The short way, which nearly every row of logits takes.  The K-th largest of the 1024 per-thread maxima is
-    // a lower bound of the K-th largest key (K threads hold a key that large), and for logits hardly more than K
-    // keys reach it.  A bisection over ONE key per thread finds it (a ballot per warp, one block barrier per bit);
-    // the keys that reach it are gathered (a few dozen shared-memory atomics) and ranked against each other, larger
-    // key first, lower column first among equals: rank r < K is output slot r.  Rows with many equal keys, where
-    // the gathered set would be large, take the bisection over all keys below instead.
-    {
-        uint32_t mk = 0u;  // padding and NaN have key 0
-#pragma unroll
-        for (int j = 0; j < kTopkPer; j++) mk = max(mk, key[j]);
-        // The K-th largest of the 32 warp maxima is such a bound too: two barriers instead of one per bit.  It is lower: of W warps with
-        // columns in any order the keys of W ln(W / (W - K)) threads reach it, 12 of 32 warps at K = 10, 22 at 16, above which nothing is
-        // tried.  Where many more do, or the gathered keys find no room (the large logits side by side in few warps), the bisection
-        // follows.  8 x 32000, us, the bisection alone | both: K = 5 8.9 | 6.2, K = 16 9.7 | 7.3, sorted rows 17.7 | 17.4.
-        for (int way = 2 * K <= (vocab + 32 * kTopkPer - 1) / (32 * kTopkPer) ? 0 : 1; way < 2; way++) {
-            uint32_t low = 0u;
-            if (way == 0) {
-                const uint32_t wm = __reduce_max_sync(0xffffffffu, mk);
-                if (lane == 0) warp_tot[wid] = (int)wm;
-                __syncthreads();
-                const uint32_t v = (uint32_t)warp_tot[lane];
-                int r = 0;
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const uint32_t u = __shfl_sync(0xffffffffu, v, j);
-                    r += u > v || (u == v && j < lane);
-                }
-                low = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, r == K - 1)) - 1);
-                if (__syncthreads_count(mk >= low) > 64) continue;
-            } else {
-#pragma unroll 1
-                for (int bit = 31; bit >= kLowBit; bit--, it++) {
-                    const uint32_t t = low | (1u << bit);
-                    const int c = __popc(__ballot_sync(0xffffffffu, mk >= t));
-                    if (lane == 0) bit_tot[it & 1][wid] = c;
-                    __syncthreads();
-                    if (__reduce_add_sync(0xffffffffu, bit_tot[it & 1][lane]) >= K) low = t;
-                }
-            }
-            if (mk >= low) {
-#pragma unroll
-                for (int j = 0; j < kTopkPer; j++) {
-                    if (j < n_mine && key[j] >= low) {
-                        const int pos = atomicAdd(&s_count, 1);
-                        if (pos < kTopkCand) {
-                            cand_key[pos] = key[j];
-                            cand_id[pos] = c0 + j;
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            const int n_c = s_count;  // >= K: K threads hold a real key >= low (or low == 0 and every column counts)
-            if (n_c <= kTopkCand) {
-                if ((int)threadIdx.x < n_c) {
-                    const uint32_t k = cand_key[threadIdx.x];
-                    const int id = cand_id[threadIdx.x];
-                    int r = 0;
-                    for (int j = 0; j < n_c; j++) r += (cand_key[j] > k) || (cand_key[j] == k && cand_id[j] < id);
-                    if (r < K) {
-                        out_val[(size_t)row * K + r] = (k == 0u) ? -INFINITY : key_value<T>(k);
-                        out_id[(size_t)row * K + r] = global_ids ? row * vocab + id : id;
-                    }
-                }
-                return;
-            }
-            __syncthreads();  // everyone has read s_count
-            if (threadIdx.x == 0) s_count = 0;
-            __syncthreads();
-        }
-    }
-
-    // 1. K-th largest key by bisection on its bits, from the top: the largest t with at least K keys >= t.  Every thread
-    // counts its 32 keys in registers, a warp adds up with one reduction, the 32 warp sums meet in shared memory (two
-    // buffers in turn: one block barrier per bit) and every thread takes the same decision, so nothing is broadcast
-    // and no shared-memory atomic is used (a 256-bin histogram of logits has a handful of hot bins: the radix form
-    // of this step spent most of its 39 us waiting for them).
-    auto block_count = [&](auto pred, int buf) {
-        int c = 0;
-#pragma unroll
-        for (int j = 0; j < kTopkPer; j++) c += (j < n_mine && pred(key[j])) ? 1 : 0;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (lane == 0) bit_tot[buf][wid] = c;
-        __syncthreads();
-        return __reduce_add_sync(0xffffffffu, bit_tot[buf][lane]);
-    };
-    uint32_t kth = 0u;
-#pragma unroll 1
-    for (int bit = 31; bit >= kLowBit; bit--, it++) {
-        const uint32_t t = kth | (1u << bit);
-        if (block_count([t](uint32_t k) { return k >= t; }, it & 1) >= K) kth = t;
-    }
-    const int need_ties = K - block_count([kth](uint32_t k) { return k > kth; }, it & 1);
-
-    // 2. gather: everything above the K-th key (any order), then the lowest-indexed ties
-    int ties = 0;
-#pragma unroll
-    for (int j = 0; j < kTopkPer; j++) {
-        if (j < n_mine && key[j] > kth) {
-            const int pos = atomicAdd(&s_count, 1);
-            cand_key[pos] = key[j];
-            cand_id[pos] = c0 + j;
-        }
-        ties += (j < n_mine && key[j] == kth);
-    }
-    __syncthreads();
-    const int n_above = s_count;  // == K - need_ties
-    {
-        int incl = ties;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((threadIdx.x & 31) >= o) incl += v;
-        }
-        if ((threadIdx.x & 31) == 31) warp_tot[threadIdx.x >> 5] = incl;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            const int v = warp_tot[threadIdx.x];
-            int inc = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, inc, o);
-                if ((int)threadIdx.x >= o) inc += u;
-            }
-            warp_tot[threadIdx.x] = inc - v;  // exclusive
-        }
-        __syncthreads();
-        int rank = warp_tot[threadIdx.x >> 5] + incl - ties;
-        if (ties > 0 && rank < need_ties) {
-#pragma unroll
-            for (int j = 0; j < kTopkPer; j++) {
-                if (j < n_mine && key[j] == kth && rank < need_ties) {
-                    cand_key[n_above + rank] = kth;
-                    cand_id[n_above + rank] = c0 + j;
-                    rank++;
-                }
-            }
-        }
-    }
-    __syncthreads();
-
-    // 3. rank sort: larger key first, lower column first among equals
-    if (threadIdx.x < K) {
-        const uint32_t k = cand_key[threadIdx.x];
-        const int id = cand_id[threadIdx.x];
-        int r = 0;
-        for (int j = 0; j < K; j++) r += (cand_key[j] > k) || (cand_key[j] == k && cand_id[j] < id);
-        out_val[(size_t)row * K + r] = (k == 0u) ? -INFINITY : key_value<T>(k);
-        out_id[(size_t)row * K + r] = global_ids ? row * vocab + id : id;
-    }
-}
-
 // The draw of (step, row) is curand_init(step, row, 0) + curand_uniform, as src/kernels/topK_sampling.cu:29-30 of the
 // reference takes it.  For row > 0 nearly all of its time is the skip-ahead to sub-sequence `row`: a linear map
 // (over GF(2)) of the 160 xorshift bits of the XORWOW state, which cuRAND applies bit by bit in one thread, 10-15 us
@@ -447,56 +256,330 @@ __global__ void skip_table_check_kernel(const uint32_t* __restrict__ tab, int* _
     }
 }
 
-__global__ void sample_kernel(const int* __restrict__ topk_id, const float* __restrict__ topk_val, int K,
-                              float temperature, int rng_step, const int* __restrict__ rng_step_dev,
-                              int vocab_size, int end_id, int literal_walk, int* __restrict__ output_id, int* __restrict__ seqlen,
-                              unsigned char* __restrict__ finished, float* __restrict__ u_out,
-                              int* __restrict__ output_id2, int* host_id, int early_seed, const uint32_t* __restrict__ skip_tab)
+// What a draw of step and row decides and where that goes
+struct SampleTo {
+    float temperature;
+    const int* step;  // device
+    int vocab, end_id, literal_walk;
+    int *id, *id2, *host_id;  // id2 and host_id may be null
+    int* seqlen;              // with finished, or both null
+    unsigned char* finished;
+    float* u;  // may be null
+    const uint32_t* skip_tab;
+};
+
+// Whole warp; the result is valid in lane 0.
+__device__ __noinline__ float draw_of(int seed, int b, const uint32_t* tab)
+{
+    float u = 0.f;
+    if (tab) {
+        u = draw_with_table(seed, b, tab);
+    } else if ((threadIdx.x & 31) == 0) {
+        curandState_t state;
+        curand_init((unsigned long long)seed, (unsigned long long)b, 0ULL, &state);
+        u = curand_uniform(&state);
+    }
+    return u;
+}
+
+// One thread; weight(i): the i-th candidate's
+template <typename W>
+__device__ __forceinline__ int walk(int K, float u, int literal_walk, W weight)
+{
+    float sum = 0.f;
+    for (int i = 0; i < K; i++) sum += weight(i);
+    float thr = u * sum;
+    for (int i = 0; i < K; i++) {
+        thr -= literal_walk ? 1.0f : weight(i);
+        if (thr < 0.f) return i;
+    }
+    return K - 1;
+}
+
+__device__ __forceinline__ void sampled(const SampleTo& to, int b, int id, float u)
+{
+    to.id[b] = id;
+    if (to.u) to.u[b] = u;
+    if (to.id2) to.id2[b] = id;
+    if (to.host_id) to.host_id[b] = id;
+    if (to.seqlen && to.finished) {
+        to.seqlen[b] = to.finished[b] ? to.seqlen[b] : to.seqlen[b] + 1;
+        to.finished[b] = (id == to.end_id) ? 1 : 0;
+    }
+}
+
+constexpr int kTopkPer = 32;  // keys per thread held in registers
+constexpr int kTopkCand = 512;  // gathered keys the short way ranks; >= kMaxK
+
+// SAMPLE: and the sampling from them.  What bounds it is the chain of one block's barriers behind the logits, most of a step's LM head being
+// hidden: the draw is taken before the logits are there, the weights of the candidates are computed side by side.  A launch less:
+// with the loads below, prompts and 16 steps of float logits (K = 1) 5755 -> 5650 and 5590 -> 5480 us.
+template <typename T, bool SAMPLE>
+__global__ void __launch_bounds__(kTopkThreads)
+topk_reg_kernel(const T* __restrict__ logits, int vocab, int K, float* __restrict__ out_val, int* __restrict__ out_id,
+                int global_ids, const SampleTo to)
+{
+    constexpr int VEC = 16 / sizeof(T);
+    pdl_launch_dependents();
+    const int row = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __shared__ int s_count;
+    __shared__ int warp_tot[kTopkThreads / 32];
+    __shared__ uint32_t cand_key[kTopkCand];
+    __shared__ int cand_id[kTopkCand];
+    __shared__ float best_val[SAMPLE ? kMaxK : 1];
+    __shared__ int best_id[SAMPLE ? kMaxK : 1];
+    // The step counter was written by work that completed long before: it is advanced by the first kernel of a step, and the layer
+    // projections between it and this kernel release their dependents only after passing their own griddepcontrol.wait.
+    float u = 0.f;
+    if (SAMPLE && wid == 0) u = draw_of(*to.step, row, to.skip_tab);
+    pdl_wait();
+    const T* x = logits + (size_t)row * vocab;
+
+    // A warp reads 512 bytes side by side.  32 columns side by side in a thread make a load of floats one of 32 cache lines: 32000 columns,
+    // K = 1, us, then | now: float 10.3 | 4.8, half 5.7 | 5.7.
+    auto col_of = [](int j) { return ((j / VEC) * kTopkThreads + (int)threadIdx.x) * VEC + j % VEC; };
+    uint32_t key[kTopkPer];
+    if (vocab % VEC == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+#pragma unroll
+        for (int j = 0; j < kTopkPer; j += VEC) {
+            uint4 raw = make_uint4(~0u, ~0u, ~0u, ~0u);  // NaN: key 0
+            if (col_of(j) < vocab) raw = *reinterpret_cast<const uint4*>(x + col_of(j));
+            const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+            for (int q = 0; q < VEC; q++) key[j + q] = logit_key<T>(e[q]);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kTopkPer; j++) key[j] = col_of(j) < vocab ? logit_key<T>(x[col_of(j)]) : 0u;
+    }
+    if (threadIdx.x == 0) s_count = 0;
+    __syncthreads();
+
+    constexpr int kLowBit = sizeof(T) == 2 ? 16 : 0;  // fp16 keys live in the upper half
+    __shared__ int bit_tot[2][kTopkThreads / 32];
+    __shared__ __align__(16) uint32_t maxima[kTopkThreads];
+    __shared__ uint32_t s_low;
+    int it = 0;
+    bool done = false;
+
+    auto put = [&](int r, uint32_t k, int id) {
+        const float v = (k == 0u) ? -INFINITY : key_value<T>(k);
+        out_val[(size_t)row * K + r] = v;
+        out_id[(size_t)row * K + r] = global_ids ? row * vocab + id : id;
+        if constexpr (SAMPLE) best_val[r] = v, best_id[r] = id;
+    };
+
+    // 0. The short way, which nearly every row of logits takes.  The K-th largest of the maxima of groups of keys is a lower bound of the
+    // K-th largest key (K groups hold a key that large), and for logits hardly more than K keys reach it: of G groups of columns in any
+    // order the keys of G ln(G / (G - K)) threads.  The groups are, up to K = 16, the 32 warps, whose maxima every warp ranks (22 threads
+    // at K = 16); above, eight lanes each, 63 threads at K = 50, and one warp bisects their 128 maxima.  The keys that reach the bound
+    // are gathered (a few dozen shared-memory atomics) and ranked against each other, larger key first, lower column first among
+    // equals: rank r < K is output slot r.  Where many more do (the large logits side by side in few groups) or the row is
+    // short, the bound comes from the maxima of all threads; rows with many equal keys, where that gathers too many as well, take the
+    // bisection over all keys below.  8 x 32000, us, with the bound of all threads and
+    // a barrier a bit | now: K = 50 half 10.1 | 9.8, float 17.3 | 10.0; sorted rows 29.5 | 31.1, 48.5 | 21.1; three values 28.2 | 27.6, 47.1 | 40.1.
+    {
+        uint32_t mk = 0u;  // padding and NaN have key 0
+#pragma unroll
+        for (int j = 0; j < kTopkPer; j++) mk = max(mk, key[j]);
+        auto filled = [&](int lanes) { return min(kTopkThreads, (vocab + VEC - 1) / VEC) / lanes; };  // whole groups of so many lanes
+        auto bisect = [&](auto n) {  // one warp: the K-th largest of 128 n maxima
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(maxima + 4 * lane);
+            uint32_t lo = 0u;
+#pragma unroll 1
+            for (int bit = 31; bit >= kLowBit; bit--) {
+                const uint32_t t = lo | (1u << bit);
+                int c = 0, d = 0;
+#pragma unroll
+                for (int i = 0; i < decltype(n)::value; i++) {
+                    uint4 m;  // again for every bit: there are no registers to keep them in
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(m.x), "=r"(m.y), "=r"(m.z), "=r"(m.w) : "r"(at + i * 512) : "memory");
+                    c += (m.x >= t) + (m.y >= t);
+                    d += (m.z >= t) + (m.w >= t);
+                }
+                if ((int)__reduce_add_sync(0xffffffffu, c + d) >= K) lo = t;
+            }
+            return lo;
+        };
+        for (int way = 2 * K <= filled(32) ? 0 : 2 * K <= filled(8) ? 1 : 2; way < 3 && !done; way = way < 2 ? 2 : 3) {
+            uint32_t low = 0u;
+            if (way == 0) {
+                const uint32_t wm = __reduce_max_sync(0xffffffffu, mk);
+                if (lane == 0) maxima[wid] = wm;
+                __syncthreads();
+                const uint32_t v = maxima[lane];
+                int r = 0;
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    const uint32_t u = __shfl_sync(0xffffffffu, v, j);
+                    r += u > v || (u == v && j < lane);
+                }
+                low = __shfl_sync(0xffffffffu, v, __ffs(__ballot_sync(0xffffffffu, r == K - 1)) - 1);
+            } else {
+                uint32_t gm = mk;
+                if (way == 1) {
+                    gm = max(gm, __shfl_xor_sync(0xffffffffu, gm, 1));
+                    gm = max(gm, __shfl_xor_sync(0xffffffffu, gm, 2));
+                    gm = max(gm, __shfl_xor_sync(0xffffffffu, gm, 4));
+                }
+                if (way == 2) maxima[threadIdx.x] = gm;
+                else if ((lane & 7) == 0) maxima[threadIdx.x / 8] = gm;
+                __syncthreads();
+                if (wid == 0) {
+                    low = way == 1 ? bisect(std::integral_constant<int, 1>{}) : bisect(std::integral_constant<int, kTopkThreads / 128>{});
+                    if (lane == 0) s_low = low;
+                }
+                __syncthreads();
+                low = s_low;
+            }
+            // twice what columns in any order lead to, and more
+            if (way < 2 && __syncthreads_count(mk >= low) > (way == 0 ? 64 : 160)) continue;
+            low = max(low, 1u);  // 0: NaN, or no column
+            if (mk >= low) {
+#pragma unroll
+                for (int j = 0; j < kTopkPer; j++) {
+                    if (key[j] >= low) {
+                        const int pos = atomicAdd(&s_count, 1);
+                        if (pos < kTopkCand) {
+                            cand_key[pos] = key[j];
+                            cand_id[pos] = col_of(j);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            const int n_c = s_count;  // >= K where K threads hold a key above 0
+            if (n_c >= K && n_c <= kTopkCand) {
+                if ((int)threadIdx.x < n_c) {
+                    const uint32_t k = cand_key[threadIdx.x];
+                    const int id = cand_id[threadIdx.x];
+                    int r = 0;
+                    for (int j = 0; j < n_c; j++) r += (cand_key[j] > k) || (cand_key[j] == k && cand_id[j] < id);
+                    if (r < K) put(r, k, id);
+                }
+                done = true;
+                break;
+            }
+            __syncthreads();  // everyone has read s_count
+            if (threadIdx.x == 0) s_count = 0;
+            __syncthreads();
+        }
+    }
+
+    if (!done) {
+        // 1. K-th largest key by bisection on its bits, from the top: the largest t with at least K keys >= t.  Every thread
+        // counts its 32 keys in registers, a warp adds up with one reduction, the 32 warp sums meet in shared memory (two
+        // buffers in turn: one block barrier per bit) and every thread takes the same decision, so nothing is broadcast
+        // and no shared-memory atomic is used (a 256-bin histogram of logits has a handful of hot bins: the radix form
+        // of this step spent most of its 39 us waiting for them).
+        auto block_count = [&](auto pred) {
+            int c = 0;
+#pragma unroll
+            for (int j = 0; j < kTopkPer; j++) c += pred(key[j]) ? 1 : 0;
+            c = __reduce_add_sync(0xffffffffu, c);
+            int* tot = bit_tot[it++ & 1];
+            if (lane == 0) tot[wid] = c;
+            __syncthreads();
+            return (int)__reduce_add_sync(0xffffffffu, tot[lane]);
+        };
+        uint32_t kth = 0u;
+#pragma unroll 1
+        for (int bit = 31; bit >= kLowBit; bit--) {
+            const uint32_t t = kth | (1u << bit);
+            if (block_count([t](uint32_t k) { return k >= t; }) >= K) kth = t;
+        }
+        const bool all_ties = block_count([kth](uint32_t k) { return k >= kth; }) == K;  // kth == 0: the places without a column count too
+
+        // 2. gather: everything above the K-th key (any order), and its ties where all of them count
+#pragma unroll
+        for (int j = 0; j < kTopkPer; j++) {
+            if (key[j] > kth || (all_ties && key[j] == kth)) {
+                const int pos = atomicAdd(&s_count, 1);
+                cand_key[pos] = key[j];
+                cand_id[pos] = col_of(j);
+            }
+        }
+        __syncthreads();
+        // else the lowest-indexed ties: a thread's VEC columns, then the threads, then the groups of columns follow each other
+        int n = s_count;
+#pragma unroll
+        for (int g = 0; g < kTopkPer / VEC; g++) {
+            if (n < K) {
+                int ties = 0;
+#pragma unroll
+                for (int q = 0; q < VEC; q++) ties += key[g * VEC + q] == kth && col_of(g * VEC + q) < vocab;
+                int incl = ties;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (lane == 31) warp_tot[wid] = incl;
+                __syncthreads();
+                const int before = __reduce_add_sync(0xffffffffu, lane < wid ? warp_tot[lane] : 0);
+                const int all = __reduce_add_sync(0xffffffffu, warp_tot[lane]);
+                int at = n + before + incl - ties;
+#pragma unroll
+                for (int q = 0; q < VEC; q++) {
+                    if (key[g * VEC + q] == kth && col_of(g * VEC + q) < vocab) {
+                        if (at < K) {
+                            cand_key[at] = kth;
+                            cand_id[at] = col_of(g * VEC + q);
+                        }
+                        at++;
+                    }
+                }
+                n += all;
+                __syncthreads();
+            }
+        }
+
+        // 3. rank sort: larger key first, lower column first among equals
+        if (threadIdx.x < K) {
+            const uint32_t k = cand_key[threadIdx.x];
+            const int id = cand_id[threadIdx.x];
+            int r = 0;
+            for (int j = 0; j < K; j++) r += (cand_key[j] > k) || (cand_key[j] == k && cand_id[j] < id);
+            put(r, k, id);
+        }
+    }
+
+    if constexpr (SAMPLE) {
+        __syncthreads();
+        if (wid > 0) return;
+        float* weight = reinterpret_cast<float*>(cand_key);
+        for (int i = lane; i < K; i += 32) weight[i] = expf((best_val[i] - best_val[0]) / to.temperature);
+        __syncwarp();
+        if (lane == 0) sampled(to, row, best_id[walk(K, u, to.literal_walk, [&](int i) { return weight[i]; })] % to.vocab, u);
+    }
+}
+
+__global__ void sample_kernel(const int* __restrict__ topk_id, const float* __restrict__ topk_val, int K, int rng_step, const SampleTo to, int early_seed)
 {
     pdl_launch_dependents();
     const int b = blockIdx.x;
     // The draw depends on (step, row) only, and seeding the generator (a sequence skip-ahead) is by far
     // the longest part of this kernel.  early_seed: do it before waiting for the candidates; the caller
-    // vouches that *rng_step_dev was written by work that completed long before (the model's step
-    // counter is advanced by the first kernel of a step, and the layer projections between it and this
-    // kernel release their dependents only after passing their own griddepcontrol.wait).
+    // vouches that *to.step was written by work that completed long before (see topk_reg_kernel).
     float u = 0.f;
-    auto draw = [&]() {  // whole warp (blockDim.x == 32); u is valid in thread 0
-        const int seed = rng_step_dev ? *rng_step_dev : rng_step;
-        if (skip_tab) {
-            u = draw_with_table(seed, b, skip_tab);
-        } else if (threadIdx.x == 0) {
-            curandState_t state;
-            curand_init((unsigned long long)seed, (unsigned long long)b, 0ULL, &state);
-            u = curand_uniform(&state);
-        }
-    };
+    auto draw = [&]() { u = draw_of(to.step ? *to.step : rng_step, b, to.skip_tab); };
     if (early_seed) draw();
     pdl_wait();
     if (!early_seed) draw();
     if (threadIdx.x != 0) return;
     const float* v = topk_val + (size_t)b * K;
     const float v0 = v[0];
-    float sum = 0.f;
-    for (int i = 0; i < K; i++) sum += expf((v[i] - v0) / temperature);
-    if (u_out) u_out[b] = u;
-    float thr = u * sum;
-    int pick = K - 1;
-    for (int i = 0; i < K; i++) {
-        thr -= literal_walk ? 1.0f : expf((v[i] - v0) / temperature);
-        if (thr < 0.f) {
-            pick = i;
-            break;
-        }
-    }
-    const int id = topk_id[(size_t)b * K + pick] % vocab_size;
-    output_id[b] = id;
-    if (output_id2) output_id2[b] = id;
-    if (host_id) host_id[b] = id;
-    if (seqlen && finished) {
-        seqlen[b] = finished[b] ? seqlen[b] : seqlen[b] + 1;
-        finished[b] = (id == end_id) ? 1 : 0;
-    }
+    const int pick = walk(K, u, to.literal_walk, [&](int i) { return expf((v[i] - v0) / to.temperature); });
+    sampled(to, b, topk_id[(size_t)b * K + pick] % to.vocab, u);
+}
+
+// Rows that topk_reg_kernel takes
+template <typename T, bool SAMPLE>
+static int topk_launch(const void* logits, int rows, int vocab, int K, float* out_val, int* out_id, int global_ids, const SampleTo& to, cudaStream_t st)
+{
+    ONELLM_CUDA(launch_pdl(topk_reg_kernel<T, SAMPLE>, dim3(rows), dim3(kTopkThreads), 0, st, (const T*)logits, vocab, K, out_val, out_id, global_ids, to));
+    ONELLM_CHECK_LAUNCH();
+    return ONELLM_OK;
 }
 
 }  // namespace onellm
@@ -512,37 +595,44 @@ extern "C" int onellm_topk(int dtype, const void* logits, int rows, int vocab, i
                    kMaxK);
     if (rows == 0) return ONELLM_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const bool in_regs = vocab <= kTopkPer * kTopkThreads;
+    ONELLM_REQUIRE(dtype == ONELLM_F16 || dtype == ONELLM_F32, ONELLM_ERR_UNSUPPORTED, "topk: dtype %d", dtype);
+    if (vocab <= kTopkPer * kTopkThreads)
+        return dtype == ONELLM_F16 ? topk_launch<__half, false>(logits, rows, vocab, K, out_val, out_id, global_ids, SampleTo{}, st)
+                                   : topk_launch<float, false>(logits, rows, vocab, K, out_val, out_id, global_ids, SampleTo{}, st);
     if (dtype == ONELLM_F16)
-        ONELLM_CUDA(launch_pdl(in_regs ? topk_reg_kernel<__half> : topk_kernel<__half>, dim3(rows), dim3(kTopkThreads), 0, st,
-                               (const __half*)logits, vocab, K, out_val, out_id, global_ids));
-    else if (dtype == ONELLM_F32)
-        ONELLM_CUDA(launch_pdl(in_regs ? topk_reg_kernel<float> : topk_kernel<float>, dim3(rows), dim3(kTopkThreads), 0, st,
-                               (const float*)logits, vocab, K, out_val, out_id, global_ids));
+        ONELLM_CUDA(launch_pdl(topk_kernel<__half>, dim3(rows), dim3(kTopkThreads), 0, st, (const __half*)logits, vocab, K, out_val, out_id, global_ids));
     else
-        ONELLM_REQUIRE(false, ONELLM_ERR_UNSUPPORTED, "topk: dtype %d", dtype);
+        ONELLM_CUDA(launch_pdl(topk_kernel<float>, dim3(rows), dim3(kTopkThreads), 0, st, (const float*)logits, vocab, K, out_val, out_id, global_ids));
     ONELLM_CHECK_LAUNCH();
     return ONELLM_OK;
 }
 
 namespace onellm {
-// Shared by the C entry point and the model driver; output_id2 (may be NULL) gets a second
-// copy of the sampled ids (the next step's input buffer), host_id (likewise) one in mapped host memory.
-int topk_sample_launch(const int* topk_id, const float* topk_val, int B, int K, float temperature, int rng_step,
-                       const int* rng_step_dev, int vocab_size, int end_id, int literal_walk, int* output_id,
-                       int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id, bool early_seed,
-                       const uint32_t* skip_table, cudaStream_t st)
+static int sample_launch(const int* topk_id, const float* topk_val, int B, int K, int rng_step, const SampleTo& to, bool early_seed, cudaStream_t st)
 {
-    ONELLM_REQUIRE(topk_id && topk_val && output_id, ONELLM_ERR_ARG, "topk_sample: null pointer");
-    ONELLM_REQUIRE(B >= 0 && K >= 1 && vocab_size > 0 && temperature > 0.f, ONELLM_ERR_ARG,
+    ONELLM_REQUIRE(topk_id && topk_val && to.id, ONELLM_ERR_ARG, "topk_sample: null pointer");
+    ONELLM_REQUIRE(B >= 0 && K >= 1 && to.vocab > 0 && to.temperature > 0.f, ONELLM_ERR_ARG,
                    "topk_sample: bad size or temperature");
-    ONELLM_REQUIRE((seqlen == nullptr) == (finished == nullptr), ONELLM_ERR_ARG,
+    ONELLM_REQUIRE((to.seqlen == nullptr) == (to.finished == nullptr), ONELLM_ERR_ARG,
                    "topk_sample: seqlen and finished must be given together");
     if (B == 0) return ONELLM_OK;
-    ONELLM_CUDA(launch_pdl(sample_kernel, dim3(B), dim3(32), 0, st, topk_id, topk_val, K, temperature, rng_step,
-                           rng_step_dev, vocab_size, end_id, literal_walk, output_id, seqlen, finished, u_out,
-                           output_id2, host_id, early_seed ? 1 : 0, skip_table));
+    ONELLM_CUDA(launch_pdl(sample_kernel, dim3(B), dim3(32), 0, st, topk_id, topk_val, K, rng_step, to, early_seed ? 1 : 0));
     return ONELLM_OK;
+}
+
+// The model driver's top-K and sampling of B rows of logits, in one launch where a row fits a block's registers.  output_id2 gets a
+// second copy of the sampled ids (the next step's input buffer), host_id one in mapped host memory.
+int sample_logits(int dtype, const void* logits, int B, int vocab, int K, float* topk_val, int* topk_id, float temperature, const int* step, int end_id,
+                  int literal_walk, int* output_id, int* seqlen, unsigned char* finished, float* u_out, int* output_id2, int* host_id,
+                  const uint32_t* skip_table, cudaStream_t st)
+{
+    const SampleTo to = {temperature, step, vocab, end_id, literal_walk, output_id, output_id2, host_id, seqlen, finished, u_out, skip_table};
+    if (vocab > kTopkPer * kTopkThreads || K < 1 || K > std::min(kMaxK, vocab) || (dtype != ONELLM_F16 && dtype != ONELLM_F32)) {
+        const int rc = onellm_topk(dtype, logits, B, vocab, K, topk_val, topk_id, 0, (void*)st);
+        return rc != ONELLM_OK ? rc : sample_launch(topk_id, topk_val, B, K, 0, to, /*early_seed=*/true, st);
+    }
+    return dtype == ONELLM_F16 ? topk_launch<__half, true>(logits, B, vocab, K, topk_val, topk_id, 0, to, st)
+                               : topk_launch<float, true>(logits, B, vocab, K, topk_val, topk_id, 0, to, st);
 }
 
 // Words a skip table for `rows` rows takes.
@@ -577,7 +667,6 @@ extern "C" int onellm_topk_sample(const int* topk_id, const float* topk_val, int
                                   int literal_walk, int* output_id, int* seqlen, unsigned char* finished,
                                   float* u_out, void* stream)
 {
-    return topk_sample_launch(topk_id, topk_val, B, K, temperature, rng_step, rng_step_dev, vocab_size, end_id,
-                              literal_walk, output_id, seqlen, finished, u_out, nullptr, nullptr, /*early_seed=*/false,
-                              /*skip_table=*/nullptr, reinterpret_cast<cudaStream_t>(stream));
+    const SampleTo to = {temperature, rng_step_dev, vocab_size, end_id, literal_walk, output_id, nullptr, nullptr, seqlen, finished, u_out, nullptr};
+    return sample_launch(topk_id, topk_val, B, K, rng_step, to, /*early_seed=*/false, reinterpret_cast<cudaStream_t>(stream));
 }
