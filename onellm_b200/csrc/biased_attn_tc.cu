@@ -4,15 +4,19 @@
 //
 // The schedule is the one of context_attn_tc_kernel (context_attn_tc.cu): a block owns 128 query rows of one
 // (sequence, head) and walks the cache in 64-row tiles; S = Q.K^T and O += P.V by tcgen05.mma with S, P and O in tensor
-// memory, four softmax warps with one query row per thread, a fifth warp that issues TMA loads and MMAs.  What differs:
+// memory, four softmax warps with one query row per thread, a warp that issues the MMAs, one that issues the loads.  What differs:
 //   - sizes are run-time numbers of 64-column chunks (key chunks in Q and K, value chunks in V and O; a size that is not
 //     a multiple of 64 is zero-filled by TMA and by the threads that write Q);
 //   - the scores of a row are turned into log2 units by the factor of its position and lose the penalty of their
-//     distance before the maximum is taken.  A tile of scores spans 191 distances: the threads read the table of the
-//     head directly, consecutive rows at consecutive addresses;
+//     distance before the maximum is taken.  A warp's rows and a tile's keys span 95 distances, which it copies to shared memory a
+//     tile ahead (read from the table by every thread, at addresses that are not aligned, they took 500 cycles of a tile);
 //   - WINDOWED: keys and values of all heads lie beside each other in one buffer that a sequence's rows are packed into, so
 //     a head is a range of columns; the tiles of a block start at the first key its first query sees, masks apply on both
 //     sides, a row may see nothing in its block's first tiles, and the output takes the gate of its token and head.
+// What bounds it is the chain of a tile in a softmax warp, 2000 cycles with another block on the SM and 1600 without penalties: maximum 560
+// (80), exponentials 700, conversions, waits and stores the rest.  The chunks of a key are a template argument: with a loop over them
+// the MMAs of a tile's scores took 750 cycles to issue.  Measured, us, one warp for loads and MMAs and the rest as said | now: 2000 tokens,
+// 16 heads of 128 and 128, 64 | 49; two prompts of 1030, window 512, 33 | 24.
 // Every mbarrier wait is bounded; on expiry the block raises the time-out flag, stops, frees its tensor memory and
 // returns.
 #include <math.h>
@@ -24,7 +28,8 @@ namespace onellm {
 
 constexpr int kBaQ = 128, kBaKV = 64;
 constexpr int kBaSoftmaxThreads = 128;
-constexpr int kBaThreads = kBaSoftmaxThreads + 32;
+constexpr int kBaThreads = kBaSoftmaxThreads + 64;
+constexpr int kBaPen = 96;                // penalties a warp reads for a tile: 32 rows less 64 keys are 95 distances
 constexpr int kBaQChunk = kBaQ * 128;    // 16 KB: 128 rows x 64 columns
 constexpr int kBaKVChunk = kBaKV * 128;  // 8 KB: 64 rows x 64 columns
 constexpr uint32_t kBaO = 128;           // tensor-memory column of O; S0 at 0, S1 at 64
@@ -48,25 +53,27 @@ __device__ __forceinline__ void ba_umma_ta(uint32_t tmem_d, uint32_t tmem_a, uin
         : "memory");
 }
 
-template <bool WINDOWED>
+template <bool WINDOWED, int KCH>  // KCH: p.kch
 __global__ void __launch_bounds__(kBaThreads, 2)
 biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v)
 {
     typedef __nv_bfloat16 bf16;
     extern __shared__ __align__(1024) unsigned char smem_raw[];  // the 128-byte swizzle works on shared-window address bits
-    const int kch = p.kch, vch = p.vch;
+    constexpr int kch = KCH;
+    const int vch = p.vch;
     const int k_tile = kch * kBaKVChunk, v_tile = vch * kBaKVChunk;
     unsigned char* sQ = smem_raw;
     unsigned char* sK = sQ + kch * kBaQChunk;  // two buffers
     unsigned char* sV = sK + 2 * k_tile;       // two buffers
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * v_tile);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    float* s_pen = reinterpret_cast<float*>(bars + 32);  // [4 warps][2][kBaPen]
     // per-tile barriers come in pairs: tile j uses slot j & 1, phase (j >> 1) & 1, so that a producer two tiles ahead
     // of a waiter cannot be taken for the tile waited for
     const uint32_t q_full = smem_u32(bars), k_full0 = smem_u32(bars + 1), s_full0 = smem_u32(bars + 3), v_full0 = smem_u32(bars + 5),
                    p_full0 = smem_u32(bars + 7), o_full0 = smem_u32(bars + 9);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.z, h = blockIdx.y, hk = h / (p.a.H / p.a.G);
+    const int b = blockIdx.y, h = blockIdx.x, hk = h / (p.a.H / p.a.G);
 
     if (smem_u32(smem_raw) & 1023u) {  // the tiles would be read with the wrong swizzle
         if (threadIdx.x == 0) atomicExch(&g_tc_timeout_flag, 1);
@@ -95,7 +102,7 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
     pdl_launch_dependents();
     pdl_wait();
     const int tok0 = p.cu[b], q_len = p.cu[b + 1] - tok0, hist = p.hist[b];
-    const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kBaQ;  // the blocks with the most cache tiles first
+    const int q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * kBaQ;  // of all heads the blocks with the most cache tiles first
     const bool active = q0 < q_len && (WINDOWED || hist + q_len <= p.a.S);
     const int q_rows = active ? min(kBaQ, q_len - q0) : 0;
     const int kv_end = hist + q0 + q_rows;
@@ -111,72 +118,74 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
         v_col = p.a.H * p.a.dk + h * p.a.dv;
     }
 
-    if (warp == 4 && active) {
-        // ---- control: the whole warp runs this code, one elected lane issues (warp-uniform control flow keeps the
-        // operands of the MMAs in uniform registers)
+    if (warp >= 4 && active) {
+        // ---- the whole warp runs this code, one elected lane issues (warp-uniform control flow keeps the operands in uniform registers)
         uint32_t leader;
         asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(leader));
         bool ok = true;
-        auto load = [&](const CUtensorMap* map, unsigned char* base, int tile_bytes, int chunks, uint32_t full0, int j, int col) {
-            const int s = j & 1;
-            if (leader) {
-                mbar_expect_tx(full0 + 8 * s, tile_bytes);
-                for (int c = 0; c < chunks; c++)
-                    tma_load_2d(smem_u32(base + s * tile_bytes + c * kBaKVChunk), map, col + 64 * c, cache_row0 + j * kBaKV, full0 + 8 * s);
+        if (warp == 5) {  // loads: K of tile j + 2 when the scores of tile j are there, V when its product is
+            auto load = [&](const CUtensorMap* map, unsigned char* base, int tile_bytes, int chunks, uint32_t full0, int j, int col) {
+                const int s = j & 1;
+                if (leader) {
+                    mbar_expect_tx(full0 + 8 * s, tile_bytes);
+                    for (int c = 0; c < chunks; c++)
+                        tma_load_2d(smem_u32(base + s * tile_bytes + c * kBaKVChunk), map, col + 64 * c, cache_row0 + j * kBaKV, full0 + 8 * s);
+                }
+                __syncwarp();
+            };
+            int n_k = 0, n_v = 0;
+            for (int j = 0; j < n_tiles && ok; j++) {
+                if (j >= 2) ok = mbar_wait_warp(s_full0 + 8 * (j & 1), (uint32_t)((j - 2) >> 1) & 1u);
+                if (!ok) break;
+                load(&map_k, sK, k_tile, kch, k_full0, n_k++, k_col);
+                if (j >= 2) ok = mbar_wait_warp(o_full0 + 8 * (j & 1), (uint32_t)((j - 2) >> 1) & 1u);
+                if (!ok) break;
+                load(&map_v, sV, v_tile, vch, v_full0, n_v++, v_col);
             }
-        };
-        auto load_k = [&](int j) { load(&map_k, sK, k_tile, kch, k_full0, j, k_col); };
-        auto load_v = [&](int j) { load(&map_v, sV, v_tile, vch, v_full0, j, v_col); };
-        auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
-        const uint32_t types = (1u << 4) | umma_operand_bits<bf16>() | ((uint32_t)(kBaQ >> 4) << 24);
-        const uint32_t idesc_s = types | ((uint32_t)(kBaKV >> 3) << 17);
-        const uint32_t idesc_o = types | (1u << 16) | ((uint32_t)(vch * 8) << 17);
-        const uint64_t dq = umma_desc(smem_u32(sQ), 16, 1024), dk = umma_desc(smem_u32(sK), 16, 1024),
-                       dv = umma_desc(smem_u32(sV), kBaKVChunk, 1024);
-        auto issue_s = [&](int j) {  // S_j = Q . K_j^T into accumulator j & 1
-            const int s = j & 1;
-            if (!wait_all(k_full0 + 8 * s, (uint32_t)(j >> 1) & 1u)) return false;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t dks = dk + (uint64_t)((s * k_tile) >> 4);
-            const uint32_t acc = tmem_base + (uint32_t)(s * kBaKV);
-            if (leader) {
-                for (int c = 0; c < kch; c++)
+            if (!ok) {
+                ring_drain(k_full0, 2, n_k);
+                ring_drain(v_full0, 2, n_v);
+            }
+        } else {  // MMAs
+            const uint32_t types = (1u << 4) | umma_operand_bits<bf16>() | ((uint32_t)(kBaQ >> 4) << 24);
+            const uint32_t idesc_s = types | ((uint32_t)(kBaKV >> 3) << 17);
+            const uint32_t idesc_o = types | (1u << 16) | ((uint32_t)(vch * 8) << 17);
+            const uint64_t dq = umma_desc(smem_u32(sQ), 16, 1024), dk = umma_desc(smem_u32(sK), 16, 1024),
+                           dv = umma_desc(smem_u32(sV), kBaKVChunk, 1024);
+            auto issue_s = [&](int j) {  // S_j = Q . K_j^T into accumulator j & 1
+                const int s = j & 1;
+                if (!mbar_wait_warp(k_full0 + 8 * s, (uint32_t)(j >> 1) & 1u)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dks = dk + (uint64_t)((s * k_tile) >> 4);
+                const uint32_t acc = tmem_base + (uint32_t)(s * kBaKV);
+                if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; kk++)
-                        umma_f16(acc, dq + (uint64_t)((c * kBaQChunk + kk * 32) >> 4), dks + (uint64_t)((c * kBaKVChunk + kk * 32) >> 4), idesc_s,
-                                 (c | kk) ? 1u : 0u);
-                umma_commit(s_full0 + 8 * s);
-            }
-            __syncwarp();
-            return true;
-        };
-        load_k(0);
-        load_v(0);
-        if (n_tiles > 1) {
-            load_k(1);
-            load_v(1);
-        }
-        ok = wait_all(q_full, 0) && issue_s(0);
-        for (int j = 0; j < n_tiles && ok; j++) {
-            const int s = j & 1;
-            if (j + 1 < n_tiles) ok = issue_s(j + 1);
-            ok = ok && wait_all(s_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);  // K buffer s is free
-            if (ok && j + 2 < n_tiles) load_k(j + 2);
-            ok = ok && wait_all(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && wait_all(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t dvs = dv + (uint64_t)((s * v_tile) >> 4);
-            if (leader) {
+                    for (int kk = 0; kk < kch * 4; kk++)
+                        umma_f16(acc, dq + (uint64_t)(((kk >> 2) * kBaQChunk + (kk & 3) * 32) >> 4),
+                                 dks + (uint64_t)(((kk >> 2) * kBaKVChunk + (kk & 3) * 32) >> 4), idesc_s, kk > 0 ? 1u : 0u);
+                    umma_commit(s_full0 + 8 * s);
+                }
+                __syncwarp();
+                return true;
+            };
+            ok = mbar_wait_warp(q_full, 0) && issue_s(0);
+            for (int j = 0; j < n_tiles && ok; j++) {
+                const int s = j & 1;
+                // the next tile's scores while the softmax warps work on this one: their accumulator was last read for tile j - 1, whose P
+                // has been waited for, by the product issued before them
+                if (j + 1 < n_tiles) ok = issue_s(j + 1);
+                ok = ok && mbar_wait_warp(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && mbar_wait_warp(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dvs = dv + (uint64_t)((s * v_tile) >> 4);
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kBaKV / 16; kk++)
-                    ba_umma_ta(tmem_base + kBaO, tmem_base + (uint32_t)(s * kBaKV + kk * 8), dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
-                               (j > 0 || kk > 0) ? 1u : 0u);
-                umma_commit(o_full0 + 8 * s);
-            }
-            __syncwarp();
-            if (j + 2 < n_tiles) {
-                ok = wait_all(o_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);  // V buffer s is free again
-                if (ok) load_v(j + 2);
+                    for (int kk = 0; kk < kBaKV / 16; kk++)
+                        ba_umma_ta(tmem_base + kBaO, tmem_base + (uint32_t)(s * kBaKV + kk * 8), dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
+                                   (j > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit(o_full0 + 8 * s);
+                }
+                __syncwarp();
             }
         }
     } else if (warp < 4 && active) {
@@ -186,34 +195,51 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
         const bool row_ok = r < q_rows;
         const uint32_t t_lane = tmem_base + ((uint32_t)(warp * 32) << 16);
         const uint32_t t_o = t_lane + kBaO;
-        const uint32_t row_off = (r >> 3) * 1024 + (r & 7) * 128;
+        auto row_off = [](int row) { return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128); };
         const float factor = WINDOWED ? p.scale_log2 : row_ok ? p.a.q_factor[pos] : 0.f;
+        // the penalties of a warp's rows and a tile's keys, by falling distance of key 0: a copy of its own per warp, two tiles in turn
         const float* pen = WINDOWED ? nullptr : p.a.penalty + (size_t)h * p.a.S;
+        float* my_pen = s_pen + warp * 2 * kBaPen;
+        float ahead[3];
+        auto fetch = [&](int kv0) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) ahead[i] = __ldg(pen + min(max(hist + q0 + warp * 32 - kv0 - 63 + 32 * i + lane, 0), p.a.S - 1));
+        };
+        if (!WINDOWED) fetch(key0);
         const int pos_c = row_ok ? pos : hist + q0;  // rows behind the end of the sequence read the penalties of its first row
         float m_ref = -INFINITY, l_run = 0.f;
         bool ok = true;
         {
-            const bf16* qrow = reinterpret_cast<const bf16*>(p.a.q) + (size_t)(tok0 + q0 + (row_ok ? r : 0)) * p.a.ld + (size_t)h * p.a.dk;
-            for (int u = 0; u < kch * 8; u++) {
-                const uint4 v = (row_ok && u * 8 < p.a.dk) ? *reinterpret_cast<const uint4*>(qrow + u * 8) : make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4*>(sQ + (u >> 3) * kBaQChunk + row_off + (((u & 7) ^ (r & 7)) << 4)) = v;
+            // a row's columns side by side in a warp (a row per thread touches 32 cache lines a load: the first tile 2 us later)
+            const bf16* q = reinterpret_cast<const bf16*>(p.a.q) + (size_t)(tok0 + q0) * p.a.ld + (size_t)h * p.a.dk;
+#pragma unroll
+            for (int i = 0; i < kch * 8; i++) {
+                const int row = (i * kBaSoftmaxThreads + r) / (kch * 8), u = (i * kBaSoftmaxThreads + r) % (kch * 8);
+                const uint4 v = (row < q_rows && u * 8 < p.a.dk) ? *reinterpret_cast<const uint4*>(q + (size_t)row * p.a.ld + u * 8) : make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(sQ + (u >> 3) * kBaQChunk + row_off(row) + (((u & 7) ^ (row & 7)) << 4)) = v;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(q_full);
         }
         for (int j = 0; j < n_tiles && ok; j++) {
+            const int kv0 = key0 + j * kBaKV;
+            if (!WINDOWED) {
+#pragma unroll
+                for (int i = 0; i < 3; i++) my_pen[(j & 1) * kBaPen + 32 * i + lane] = ahead[i];
+                __syncwarp();
+                fetch(kv0 + kBaKV);
+            }
             ok = mbar_wait(s_full0 + 8 * (j & 1), (uint32_t)(j >> 1) & 1u);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int kv0 = key0 + j * kBaKV;
             const bool need_mask = kv0 + kBaKV - 1 > hist + q0 || (WINDOWED && kv0 <= hist + q0 + q_rows - 1 - p.window);
             uint32_t sv[64];
             tmem_ld32(t_lane + (uint32_t)((j & 1) * kBaKV), *reinterpret_cast<uint32_t(*)[32]>(&sv[0]));
             tmem_ld32(t_lane + (uint32_t)((j & 1) * kBaKV + 32), *reinterpret_cast<uint32_t(*)[32]>(&sv[32]));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-            const float* pd = pen + (pos_c - kv0);  // penalty of the tile's first key; key i: pd[-i]
+            const float* pd = my_pen + (j & 1) * kBaPen + 63 + lane;  // penalty of the tile's first key; key i: pd[-i]
             if constexpr (WINDOWED) {
                 if (need_mask) {
                     const int last = pos_c - kv0, before = last - p.window;  // visible: before < i <= last
@@ -227,14 +253,14 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
 #pragma unroll
                 for (int i = 0; i < 64; i++) {
                     float s = -INFINITY;
-                    if (kv0 + i <= pos_c) s = fmaf(__uint_as_float(sv[i]), factor, -__ldg(pd - i));
+                    if (kv0 + i <= pos_c) s = fmaf(__uint_as_float(sv[i]), factor, -pd[-i]);
                     sv[i] = __float_as_uint(s);
                     mx4[i & 3] = fmaxf(mx4[i & 3], s);
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < 64; i++) {
-                    const float s = fmaf(__uint_as_float(sv[i]), factor, -__ldg(pd - i));
+                    const float s = fmaf(__uint_as_float(sv[i]), factor, -pd[-i]);
                     sv[i] = __float_as_uint(s);
                     mx4[i & 3] = fmaxf(mx4[i & 3], s);
                 }
@@ -286,7 +312,7 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
                 if (!ok) break;
                 if (r < kBaKV && kv0 + r >= kv_end)
                     for (int u = 0; u < vch * 8; u++)
-                        *reinterpret_cast<uint4*>(sV + (j & 1) * v_tile + (u >> 3) * kBaKVChunk + row_off + (u & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        *reinterpret_cast<uint4*>(sV + (j & 1) * v_tile + (u >> 3) * kBaKVChunk + row_off(r) + (u & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -327,14 +353,23 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
 
 static const TimeoutFlag timeout_flag(tc_flag_read_clear, tc_flag_address);
 
+template <bool WINDOWED, int KCH>
+static int ba_launch(const BaParams& p, int B, int max_new, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t st)
+{
+    const int smem = p.kch * kBaQChunk + 2 * (p.kch + p.vch) * kBaKVChunk + 256 + (WINDOWED ? 0 : 4 * 2 * kBaPen * (int)sizeof(float));
+    static DeviceOnce attr;
+    ONELLM_CUDA(attr.run([] { return cudaFuncSetAttribute(biased_attn_tc_kernel<WINDOWED, KCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }));
+    ONELLM_CUDA(launch_pdl(biased_attn_tc_kernel<WINDOWED, KCH>, dim3(p.a.H, B, (max_new + kBaQ - 1) / kBaQ), dim3(kBaThreads), smem, st, p, map_k, map_v));
+    return ONELLM_OK;
+}
+
 template <bool WINDOWED>
 static int ba_launch(const BaParams& p, int B, int max_new, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t st)
 {
-    const int smem = p.kch * kBaQChunk + 2 * (p.kch + p.vch) * kBaKVChunk + 256;
-    static DeviceOnce attr;
-    ONELLM_CUDA(attr.run([] { return cudaFuncSetAttribute(biased_attn_tc_kernel<WINDOWED>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }));
-    ONELLM_CUDA(launch_pdl(biased_attn_tc_kernel<WINDOWED>, dim3((max_new + kBaQ - 1) / kBaQ, p.a.H, B), dim3(kBaThreads), smem, st, p, map_k, map_v));
-    return ONELLM_OK;
+    return p.kch == 1   ? ba_launch<WINDOWED, 1>(p, B, max_new, map_k, map_v, st)
+           : p.kch == 2 ? ba_launch<WINDOWED, 2>(p, B, max_new, map_k, map_v, st)
+           : p.kch == 3 ? ba_launch<WINDOWED, 3>(p, B, max_new, map_k, map_v, st)
+                        : ba_launch<WINDOWED, 4>(p, B, max_new, map_k, map_v, st);
 }
 
 int biased_attn_tc_launch(const BiasedAttn& a, const TokenPositions& tp, int max_new, cudaStream_t st)

@@ -19,7 +19,11 @@
 //                         2^8), and only then does a thread wait for the previous product and rescale O in place.
 // The MMAs of one thread run in issue order, which is what lets S of tile j + 2 overwrite the accumulator P of tile j
 // was read from without a wait in between.
-// A fifth warp issues the TMA loads (K and V tiles double-buffered) and the MMAs.  96 KB of shared memory and 256
+// A fifth warp issues the MMAs and a sixth the TMA loads (K and V tiles double-buffered).  With both in one warp the product of a tile
+// was waited for, to reuse its V buffer, before the scores of the next but one were issued: a tile took the warp 3000 cycles, where
+// the softmax warps need 1600.  The blocks with the most tiles start first, of all heads and sequences; head by head, the last
+// ones left most SMs idle for up to 30 tiles.  Prompts of 2040 and 1777 tokens, 32 heads, us: 121, with the sixth warp 103, in this
+// order 86.  96 KB of shared memory and 256
 // columns of tensor memory per block: two blocks share an SM, so one block's start-up and drain hide under the
 // other's steady state.  Every mbarrier wait is bounded; on expiry the block raises the time-out flag, stops, frees
 // its tensor memory and returns.
@@ -31,7 +35,7 @@ namespace onellm {
 
 constexpr int kAtQ = 128, kAtKV = 64, kAtD = 128;
 constexpr int kAtSoftmaxThreads = 128;              // one query row per thread
-constexpr int kAtThreads = kAtSoftmaxThreads + 32;  // + one control warp (TMA and MMA issue)
+constexpr int kAtThreads = kAtSoftmaxThreads + 64;  // + a warp that issues the MMAs and one that issues the loads
 constexpr int kAtQTile = kAtQ * kAtD * 2;           // 32 KB: two 64-column chunks of [128 rows x 128 bytes]
 constexpr int kAtQChunk = kAtQTile / 2;
 constexpr int kAtKVTile = kAtKV * kAtD * 2;         // 16 KB: two 64-column chunks of [64 rows x 128 bytes]
@@ -72,7 +76,7 @@ context_attn_tc_kernel(const __half* __restrict__ q, long q_ld, const __grid_con
     const uint32_t q_full = smem_u32(bars), k_full0 = smem_u32(bars + 1), s_full0 = smem_u32(bars + 3), v_full0 = smem_u32(bars + 5),
                    p_full0 = smem_u32(bars + 7), o_full0 = smem_u32(bars + 9);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.z, h = blockIdx.y, hk = h / (H / Hkv);
+    const int b = blockIdx.y, h = blockIdx.x, hk = h / (H / Hkv);
 
     if (smem_u32(smem_raw) & 1023u) {  // never seen; the tiles would be read with the wrong swizzle
         if (threadIdx.x == 0) atomicExch(&g_tc_timeout_flag, 1);
@@ -101,100 +105,94 @@ context_attn_tc_kernel(const __half* __restrict__ q, long q_ld, const __grid_con
     pdl_launch_dependents();
     pdl_wait();  // q and the cache rows come from the kernel before this one
     const int tok0 = cu_seqlens[b], q_len = cu_seqlens[b + 1] - tok0, hist = history[b];
-    // the blocks with the most cache tiles first: the last query rows of a sequence
-    const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kAtQ;
+    // the blocks with the most cache tiles first: the last query rows of every sequence and head
+    const int q0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * kAtQ;
     const bool active = q0 < q_len;  // uniform over the block
     const int q_rows = active ? min(kAtQ, q_len - q0) : 0;
     const int kv_end = hist + q0 + q_rows;  // rows any query of this block may attend
     const int n_tiles = active ? (kv_end + kAtKV - 1) / kAtKV : 0;
     const int cache_row0 = (b * Hkv + hk) * S_max;
 
-    if (warp == 4 && active) {
-        // ---- control: TMA loads and MMA issue.  The whole warp runs this code and one elected lane issues the
+    if (warp >= 4 && active) {
+        // ---- TMA loads and MMA issue.  The whole warp runs this code and one elected lane issues the
         // single-thread instructions: with warp-uniform control flow the descriptors and addresses stay in uniform
         // registers, which is where tcgen05.mma takes them from (under a divergent `lane == 0` branch every operand
         // of every MMA was moved there one by one, ~100 cycles per instruction).
         uint32_t leader;
         asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(leader));
         bool ok = true;
-        auto load_k = [&](int j) {
-            const int s = j & 1;
-            if (leader) {
-                mbar_expect_tx(k_full0 + 8 * s, kAtKVTile);
+        if (warp == 5) {  // loads: K of tile j + 2 when the scores of tile j are there, V when its product is
+            auto load = [&](const CUtensorMap* map, unsigned char* base, uint32_t full0, int j) {
+                const int s = j & 1;
+                if (leader) {
+                    mbar_expect_tx(full0 + 8 * s, kAtKVTile);
 #pragma unroll
-                for (int c = 0; c < 2; c++)
-                    tma_load_2d(smem_u32(sK + s * kAtKVTile + c * kAtKVChunk), &map_k, 64 * c, cache_row0 + j * kAtKV, k_full0 + 8 * s);
-            }
-        };
-        auto load_v = [&](int j) {
-            const int s = j & 1;
-            if (leader) {
-                mbar_expect_tx(v_full0 + 8 * s, kAtKVTile);
-#pragma unroll
-                for (int c = 0; c < 2; c++)
-                    tma_load_2d(smem_u32(sV + s * kAtKVTile + c * kAtKVChunk), &map_v, 64 * c, cache_row0 + j * kAtKV, v_full0 + 8 * s);
-            }
-        };
-        auto wait_all = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
-        // instruction descriptors: D = f32, A = B = f16, M = 128; S: N = 64, B K-major; O: N = 128, B MN-major
-        const uint32_t idesc_s = (1u << 4) | (0u << 16) | ((uint32_t)(kAtKV >> 3) << 17) | ((uint32_t)(kAtQ >> 4) << 24);
-        const uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(kAtD >> 3) << 17) | ((uint32_t)(kAtQ >> 4) << 24);
-        // Shared-memory descriptors are built once; a step inside a tile only adds (bytes >> 4) to the address field in
-        // the low word (the field holds any shared-memory address, so the add never carries out of it).
-        const uint64_t dq = umma_desc(smem_u32(sQ), 16, 1024), dk = umma_desc(smem_u32(sK), 16, 1024),
-                       dv = umma_desc(smem_u32(sV), kAtKVChunk, 1024);
-        auto issue_s = [&](int j) {  // S_j = Q . K_j^T into accumulator j & 1
-            const int s = j & 1;
-            if (!wait_all(k_full0 + 8 * s, (uint32_t)(j >> 1) & 1u)) return false;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t dks = dk + (uint64_t)(s * (kAtKVTile >> 4));
-            const uint32_t acc = tmem_base + (uint32_t)(s * kAtKV);
-            if (leader) {
-#pragma unroll
-                for (int kk = 0; kk < kAtD / 16; kk++) {
-                    // both K-major: 64-column chunk kk/4, 32 bytes per 16 k inside the 128-byte row, 8-row groups 1024 bytes apart
-                    umma_f16(acc, dq + (uint64_t)(((kk >> 2) * kAtQChunk + (kk & 3) * 32) >> 4),
-                             dks + (uint64_t)(((kk >> 2) * kAtKVChunk + (kk & 3) * 32) >> 4), idesc_s, kk > 0 ? 1u : 0u);
+                    for (int c = 0; c < 2; c++)
+                        tma_load_2d(smem_u32(base + s * kAtKVTile + c * kAtKVChunk), map, 64 * c, cache_row0 + j * kAtKV, full0 + 8 * s);
                 }
-                umma_commit(s_full0 + 8 * s);
+                __syncwarp();
+            };
+            int n_k = 0, n_v = 0;
+            for (int j = 0; j < n_tiles; j++) {
+                if (j >= 2) ok = mbar_wait_warp(s_full0 + 8 * (j & 1), (uint32_t)((j - 2) >> 1) & 1u);
+                if (!ok) break;
+                load(&map_k, sK, k_full0, n_k++);
+                if (j >= 2) ok = mbar_wait_warp(o_full0 + 8 * (j & 1), (uint32_t)((j - 2) >> 1) & 1u);
+                if (!ok) break;
+                load(&map_v, sV, v_full0, n_v++);
             }
-            __syncwarp();
-            return true;
-        };
-        load_k(0);
-        load_v(0);
-        if (n_tiles > 1) {
-            load_k(1);
-            load_v(1);
-        }
-        ok = wait_all(q_full, 0) && issue_s(0);
-        for (int j = 0; j < n_tiles && ok; j++) {
-            const int s = j & 1;
-            // the next tile's scores while the softmax warps work on this one (its accumulator was last read for
-            // tile j - 1, whose P has been waited for in the previous round)
-            if (j + 1 < n_tiles) ok = issue_s(j + 1);
-            // K buffer s is free once S_j is complete
-            ok = ok && wait_all(s_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
-            if (ok && j + 2 < n_tiles) load_k(j + 2);
-            ok = ok && wait_all(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && wait_all(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t dvs = dv + (uint64_t)(s * (kAtKVTile >> 4));
-            if (leader) {
+            if (!ok) {
+                ring_drain(k_full0, 2, n_k);
+                ring_drain(v_full0, 2, n_v);
+            }
+        } else {  // MMAs
+            // instruction descriptors: D = f32, A = B = f16, M = 128; S: N = 64, B K-major; O: N = 128, B MN-major
+            const uint32_t idesc_s = (1u << 4) | (0u << 16) | ((uint32_t)(kAtKV >> 3) << 17) | ((uint32_t)(kAtQ >> 4) << 24);
+            const uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(kAtD >> 3) << 17) | ((uint32_t)(kAtQ >> 4) << 24);
+            // Shared-memory descriptors are built once; a step inside a tile only adds (bytes >> 4) to the address field in
+            // the low word (the field holds any shared-memory address, so the add never carries out of it).
+            const uint64_t dq = umma_desc(smem_u32(sQ), 16, 1024), dk = umma_desc(smem_u32(sK), 16, 1024),
+                           dv = umma_desc(smem_u32(sV), kAtKVChunk, 1024);
+            auto issue_s = [&](int j) {  // S_j = Q . K_j^T into accumulator j & 1
+                const int s = j & 1;
+                if (!mbar_wait_warp(k_full0 + 8 * s, (uint32_t)(j >> 1) & 1u)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dks = dk + (uint64_t)(s * (kAtKVTile >> 4));
+                const uint32_t acc = tmem_base + (uint32_t)(s * kAtKV);
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kAtKV / 16; kk++) {
-                    // O += P . V_tile.  A = P, K-major over the 64 cache rows of the tile (one 128-byte row per query); B =
-                    // V_tile, MN-major: 64-column chunks 8 KB apart (LBO), 8-row groups 1024 bytes apart (SBO), 16 rows =
-                    // 2048 bytes further
-                    umma_f16_ta(tmem_base + 128u, tmem_base + (uint32_t)(s * kAtKV + kk * 8), dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
-                             (j > 0 || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < kAtD / 16; kk++) {
+                        // both K-major: 64-column chunk kk/4, 32 bytes per 16 k inside the 128-byte row, 8-row groups 1024 bytes apart
+                        umma_f16(acc, dq + (uint64_t)(((kk >> 2) * kAtQChunk + (kk & 3) * 32) >> 4),
+                                 dks + (uint64_t)(((kk >> 2) * kAtKVChunk + (kk & 3) * 32) >> 4), idesc_s, kk > 0 ? 1u : 0u);
+                    }
+                    umma_commit(s_full0 + 8 * s);
                 }
-                umma_commit(o_full0 + 8 * s);
-            }
-            __syncwarp();
-            if (j + 2 < n_tiles) {
-                ok = wait_all(o_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);  // V buffer s is free again
-                if (ok) load_v(j + 2);
+                __syncwarp();
+                return true;
+            };
+            ok = mbar_wait_warp(q_full, 0) && issue_s(0);
+            for (int j = 0; j < n_tiles && ok; j++) {
+                const int s = j & 1;
+                // the next tile's scores while the softmax warps work on this one (its accumulator was last read for
+                // tile j - 1, whose P has been waited for in the previous round, by the product issued before them)
+                if (j + 1 < n_tiles) ok = issue_s(j + 1);
+                ok = ok && mbar_wait_warp(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && mbar_wait_warp(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t dvs = dv + (uint64_t)(s * (kAtKVTile >> 4));
+                if (leader) {
+#pragma unroll
+                    for (int kk = 0; kk < kAtKV / 16; kk++) {
+                        // O += P . V_tile.  A = P, K-major over the 64 cache rows of the tile (one 128-byte row per query); B =
+                        // V_tile, MN-major: 64-column chunks 8 KB apart (LBO), 8-row groups 1024 bytes apart (SBO), 16 rows =
+                        // 2048 bytes further
+                        umma_f16_ta(tmem_base + 128u, tmem_base + (uint32_t)(s * kAtKV + kk * 8), dvs + (uint64_t)((kk * 2048) >> 4), idesc_o,
+                                    (j > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    umma_commit(o_full0 + 8 * s);
+                }
+                __syncwarp();
             }
         }
     } else if (warp < 4 && active) {
@@ -211,11 +209,12 @@ context_attn_tc_kernel(const __half* __restrict__ q, long q_ld, const __grid_con
             // the query row into the Q tile, in the swizzled K-major form a TMA load would give it (rows behind the
             // end of the sequence are zero): the packed q buffer has no row count the host could put into a tensor map
             // without reading cu_seqlens back
-            const __half* qrow = q + (size_t)(tok0 + q0 + r) * q_ld + (size_t)h * kAtD;
+            const __half* rows = q + (size_t)(tok0 + q0) * q_ld + (size_t)h * kAtD;
 #pragma unroll
-            for (int u = 0; u < 16; u++) {
-                const uint4 v = row_ok ? *reinterpret_cast<const uint4*>(qrow + u * 8) : make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4*>(sQ + (u >> 3) * kAtQChunk + row_off + (((u & 7) ^ (r & 7)) << 4)) = v;
+            for (int i = 0; i < 16; i++) {  // a row's columns side by side in a warp
+                const int row = i * 8 + (r >> 4), u = r & 15;
+                const uint4 v = row < q_rows ? *reinterpret_cast<const uint4*>(rows + (size_t)row * q_ld + u * 8) : make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(sQ + (u >> 3) * kAtQChunk + (row >> 3) * 1024 + (row & 7) * 128 + (((u & 7) ^ (row & 7)) << 4)) = v;
             }
             fence_async_smem();
             mbar_arrive(q_full);
@@ -352,7 +351,7 @@ int context_attn_tc_launch(const __half* q, long q_ld, const __half* k_cache, co
     if (rc) return rc;
     static DeviceOnce smem_attr;
     ONELLM_CUDA(smem_attr.run([] { return cudaFuncSetAttribute(context_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtSmemBytes); }));
-    const dim3 grid((max_q_len + kAtQ - 1) / kAtQ, H, B);
+    const dim3 grid(H, B, (max_q_len + kAtQ - 1) / kAtQ);
     ONELLM_CUDA(launch_pdl(context_attn_tc_kernel, grid, dim3(kAtThreads), kAtSmemBytes, st, q, q_ld, map_k, map_v, cu_seqlens, history, H,
                            Hkv, S_max, scale * 1.4426950408889634f, out));
     return ONELLM_OK;
