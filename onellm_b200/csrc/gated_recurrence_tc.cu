@@ -55,7 +55,7 @@ struct GrChunks {
     unsigned char* v;     // [dv / 64] tiles of tokens x values
     float* vec;           // [dk / 64][4][64]: b_m, b / b_m, and a, c of S <- a S + c S
     float* A;             // [128][128] the plain table, where `notes` says so
-    int* bad;             // [dv] first token whose value is not finite, or 128
+    int* bad;             // [dv] first token whose value is not finite, or 128; there only for a half of the columns that the notes name
     int4* notes;          // x: the chunk has the plain table; y, z: the first, the second half of the columns has values that are not finite
 };
 static size_t gc_chunk_bytes(int dk, int dv)
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(free0 + 8 * (i & 1));  // the accumulators and the vectors
-            if ((notes.y | notes.z) && ck.bad[at * dv + v] < kGcTok) {
+            if ((v < dv / 2 ? notes.y : notes.z) && ck.bad[at * dv + v] < kGcTok) {
 #pragma unroll
                 for (int c = 0; c < kCols; c++) S[c] = __uint_as_float(0x7fffffffu);
             }
@@ -905,7 +905,7 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(o_read);
-                if (notes.y | notes.z) {
+                if (vt * 128 + half * 64 < dv / 2 ? notes.y : notes.z) {  // 64 columns lie in one of the halves
 #pragma unroll
                     for (int j = 0; j < 64; j++)
                         if (ck.bad[at * dv + vt * 128 + half * 64 + j] <= row) o[j] = __uint_as_float(0x7fffffffu);

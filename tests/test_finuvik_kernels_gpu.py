@@ -264,12 +264,14 @@ def test_query_temperature_at_its_edges(cuda, ob, kind):
 
 
 # ---- recurrence --------------------------------------------------------------------------------------------
-def run_recurrence(ob, d, H, dk, dv, q, z, v, zb, lower, w, state, tp, B, eps=1e-5, width=None, scale_out=1.0):
+def run_recurrence(ob, d, H, dk, dv, q, z, v, zb, lower, w, state, tp, B, eps=1e-5, width=None, scale_out=1.0, left=None):
     T = len(q)
     row = d.up(np.concatenate([q.reshape(T, -1), z.reshape(T, -1), v.reshape(T, -1)], 1))
     es, p = row.element_size(), row.data_ptr()
     out = d.zeros(T, H * dv + 32)
     work = d.zeros(ob.gated_recurrence_workspace(T, H, dk, dv) // 4, f32=True) + float("nan")
+    if left is not None:  # the byte that an earlier user of the work space left behind
+        work.view(d.torch.uint8).fill_(left)
     g = ob.GatedRecurrence(d.dtype, H, dk, dv, p, p + H * dk * es, p + 2 * H * dk * es, row.shape[1], d.f32(zb).data_ptr(),
                            d.f32(lower).data_ptr(), d.f32(w).data_ptr(), eps, width or dv, state.data_ptr(), out.data_ptr() + 16 * es,
                            H * dv + 32, scale_out, work.data_ptr())

@@ -389,7 +389,7 @@ def test_window_attention_of_a_context_pass(cuda, ob, H, dk, dv, window):
 
 
 # ---- gated linear attention --------------------------------------------------------------------------------
-def run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, tau, q_scale, eps=1e-5, width=None, scale_out=1.0, gated=True):
+def run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, tau, q_scale, eps=1e-5, width=None, scale_out=1.0, gated=True, left=None):
     q, k, v, r, g = x
     T, rank = len(q), r.shape[1]
     parts = [q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1), g.reshape(T, -1), padded(r, pad(rank, 8))]
@@ -400,6 +400,8 @@ def run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, tau, q_scale, eps=1e-5, wi
         at += p.shape[1]
     out = d.zeros(T, H * dv + 32)
     work = d.zeros(ob.gated_recurrence_workspace(T, H, dk, dv, ob.GR_KEYED) // 4, f32=True) + float("nan")
+    if left is not None:  # the byte that an earlier user of the work space left behind
+        work.view(d.torch.uint8).fill_(left)
     a = ob.GatedRecurrence(d.dtype, H, dk, dv, q=ptr[0], v=ptr[2], ld=at, zb=d.f32(zb).data_ptr(), w=d.f32(w).data_ptr(), eps=eps, norm_width=width or dv,
                            state=state.data_ptr(), out=out.data_ptr() + 16 * es, out_ld=H * dv + 32, out_scale=scale_out, work=work.data_ptr(),
                            kind=ob.GR_KEYED, k=ptr[1], r=ptr[4], rank=rank, A=d.f32(A).data_ptr(), inv_tau=1.0 / tau, q_scale=q_scale,

@@ -92,3 +92,32 @@ def test_what_is_not_finite_reaches_its_own_and_later_tokens_only(cuda, ob, what
         assert rel_err(got[t + 1:], clean[t + 1:]) < TOL and rel_err(host(states[1]), host(states[0])) < STATE
     else:
         assert np.isnan(got[t + 1:]).any(-1).all() and not np.isfinite(host(states[1])).all()
+
+
+@pytest.mark.parametrize("left", [0x00, 0x01, 0xff])
+@pytest.mark.parametrize("dv,col", [(128, 0), (128, 100), (256, 5), (256, 130), (384, 130), (384, 200)])
+@pytest.mark.parametrize("keyed", [False, True])
+def test_a_value_that_is_not_finite_is_its_column_alone(cuda, ob, left, dv, col, keyed):
+    # in either half of a head's columns (which two blocks look through) and in its second tile, whatever the work space holds
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(dv + col)
+    H, dk, n, rank, t = 2, 64, 400, 4, 200
+    x = [rounded(rng.standard_normal(s), "bf16") for s in ((n, H, dk), (n, H, dk), (n, H, dv), (n, rank), (n, H, dv))]
+    A, zb, w = rng.standard_normal((H * dk, rank)), np.ones(H * dk), np.ones(dv)
+
+    def run(state):
+        tp = positions(ob, d, [n], [0])
+        if keyed:
+            return run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, 16.0, 1.0, gated=False, left=left)
+        return run_recurrence(ob, d, H, dk, dv, x[0], x[1], x[2], zb, np.zeros(H * dk), w, state, tp, 1, left=left)
+
+    states = [d.zeros(1, H, dk, dv, f32=True) for _ in range(2)]
+    clean = run(states[0])
+    x[2][t, 0, col] = np.inf
+    got = run(states[1])
+    assert np.array_equal(got[:t], clean[:t]) and np.array_equal(got[:, 1], clean[:, 1])
+    assert np.isnan(got[t:, 0]).any(-1).all()
+    was, now = (host(s)[0] for s in states)
+    others = np.arange(dv) != col
+    assert np.array_equal(now[1], was[1]) and np.array_equal(now[0][:, others], was[0][:, others])
+    assert not np.isfinite(now[0][:, col]).any()
