@@ -226,23 +226,24 @@ __device__ __noinline__ void gc_direct(const GrParams& pp, const GrChunks& ck, s
     }
 }
 
-// Half the value columns of a chunk in tiles, zero behind its last token and where they are not finite
-__device__ __forceinline__ void gc_values(const GatedRecurrence& p, const GrChunks& ck, size_t at, int h, int half, int t0, int n, int* s_bad)
+// Half the value columns of a chunk in tiles, zero behind its last token and where they are not finite; whether any of the others is too
+// large for the quotients: k~ of up to 2^80 times 2^20, times 2^20 and 64 tokens, is all that float holds.
+__device__ __forceinline__ bool gc_values(const GatedRecurrence& p, const GrChunks& ck, size_t at, int h, int half, int t0, int n, int* s_bad)
 {
     const int tid = threadIdx.x, dv = p.dv / 2, groups = dv / 4;
     for (int e = tid; e < dv; e += blockDim.x) s_bad[e] = kGcTok;
     __syncthreads();
     const bf16* src = reinterpret_cast<const bf16*>(p.v) + (size_t)t0 * p.ld + (size_t)h * p.dv + half * dv;
     unsigned char* dst = ck.v + (at * 2 + half) * (dv / 64) * kGcTile;
-    bool bad = false;
+    bool bad = false, large = false;
 #pragma unroll 8
     for (int e = tid; e < kGcTok * groups; e += blockDim.x) {
         const int t = e / groups, col = (e % groups) * 4;
         uint2 x = make_uint2(0u, 0u);
         if (t < n) x = *reinterpret_cast<const uint2*>(src + (size_t)t * p.ld + col);
-        // a half whose exponent is all ones
-        const uint32_t ones = (((x.x & 0x7f807f80u) + 0x00800080u) | ((x.y & 0x7f807f80u) + 0x00800080u)) & 0x80008000u;
-        if (ones) {
+        // a half of kGcMost or more: its exponent's field reaches 147; all ones where it is not finite
+        const uint32_t most = (((x.x & 0x7f807f80u) + 0x36803680u) | ((x.y & 0x7f807f80u) + 0x36803680u)) & 0x80008000u;
+        if (most) {
             uint32_t w[2] = {x.x, x.y};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -250,10 +251,12 @@ __device__ __forceinline__ void gc_values(const GatedRecurrence& p, const GrChun
                 if ((w[j >> 1] & top) == top) {
                     w[j >> 1] &= ~part;
                     atomicMin(&s_bad[col + j], t);
+                    bad = true;
+                } else {
+                    large |= ((w[j >> 1] & top) >> (16 * (j & 1))) >= 0x4980u;
                 }
             }
             x = make_uint2(w[0], w[1]);
-            bad = true;
         }
         *reinterpret_cast<uint2*>(dst + (size_t)(col >> 6) * kGcTile + gc_at(t, col & 63)) = x;
     }
@@ -261,9 +264,10 @@ __device__ __forceinline__ void gc_values(const GatedRecurrence& p, const GrChun
     if (any)
         for (int e = tid; e < dv; e += blockDim.x) ck.bad[at * p.dv + half * dv + e] = s_bad[e];
     if (tid == 0) (half ? ck.notes[at].z : ck.notes[at].y) = any;
+    return __syncthreads_or(large);
 }
 
-// Grid (slots, H, 4), 2 dk threads, clusters of two.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
+// Grid (slots, H, 4), 2 dk threads, clusters of the four.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
 // channels and a quarter of the tokens, in the order outward from the middle.  z = 2 and 3: the values.
 // The loops are short on purpose: straight-line code is fetched once per block, by all SMs at the same time.
 template <bool KEYED>
@@ -278,12 +282,15 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
     pdl_wait();
     pdl_launch_dependents();
     int b, i;
-    if (!gc_locate(pp.tp.cu, pp.tp.B, blockIdx.x, b, i)) return;  // the same in both blocks of a cluster
+    if (!gc_locate(pp.tp.cu, pp.tp.B, blockIdx.x, b, i)) return;  // the same in all blocks of a cluster
     const int tid = threadIdx.x, h = blockIdx.y, dk = p.dk;
     const int t0 = pp.tp.cu[b] + i * kGcTok, n = min(kGcTok, pp.tp.cu[b + 1] - t0);
     const size_t at = (size_t)h * ck.slots + blockIdx.x;
     if (blockIdx.z >= 2) {
-        gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm));
+        const bool large = gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm));
+        if (tid == 0) s_odd = large;
+        cluster.sync();
+        cluster.sync();  // the first block may still be reading it
         return;
     }
     const bool back = blockIdx.z == 0;
@@ -420,7 +427,7 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
     }
     const int mine = __syncthreads_or(odd);
     if (tid == 0) s_odd = mine;
-    cluster.sync();  // everything that either block has written
+    cluster.sync();  // everything that the blocks have written
     if (back) {
         const float *hi = cluster.map_shared_rank(s_all[0], 1), *lo = cluster.map_shared_rank(s_all[1], 1);
         for (int e = tid; e < dk; e += blockDim.x) {
@@ -432,7 +439,8 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
             all.times(hi[e], lo[e]);
             decay_form(all, vec[128], vec[192]);
         }
-        const bool direct = mine || *cluster.map_shared_rank(&s_odd, 1);
+        bool direct = mine;
+        for (int r = 1; r < 4; r++) direct |= *cluster.map_shared_rank(&s_odd, r) != 0;
         if (tid == 0) ck.notes[at].x = direct;
         if (direct) gc_direct<KEYED>(pp, ck, at, h, t0, n, sm);
     }
@@ -1082,7 +1090,7 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     const long clusters = std::min((long)go_clusters(nv), (long)slots * g.H);
     // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
     const bool narrow = (long)(dk / 32) * nv * g.H * B <= num_sms();
-    ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
+    ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 4), st, p, ck));
     ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(dk / (narrow ? 32 : 64), nv * g.H, B), kGsBlock, kGsSmem, dim3(1),
                           st, p, ck));
     ONELLM_CUDA(gc_launch(gr_chunk_output_kernel, dim3(nv, (unsigned)clusters), kGoBlock, kGoSmem, dim3(nv), st, p, ck));

@@ -121,3 +121,31 @@ def test_a_value_that_is_not_finite_is_its_column_alone(cuda, ob, left, dv, col,
     others = np.arange(dv) != col
     assert np.array_equal(now[1], was[1]) and np.array_equal(now[0][:, others], was[0][:, others])
     assert not np.isfinite(now[0][:, col]).any()
+
+
+@pytest.mark.parametrize("keyed", [False, True])
+@pytest.mark.parametrize("size", [2.0 ** 20, 2.0 ** 50])
+def test_large_values_beside_channels_that_nearly_forget(cuda, ob, keyed, size):
+    # half a chunk keeps 2^-79 of some channels: a key over that share, times such a value, is beyond float, the state is not
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(3)
+    H, dk, dv, n = 2, 64, 128, 300
+    x = [rounded(rng.standard_normal(s), "bf16") for s in ((n, H, dk), (n, H, dk), (n, H, dv), (n, 4), (n, H, dv))]
+    x[2][:, 1, 64:] *= size  # of one head and one half of its columns
+    w, zb = np.ones(dv), np.full(H * dk, 4.0)
+    keep = 2.0 ** (-79 / 64)  # of a channel and token
+    zb[::16] = np.log(keep / (1 - keep))
+    state, ref_state = d.zeros(1, H, dk, dv, f32=True), np.zeros((H, dk, dv))
+    tp = positions(ob, d, [n], [0])
+    if keyed:
+        A = np.zeros((H * dk, 4))
+        got = run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, 1.0, 1.0, gated=False)
+        ref = ref_gla(x, A, zb, w, ref_state, 1.0, 1.0, gated=False)
+    else:
+        x[1][:] = 0.0
+        got = run_recurrence(ob, d, H, dk, dv, x[0], x[1], x[2], zb, np.zeros(H * dk), w, state, tp, 1)
+        ref = ref_recurrence(x[0], x[1], x[2], zb, np.zeros(H * dk), w, ref_state)
+    for h in range(H):
+        assert rel_err(got[:, h], ref[:, h]) < TOL
+        for half in (slice(0, 64), slice(64, 128)):
+            assert rel_err(host(state)[0, h][:, half], ref_state[h][:, half]) < STATE
