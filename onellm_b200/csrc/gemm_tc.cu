@@ -815,6 +815,26 @@ static SplitPlan plan_split(int M, int N, int K, bool dual, bool pairs)
     return plan;
 }
 
+// Blocks of the launch's kernel that are sure to run at once in clusters of `size`, asked once per device.  The calculator answers one block
+// per SM for a kernel with tensor memory; two fit.
+template <typename Kern>
+static int split_places(Kern kern, const cudaLaunchConfig_t& cfg, int size)
+{
+    static std::mutex mu;
+    static std::map<std::tuple<const void*, int, int>, int> known;  // the kernels share their type
+    std::lock_guard<std::mutex> lock(mu);
+    int& n = known[std::make_tuple((const void*)kern, size, current_device())];
+    if (n == 0) {
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
+            (void)cudaGetLastError();
+            clusters = num_sms() / size;
+        }
+        n = 2 * clusters * size;
+    }
+    return n;
+}
+
 template <typename T, int MODE>
 static cudaError_t launch_split(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& b2, T* y, int M, int N, int K, const TcEpilogue& epi,
                                 const SplitPlan& plan, cudaStream_t st)
@@ -843,10 +863,13 @@ static cudaError_t launch_split(const CUtensorMap& a, const CUtensorMap& b, cons
     cfg.dynamicSmemBytes = kSplitSmem;
     cfg.stream = st;
     cfg.attrs = at;
-    // Clusters that start beside the last blocks of the kernel in front take places of a GPC such that the last of them find no room for all
-    // their blocks until others are through: every second o_proj or down projection behind 238 tokens took 29 instead of 19, 52 instead
-    // of 33 us.  They wait for the kernel's end; blocks alone and in twos fit anywhere and start early.
-    cfg.numAttrs = at[0].val.clusterDim.x * at[0].val.clusterDim.y > 2 ? 1 : 2;
+    // Clusters that only just fit beside each other wait for the end of the kernel in front: started beside its last blocks they take places of a
+    // GPC such that the last of them find no room for all their blocks until others are through (129 to 256 tokens, 4096 outputs, 32 clusters of
+    // eight where 30 are sure to fit: every second projection took 29 instead of 19, 52 instead of 33 us).  All others start early.  Four layers
+    // of 4096 (2048, 5120), us, all behind the end | as here: 130 tokens 781 | 781 (475 | 461, 947 | 928), 66 tokens 719 | 687 (460 | 433, 892 | 889).
+    const int size = at[0].val.clusterDim.x * at[0].val.clusterDim.y;
+    cfg.numAttrs = 1;
+    if (size <= 2 || (int)(cfg.gridDim.x * cfg.gridDim.y) <= split_places(kern, cfg, size)) cfg.numAttrs = 2;
     note_launch();
     return cudaLaunchKernelEx(&cfg, kern, a, b, b2, y, M, N, K, epi, tiles_n, plan.per);
 }
