@@ -55,14 +55,16 @@ struct GrChunks {
     unsigned char* v;     // [dv / 64] tiles of tokens x values
     float* vec;           // [dk / 64][4][64]: b_m, b / b_m, and a, c of S <- a S + c S
     float* A;             // [128][128] the plain table, where `notes` says so
-    int* bad;             // [dv] first token whose value is not finite, or 128; there only for a half of the columns that the notes name
-    int4* notes;          // x: the chunk has the plain table; y, z: the first, the second half of the columns has values that are not finite
+    int* bad;             // [2][dv] first token of the chunk's half whose value is not finite, or 128; there only for a half that the notes name
+    int4* notes;          // x: the chunk has the plain table; y, z: the first, the second half of the tokens has values that are not finite;
+                          // w: these values have been divided by 2 to the power of the low, the high half word
 };
 static size_t gc_chunk_bytes(int dk, int dv)
 {
     return (size_t)2 * 3 * kGcTok * dk * 2 + (size_t)3 * dv * dk * 2 + (size_t)kGcTok * dv * 2 + (size_t)4 * dk * 4 + (size_t)kGcTok * kGcTok * 4 +
-           (size_t)dv * 4 + 16;
+           (size_t)2 * dv * 4 + 16;
 }
+__device__ __forceinline__ float two_to(int e) { return __int_as_float((127 + e) << 23); }
 // place of an element in a tile
 __device__ __forceinline__ uint32_t gc_at(int row, int col) { return (uint32_t)(row * 128 + (((col >> 3) ^ (row & 7)) << 4) + (col & 7) * 2); }
 
@@ -226,22 +228,26 @@ __device__ __noinline__ void gc_direct(const GrParams& pp, const GrChunks& ck, s
     }
 }
 
-// Half the value columns of a chunk in tiles, zero behind its last token and where they are not finite; whether any of the others is too
-// large for the quotients: k~ of up to 2^80 times 2^20, times 2^20 and 64 tokens, is all that float holds.
-__device__ __forceinline__ bool gc_values(const GatedRecurrence& p, const GrChunks& ck, size_t at, int h, int half, int t0, int n, int* s_bad)
+// The values of half a chunk's tokens in tiles, zero behind its last token and where they are not finite.  Where any is kGcMost or more, all are
+// divided by the power of two that brings them below: k~ is up to 2^80 times 2^20, and that times 2^20 and 64 tokens is all that float holds.
+// (By halves of the tokens, each with a power of its own: a block with half the columns of all of them had to hear of the other half's, at 4 us
+// of 82 by looking through that as well, 9 by a word of the other block.)
+__device__ __forceinline__ void gc_values(const GatedRecurrence& p, const GrChunks& ck, size_t at, int h, int half, int t0, int n, int* s_bad, int* s_most)
 {
-    const int tid = threadIdx.x, dv = p.dv / 2, groups = dv / 4;
+    const int tid = threadIdx.x, dv = p.dv, groups = dv / 4, from = half * (kGcTok / 2);
     for (int e = tid; e < dv; e += blockDim.x) s_bad[e] = kGcTok;
+    if (tid == 0) *s_most = 0;
     __syncthreads();
-    const bf16* src = reinterpret_cast<const bf16*>(p.v) + (size_t)t0 * p.ld + (size_t)h * p.dv + half * dv;
-    unsigned char* dst = ck.v + (at * 2 + half) * (dv / 64) * kGcTile;
-    bool bad = false, large = false;
+    const bf16* src = reinterpret_cast<const bf16*>(p.v) + (size_t)t0 * p.ld + (size_t)h * dv;
+    unsigned char* dst = ck.v + at * (dv / 64) * kGcTile;
+    auto place = [&](int e) { return reinterpret_cast<uint2*>(dst + (size_t)((e % groups) * 4 >> 6) * kGcTile + gc_at(from + e / groups, (e % groups) * 4 & 63)); };
+    bool bad = false;
 #pragma unroll 8
-    for (int e = tid; e < kGcTok * groups; e += blockDim.x) {
-        const int t = e / groups, col = (e % groups) * 4;
+    for (int e = tid; e < kGcTok / 2 * groups; e += blockDim.x) {
+        const int t = from + e / groups, col = (e % groups) * 4;
         uint2 x = make_uint2(0u, 0u);
         if (t < n) x = *reinterpret_cast<const uint2*>(src + (size_t)t * p.ld + col);
-        // a half of kGcMost or more: its exponent's field reaches 147; all ones where it is not finite
+        // a value whose exponent's field reaches 147, kGcMost or more; all ones where it is not finite
         const uint32_t most = (((x.x & 0x7f807f80u) + 0x36803680u) | ((x.y & 0x7f807f80u) + 0x36803680u)) & 0x80008000u;
         if (most) {
             uint32_t w[2] = {x.x, x.y};
@@ -253,21 +259,31 @@ __device__ __forceinline__ bool gc_values(const GatedRecurrence& p, const GrChun
                     atomicMin(&s_bad[col + j], t);
                     bad = true;
                 } else {
-                    large |= ((w[j >> 1] & top) >> (16 * (j & 1))) >= 0x4980u;
+                    atomicMax(s_most, (int)((w[j >> 1] & top) >> (16 * (j & 1))));
                 }
             }
             x = make_uint2(w[0], w[1]);
         }
-        *reinterpret_cast<uint2*>(dst + (size_t)(col >> 6) * kGcTile + gc_at(t, col & 63)) = x;
+        *place(e) = x;
     }
     const bool any = __syncthreads_or(bad);
+    const int down = max((*s_most >> 7) - 146, 0);
     if (any)
-        for (int e = tid; e < dv; e += blockDim.x) ck.bad[at * p.dv + half * dv + e] = s_bad[e];
-    if (tid == 0) (half ? ck.notes[at].z : ck.notes[at].y) = any;
-    return __syncthreads_or(large);
+        for (int e = tid; e < dv; e += blockDim.x) ck.bad[(at * 2 + half) * dv + e] = s_bad[e];
+    if (down) {
+        const float scale = two_to(-down);
+        for (int e = tid; e < kGcTok / 2 * groups; e += blockDim.x) {  // what this thread has written
+            const float2 a = unpack2<bf16>(place(e)->x), b = unpack2<bf16>(place(e)->y);
+            *place(e) = make_uint2(pack2<bf16>(a.x * scale, a.y * scale), pack2<bf16>(b.x * scale, b.y * scale));
+        }
+    }
+    if (tid == 0) {
+        (half ? ck.notes[at].z : ck.notes[at].y) = any;
+        reinterpret_cast<short*>(&ck.notes[at].w)[half] = (short)down;
+    }
 }
 
-// Grid (slots, H, 4), 2 dk threads, clusters of the four.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
+// Grid (slots, H, 4), 2 dk threads, clusters of two.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
 // channels and a quarter of the tokens, in the order outward from the middle.  z = 2 and 3: the values.
 // The loops are short on purpose: straight-line code is fetched once per block, by all SMs at the same time.
 template <bool KEYED>
@@ -282,15 +298,12 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
     pdl_wait();
     pdl_launch_dependents();
     int b, i;
-    if (!gc_locate(pp.tp.cu, pp.tp.B, blockIdx.x, b, i)) return;  // the same in all blocks of a cluster
+    if (!gc_locate(pp.tp.cu, pp.tp.B, blockIdx.x, b, i)) return;  // the same in both blocks of a cluster
     const int tid = threadIdx.x, h = blockIdx.y, dk = p.dk;
     const int t0 = pp.tp.cu[b] + i * kGcTok, n = min(kGcTok, pp.tp.cu[b + 1] - t0);
     const size_t at = (size_t)h * ck.slots + blockIdx.x;
     if (blockIdx.z >= 2) {
-        const bool large = gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm));
-        if (tid == 0) s_odd = large;
-        cluster.sync();
-        cluster.sync();  // the first block may still be reading it
+        gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm), &s_odd);
         return;
     }
     const bool back = blockIdx.z == 0;
@@ -427,7 +440,7 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
     }
     const int mine = __syncthreads_or(odd);
     if (tid == 0) s_odd = mine;
-    cluster.sync();  // everything that the blocks have written
+    cluster.sync();  // everything that either block has written
     if (back) {
         const float *hi = cluster.map_shared_rank(s_all[0], 1), *lo = cluster.map_shared_rank(s_all[1], 1);
         for (int e = tid; e < dk; e += blockDim.x) {
@@ -439,8 +452,7 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
             all.times(hi[e], lo[e]);
             decay_form(all, vec[128], vec[192]);
         }
-        bool direct = mine;
-        for (int r = 1; r < 4; r++) direct |= *cluster.map_shared_rank(&s_odd, r) != 0;
+        const bool direct = mine || *cluster.map_shared_rank(&s_odd, 1);
         if (tid == 0) ck.notes[at].x = direct;
         if (direct) gc_direct<KEYED>(pp, ck, at, h, t0, n, sm);
     }
@@ -557,12 +569,13 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
         float* state = p.state + (((size_t)b * p.H + h) * dk + blockIdx.x * COLS + c0) * dv + v;
         const bool fresh = pp.tp.hist[b] == 0;
         float S[kCols];
-        int4 notes = ck.notes[at0];
+        auto is_rare = [&](size_t at) { return (ck.notes[at].y | ck.notes[at].z | ck.notes[at].w) != 0; };
+        bool rare = is_rare(at0);
 #pragma unroll
         for (int c = 0; c < kCols; c++) S[c] = fresh ? 0.f : state[(size_t)c * dv];
         for (int i = 0; i < n_chunk; i++) {
             const size_t at = at0 + i;
-            const int4 next = i + 1 < n_chunk ? ck.notes[at + 1] : make_int4(0, 0, 0, 0);
+            const bool next = i + 1 < n_chunk && is_rare(at + 1);
             bool there = ok && mbar_wait_warp(vec0 + 8 * (i & 3), (uint32_t)(i >> 2) & 1u);
             const float4* vec = reinterpret_cast<const float4*>(s_vec + (i & 3) * kGsVec) + (from_col + c0) / 4;  // + 16: the next vector
             // the pieces of the chunk in front have been read out of shared memory before anyone writes the next ones; half rows have two places
@@ -605,9 +618,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
             if (!there) ok = false;  // goes on to the barriers of the others, with nothing stored at the end
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = t_lane + (uint32_t)((i & 1) * 4 * COLS);
-            float add[kCols];
-#pragma unroll
-            for (int e = 0; e < 4; e += 2) {
+            auto sums = [&](int e, float(&two)[kCols]) {  // of 64 tokens
                 uint32_t x[kCols], y[kCols];
                 if constexpr (kCols == 16) {
                     tmem_ld16(acc + (uint32_t)(e * COLS), x);
@@ -618,29 +629,38 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
+                for (int c = 0; c < kCols; c++) two[c] = __uint_as_float(x[c]) + __uint_as_float(y[c]);
+            };
+            float add[kCols], more[kCols];
+            sums(0, add);
+            sums(2, more);
+            if (!rare) {
+#pragma unroll
+                for (int e = 0; e < kCols / 4; e++) {
+                    const float4 be = vec[16 + e], al = vec[32 + e], ga = vec[48 + e];
+                    const float fe[4] = {be.x, be.y, be.z, be.w}, fa[4] = {al.x, al.y, al.z, al.w}, fg[4] = {ga.x, ga.y, ga.z, ga.w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const int c = 4 * e + j;
+                        S[c] = fmaf(fe[j], add[c] + more[c], fmaf(fa[j], S[c], fg[j] * S[c]));
+                    }
+                }
+            } else {  // values that are not finite, or have been divided: each half's sums by themselves, behind their factor
+                const float* f = reinterpret_cast<const float*>(vec);
+                const int4 notes = ck.notes[at];
+                const bool bad = (notes.y && ck.bad[at * 2 * dv + v] < kGcTok) || (notes.z && ck.bad[(at * 2 + 1) * dv + v] < kGcTok);
+#pragma unroll
                 for (int c = 0; c < kCols; c++) {
-                    const float two = __uint_as_float(x[c]) + __uint_as_float(y[c]);
-                    add[c] = e == 0 ? two : add[c] + two;
+                    const float kept = fmaf(f[128 + c], S[c], f[192 + c] * S[c]);
+                    S[c] = bad       ? __uint_as_float(0x7fffffffu)
+                           : notes.w ? fmaf(f[64 + c] * add[c], two_to(notes.w & 0xffff), fmaf(f[64 + c] * more[c], two_to(notes.w >> 16), kept))
+                                     : fmaf(f[64 + c], add[c] + more[c], kept);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int e = 0; e < kCols / 4; e++) {
-                const float4 be = vec[16 + e], al = vec[32 + e], ga = vec[48 + e];
-                const float fe[4] = {be.x, be.y, be.z, be.w}, fa[4] = {al.x, al.y, al.z, al.w}, fg[4] = {ga.x, ga.y, ga.z, ga.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int c = 4 * e + j;
-                    S[c] = fmaf(fe[j], add[c], fmaf(fa[j], S[c], fg[j] * S[c]));
-                }
-            }
             __syncwarp();
             if (lane == 0) mbar_arrive(free0 + 8 * (i & 1));  // the accumulators and the vectors
-            if ((v < dv / 2 ? notes.y : notes.z) && ck.bad[at * dv + v] < kGcTok) {
-#pragma unroll
-                for (int c = 0; c < kCols; c++) S[c] = __uint_as_float(0x7fffffffu);
-            }
-            notes = next;
+            rare = next;
         }
         if (ok) {
 #pragma unroll
@@ -882,6 +902,10 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
 #pragma unroll
                         for (int j = 0; j < 16; j++) a[j] = j0 + j <= last ? src[j] : 0.f;
                     }
+                    if (notes.w) {  // a warp's columns are the tokens of one of the halves
+#pragma unroll
+                        for (int j = 0; j < 16; j++) a[j] *= two_to(half ? notes.w >> 16 : notes.w & 0xffff);
+                    }
 #pragma unroll
                     for (int j = 0; j < 8; j++)
                         split_pair(j0 + 2 * j <= last ? a[2 * j] : 0.f, j0 + 2 * j + 1 <= last ? a[2 * j + 1] : 0.f, p0[j], p1[j], p2[j], rest);
@@ -913,10 +937,12 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(o_read);
-                if (vt * 128 + half * 64 < dv / 2 ? notes.y : notes.z) {  // 64 columns lie in one of the halves
+                for (int e = 0; e < 2; e++) {
+                    if (!(e ? notes.z : notes.y)) continue;
+                    const int* bad = ck.bad + (at * 2 + e) * dv + vt * 128 + half * 64;
 #pragma unroll
                     for (int j = 0; j < 64; j++)
-                        if (ck.bad[at * dv + vt * 128 + half * 64 + j] <= row) o[j] = __uint_as_float(0x7fffffffu);
+                        if (bad[j] <= row) o[j] = __uint_as_float(0x7fffffffu);
                 }
 #pragma unroll
                 for (int j = 0; j < 64; j++) ss = fmaf(o[j], o[j], ss);
@@ -1069,7 +1095,7 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     ck.v = take((size_t)kGcTok * dv * 2);
     ck.vec = reinterpret_cast<float*>(take((size_t)4 * dk * 4));
     ck.A = reinterpret_cast<float*>(take((size_t)kGcTok * kGcTok * 4));
-    ck.bad = reinterpret_cast<int*>(take((size_t)dv * 4));
+    ck.bad = reinterpret_cast<int*>(take((size_t)2 * dv * 4));
     ck.notes = reinterpret_cast<int4*>(take(16));
 
     const size_t prep = std::max((size_t)kGcTok / 2 * (dk + (keyed ? g.rank : 0)), (size_t)5 * kGcTok * kGcDirect) * sizeof(float);
@@ -1090,7 +1116,7 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     const long clusters = std::min((long)go_clusters(nv), (long)slots * g.H);
     // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
     const bool narrow = (long)(dk / 32) * nv * g.H * B <= num_sms();
-    ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 4), st, p, ck));
+    ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
     ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(dk / (narrow ? 32 : 64), nv * g.H, B), kGsBlock, kGsSmem, dim3(1),
                           st, p, ck));
     ONELLM_CUDA(gc_launch(gr_chunk_output_kernel, dim3(nv, (unsigned)clusters), kGoBlock, kGoSmem, dim3(nv), st, p, ck));
