@@ -16,14 +16,18 @@
 //
 // Three launches (us at 1 x 2000 tokens, 16 heads of 128 x 128, TIED | 2 x 1030 tokens, 4 heads of 256 x 512, KEYED):
 //   1. gr_chunk_prepare_kernel (26 | 37): gates, their products outward from the middle of the chunk, the pieces of q~ and k~, a copy of the
-//      values in whole chunks.  A chunk that forgets too much has q b_t and k b / b_j instead, and its (q_t . k_j) table by plain
-//      multiply-adds along the gates: slower, never out of range.  Bound by the instructions (70 per channel and token).
+//      values in whole chunks.  A channel that forgets too much has q b_t and k b / b_j instead.  Bound by the instructions (70 per
+//      channel and token).
 //   2. gr_chunk_state_kernel (29 | 24): a block keeps 32 or 64 key channels x 128 value columns of a state in registers and walks the
 //      chunks; it leaves the pieces of b_m S in front of every chunk.  Bound by the chain of a chunk: products into registers, update, split.
+//      Blocks behind these make the parts of the tables (q_t . k_j) that channels without quotients owe, see gd_table.
 //   3. gr_chunk_output_kernel (26 | 58): a block makes 128 tokens x 128 value columns of the output: q~ . k~, q~ . S, then, behind the mask,
 //      the first times V with the pieces of the table in tensor memory; RMS norm over the head (a cluster's blocks share the sums) and gate.
 //      Bound by its operands: 6 bytes a float, 320 KB (608 KB) for 7680 (13800) cycles of products.
-// All three 82 | 118 us; token by token 254 | 246.  Error of the state against 64 bits 9.7e-8 | 8.2e-8 (9.3e-8 | 1.1e-7), of the outputs
+// All three 84.5 | 119.6 us; token by token 255 | 244.  With one channel a head that forgets too much 115 | 163, where the gates are sigmoids of
+// normal numbers 181 | 202, where all channels do 239 | 234.  A short call with such channels is slower than token by token, which no rule
+// on sizes can know: 1 x 288 tokens 38 | 57 us without, 59 | 81, 82 | 99 and 103 | 119 with them, token by token 42 | 73; 1 x 768 tokens TIED 48
+// without, 73, 110 and 132, token by token 101.  Error of the state against 64 bits 9.7e-8 | 8.2e-8 (9.3e-8 | 1.1e-7), of the outputs
 // 1.66e-3 both, the rounding to bfloat16.
 // A value that is not finite would reach the chunk's earlier tokens through a product with zero: the copy has zero there, and the
 // column is NaN from its token on.
@@ -44,25 +48,26 @@ constexpr int kGcTok = 128;                        // tokens of a chunk
 constexpr int kGcMaxDk = 256, kGcMaxDv = 1024, kGcMaxRank = 64;
 constexpr int kGcTile = kGcTok * 64 * 2;           // bytes of 128 rows of 64 columns
 constexpr float kGcLeast = 0x1p-80f, kGcMost = 0x1p20f;
-constexpr int kGcDirect = 16;                      // channels at a time of the plain table
 
 // What the launches hand on, for chunk s of head h at index `at` = h * slots + s.  Operands lie as the tensor cores read them, in tiles of
 // 128 rows x 64 columns (16 KB, 128-byte rows swizzled), so that one copy of contiguous bytes brings them in.
 struct GrChunks {
-    int slots;            // chunks of all sequences, at most
+    int slots, heads;     // chunks of all sequences, at most; heads
     unsigned char *q, *k; // [dk / 64][3 pieces] tiles of tokens x channels
     unsigned char* s;     // [dv / 128][dk / 64][3 pieces] tiles of values x channels: b_m times the state in front of the chunk
     unsigned char* v;     // [dv / 64] tiles of tokens x values
     float* vec;           // [dk / 64][4][64]: b_m, b / b_m, and a, c of S <- a S + c S
-    float* A;             // [128][128] the plain table, where `notes` says so
+    float* A;             // [128][128] a table by multiply-adds, where `notes` says so
+    float* gate;          // [128][dk] 1 - f of the channels it has
+    uint32_t* fast;       // [8] bits of these channels, there only where `notes` says so
     int* bad;             // [2][dv] first token of the chunk's half whose value is not finite, or 128; there only for a half that the notes name
-    int4* notes;          // x: the chunk has the plain table; y, z: the first, the second half of the tokens has values that are not finite;
+    int4* notes;          // x: 1 A is the chunk's table, 2 A is added to it; y, z: the first, the second half of the tokens has values that are not finite;
                           // w: these values have been divided by 2 to the power of the low, the high half word
 };
 static size_t gc_chunk_bytes(int dk, int dv)
 {
     return (size_t)2 * 3 * kGcTok * dk * 2 + (size_t)3 * dv * dk * 2 + (size_t)kGcTok * dv * 2 + (size_t)4 * dk * 4 + (size_t)kGcTok * kGcTok * 4 +
-           (size_t)2 * dv * 4 + 16;
+           (size_t)2 * dv * 4 + (size_t)4 * kGcTok * dk + 32 + 16;
 }
 __device__ __forceinline__ float two_to(int e) { return __int_as_float((127 + e) << 23); }
 // place of an element in a tile
@@ -152,82 +157,6 @@ __device__ __forceinline__ void gc_store_pieces(unsigned char* dst, float lo, fl
     *reinterpret_cast<uint32_t*>(dst + 2 * kGcTile) = p2;
 }
 
-// The form of a chunk without quotients: q b_t, k b / b_j and the table (q_t . k_j) by multiply-adds along the gates, 16 channels at a time.
-template <bool KEYED>
-__device__ __noinline__ void gc_direct(const GrParams& pp, const GrChunks& ck, size_t at, int h, int t0, int n, float* sm)
-{
-    const GatedRecurrence& p = pp.g;
-    float *q = sm, *k = q + kGcTok * kGcDirect, *d = k + kGcTok * kGcDirect, *qb = d + kGcTok * kGcDirect, *kb = qb + kGcTok * kGcDirect;
-    const int tid = threadIdx.x, dk = p.dk;
-    for (int c0 = 0; c0 < dk; c0 += kGcDirect) {
-        __syncthreads();
-        for (int e = tid; e < kGcTok * kGcDirect; e += blockDim.x) {
-            const int t = e / kGcDirect, c = h * dk + c0 + e % kGcDirect;
-            float qv = 0.f, kv = 0.f, dv = 0.f;
-            if (t < n) {
-                const size_t row = (size_t)(t0 + t) * p.ld;
-                qv = to_float(reinterpret_cast<const bf16*>(p.q)[row + c]);
-                if constexpr (KEYED) {
-                    float z = p.zb[c];
-                    const bf16* r = reinterpret_cast<const bf16*>(p.r) + row;
-                    for (int j = 0; j < p.rank; j++) z = fmaf(p.A[(size_t)c * p.rank + j], to_float(r[j]), z);
-                    dv = gc_forget<true>(p, z, 0.f, 0.f);
-                    qv *= p.q_scale;
-                    kv = to_float(reinterpret_cast<const bf16*>(p.k)[row + c]);
-                } else {
-                    dv = gc_forget<false>(p, to_float(reinterpret_cast<const bf16*>(p.z)[row + c]), p.zb[c], p.lower[c]);
-                    qv = silu_of<bf16>(qv);
-                    kv = dv;
-                }
-            }
-            q[e] = qv, k[e] = kv, d[e] = dv;
-        }
-        __syncthreads();
-        if (tid < kGcDirect) {
-            GateProduct b;
-            for (int t = 0; t < kGcTok; t++) {
-                b.times(d[t * kGcDirect + tid]);
-                qb[t * kGcDirect + tid] = q[t * kGcDirect + tid] * b.value();
-            }
-            float* vec = ck.vec + at * 4 * dk + (c0 >> 6) * 256 + (c0 & 63) + tid;
-            vec[0] = 1.f;
-            vec[64] = 1.f;
-            decay_form(b, vec[128], vec[192]);
-        } else if (tid >= 32 && tid < 32 + kGcDirect) {
-            GateProduct b;
-            for (int t = kGcTok - 1; t >= 0; t--) {
-                const int e = t * kGcDirect + tid - 32;
-                kb[e] = k[e] * b.value();
-                b.times(d[e]);
-            }
-        }
-        __syncthreads();
-        for (int e = tid; e < kGcTok * kGcDirect / 2; e += blockDim.x) {
-            const int t = e / (kGcDirect / 2), c = (e % (kGcDirect / 2)) * 2;
-            const size_t dst = (at * (dk / 64) + (c0 >> 6)) * 3 * kGcTile + gc_at(t, (c0 & 63) + c);
-            gc_store_pieces(ck.q + dst, qb[t * kGcDirect + c], qb[t * kGcDirect + c + 1]);
-            gc_store_pieces(ck.k + dst, kb[t * kGcDirect + c], kb[t * kGcDirect + c + 1]);
-        }
-        if (tid < kGcTok) {  // a thread has the column of token j
-            const int j = tid;
-            float w[kGcDirect];
-#pragma unroll
-            for (int c = 0; c < kGcDirect; c++) w[c] = k[j * kGcDirect + c];
-            for (int t = j & ~31; t < n; t++) {
-                if (t < j) continue;
-                float s = 0.f;
-#pragma unroll
-                for (int c = 0; c < kGcDirect; c++) {
-                    if (t > j) w[c] = fmaf(-d[t * kGcDirect + c], w[c], w[c]);
-                    s = fmaf(q[t * kGcDirect + c], w[c], s);
-                }
-                float* a = ck.A + (at * kGcTok + t) * kGcTok + j;
-                *a = c0 == 0 ? s : *a + s;
-            }
-        }
-    }
-}
-
 // The values of half a chunk's tokens in tiles, zero behind its last token and where they are not finite.  Where any is kGcMost or more, all are
 // divided by the power of two that brings them below: k~ is up to 2^80 times 2^20, and that times 2^20 and 64 tokens is all that float holds.
 // (By halves of the tokens, each with a power of its own: a block with half the columns of all of them had to hear of the other half's, at 4 us
@@ -291,9 +220,10 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
 {
     constexpr int kSegs = 4, kHalf = kGcTok / 2, kSeg = kHalf / kSegs, kBatch = 4;
     const GatedRecurrence& p = pp.g;
-    extern __shared__ __align__(16) float sm[];  // 1 - f [16][2 dk threads][2], the gate's low-rank input [64][rank]; the direct form's
+    extern __shared__ __align__(16) float sm[];  // 1 - f [16][2 dk threads][2], the gate's low-rank input [64][rank]
     __shared__ float s_hi[kSegs][kGcMaxDk], s_lo[kSegs][kGcMaxDk], s_all[2][kGcMaxDk];
-    __shared__ int s_odd;
+    __shared__ uint32_t s_fast[kGcMaxDk / 32];
+    __shared__ int s_odd;  // 1: something is too large or not a number, 2: a channel forgets too much
     cg::cluster_group cluster = cg::this_cluster();
     pdl_wait();
     pdl_launch_dependents();
@@ -306,6 +236,7 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
         gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm), &s_odd);
         return;
     }
+    if (tid == 0) s_odd = 0;
     const bool back = blockIdx.z == 0;
     const int seg = tid / (dk / 2), c = (tid % (dk / 2)) * 2, hc = h * dk + c;
     const int first = back ? kHalf - 1 - seg * kSeg : kHalf + seg * kSeg, dir = back ? -1 : 1;
@@ -431,30 +362,94 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
             gc_store_pieces(k_dst + to, k.x * (back ? f0 : r0), k.y * (back ? f1 : r1));
         }
     }
+    bool less = false;
     odd |= !(__low2float(most) < kGcMost && __high2float(most) < kGcMost);
     if (KEYED) odd |= !(fabsf(p.q_scale) < kGcMost);
     if (seg == kSegs - 1) {  // these have come to the end of the chunk's half
-        odd |= !(b0.hi >= kGcLeast && b1.hi >= kGcLeast);
+        less = b0.hi < kGcLeast || b1.hi < kGcLeast;
+        odd |= !(b0.hi >= 0.f && b1.hi >= 0.f);
         *reinterpret_cast<float2*>(&s_all[0][c]) = make_float2(b0.hi, b1.hi);
         *reinterpret_cast<float2*>(&s_all[1][c]) = make_float2(b0.lo, b1.lo);
     }
-    const int mine = __syncthreads_or(odd);
-    if (tid == 0) s_odd = mine;
+    if (odd || less) atomicOr(&s_odd, odd ? 1 : 2);
     cluster.sync();  // everything that either block has written
+    const int notes = s_odd | *cluster.map_shared_rank(&s_odd, back ? 1 : 0);
+    const float *back_hi = cluster.map_shared_rank(s_all[0], 0), *front_hi = cluster.map_shared_rank(s_all[0], 1);
+    if (notes) {  // channels without quotients: see gd_table
+        if (tid < dk) {
+            const bool in = (notes & 1) || !(back_hi[tid] >= kGcLeast && front_hi[tid] >= kGcLeast);
+            const uint32_t bits = __ballot_sync(0xffffffffu, in);
+            if ((tid & 31) == 0) {
+                s_fast[tid >> 5] = bits;
+                if (back) ck.fast[at * 8 + (tid >> 5)] = bits;
+            }
+        }
+        __syncthreads();
+    }
     if (back) {
-        const float *hi = cluster.map_shared_rank(s_all[0], 1), *lo = cluster.map_shared_rank(s_all[1], 1);
+        const float* front_lo = cluster.map_shared_rank(s_all[1], 1);
         for (int e = tid; e < dk; e += blockDim.x) {
             GateProduct all;
             float* vec = ck.vec + at * 4 * dk + (e >> 6) * 256 + (e & 63);
+            const bool plain = notes && (s_fast[e >> 5] >> (e & 31)) & 1u;
             all.times(s_all[0][e], s_all[1][e]);
-            vec[0] = all.value();
-            vec[64] = hi[e] + lo[e];
-            all.times(hi[e], lo[e]);
+            vec[0] = plain ? 1.f : all.value();
+            vec[64] = plain ? 1.f : front_hi[e] + front_lo[e];
+            all.times(front_hi[e], front_lo[e]);
             decay_form(all, vec[128], vec[192]);
         }
-        const bool direct = mine || *cluster.map_shared_rank(&s_odd, 1);
-        if (tid == 0) ck.notes[at].x = direct;
-        if (direct) gc_direct<KEYED>(pp, ck, at, h, t0, n, sm);
+        if (tid == 0) ck.notes[at].x = notes & 1 ? 1 : notes;
+    }
+    const uint32_t mine = notes ? s_fast[c >> 5] >> (c & 31) & 3u : 0u;
+    if (mine) {
+        // q b_t and k b / b_j: one of them takes the gates between its token and the other half, and that half's, on the way out from the middle of
+        // the chunk, the other one those on the far side of its token, on the way back.  The front half has q on the way out.
+#pragma unroll 1
+        for (int way = 0; way < 2; way++) {
+            const bool out = way == 0, is_q = back != out;
+            b0 = GateProduct(), b1 = GateProduct();
+            if (out) {
+                const float *hi = back ? front_hi : back_hi, *lo = cluster.map_shared_rank(s_all[1], back ? 1 : 0);
+                b0.times(hi[c], lo[c]);
+                b1.times(hi[c + 1], lo[c + 1]);
+            }
+#pragma unroll 1
+            for (int s = out ? 0 : seg + 1; s < (out ? seg : kSegs); s++) {
+                b0.times(s_hi[s][c], s_lo[s][c]);
+                b1.times(s_hi[s][c + 1], s_lo[s][c + 1]);
+            }
+#pragma unroll 1
+            for (int o0 = 0; o0 < kSeg; o0 += 8) {
+                uint32_t w[8];
+                if (is_q || KEYED) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const int t = first + dir * (out ? o0 + j : kSeg - 1 - o0 - j);
+                        w[j] = t < n ? *reinterpret_cast<const uint32_t*>((is_q ? qp : kp) + (size_t)t * p.ld) : 0u;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int o = out ? o0 + j : kSeg - 1 - o0 - j, t = first + dir * o;
+                    const float2 x = d[o * D];
+                    float2 y = x;
+                    if (is_q || KEYED) y = unpack2<bf16>(w[j]);
+                    if (is_q) y = KEYED ? make_float2(y.x * p.q_scale, y.y * p.q_scale) : make_float2(silu_of<bf16>(y.x), silu_of<bf16>(y.y));
+                    const float f0 = b0.value(), f1 = b1.value();
+                    b0.times(x.x);
+                    b1.times(x.y);
+                    uint32_t piece[3], rest = 0u;
+                    split_pair(y.x * (is_q ? b0.value() : f0), y.y * (is_q ? b1.value() : f1), piece[0], piece[1], piece[2], rest);
+                    unsigned char* to = (is_q ? q_dst : k_dst) + (t * 128 + ((c16 ^ (t & 7)) << 4));
+#pragma unroll
+                    for (int e = 0; e < 3; e++) {
+                        if (mine == 3u) *reinterpret_cast<uint32_t*>(to + e * kGcTile) = piece[e];
+                        else *reinterpret_cast<unsigned short*>(to + e * kGcTile + (mine & 2u)) = (unsigned short)(mine == 1u ? piece[e] : piece[e] >> 16);
+                    }
+                    if (out) *reinterpret_cast<float2*>(ck.gate + (at * kGcTok + t) * dk + c) = x;
+                }
+            }
+        }
     }
     cluster.sync();  // the other block may still be reading this one's products
 }
@@ -470,7 +465,196 @@ constexpr int kGsSmem = kGsDepth * kGsStage + 3 * kGcTile + 4 * kGsVec;
 
 __device__ __forceinline__ void gs_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kGsWarps * 32) : "memory"); }  // the warps that hold the state
 
-// grid (dk / COLS, dv / 128 * H, B)
+// ---- channels without quotients
+// A channel that forgets too much (below 2^-80 in half a chunk) has q b_t and k b / b_j in the place of q~ and k~, with the middle of the chunk at one.
+// The table's product makes no more than 2^-80 of what is due of those, and the channel's own part of the table, by multiply-adds along the
+// gates, is added to it.  Where q or k is too large or a gate is not a number, all channels of the chunk go that way and the sums
+// here take the table's place.  The blocks behind those of the states make these parts of the table while those walk the chunks: several blocks to a
+// chunk and head where there are few.  A warp has a strip of 8 tokens, its lanes the tokens in front: 32 at a time by what they are worth at the
+// end of their 32, but for the strip's own 32, along the gates.  32 channels at a time, their values requested one group ahead.
+constexpr int kGdGroup = 32, kGdRow = kGcTok + 4;
+static_assert(6 * kGdGroup * kGdRow * 4 <= kGsSmem, "the blocks of the states have room for it");
+struct GdShared {
+    unsigned short list[kGcMaxDk];
+    int count;
+    __align__(16) float strip[kGdGroup][16];  // products of a strip's gates
+};
+
+template <bool KEYED>
+__device__ __noinline__ void gd_table(const GrParams& pp, const GrChunks& ck, unsigned char* smem, GdShared& g, int block, int blocks)
+{
+    const GatedRecurrence& p = pp.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dk = p.dk;
+    // k to the end of its strip, to the end of its 32 tokens; 1 - f, q, q from its strip's start on, k
+    constexpr int kArray = kGdGroup * kGdRow;
+    float *near_end = reinterpret_cast<float*>(smem), *tile_end = near_end + kArray;
+    const int chunks = gc_count(pp.tp.cu, pp.tp.B), pairs = chunks * ck.heads, parts = 4 * pairs <= blocks ? 4 : 2 * pairs <= blocks ? 2 : 1;
+    const int c = lane, s = warp;  // a thread's channel of the group and strip while the operands are made
+    for (int work = block; work < pairs * parts; work += blocks) {
+        const int pair = work / parts, part = work % parts, slot = pair % chunks, h = pair / chunks;
+        const size_t at = (size_t)h * ck.slots + slot;
+        if (ck.notes[at].x == 0) continue;
+        int b = 0, i = 0;
+        (void)gc_locate(pp.tp.cu, pp.tp.B, slot, b, i);
+        const int t0 = pp.tp.cu[b] + i * kGcTok, n = min(kGcTok, pp.tp.cu[b + 1] - t0);
+        gs_sync();
+        if (warp == 0) {
+            uint32_t bits = lane < dk / 32 ? ck.fast[at * 8 + lane] : 0u;
+            int to = __popc(bits);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, to, o);
+                if (lane >= o) to += up;
+            }
+            if (lane == 31) g.count = to;
+            to -= __popc(bits);
+            for (; bits; bits &= bits - 1) g.list[to++] = (unsigned short)(lane * 32 + __ffs(bits) - 1);
+        }
+        gs_sync();
+        const int channels = g.count;
+        // each quarter of the SM has a strip of every 32 tokens (of some 2 or 4 parts; two or four warps to a strip then)
+        const int each = 4 / parts, sub = (warp & 3) / each, I = warp >> 2, x = part + parts * ((warp & 3) % each), strip = 4 * I + x;
+        const int r = lane >> 3, entry = r == x ? lane & 7 : -1;  // the lane's token lies in strip r of the strip's 32 tokens
+        float acc[4][8];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int t = 0; t < 8; t++) acc[e][t] = 0.f;
+        const unsigned short *q0 = reinterpret_cast<const unsigned short*>(p.q), *k0 = reinterpret_cast<const unsigned short*>(p.k);
+        unsigned short qr[8], kr[KEYED ? 8 : 1];
+        float dr[8];
+        auto fetch = [&](int g0) {
+            const int ch = g.list[min(g0 + c, channels - 1)];
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+                const size_t from = (size_t)(t0 + min(8 * s + t, n - 1)) * p.ld + h * dk + ch;
+                dr[t] = ck.gate[(at * kGcTok + 8 * s + t) * dk + ch];
+                qr[t] = q0[from];
+                if constexpr (KEYED) kr[t] = k0[from];
+            }
+        };
+        auto value = [](unsigned short v) { return __uint_as_float((uint32_t)v << 16); };
+        fetch(0);
+#pragma unroll 1
+        for (int g0 = 0; g0 < channels; g0 += kGdGroup) {
+            gs_sync();
+            const int row = c * kGdRow + 8 * s;
+            auto put = [&](int array, const float(&v)[8]) {
+                float* to = near_end + array * kArray + row;
+                *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4*>(to + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            };
+            float end[8], left = 1.f;
+            {
+                float d[8], k[8], q[8], qa[8], on = 1.f;
+#pragma unroll
+                for (int t = 0; t < 8; t++) {
+                    const bool in = g0 + c < channels && 8 * s + t < n;
+                    d[t] = in ? dr[t] : 0.f;
+                    k[t] = !in ? 0.f : KEYED ? value(kr[KEYED ? t : 0]) : d[t];
+                    q[t] = !in ? 0.f : KEYED ? value(qr[t]) * p.q_scale : silu_of<bf16>(value(qr[t]));
+                    on = fmaf(-d[t], on, on);
+                    qa[t] = q[t] * on;
+                }
+#pragma unroll
+                for (int t = 7; t >= 0; t--) {
+                    end[t] = k[t] * left;
+                    left = fmaf(-d[t], left, left);
+                }
+                g.strip[c][s] = left;
+                put(0, end);
+                put(2, d);
+                put(3, q);
+                put(4, qa);
+                put(5, k);
+            }
+            if (g0 + kGdGroup < channels) fetch(g0 + kGdGroup);
+            gs_sync();
+            {
+                float f = 1.f;  // from the strip's end to the end of its 32 tokens
+                for (int m = s + 1; m < (s | 3) + 1; m++) f *= g.strip[c][m];
+#pragma unroll
+                for (int t = 0; t < 8; t++) end[t] *= f;
+                put(1, end);
+            }
+            gs_sync();
+            const int last = min(kGdGroup, channels - g0);
+#pragma unroll 1
+            for (int c0 = sub; c0 < last; c0 += 2 * parts) {  // two channels at a time (zeros behind the last one), for their chains' sake
+                float w[2], fac[2], d[2][8], q[2][8], own_k[2];
+                const float* ops[2];
+                auto get = [&](float(&v)[8], const float* from) {
+                    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(from);
+                    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(from + 4);
+                };
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int cc = c0 + u * parts;
+                    const float4 gate = *reinterpret_cast<const float4*>(&g.strip[cc][4 * I]);
+                    ops[u] = near_end + cc * kGdRow + 8 * strip;
+                    w[u] = r < x ? near_end[cc * kGdRow + 32 * I + lane] : 0.f;
+                    w[u] *= (r < 1 && x > 1 ? gate.y : 1.f) * (r < 2 && x > 2 ? gate.z : 1.f);
+                    fac[u] = (x > 0 ? gate.x : 1.f) * (x > 1 ? gate.y : 1.f) * (x > 2 ? gate.z : 1.f);
+                    own_k[u] = ops[u][5 * kArray + (lane & 7)];
+                    get(d[u], ops[u] + 2 * kArray);
+                    get(q[u], ops[u] + 3 * kArray);
+                }
+#pragma unroll
+                for (int t = 0; t < 8; t++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        w[u] = t == entry ? own_k[u] : fmaf(-d[u][t], w[u], w[u]);
+                        acc[0][t] = fmaf(q[u][t], w[u], acc[0][t]);
+                    }
+#pragma unroll
+                for (int u = 0; u < 2; u++) get(q[u], ops[u] + 4 * kArray);
+#pragma unroll
+                for (int e = 1; e < 4; e++) {  // the 32 tokens e in front
+                    if (e <= I) {
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const int cc = c0 + u * parts;
+                            w[u] = tile_end[cc * kGdRow + 32 * (I - e) + lane] * fac[u];
+                            const float4 tile = *reinterpret_cast<const float4*>(&g.strip[cc][4 * (I - e)]);
+                            fac[u] *= (tile.x * tile.y) * (tile.z * tile.w);
+                        }
+#pragma unroll
+                        for (int t = 0; t < 8; t++) acc[e][t] = fmaf(q[1][t], w[1], fmaf(q[0][t], w[0], acc[e][t]));
+                    }
+                }
+            }
+        }
+        if (parts > 1) {  // the warps of a strip
+            gs_sync();
+            float* sums = near_end + (I * each + (warp & 3) % each) * (parts - 1) * 1024 + lane;
+            if (sub > 0) {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+#pragma unroll
+                    for (int t = 0; t < 8; t++) sums[(sub - 1) * 1024 + (e * 8 + t) * 32] = acc[e][t];
+            }
+            gs_sync();
+            if (sub == 0) {
+                for (int o = 0; o < parts - 1; o++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+#pragma unroll
+                        for (int t = 0; t < 8; t++) acc[e][t] += sums[o * 1024 + (e * 8 + t) * 32];
+            }
+        }
+        if (sub == 0) {
+            float* a = ck.A + (at * kGcTok + 8 * strip) * kGcTok + lane;
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (e <= I) {
+#pragma unroll
+                    for (int t = 0; t < 8; t++) a[t * kGcTok + 32 * (I - e)] = acc[e][t];
+                }
+        }
+    }
+}
+
+// grid: dk / COLS x dv / 128 * heads x sequences blocks for the states, the first index fastest, and the ones of gd_table behind them
 template <int COLS>
 __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __grid_constant__ GrParams pp, const __grid_constant__ GrChunks ck)
 {
@@ -480,9 +664,20 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
     unsigned char *s_out = smem + kGsDepth * kGsStage, *s_vec = s_out + 3 * kGcTile;
     __shared__ __align__(8) uint64_t bars[14];  // stage is there (4), its products are done (4), accumulators are read (2), vectors are there (4)
     __shared__ uint32_t tmem_slot;
+    __shared__ GdShared s_gd;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, dk = p.dk, dv = p.dv, nd = dk / 64, nv = dv / 128;
-    const int slice = blockIdx.x * COLS / 64, from_col = blockIdx.x * COLS % 64;  // tiles have 64 channels
-    const int h = blockIdx.y / nv, vt = blockIdx.y % nv, b = blockIdx.z;
+    const int states = dk / COLS * nv * ck.heads * pp.tp.B;
+    if ((int)blockIdx.x >= states) {
+        pdl_wait();
+        pdl_launch_dependents();
+        if (warp >= kGsWarps) return;
+        if (p.kind == ONELLM_GR_KEYED) gd_table<true>(pp, ck, smem, s_gd, blockIdx.x - states, gridDim.x - states);
+        else gd_table<false>(pp, ck, smem, s_gd, blockIdx.x - states, gridDim.x - states);
+        return;
+    }
+    const int cols = blockIdx.x % (dk / COLS), hv = blockIdx.x / (dk / COLS) % (nv * ck.heads);
+    const int slice = cols * COLS / 64, from_col = cols * COLS % 64;  // tiles have 64 channels
+    const int h = hv / nv, vt = hv % nv, b = blockIdx.x / (dk / COLS) / (nv * ck.heads);
     const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + 4), free0 = smem_u32(bars + 8), vec0 = smem_u32(bars + 10);
     const uint32_t ring = smem_u32(smem);
     bool ok = (ring & 1023u) == 0;
@@ -566,7 +761,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
     } else if (ok && n_chunk > 0) {
         const int q = warp & 3, part = warp >> 2, row = q * 32 + lane, v = vt * 128 + row, c0 = part * kCols;
         const uint32_t t_lane = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
-        float* state = p.state + (((size_t)b * p.H + h) * dk + blockIdx.x * COLS + c0) * dv + v;
+        float* state = p.state + (((size_t)b * p.H + h) * dk + cols * COLS + c0) * dv + v;
         const bool fresh = pp.tp.hist[b] == 0;
         float S[kCols];
         auto is_rare = [&](size_t at) { return (ck.notes[at].y | ck.notes[at].z | ck.notes[at].w) != 0; };
@@ -884,6 +1079,7 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
             (void)gc_locate(pp.tp.cu, pp.tp.B, s, b, i);
             const int t0 = pp.tp.cu[b] + i * kGcTok, n = min(kGcTok, pp.tp.cu[b + 1] - t0);
             const int4 notes = ck.notes[at];
+            if (k == 0 && notes.x) pdl_wait();  // the state kernel has made a table
             if (ok) ok = mbar_wait_warp(t_done, phase);
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -900,7 +1096,8 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
                     if (notes.x) {
                         const float* src = ck.A + (at * kGcTok + row) * kGcTok + j0;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) a[j] = j0 + j <= last ? src[j] : 0.f;
+                        for (int j = 0; j < 16; j++)
+                            if (j0 + j <= last) a[j] = notes.x == 1 ? src[j] : a[j] + src[j];
                     }
                     if (notes.w) {  // a warp's columns are the tokens of one of the halves
 #pragma unroll
@@ -1013,7 +1210,7 @@ bool gr_chunked_takes(const GatedRecurrence& g, const TokenPositions& tp, int B,
     const bool keyed = g.kind == ONELLM_GR_KEYED;
     const int least = (long)B * g.H * (g.dv / 32) > num_sms() ? kGcLeastTokensFull : kGcLeastTokens;
     return g.dtype == ONELLM_BF16 && tp.cu && g.dk % 64 == 0 && g.dk <= kGcMaxDk && g.dv % 128 == 0 && g.dv <= kGcMaxDv && (!keyed || g.rank <= kGcMaxRank) &&
-           (long)tokens >= (long)least * B && gc_slots(tokens, B) < (1 << 24) && (long)g.H * (g.dv / 128) <= 65535 && multiple(g.q, 4) &&
+           (long)tokens >= (long)least * B && gc_slots(tokens, B) < (1 << 24) && g.H <= 65535 && (long)g.H * (g.dv / 128) * (g.dk / 32) * B < (1 << 30) && multiple(g.q, 4) &&
            multiple(keyed ? g.k : g.z, 4) && multiple(g.v, 8) && multiple(g.zb, 8) && multiple(keyed ? g.A : g.lower, 16) && multiple(g.g, 16) &&
            multiple(g.out, 16) && g.out_ld % 8 == 0;
 }
@@ -1025,7 +1222,8 @@ size_t gr_chunked_workspace(int tokens, int H, int dk, int dv)
 }
 
 // Clusters of `nv` output blocks that run at once, asked once per device: a GPC of 18 SMs has room for four clusters of four, and a
-// cluster more than there is room for would run when the others are through (4 heads of 256 x 512, 2 x 1030 tokens: 84 us instead of 42).
+// cluster more than there is room for would run when the others are through (4 heads of 256 x 512, 2 x 1030 tokens, 37 clusters where 34 run at
+// once: all three launches 144 us instead of 119).
 static int go_clusters(int nv)
 {
     static std::mutex mu;
@@ -1083,6 +1281,7 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     const size_t n = (size_t)slots * g.H;
     GrChunks ck;
     ck.slots = slots;
+    ck.heads = g.H;
     unsigned char* w = static_cast<unsigned char*>(g.work);
     auto take = [&](size_t bytes) {
         unsigned char* r = w;
@@ -1096,9 +1295,11 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     ck.vec = reinterpret_cast<float*>(take((size_t)4 * dk * 4));
     ck.A = reinterpret_cast<float*>(take((size_t)kGcTok * kGcTok * 4));
     ck.bad = reinterpret_cast<int*>(take((size_t)2 * dv * 4));
+    ck.gate = reinterpret_cast<float*>(take((size_t)4 * kGcTok * dk));
+    ck.fast = reinterpret_cast<uint32_t*>(take(32));
     ck.notes = reinterpret_cast<int4*>(take(16));
 
-    const size_t prep = std::max((size_t)kGcTok / 2 * (dk + (keyed ? g.rank : 0)), (size_t)5 * kGcTok * kGcDirect) * sizeof(float);
+    const size_t prep = (size_t)kGcTok / 2 * (dk + (keyed ? g.rank : 0)) * sizeof(float);
     auto k1 = keyed ? gr_chunk_prepare_kernel<true> : gr_chunk_prepare_kernel<false>;
     static DeviceOnce attr;
     ONELLM_CUDA(attr.run([] {
@@ -1116,9 +1317,9 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
     const long clusters = std::min((long)go_clusters(nv), (long)slots * g.H);
     // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
     const bool narrow = (long)(dk / 32) * nv * g.H * B <= num_sms();
+    const unsigned states = (unsigned)(dk / (narrow ? 32 : 64) * nv * g.H * B);
     ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
-    ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(dk / (narrow ? 32 : 64), nv * g.H, B), kGsBlock, kGsSmem, dim3(1),
-                          st, p, ck));
+    ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(states + num_sms()), kGsBlock, kGsSmem, dim3(1), st, p, ck));
     ONELLM_CUDA(gc_launch(gr_chunk_output_kernel, dim3(nv, (unsigned)clusters), kGoBlock, kGoSmem, dim3(nv), st, p, ck));
     return ONELLM_OK;
 }

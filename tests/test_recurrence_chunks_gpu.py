@@ -149,3 +149,32 @@ def test_large_values_beside_channels_that_nearly_forget(cuda, ob, keyed, size):
         assert rel_err(got[:, h], ref[:, h]) < TOL
         for half in (slice(0, 64), slice(64, 128)):
             assert rel_err(host(state)[0, h][:, half], ref_state[h][:, half]) < STATE
+
+
+@pytest.mark.parametrize("dk,fast", [(64, 1), (64, 64), (128, 17), (128, 40), (192, 25), (192, 192), (256, 1), (256, 33), (256, 256)])
+@pytest.mark.parametrize("keyed", [False, True])
+def test_channels_that_forget(cuda, ob, dk, fast, keyed):
+    # so many channels of one head below 2^-80 in half a chunk, none of the other: one of a pair, more than a group takes, all
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(dk + fast)
+    H, dv, counts = 2, 128, [300, 1, 600]
+    n = sum(counts)
+    x = [rounded(rng.standard_normal(s), "bf16") for s in ((n, H, dk), (n, H, dk), (n, H, dv), (n, 4), (n, H, dv))]
+    w, zb, A = np.ones(dv), np.full((H, dk), 4.0), fr.round_bf16(rng.standard_normal((H * dk, 4)) * 0.2)
+    zb[1, rng.permutation(dk)[:fast]] = -2.0
+    state, ref_state = d.zeros(3, H, dk, dv, f32=True), [np.zeros((H, dk, dv)) for _ in counts]
+    tp = positions(ob, d, counts, [0, 0, 0])
+    if keyed:
+        got = run_gla(ob, d, H, dk, dv, x, A, zb.ravel(), w, state, tp, 1.0, 1.0, gated=False)
+    else:
+        got = run_recurrence(ob, d, H, dk, dv, x[0], x[1], x[2], zb.ravel(), np.zeros(H * dk), w, state, tp, 3)
+    at = 0
+    for b, m in enumerate(counts):
+        y = [a[at:at + m] for a in x]
+        if keyed:
+            ref = ref_gla(y, A, zb.ravel(), w, ref_state[b], 1.0, 1.0, gated=False)
+        else:
+            ref = ref_recurrence(y[0], y[1], y[2], zb.ravel(), np.zeros(H * dk), w, ref_state[b])
+        assert rel_err(got[at:at + m], ref) < TOL
+        assert rel_err(host(state[b]), ref_state[b]) < STATE
+        at += m
