@@ -171,9 +171,9 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
             ok = mbar_wait_warp(q_full, 0) && issue_s(0);
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int s = j & 1;
-                // the next tile's scores while the softmax warps work on this one: their accumulator was last read for tile j - 1, whose P
-                // has been waited for, by the product issued before them
-                if (j + 1 < n_tiles) ok = issue_s(j + 1);
+                // the next tile's scores while the softmax warps work on this one; their accumulator holds P of tile j - 1 until its product is done
+                if (j >= 1 && j + 1 < n_tiles) ok = mbar_wait_warp(o_full0 + 8 * (s ^ 1), (uint32_t)((j - 1) >> 1) & 1u);
+                if (ok && j + 1 < n_tiles) ok = issue_s(j + 1);
                 ok = ok && mbar_wait_warp(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && mbar_wait_warp(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -17,8 +17,9 @@
 //                         columns) over all tiles.  `ref` is the row maximum the exponentials are taken against; it
 //                         follows the true running maximum only when that has grown by more than 8 (P stays below
 //                         2^8), and only then does a thread wait for the previous product and rescale O in place.
-// The MMAs of one thread run in issue order, which is what lets S of tile j + 2 overwrite the accumulator P of tile j
-// was read from without a wait in between.
+// S of tile j + 1 overwrites the columns that P of tile j - 1 is read from.  Only MMAs of the same shape and accumulator are promised to
+// run in the order of their issue, so the product is waited for first.  The wait is short: the product was issued when the softmax
+// warps turned to tile j, which takes them three times as long.
 // A fifth warp issues the MMAs and a sixth the TMA loads (K and V tiles double-buffered).  With both in one warp the product of a tile
 // was waited for, to reuse its V buffer, before the scores of the next but one were issued: a tile took the warp 3000 cycles, where
 // the softmax warps need 1600.  The blocks with the most tiles start first, of all heads and sequences; head by head, the last
@@ -174,9 +175,9 @@ context_attn_tc_kernel(const __half* __restrict__ q, long q_ld, const __grid_con
             ok = mbar_wait_warp(q_full, 0) && issue_s(0);
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int s = j & 1;
-                // the next tile's scores while the softmax warps work on this one (its accumulator was last read for
-                // tile j - 1, whose P has been waited for in the previous round, by the product issued before them)
-                if (j + 1 < n_tiles) ok = issue_s(j + 1);
+                // the next tile's scores while the softmax warps work on this one; their accumulator holds P of tile j - 1 until its product is done
+                if (j >= 1 && j + 1 < n_tiles) ok = mbar_wait_warp(o_full0 + 8 * (s ^ 1), (uint32_t)((j - 1) >> 1) & 1u);
+                if (ok && j + 1 < n_tiles) ok = issue_s(j + 1);
                 ok = ok && mbar_wait_warp(v_full0 + 8 * s, (uint32_t)(j >> 1) & 1u) && mbar_wait_warp(p_full0 + 8 * s, (uint32_t)(j >> 1) & 1u);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

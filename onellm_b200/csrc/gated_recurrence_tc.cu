@@ -887,20 +887,20 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
     const GatedRecurrence& p = pp.g;
     extern __shared__ __align__(1024) unsigned char smem[];
     // tile is there (14), tile has been used (14), table is done, pieces of the table are there, output is done, output is read, sums of the
-    // cluster are there, everything issued by a block that gave up is done
-    __shared__ __align__(8) uint64_t bars[2 * kGoRing + 6];
+    // cluster are there, everything issued by a block that gave up is done, products with the state are done
+    __shared__ __align__(8) uint64_t bars[2 * kGoRing + 7];
     __shared__ uint32_t tmem_slot;
     __shared__ float s_part[kGcTok], s_sum[2][kGcTok], s_w[128];
     cg::cluster_group cluster = cg::this_cluster();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, dk = p.dk, dv = p.dv, nd = dk / 64, nv = dv / 128;
     const int vt = blockIdx.x;
     const uint32_t full0 = smem_u32(bars), used0 = full0 + 8 * kGoRing, t_done = used0 + 8 * kGoRing, p_full = t_done + 8, o_done = t_done + 16,
-                   o_read = t_done + 24, sums = t_done + 32, end = t_done + 40;
+                   o_read = t_done + 24, sums = t_done + 32, end = t_done + 40, s_done = t_done + 48;
     const uint32_t ring = smem_u32(smem);
     bool ok = (ring & 1023u) == 0;
     if (!ok && tid == 0) atomicExch(&g_tc_timeout_flag, 1);
     if (tid == 0) {
-        for (int s = 0; s < 2 * kGoRing + 6; s++) {
+        for (int s = 0; s < 2 * kGoRing + 7; s++) {
             const int e = s - 2 * kGoRing;
             mbar_init(full0 + 8 * s, e == 1 || e == 3 ? kGoWarps : e == 4 ? kGoWarps * nv : 1);
         }
@@ -1000,7 +1000,11 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
             if (ok && leader) umma_commit(used0 + 8 * a);
             __syncwarp();
         };
+        // Only MMAs of the same shape and accumulator are promised to run in the order of their issue.  Two places need another order and wait: the
+        // table's product of a pair overwrites the pieces that the last one of the pair in front reads, and that one, 64 columns wide, adds to sums of
+        // products 128 wide.
         for (int k = 0; k < mine && ok; k++) {
+            if (k > 0) ok = mbar_wait_warp(o_done, (uint32_t)(k - 1) & 1u);
 #pragma unroll 1
             for (int d = 0; d < nd && ok; d++) {
                 const uint32_t more = d > 0;
@@ -1036,11 +1040,15 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
                 release(s0);
                 const int s2 = next();
                 product(q0, s2, kGoStateLow, 1u);
+                if (d == nd - 1) {
+                    if (ok && leader) umma_commit(s_done);
+                    __syncwarp();
+                }
                 release(q0);
                 release(s2);
             }
             const int v0 = next(), v1 = next();
-            ok = ok && mbar_wait_warp(p_full, (uint32_t)k & 1u);
+            ok = ok && mbar_wait_warp(s_done, (uint32_t)k & 1u) && mbar_wait_warp(p_full, (uint32_t)k & 1u);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (leader) {
