@@ -49,10 +49,11 @@ constexpr int kGcMaxDk = 256, kGcMaxDv = 1024, kGcMaxRank = 64;
 constexpr int kGcTile = kGcTok * 64 * 2;           // bytes of 128 rows of 64 columns
 constexpr float kGcLeast = 0x1p-80f, kGcMost = 0x1p20f;
 
-// What the launches hand on, for chunk s of head h at index `at` = h * slots + s.  Operands lie as the tensor cores read them, in tiles of
+// What the launches hand on, for chunk s of the pass's head h at index `at` = h * slots + s.  Operands lie as the tensor cores read them, in tiles of
 // 128 rows x 64 columns (16 KB, 128-byte rows swizzled), so that one copy of contiguous bytes brings them in.
 struct GrChunks {
-    int slots, heads;     // chunks of all sequences, at most; heads
+    int slots;            // chunks of all sequences, at most
+    int head0, heads;     // of this pass
     unsigned char *q, *k; // [dk / 64][3 pieces] tiles of tokens x channels
     unsigned char* s;     // [dv / 128][dk / 64][3 pieces] tiles of values x channels: b_m times the state in front of the chunk
     unsigned char* v;     // [dv / 64] tiles of tokens x values
@@ -212,7 +213,7 @@ __device__ __forceinline__ void gc_values(const GatedRecurrence& p, const GrChun
     }
 }
 
-// Grid (slots, H, 4), 2 dk threads, clusters of two.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
+// Grid (slots, heads, 4), 2 dk threads, clusters of two.  z = 0 and 1 have the tokens in front of and behind the middle of the chunk: a thread two
 // channels and a quarter of the tokens, in the order outward from the middle.  z = 2 and 3: the values.
 // The loops are short on purpose: straight-line code is fetched once per block, by all SMs at the same time.
 template <bool KEYED>
@@ -229,9 +230,9 @@ __global__ void __launch_bounds__(512, 2) gr_chunk_prepare_kernel(const __grid_c
     pdl_launch_dependents();
     int b, i;
     if (!gc_locate(pp.tp.cu, pp.tp.B, blockIdx.x, b, i)) return;  // the same in both blocks of a cluster
-    const int tid = threadIdx.x, h = blockIdx.y, dk = p.dk;
+    const int tid = threadIdx.x, h = ck.head0 + blockIdx.y, dk = p.dk;
     const int t0 = pp.tp.cu[b] + i * kGcTok, n = min(kGcTok, pp.tp.cu[b + 1] - t0);
-    const size_t at = (size_t)h * ck.slots + blockIdx.x;
+    const size_t at = (size_t)blockIdx.y * ck.slots + blockIdx.x;
     if (blockIdx.z >= 2) {
         gc_values(p, ck, at, h, blockIdx.z - 2, t0, n, reinterpret_cast<int*>(sm), &s_odd);
         return;
@@ -527,7 +528,7 @@ __device__ __noinline__ void gd_table(const GrParams& pp, const GrChunks& ck, un
             const int ch = g.list[min(g0 + c, channels - 1)];
 #pragma unroll
             for (int t = 0; t < 8; t++) {
-                const size_t from = (size_t)(t0 + min(8 * s + t, n - 1)) * p.ld + h * dk + ch;
+                const size_t from = (size_t)(t0 + min(8 * s + t, n - 1)) * p.ld + (ck.head0 + h) * dk + ch;
                 dr[t] = ck.gate[(at * kGcTok + 8 * s + t) * dk + ch];
                 qr[t] = q0[from];
                 if constexpr (KEYED) kr[t] = k0[from];
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
     }
     const int cols = blockIdx.x % (dk / COLS), hv = blockIdx.x / (dk / COLS) % (nv * ck.heads);
     const int slice = cols * COLS / 64, from_col = cols * COLS % 64;  // tiles have 64 channels
-    const int h = hv / nv, vt = hv % nv, b = blockIdx.x / (dk / COLS) / (nv * ck.heads);
+    const int h = ck.head0 + hv / nv, vt = hv % nv, b = blockIdx.x / (dk / COLS) / (nv * ck.heads);
     const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + 4), free0 = smem_u32(bars + 8), vec0 = smem_u32(bars + 10);
     const uint32_t ring = smem_u32(smem);
     bool ok = (ring & 1023u) == 0;
@@ -697,7 +698,7 @@ __global__ void __launch_bounds__(kGsBlock, 1) gr_chunk_state_kernel(const __gri
     pdl_wait();
     pdl_launch_dependents();
     const int n_chunk = (pp.tp.cu[b + 1] - pp.tp.cu[b] + kGcTok - 1) / kGcTok;
-    const size_t at0 = (size_t)h * ck.slots + gc_count(pp.tp.cu, b);  // behind the chunks of the sequences in front
+    const size_t at0 = (size_t)(h - ck.head0) * ck.slots + gc_count(pp.tp.cu, b);  // behind the chunks of the sequences in front
 
     const int n_half = 2 * n_chunk;
     auto slot = [](int j) { return j & (kGsDepth - 1); };
@@ -917,13 +918,13 @@ __global__ void __launch_bounds__(kGoBlock, 1) gr_chunk_output_kernel(const __gr
     // No block of this kernel starts before every block of the state kernel is behind its wait for the prepare kernel: what that one wrote
     // is there.  The wait for the states comes in front of their first load (and of the first store).
     const int chunks = gc_count(pp.tp.cu, pp.tp.B);
-    const long n_work = (long)chunks * p.H;
+    const long n_work = (long)chunks * ck.heads;
     const int mine = n_work > blockIdx.y ? (int)((n_work - 1 - blockIdx.y) / gridDim.y) + 1 : 0;  // the same in all blocks of a cluster
     auto place = [&](int k, int& s, int& h) {  // of the k-th pair of this cluster
         const long w = blockIdx.y + (long)k * gridDim.y;
-        h = (int)(w / chunks);
         s = (int)(w % chunks);
-        return (size_t)h * ck.slots + s;
+        h = ck.head0 + (int)(w / chunks);
+        return (size_t)(h - ck.head0) * ck.slots + s;
     };
 
     // The tiles of a pair in the order of their use: of 64 channels q~0 k~0 k~1 q~1 k~2 q~2 S0 S1 S2 (pieces), then of the next; V at the end.
@@ -1212,6 +1213,25 @@ constexpr int kGcLeastTokens = 288, kGcLeastTokensFull = 192;
 
 static long gc_slots(int tokens, int B) { return (long)tokens / kGcTok + B; }
 
+// Heads that go through the three launches together, 0: the call is not for them.  A chunk of a head takes 1.7 to 2.1 times the token by token form's
+// vectors of it, and more where sequences end within chunks, so a call takes no more than the larger of that form's work space and kGcSpace, and
+// goes through its heads in passes where all of them would need more.  32 heads of 128 x 128 and 8 of 256 x 512 find room in it for 2000
+// tokens; a pass of as much fills the chip.
+constexpr size_t kGcSpace = (size_t)256 << 20;
+constexpr size_t kGcPad = 10 * 16;  // the parts of the work space begin on multiples of 16 bytes
+static int gc_heads(int kind, int tokens, int B, int H, int dk, int dv)
+{
+    const size_t space = gated_recurrence_workspace(kind, tokens, H, dk, dv) - kGcPad, head = (size_t)gc_slots(tokens, B) * gc_chunk_bytes(dk, dv);
+    const int most = (int)std::min<size_t>(space / head, H), passes = most > 0 ? (H + most - 1) / most : 0;
+    return passes > 0 ? (H + passes - 1) / passes : 0;
+}
+
+size_t gr_chunked_workspace(int tokens, int H, int dk, int dv)
+{
+    if (dk % 64 != 0 || dk > kGcMaxDk || dv % 128 != 0 || dv > kGcMaxDv || tokens < kGcLeastTokensFull) return 0;
+    return std::min(kGcSpace, (size_t)gc_slots(tokens, tokens / kGcLeastTokensFull) * H * gc_chunk_bytes(dk, dv) + kGcPad);
+}
+
 bool gr_chunked_takes(const GatedRecurrence& g, const TokenPositions& tp, int B, int tokens)
 {
     const auto multiple = [](const void* p, uintptr_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
@@ -1220,13 +1240,7 @@ bool gr_chunked_takes(const GatedRecurrence& g, const TokenPositions& tp, int B,
     return g.dtype == ONELLM_BF16 && tp.cu && g.dk % 64 == 0 && g.dk <= kGcMaxDk && g.dv % 128 == 0 && g.dv <= kGcMaxDv && (!keyed || g.rank <= kGcMaxRank) &&
            (long)tokens >= (long)least * B && gc_slots(tokens, B) < (1 << 24) && g.H <= 65535 && (long)g.H * (g.dv / 128) * (g.dk / 32) * B < (1 << 30) && multiple(g.q, 4) &&
            multiple(keyed ? g.k : g.z, 4) && multiple(g.v, 8) && multiple(g.zb, 8) && multiple(keyed ? g.A : g.lower, 16) && multiple(g.g, 16) &&
-           multiple(g.out, 16) && g.out_ld % 8 == 0;
-}
-
-size_t gr_chunked_workspace(int tokens, int H, int dk, int dv)
-{
-    if (dk % 64 != 0 || dk > kGcMaxDk || dv % 128 != 0 || dv > kGcMaxDv || tokens < kGcLeastTokensFull) return 0;
-    return (size_t)gc_slots(tokens, tokens / kGcLeastTokensFull) * H * gc_chunk_bytes(dk, dv) + 256;
+           multiple(g.out, 16) && g.out_ld % 8 == 0 && gc_heads(g.kind, tokens, B, g.H, g.dk, g.dv) > 0;
 }
 
 // Clusters of `nv` output blocks that run at once, asked once per device: a GPC of 18 SMs has room for four clusters of four, and a
@@ -1285,11 +1299,10 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
 {
     const GatedRecurrence& g = p.g;
     const bool keyed = g.kind == ONELLM_GR_KEYED;
-    const int dk = g.dk, dv = g.dv, slots = (int)gc_slots(tokens, B), nv = dv / 128;
-    const size_t n = (size_t)slots * g.H;
+    const int dk = g.dk, dv = g.dv, slots = (int)gc_slots(tokens, B), nv = dv / 128, heads = gc_heads(g.kind, tokens, B, g.H, dk, dv);
+    const size_t n = (size_t)slots * heads;
     GrChunks ck;
     ck.slots = slots;
-    ck.heads = g.H;
     unsigned char* w = static_cast<unsigned char*>(g.work);
     auto take = [&](size_t bytes) {
         unsigned char* r = w;
@@ -1322,13 +1335,16 @@ int gr_chunked(const GrParams& p, int B, int tokens, cudaStream_t st)
             if (e == cudaSuccess) e = prefer_max_shared(k);
         return e;
     }));
-    const long clusters = std::min((long)go_clusters(nv), (long)slots * g.H);
-    // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
-    const bool narrow = (long)(dk / 32) * nv * g.H * B <= num_sms();
-    const unsigned states = (unsigned)(dk / (narrow ? 32 : 64) * nv * g.H * B);
-    ONELLM_CUDA(gc_launch(k1, dim3(slots, g.H, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
-    ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(states + num_sms()), kGsBlock, kGsSmem, dim3(1), st, p, ck));
-    ONELLM_CUDA(gc_launch(gr_chunk_output_kernel, dim3(nv, (unsigned)clusters), kGoBlock, kGoSmem, dim3(nv), st, p, ck));
+    for (ck.head0 = 0; ck.head0 < g.H; ck.head0 += heads) {
+        ck.heads = std::min(heads, g.H - ck.head0);
+        const long clusters = std::min((long)go_clusters(nv), (long)slots * ck.heads);
+        // 32 channels a block where there is an SM for each of them: a chunk's step is as long as the work of a thread
+        const bool narrow = (long)(dk / 32) * nv * ck.heads * B <= num_sms();
+        const unsigned states = (unsigned)(dk / (narrow ? 32 : 64) * nv * ck.heads * B);
+        ONELLM_CUDA(gc_launch(k1, dim3(slots, ck.heads, 4), 2 * dk, prep, dim3(1, 1, 2), st, p, ck));
+        ONELLM_CUDA(gc_launch(narrow ? gr_chunk_state_kernel<32> : gr_chunk_state_kernel<64>, dim3(states + num_sms()), kGsBlock, kGsSmem, dim3(1), st, p, ck));
+        ONELLM_CUDA(gc_launch(gr_chunk_output_kernel, dim3(nv, (unsigned)clusters), kGoBlock, kGoSmem, dim3(nv), st, p, ck));
+    }
     return ONELLM_OK;
 }
 

@@ -178,3 +178,33 @@ def test_channels_that_forget(cuda, ob, dk, fast, keyed):
         assert rel_err(got[at:at + m], ref) < TOL
         assert rel_err(host(state[b]), ref_state[b]) < STATE
         at += m
+
+
+@pytest.mark.parametrize("keyed,H,dk,dv,B", [(False, 8, 256, 128, 40), (True, 2, 64, 256, 70), (False, 3, 64, 128, 33), (True, 1, 128, 512, 1)])
+def test_many_chunks(cuda, ob, keyed, H, dk, dv, B):
+    # Clusters of the output kernel take several (chunk, head) pairs; a warp looks through the sequences more than once; the first case goes
+    # through its heads in three passes.
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(B)
+    counts = rng.integers(300, 725, B) if B > 1 else np.array([8000])
+    T, ends = int(counts.sum()), np.cumsum(counts)
+    x = [rounded(rng.standard_normal(s).astype(np.float32), "bf16") for s in ((T, H, dk), (T, H, dk), (T, H, dv), (T, 4), (T, H, dv))]
+    w, zb = fr.round_bf16(1 + 0.3 * rng.standard_normal(dv)), fr.round_bf16(rng.uniform(-1, 6, H * dk))
+    A, lower = fr.round_bf16(rng.standard_normal((H * dk, 4)) * 0.3), np.zeros(H * dk)
+    state = d.zeros(B, H, dk, dv, f32=True)
+    tp = positions(ob, d, counts, [0] * B)
+    if keyed:
+        got = run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, 16.0, 1.0)
+    else:
+        got = run_recurrence(ob, d, H, dk, dv, x[0], x[1], x[2], zb, lower, w, state, tp, B)
+    for b in sorted({0, 1, 31, 32, 33, B // 2, B - 1} & set(range(B))):
+        s = slice(int(ends[b] - counts[b]), int(ends[b]))
+        for h in {0, H // 2, H - 1}:
+            ch, ref_state = slice(h * dk, (h + 1) * dk), np.zeros((1, dk, dv))
+            y = [a[s, h:h + 1] for a in x[:3]]
+            if keyed:
+                ref = ref_gla(y + [x[3][s], x[4][s, h:h + 1]], A[ch], zb[ch], w, ref_state, 16.0, 1.0)
+            else:
+                ref = ref_recurrence(*y, zb[ch], lower[ch], w, ref_state)
+            assert rel_err(got[s, h:h + 1], ref) < TOL, (b, h)
+            assert rel_err(host(state[b, h:h + 1]), ref_state) < STATE, (b, h)
