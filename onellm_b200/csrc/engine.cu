@@ -224,6 +224,21 @@ int Engine::enqueue_step(int mode, int step_bound, int prompt_len)
     return ONELLM_OK;
 }
 
+// A step that no graph holds.  One that fails behind its first kernel has moved the device's step counter: it goes back to the cached
+// positions, or the next step would be a position too far on and read the ids of another turn of the mail.
+int Engine::run_eagerly(int mode, int step_bound, int prompt_len)
+{
+    const long before = launches_noted();
+    const int rc = enqueue_step(mode, step_bound, prompt_len);
+    if (rc != ONELLM_OK) {
+        (void)cudaMemcpyAsync(d_step, &cur_len, sizeof(int), cudaMemcpyHostToDevice, stream);
+        return rc;
+    }
+    launches += launches_noted() - before;
+    cur_len++;
+    return ONELLM_OK;
+}
+
 // Runs one step (attending cur_len + 1 rows) and advances cur_len.
 int Engine::run_step(int mode, int prompt_len, const int* host_ids)
 {
@@ -247,13 +262,7 @@ int Engine::run_step(int mode, int prompt_len, const int* host_ids)
     mail.unread++;
     int bound = (step + 255) / 256 * 256;
     bound = std::min({bound, max_seq_len, span_cap});
-    if (!use_graphs) {
-        const long before = launches_noted();
-        RC(enqueue_step(mode, bound, prompt_len));
-        launches += launches_noted() - before;
-        cur_len++;
-        return ONELLM_OK;
-    }
+    if (!use_graphs) return run_eagerly(mode, bound, prompt_len);
     const long key = ((long)bound << 20) | ((long)batch << 8) | ((long)mode << 4) | (top_k > 1 ? 1 : 0);
     // prompt_len, top_k, temperature are baked into the captured nodes: changing them drops the cache
     auto it = graphs.find(key);
@@ -261,11 +270,7 @@ int Engine::run_step(int mode, int prompt_len, const int* host_ids)
         // first step of this shape runs eagerly: the launch planners query occupancy and set
         // function attributes once per kernel, which must not happen inside a stream capture
         warmed[key] = 1;
-        const long before = launches_noted();
-        RC(enqueue_step(mode, bound, prompt_len));
-        launches += launches_noted() - before;
-        cur_len++;
-        return ONELLM_OK;
+        return run_eagerly(mode, bound, prompt_len);
     }
     if (it == graphs.end()) {
         const long before = launches_noted();  // what the capture records = the nodes of one replay

@@ -123,6 +123,7 @@ struct Engine {
     // ---- the generation loop
     int sample(const void* row_logits);
     int enqueue_step(int mode, int step_bound, int prompt_len);
+    int run_eagerly(int mode, int step_bound, int prompt_len);
     int run_step(int mode, int prompt_len, const int* host_ids = nullptr);  // host_ids: the step's input ids, else the ones sampled last
     // step: what the step counter is to be; first: the sequences begin with this pass
     int prefill_context(int B, const int* lens, int step, bool first);

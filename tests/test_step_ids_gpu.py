@@ -38,3 +38,35 @@ def test_steps_read_their_own_ids(ob, cuda, graphs, batch, steps):
         assert np.array_equal(got, out)
         assert np.array_equal(m.logits(batch), want)
     m.close()
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+@pytest.mark.parametrize("behind", [0, 3])
+def test_a_step_after_one_that_failed_reads_its_own_ids(ob, cuda, graphs, behind):
+    # a step fails behind its layers where fewer logits than candidates are asked for; the next one is at the same position
+    m = ob.Llama(**dict(CFG, vocab_size=40))
+    m.init_random(3, 0.05)
+    m.set_graphs(graphs)
+    rng = np.random.default_rng(behind)
+    prompt = rng.integers(0, 40, (2, 5)).astype(np.int32)
+    ids = rng.integers(0, 40, (behind + 3, 2)).astype(np.int32)
+    out = np.zeros(2, np.int32)
+
+    def steps(fail):
+        m.set_sampling(1)
+        m.prefill(prompt)
+        rows = []
+        for t in range(len(ids)):
+            if fail and t == behind:
+                m.set_sampling(64)
+                for _ in range(2):
+                    with pytest.raises(ob.OnellmError):
+                        m.decode_step((ids[t] + 1) % 40, out)
+                m.set_sampling(1)
+            m.decode_step(ids[t], out)
+            rows.append(m.logits(2))
+        return np.array(rows)
+
+    want = steps(False)
+    assert np.array_equal(steps(True), want)
+    m.close()
