@@ -206,7 +206,9 @@ biased_attn_tc_kernel(const BaParams p, const __grid_constant__ CUtensorMap map_
             for (int i = 0; i < 3; i++) ahead[i] = __ldg(pen + min(max(hist + q0 + warp * 32 - kv0 - 63 + 32 * i + lane, 0), p.a.S - 1));
         };
         if (!WINDOWED) fetch(key0);
-        const int pos_c = row_ok ? pos : hist + q0;  // rows behind the end of the sequence read the penalties of its first row
+        // Rows behind the end of the sequence are masked as its first row; what keeps their penalties in range are the distances cut off in fetch.
+        // They have a factor of zero and nothing of them is stored.
+        const int pos_c = row_ok ? pos : hist + q0;
         float m_ref = -INFINITY, l_run = 0.f;
         bool ok = true;
         {

@@ -27,8 +27,8 @@
 // All three 84.5 | 119.6 us; token by token 255 | 244.  With one channel a head that forgets too much 115 | 163, where the gates are sigmoids of
 // normal numbers 181 | 202, where all channels do 239 | 234.  A short call with such channels is slower than token by token, which no rule
 // on sizes can know: 1 x 288 tokens 38 | 57 us without, 59 | 81, 82 | 99 and 103 | 119 with them, token by token 42 | 73; 1 x 768 tokens TIED 48
-// without, 73, 110 and 132, token by token 101.  Error of the state against 64 bits 9.7e-8 | 8.2e-8 (9.3e-8 | 1.1e-7), of the outputs
-// 1.66e-3 both, the rounding to bfloat16.
+// without, 73, 110 and 132, token by token 101.  Error of the state against 64 bits 9.7e-8 | 8.3e-8 (9.3e-8 | 1.1e-7; sigmoids of normal numbers
+// 8.7e-8 | 6.3e-8, 7.0e-8 | 5.3e-8), of the outputs 1.66e-3 both, the rounding to bfloat16.
 // A value that is not finite would reach the chunk's earlier tokens through a product with zero: the copy has zero there, and the
 // column is NaN from its token on.
 #include <cooperative_groups.h>

@@ -552,8 +552,10 @@ static StagedPlan plan_staged(int N, int K, bool tp)
         // clusters of eight where 33 fit took 10 us longer than 32 of seven in a design's decode steps (19200 x 4096, 16 tokens: as if
         // in two waves), elsewhere about as long; called alone one right behind the other they are the faster by 9 %.
         // Rates (KB a us and SM with one to four blocks) and cost per range (us) are fitted to a sweep over all splits and seven depths
-        // of 26 shapes with 4, 12 and 24 tokens, weights from memory.  Behind the best plan of each: 3 % on average, 12 % at most (two
-        // rules by blocks and bytes on their way alone: 8 % and 51 %, 7 % and 31 %).
+        // of 26 shapes with 4, 12 and 24 tokens, weights from memory, when the partial sums of up to 16 tokens were still read from the peers;
+        // pushed, a range costs less than it says here.  Behind the best plan of each with 1, 4 and 12 tokens: 4.4 % on average, 16 % at most
+        // (2048 x 2048 pairs, six ranges instead of eight), for which the sums of all shapes would be taken in another order.  (When fitted 3 %
+        // and 12 %; two rules by blocks and bytes on their way alone: 8 % and 51 %, 7 % and 31 %.)
         constexpr int kClass = MB >= 4 ? 2 : MB >= 2 ? 1 : 0;
         constexpr double kRange[3][2] = {{0.03, 0.20}, {0.05, 0.32}, {0.21, 0.81}};
         constexpr double kRate[3][2][4] = {{{29, 46, 49, 49}, {43, 60, 54, 54}}, {{26, 41, 45, 45}, {38, 54, 50, 50}}, {{19.4, 29, 31.5, 33}, {32, 43, 41, 41}}};
