@@ -1215,9 +1215,9 @@ static long gc_slots(int tokens, int B) { return (long)tokens / kGcTok + B; }
 
 // Heads that go through the three launches together, 0: the call is not for them.  A chunk of a head takes 1.7 to 2.1 times the token by token form's
 // vectors of it, and more where sequences end within chunks, so a call takes no more than the larger of that form's work space and kGcSpace, and
-// goes through its heads in passes where all of them would need more.  32 heads of 128 x 128 and 8 of 256 x 512 find room in it for 2000
-// tokens; a pass of as much fills the chip.
-constexpr size_t kGcSpace = (size_t)256 << 20;
+// goes through its heads in passes where all of them would need more.  With 256 MB, 8 x 512 tokens of 32 heads of 128 x 128 went in three passes, 302 us
+// instead of 233.
+constexpr size_t kGcSpace = (size_t)1 << 30;
 constexpr size_t kGcPad = 10 * 16;  // the parts of the work space begin on multiples of 16 bytes
 static int gc_heads(int kind, int tokens, int B, int H, int dk, int dv)
 {

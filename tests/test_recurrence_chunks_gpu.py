@@ -183,7 +183,7 @@ def test_channels_that_forget(cuda, ob, dk, fast, keyed):
 @pytest.mark.parametrize("keyed,H,dk,dv,B", [(False, 8, 256, 128, 40), (True, 2, 64, 256, 70), (False, 3, 64, 128, 33), (True, 1, 128, 512, 1)])
 def test_many_chunks(cuda, ob, keyed, H, dk, dv, B):
     # Clusters of the output kernel take several (chunk, head) pairs; a warp looks through the sequences more than once; the first case goes
-    # through its heads in three passes.
+    # through its heads in two passes.
     d = Dev(cuda, ob, "bf16")
     rng = np.random.default_rng(B)
     counts = rng.integers(300, 725, B) if B > 1 else np.array([8000])
