@@ -24,7 +24,7 @@
 //   3. gr_chunk_output_kernel (26 | 58): a block makes 128 tokens x 128 value columns of the output: q~ . k~, q~ . S, then, behind the mask,
 //      the first times V with the pieces of the table in tensor memory; RMS norm over the head (a cluster's blocks share the sums) and gate.
 //      Bound by its operands: 6 bytes a float, 320 KB (608 KB) for 7680 (13800) cycles of products.
-// All three 84.5 | 119.6 us; token by token 255 | 244.  With one channel a head that forgets too much 115 | 163, where the gates are sigmoids of
+// All three 85 | 121 us; token by token 255 | 244.  With one channel a head that forgets too much 115 | 163, where the gates are sigmoids of
 // normal numbers 181 | 202, where all channels do 239 | 234.  A short call with such channels is slower than token by token, which no rule
 // on sizes can know: 1 x 288 tokens 38 | 57 us without, 59 | 81, 82 | 99 and 103 | 119 with them, token by token 42 | 73; 1 x 768 tokens TIED 48
 // without, 73, 110 and 132, token by token 101.  Error of the state against 64 bits 9.7e-8 | 8.3e-8 (9.3e-8 | 1.1e-7; sigmoids of normal numbers
@@ -491,6 +491,10 @@ __device__ __noinline__ void gd_table(const GrParams& pp, const GrChunks& ck, un
     float *near_end = reinterpret_cast<float*>(smem), *tile_end = near_end + kArray;
     const int chunks = gc_count(pp.tp.cu, pp.tp.B), pairs = chunks * ck.heads, parts = 4 * pairs <= blocks ? 4 : 2 * pairs <= blocks ? 2 : 1;
     const int c = lane, s = warp;  // a thread's channel of the group and strip while the operands are made
+    bool any = false;  // most calls have none: looked for all at once (one after the other 2 x 1030 tokens of 32 heads took 137.6 us, so 133.6)
+    for (int work = block + lane * blocks; work < pairs * parts; work += 32 * blocks)
+        any |= ck.notes[(size_t)(work / parts / chunks) * ck.slots + work / parts % chunks].x != 0;
+    if (!__any_sync(0xffffffffu, any)) return;
     for (int work = block; work < pairs * parts; work += blocks) {
         const int pair = work / parts, part = work % parts, slot = pair % chunks, h = pair / chunks;
         const size_t at = (size_t)h * ck.slots + slot;
