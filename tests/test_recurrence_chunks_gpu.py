@@ -10,8 +10,9 @@ from tests.test_fuposun_kernels_gpu import ref_gla, run_gla
 
 pytestmark = pytest.mark.gpu
 TOL = 1.2e-2
-# The state is float and its sums are taken as closely as float adds them; the outputs are rounded to bfloat16.
-STATE = 2e-6
+# The state is float and its sums are taken as closely as float adds them: 1e-7 for the gates of a trained model, up to 4.4e-7 where hundreds
+# of gates are the same one close to 1, 3e-7 where all terms have one sign.  The outputs are rounded to bfloat16.
+STATE = 1e-6
 
 
 def positions(ob, d, counts, hist):
@@ -208,3 +209,23 @@ def test_many_chunks(cuda, ob, keyed, H, dk, dv, B):
                 ref = ref_recurrence(*y, zb[ch], lower[ch], w, ref_state)
             assert rel_err(got[s, h:h + 1], ref) < TOL, (b, h)
             assert rel_err(host(state[b, h:h + 1]), ref_state) < STATE, (b, h)
+
+
+@pytest.mark.parametrize("keyed", [False, True])
+def test_state_from_operands_of_one_sign(cuda, ob, keyed):
+    # where every term adds up, so do the errors that the tensor cores make when they cut sums off
+    d = Dev(cuda, ob, "bf16")
+    rng = np.random.default_rng(11)
+    H, dk, dv, n = 2, 128, 128, 1500
+    x = [rounded(np.abs(rng.standard_normal(s)) if i in (1, 2) and (keyed or i == 2) else rng.standard_normal(s), "bf16")
+         for i, s in enumerate(((n, H, dk), (n, H, dk), (n, H, dv), (n, 4), (n, H, dv)))]
+    A, zb, w = fr.round_bf16(rng.standard_normal((H * dk, 4)) * 0.3), fr.round_bf16(rng.uniform(2, 7, H * dk)), np.ones(dv)
+    state, ref_state = d.zeros(1, H, dk, dv, f32=True), np.zeros((H, dk, dv))
+    tp = positions(ob, d, [n], [0])
+    if keyed:
+        run_gla(ob, d, H, dk, dv, x, A, zb, w, state, tp, 4.0, 1.0)
+        ref_gla(x, A, zb, w, ref_state, 4.0, 1.0)
+    else:
+        run_recurrence(ob, d, H, dk, dv, x[0], x[1], x[2], zb, np.zeros(H * dk), w, state, tp, 1)
+        ref_recurrence(x[0], x[1], x[2], zb, np.zeros(H * dk), w, ref_state)
+    assert rel_err(host(state)[0], ref_state) < STATE
